@@ -484,6 +484,23 @@ int adamas_append_decode_rope_fused(void* q, void* k, const void* v, void* q_cod
                             thresholds3_host, dtype, stream, rope, nullptr, num_q_heads);
 }
 
+static int rope_impl(void* q, void* k, int64_t seq_len, int num_q_heads, int num_kv_heads, int64_t past_kv_len,
+                     const RopeParams& rp, int dtype, adamas_stream_t stream) {
+  const DeviceInfo* di = nullptr;
+  if (int rc = get_device_info(&di)) return rc;
+  // kRopeTokens tokens per block once that still gives every SM several blocks; one per block below
+  const int tpb = seq_len >= static_cast<int64_t>(8) * kRopeTokens * di->num_sms ? kRopeTokens : 1;
+  const unsigned blocks = static_cast<unsigned>((seq_len + tpb - 1) / tpb);
+  const int seq = static_cast<int>(seq_len), past = static_cast<int>(past_kv_len);
+  if (dtype == ADAMAS_F16)
+    rope_kernel<__half><<<blocks, kRopeThreads, 0, to_stream(stream)>>>(
+        static_cast<__half*>(q), static_cast<__half*>(k), seq, num_q_heads, num_kv_heads, past, tpb, rp);
+  else
+    rope_kernel<__nv_bfloat16><<<blocks, kRopeThreads, 0, to_stream(stream)>>>(
+        static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), seq, num_q_heads, num_kv_heads, past, tpb, rp);
+  return check_launch("rope_kernel");
+}
+
 int adamas_apply_rope_in_place(void* q, void* k, int64_t seq_len, int num_q_heads, int num_kv_heads,
                                int head_dim, int64_t past_kv_len, float rope_scale, float rope_theta,
                                int dtype, adamas_stream_t stream) {
@@ -495,18 +512,8 @@ int adamas_apply_rope_in_place(void* q, void* k, int64_t seq_len, int num_q_head
                  "positions must stay below 2^24 (exact in fp32)");
   if (seq_len == 0) return ADAMAS_OK;
   ADAMAS_REQUIRE(q && k, "null pointer");
-  const int64_t rows_q = seq_len * num_q_heads, rows_k = seq_len * num_kv_heads;
-  const unsigned blocks = rows_to_blocks(rows_q + rows_k);
-  const RopeParams rp{1.0f / rope_scale, rope_theta, nullptr, 1.f};
-  if (dtype == ADAMAS_F16)
-    rope_kernel<__half><<<blocks, 256, 0, to_stream(stream)>>>(static_cast<__half*>(q), static_cast<__half*>(k),
-                                                              rows_q, rows_k, num_q_heads, num_kv_heads,
-                                                              static_cast<int>(past_kv_len), rp);
-  else
-    rope_kernel<__nv_bfloat16><<<blocks, 256, 0, to_stream(stream)>>>(
-        static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), rows_q, rows_k, num_q_heads,
-        num_kv_heads, static_cast<int>(past_kv_len), rp);
-  return check_launch("rope_kernel");
+  return rope_impl(q, k, seq_len, num_q_heads, num_kv_heads, past_kv_len,
+                   RopeParams{1.0f / rope_scale, rope_theta, nullptr, 1.f}, dtype, stream);
 }
 
 int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n_tokens, void* kv_data,
@@ -1685,18 +1692,8 @@ int adamas_apply_rope_table_in_place(void* q, void* k, int64_t seq_len, int num_
                  "positions must stay below 2^24 (exact in fp32)");
   if (seq_len == 0) return ADAMAS_OK;
   ADAMAS_REQUIRE(q && k && inv_freq_dev, "null pointer");
-  const int64_t rows_q = seq_len * num_q_heads, rows_k = seq_len * num_kv_heads;
-  const unsigned blocks = rows_to_blocks(rows_q + rows_k);
-  const RopeParams rp{1.f, 1e4f, inv_freq_dev, mscale};
-  if (dtype == ADAMAS_F16)
-    rope_kernel<__half><<<blocks, 256, 0, to_stream(stream)>>>(static_cast<__half*>(q), static_cast<__half*>(k),
-                                                              rows_q, rows_k, num_q_heads, num_kv_heads,
-                                                              static_cast<int>(past_kv_len), rp);
-  else
-    rope_kernel<__nv_bfloat16><<<blocks, 256, 0, to_stream(stream)>>>(
-        static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), rows_q, rows_k, num_q_heads,
-        num_kv_heads, static_cast<int>(past_kv_len), rp);
-  return check_launch("rope_kernel");
+  return rope_impl(q, k, seq_len, num_q_heads, num_kv_heads, past_kv_len, RopeParams{1.f, 1e4f, inv_freq_dev, mscale},
+                   dtype, stream);
 }
 
 int adamas_merge_states(const float* o_parts, const float* lse_parts, int num_parts, int num_heads,
