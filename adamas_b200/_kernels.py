@@ -4,7 +4,9 @@
 Same function names, argument order and meaning, and the same error behaviour (bad shapes,
 dtypes or devices raise ``RuntimeError``, as ``TORCH_CHECK`` does).  Each function checks its
 tensors and hands raw device pointers to the C ABI in ``libadamas_b200.so``; torch is used for
-memory and streams only.  All launches go to torch's current CUDA stream.
+memory and streams only.  All launches go to torch's current CUDA stream.  The operators that a
+decode loop calls for every layer do so in the extension module ``_native`` (csrc/binding.cpp), the
+others through ctypes.
 """
 from __future__ import annotations
 
@@ -16,8 +18,10 @@ import torch
 
 from . import _lib
 from ._lib import lib
+from . import _native     # the per-layer operators (csrc/binding.cpp); needs torch and the library loaded
 
 NHD, HND = 0, 1
+_METRICS = {"l1": _lib.METRIC_L1, "xor": _lib.METRIC_XOR}
 DEFAULT_THRESHOLDS = (-10.0, 0.0, 10.0)
 
 
@@ -87,29 +91,14 @@ def hadamard_transform(x: torch.Tensor, inplace: bool = False, scale: Optional[f
     """Stand-in for ``faster_hadamard_transform.hadamard_transform`` (call sites
     adamas/models/Adamas.py:120,150): Walsh-Hadamard transform of the last dimension (128),
     scaled by 1/sqrt(128) unless `scale` is given, result in x.dtype."""
-    _check_input(x, "x")
-    _require(x.size(-1) == 128, "hadamard_transform supports a last dimension of 128")
-    y = x if inplace else torch.empty_like(x)
-    rows = x.numel() // 128
-    s = 1.0 / math.sqrt(128.0) if scale is None else float(scale)
-    _lib.check(lib.adamas_hadamard_transform(_ptr(x), _ptr(y), rows, 128, s,
-                                             _dtype_code(x.dtype, "hadamard_transform"), _stream()),
-               "hadamard_transform")
-    return y
+    return _native.hadamard_transform(x, inplace, scale)
 
 
 def apply_rope_in_place(q: torch.Tensor, k: torch.Tensor, past_kv_len: int, rope_scale: float = 1.0,
                         rope_theta: float = 1e4) -> None:
     """adamas/ops/csrc/page.cu:228-269.  q [N,Hq,D], k [N,Hk,D] rotated in place; token s has
     position past_kv_len + s; linear position scaling by rope_scale."""
-    _check_input(q, "q", 3)
-    _check_input(k, "k", 3)
-    _require(q.size(0) == k.size(0) and q.size(2) == k.size(2) == 128 and q.dtype == k.dtype,
-             "q and k must be [N, H, 128] of one dtype")
-    _lib.check(lib.adamas_apply_rope_in_place(_ptr(q), _ptr(k), q.size(0), q.size(1), k.size(1), 128,
-                                              int(past_kv_len), float(rope_scale), float(rope_theta),
-                                              _dtype_code(q.dtype, "apply_rope_in_place"), _stream()),
-               "apply_rope_in_place")
+    _native.apply_rope_in_place(q, k, past_kv_len, rope_scale, rope_theta)
 
 
 def bucketize_pack(h: torch.Tensor, o: torch.Tensor, thresholds=None) -> None:
@@ -194,18 +183,8 @@ def append_kv_cache_decode(k, v, h, o, kv_data, kv_indices, kv_indptr, kv_last_p
                            hadamard_last_page_idx, layout, thresholds=None) -> None:
     """adamas/ops/csrc/page.cu:6-109.  k, v [1,H,D]; h [2,H,D] = Hadamard(q), Hadamard(k);
     o [1,H,D/8] receives the packed query code.  The indptr tensors are [0, len(indices)]."""
-    num_heads, head_dim, page_size = _check_append(k, v, kv_data, kv_indices, hadamard_data, hadamard_indices, layout)
-    _check_input(h, "h", 3)
-    _check_input(o, "o", 3)
-    _require(k.size(0) == 1 and v.size(0) == 1 and h.size(0) == 2 and o.size(0) == 1, "decode appends one token")
-    _require(h.size(1) == num_heads and h.size(2) == head_dim and h.dtype == k.dtype, "h must be [2, H, D] in k.dtype")
-    _require(o.size(1) == num_heads and o.size(2) == head_dim // 8 and o.element_size() == 2, "o must be [1, H, D/8] 16-bit")
-    _lib.check(lib.adamas_append_decode(
-        _ptr(k), _ptr(v), _ptr(h), _ptr(o),
-        _ptr(kv_data), _ptr(kv_indices), kv_indices.numel(), int(kv_last_page_len),
-        _ptr(hadamard_data), _ptr(hadamard_indices), hadamard_indices.numel(), int(hadamard_last_page_len),
-        num_heads, head_dim, page_size, _lib.thresholds_arg(thresholds),
-        _dtype_code(k.dtype, "Append_kv_cache_decode"), _stream()), "Append_kv_cache_decode")
+    _native.append_kv_cache_decode(k, v, h, o, kv_data, kv_indices, kv_last_page_len, hadamard_data, hadamard_indices,
+                                   hadamard_last_page_len, layout, thresholds)
 
 
 def append_kv_cache_decode_fused(q, k, v, o, kv_data, kv_indices, kv_last_page_len, hadamard_data,
@@ -215,29 +194,8 @@ def append_kv_cache_decode_fused(q, k, v, o, kv_data, kv_indices, kv_last_page_l
     (adamas/models/Adamas.py:145-161).  With rope=(rope_scale, rope_theta), or a frequency table
     {"inv_freq": tensor[64], "mscale": float}, q and k arrive un-rotated and are rotated in place first
     (also replaces apply_rope_in_place, Adamas.py:113).  q may have a multiple of k's heads."""
-    num_heads, head_dim, page_size = _check_append(k, v, kv_data, kv_indices, hadamard_data, hadamard_indices, layout)
-    _check_input(q, "q", 3)
-    _check_input(o, "o", 3)
-    _require(k.size(0) == 1, "k, v must be [1, H, D]")
-    q_heads = _query_heads(q, k, "append_kv_cache_decode_fused")
-    _require(o.size(1) == q_heads and o.size(2) == head_dim // 8 and o.element_size() == 2, "o must be [1, Hq, D/8] 16-bit")
-    s = 1.0 / math.sqrt(head_dim) if scale is None else float(scale)
-    if rope is not None:
-        rs, rt, inv_freq, mscale = _rope_args(rope)
-        _lib.check(lib.adamas_append_decode_rope_fused(
-            _ptr(q), _ptr(k), _ptr(v), _ptr(o),
-            _ptr(kv_data), _ptr(kv_indices), kv_indices.numel(), int(kv_last_page_len),
-            _ptr(hadamard_data), _ptr(hadamard_indices), hadamard_indices.numel(), int(hadamard_last_page_len),
-            num_heads, q_heads, head_dim, page_size, s, _lib.thresholds_arg(thresholds), rs if inv_freq is None else 1.0,
-            rt if inv_freq is None else 1e4, _ptr(inv_freq), mscale,
-            _dtype_code(k.dtype, "append_kv_cache_decode_rope_fused"), _stream()), "append_kv_cache_decode_rope_fused")
-        return
-    _lib.check(lib.adamas_append_decode_fused(
-        _ptr(q), _ptr(k), _ptr(v), _ptr(o),
-        _ptr(kv_data), _ptr(kv_indices), kv_indices.numel(), int(kv_last_page_len),
-        _ptr(hadamard_data), _ptr(hadamard_indices), hadamard_indices.numel(), int(hadamard_last_page_len),
-        num_heads, q_heads, head_dim, page_size, s, _lib.thresholds_arg(thresholds),
-        _dtype_code(k.dtype, "append_kv_cache_decode_fused"), _stream()), "append_kv_cache_decode_fused")
+    _native.append_kv_cache_decode_fused(q, k, v, o, kv_data, kv_indices, kv_last_page_len, hadamard_data, hadamard_indices,
+                                         hadamard_last_page_len, layout, scale, thresholds, rope)
 
 
 def append_kv_cache_prefill(k, v, h, kv_data, kv_indices, kv_indptr, kv_last_page_len, kv_last_page_idx,
@@ -245,17 +203,8 @@ def append_kv_cache_prefill(k, v, h, kv_data, kv_indices, kv_indptr, kv_last_pag
                             hadamard_last_page_idx, layout, scale=None, thresholds=None) -> None:
     """adamas/ops/csrc/page.cu:111-226.  k, v, h [N,H,D]; h = Hadamard(k).  Passing h=None
     computes the transform inside the same launch."""
-    num_heads, head_dim, page_size = _check_append(k, v, kv_data, kv_indices, hadamard_data, hadamard_indices, layout)
-    if h is not None:
-        _check_input(h, "h", 3)
-        _require(tuple(h.shape) == tuple(k.shape) and h.dtype == k.dtype, "h must match k")
-    s = 1.0 / math.sqrt(head_dim) if scale is None else float(scale)
-    _lib.check(lib.adamas_append_prefill(
-        _ptr(k), _ptr(v), _ptr(h), k.size(0),
-        _ptr(kv_data), _ptr(kv_indices), kv_indices.numel(), int(kv_last_page_len),
-        _ptr(hadamard_data), _ptr(hadamard_indices), hadamard_indices.numel(), int(hadamard_last_page_len),
-        num_heads, head_dim, page_size, s, _lib.thresholds_arg(thresholds),
-        _dtype_code(k.dtype, "Append_kv_cache_prefill"), _stream()), "Append_kv_cache_prefill")
+    _native.append_kv_cache_prefill(k, v, h, kv_data, kv_indices, kv_last_page_len, hadamard_data, hadamard_indices,
+                                    hadamard_last_page_len, layout, scale, thresholds)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -270,28 +219,8 @@ def estimate_attn_score(q, o, metadata_data, metadata_indices, metadata_indptr, 
     (a sequence shard that does not hold the newest token).  `hist` (a zeroed histogram_scratch(H))
     additionally receives the per-slice counts that select_attend(..., hist_ready=True) reads;
     hist_slices = select_attend_slices(n, k, H) of that call."""
-    _nhd_only(layout)
-    _check_input(q, "q", 3)
-    _check_rows(o, "o")
-    _check_input(metadata_data, "hadamard_data", 5)
-    _check_input(metadata_indices, "hadamard_indices", 1)
-    _require(q.size(0) == 1, "q.size(0) must be 1")
-    _require(metadata_indices.dtype == torch.int32, "hadamard_indices must be int32")
-    q_heads, code_words = q.size(1), q.size(2)
-    page_size = metadata_data.size(2)
-    num_heads = metadata_data.size(3)          # heads of the cache; q_heads is a multiple of it
-    _require(q_heads >= num_heads and q_heads % num_heads == 0 and metadata_data.size(4) == code_words
-             and code_words == 16, "hadamard_data must be [pages, 1, page_size, num_heads, 16], q [1, Hq, 16]")
-    _require(q.element_size() == 2 and metadata_data.element_size() == 2, "codes must be 16-bit words")
-    n = (metadata_indices.numel() - 1) * page_size + int(metadata_last_page_len) - (1 if exclude_last else 0)
-    _require(o.size(0) == q_heads and o.size(1) == n, f"o must be [{q_heads}, {n}]")
-    _lib.check(lib.adamas_estimate(
-        _ptr(q), _ptr(metadata_data), _ptr(metadata_indices), metadata_indices.numel(),
-        int(metadata_last_page_len), page_size, num_heads, q_heads, code_words * 8, _ptr(o), o.stride(0),
-        _value_format(o.dtype, "Estimate_attn_score"),
-        {"l1": _lib.METRIC_L1, "xor": _lib.METRIC_XOR}[metric], 1 if exclude_last else 0,
-        _ptr(_check_hist(hist, q_heads)), int(hist_slices), _stream()),
-        "Estimate_attn_score")
+    _native.estimate_attn_score(q, o, metadata_data, metadata_indices, metadata_last_page_len, layout, _METRICS[metric],
+                                exclude_last, hist, hist_slices)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -303,45 +232,14 @@ def topk_filtering(estimated_value, estimated_indices, d_out, indices_out, buf, 
     estimated_indices [H, n] to indices_out [H, k].  `buf` (the reference's radix scratch) is
     accepted and unused.  Unlike the reference the result is deterministic: equal values are taken
     lowest position first and rows are emitted in ascending position order."""
-    _check_rows(estimated_value, "estimated_value")
-    _check_rows(estimated_indices, "estimated_indices")
-    _check_rows(d_out, "d_out")
-    _check_rows(indices_out, "indices_out")
-    _require(d_out.stride(0) == indices_out.stride(0), "d_out and indices_out must share a row stride")
-    rows, n = estimated_value.shape
-    k = int(page_budget)
-    _require(tuple(estimated_indices.shape) == (rows, n), "estimated_indices must match estimated_value")
-    _require(estimated_indices.dtype == torch.int32 and indices_out.dtype == torch.int32, "indices must be int32")
-    _require(n >= k, "num_pages must be >= page_budget")
-    _require(d_out.size(1) == k and indices_out.size(1) == k, "outputs must have page_budget columns")
-    _require(d_out.size(0) == rows and indices_out.size(0) == rows, "outputs must have one row per head")
-    _require(d_out.dtype == estimated_value.dtype, "d_out must have the dtype of estimated_value")
-    _lib.check(lib.adamas_topk(
-        _ptr(estimated_value), _value_format(estimated_value.dtype, "Top-k filtering"), estimated_value.stride(0), n,
-        _ptr(estimated_indices), estimated_indices.stride(0), 1, rows, k,
-        _ptr(d_out), _ptr(indices_out), indices_out.stride(0), _stream()), "Top-k filtering")
+    _native.topk_filtering(estimated_value, estimated_indices, d_out, indices_out, page_budget)
 
 
 def topk_select(values, k, indices_out, values_out=None, page_table=None, page_size=1) -> None:
     """Token-granular select used when page_size > 1: positions p of the k smallest values per row
     are mapped through one page table shared by all rows, out = page_table[p // page_size] *
     page_size + p % page_size (or p itself when page_table is None)."""
-    _check_rows(values, "values")
-    _check_rows(indices_out, "indices_out")
-    rows, n = values.shape
-    _require(indices_out.dtype == torch.int32 and indices_out.size(0) == rows and indices_out.size(1) >= k,
-             "indices_out must be int32 [rows, >=k]")
-    if values_out is not None:
-        _check_rows(values_out, "values_out")
-        _require(values_out.dtype == values.dtype and values_out.stride(0) == indices_out.stride(0),
-                 "values_out must match values.dtype and the row stride of indices_out")
-    if page_table is not None:
-        _check_input(page_table, "page_table", 1)
-        _require(page_table.dtype == torch.int32 and page_table.numel() * page_size >= n, "page_table too short")
-    _lib.check(lib.adamas_topk(
-        _ptr(values), _value_format(values.dtype, "topk_select"), values.stride(0), n,
-        _ptr(page_table), 0, int(page_size), rows, int(k),
-        _ptr(values_out), _ptr(indices_out), indices_out.stride(0), _stream()), "topk_select")
+    _native.topk_select(values, k, indices_out, values_out, page_table, page_size)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -369,14 +267,15 @@ class BatchDecodeWithPagedKVCachePyTorchWrapper:
             self._handle = None
 
     def begin_forward(self, indptr, num_qo_heads, num_kv_heads, head_dim, page_size, empty_data) -> None:
-        _require(indptr.dim() == 1 and indptr.dtype == torch.int32 and indptr.is_contiguous(),
+        _require(indptr is None or (indptr.dim() == 1 and indptr.dtype == torch.int32 and indptr.is_contiguous()),
                  "indptr must be a contiguous 1D int32 tensor")
         _require(num_qo_heads >= num_kv_heads >= 1 and num_qo_heads % num_kv_heads == 0,
                  "num_qo_heads must be a multiple of num_kv_heads")
         self._cfg = (int(num_qo_heads), int(head_dim), int(page_size),
                      _dtype_code(empty_data.dtype, "BatchDecodeWithPagedKVCache"))
         self._kv_heads = int(num_kv_heads)
-        self._batch = max(1, indptr.numel() - 1)      # the reference's indptr has one entry per sequence, plus one
+        # (the reference's indptr has one entry per sequence, plus one; None: a single sequence)
+        self._batch = 1 if indptr is None else max(1, indptr.numel() - 1)
         self._started = True
         self._planned_tokens = 0   # scratch is sized on the first forward, from the index tensor
 
@@ -397,14 +296,17 @@ class BatchDecodeWithPagedKVCachePyTorchWrapper:
         there unrounded instead of into `o` (partial result of a sequence shard)."""
         if not self._started:
             raise RuntimeError("BatchDecodeWithPagedKVCache failed with error: forward called before begin_forward")
-        _check_input(q, "q", 3)
+        num_heads, head_dim, page_size, dt = self._cfg
         if o_f32 is None:
-            _check_input(o, "o", 3)
+            self._planned_tokens = _native.decode_forward(
+                self._handle.value, q, o, lse, paged_kv_data, paged_kv_indices, paged_kv_last_page_len,
+                paged_kv_last_page_idx, token_granular, num_heads, self._kv_heads, head_dim, page_size, dt,
+                self._planned_tokens, self._batch, tail_len)
+            return
+        _check_input(q, "q", 3)
         _check_input(paged_kv_data, "paged_kv_data", 5)
         _check_rows(paged_kv_indices, "paged_kv_indices")
-        num_heads, head_dim, page_size, dt = self._cfg
         _require(q.size(0) == 1 and q.size(1) == num_heads and q.size(2) == head_dim, "q must be [1, H, D]")
-        _require(o_f32 is not None or (tuple(o.shape) == tuple(q.shape) and o.dtype == q.dtype), "o must match q")
         _require(paged_kv_data.size(1) == 2 and paged_kv_data.size(2) == page_size
                  and paged_kv_data.size(3) == self._kv_heads and paged_kv_data.size(4) == head_dim,
                  "paged_kv_data must be [pages, 2, page_size, H_kv, D]")
@@ -422,22 +324,14 @@ class BatchDecodeWithPagedKVCachePyTorchWrapper:
             _lib.check(lib.adamas_decode_begin_forward(self._handle, n_tokens, self._batch, self._kv_heads, num_heads,
                                                        head_dim, page_size, dt, _stream()), "BatchDecodeWithPagedKVCache")
             self._planned_tokens = n_tokens
-        if lse is not None:
-            _require(lse.is_cuda and lse.dtype == torch.float32 and lse.numel() == num_heads and lse.is_contiguous(),
-                     "lse must be a contiguous float32 CUDA tensor of H elements")
-        if o_f32 is not None:
-            _require(lse is not None and o_f32.is_cuda and o_f32.dtype == torch.float32 and o_f32.is_contiguous()
-                     and o_f32.numel() == num_heads * head_dim, "o_f32 must be float32 [H, D] and lse given")
-            _lib.check(lib.adamas_decode_forward_partial(
-                self._handle, _ptr(q), _ptr(o_f32), _ptr(lse), _ptr(paged_kv_data), _ptr(paged_kv_indices),
-                paged_kv_indices.stride(0), n_idx, unit, int(paged_kv_last_page_idx), int(paged_kv_last_page_len),
-                tail, 1.0 / math.sqrt(head_dim), _stream()), "BatchDecodeWithPagedKVCache")
-            return
-        _lib.check(lib.adamas_decode_forward(
-            self._handle, _ptr(q), _ptr(o), _ptr(lse), _ptr(paged_kv_data), _ptr(paged_kv_indices),
-            paged_kv_indices.stride(0), n_idx, unit, int(paged_kv_last_page_idx), int(paged_kv_last_page_len), tail,
-            1.0 / math.sqrt(head_dim), _stream()), "BatchDecodeWithPagedKVCache")
-
+        _require(lse is not None and lse.is_cuda and lse.dtype == torch.float32 and lse.numel() == num_heads
+                 and lse.is_contiguous(), "lse must be a contiguous float32 CUDA tensor of H elements")
+        _require(o_f32.is_cuda and o_f32.dtype == torch.float32 and o_f32.is_contiguous()
+                 and o_f32.numel() == num_heads * head_dim, "o_f32 must be float32 [H, D] and lse given")
+        _lib.check(lib.adamas_decode_forward_partial(
+            self._handle, _ptr(q), _ptr(o_f32), _ptr(lse), _ptr(paged_kv_data), _ptr(paged_kv_indices),
+            paged_kv_indices.stride(0), n_idx, unit, int(paged_kv_last_page_idx), int(paged_kv_last_page_len),
+            tail, 1.0 / math.sqrt(head_dim), _stream()), "BatchDecodeWithPagedKVCache")
 
     def dense_step_dev(self, q, k, v, o, q_code, kv_data, kv_indices, hadamard_data, hadamard_indices,
                        seq_len: torch.Tensor, max_seq_len: int, scale: Optional[float] = None, thresholds=None,
@@ -578,31 +472,9 @@ def decode_step(q, k, v, o, q_code, kv_data, kv_indices, kv_last_page_len, kv_la
     or 64 heads, else three, for what adamas/models/Adamas.py:145-200 does with seven).  Needs context > budget.  `hist`: a histogram_scratch(H), all zero between steps.  With
     rope=(rope_scale, rope_theta) or {"inv_freq": tensor[64], "mscale": float} q and k arrive un-rotated
     and are rotated in place first.  q, o may have a multiple of k's heads (grouped-query attention)."""
-    num_heads, head_dim, page_size = _check_append(k, v, kv_data, kv_indices, hadamard_data, hadamard_indices, NHD)
-    _check_input(q, "q", 3)
-    _check_input(o, "o", 3)
-    _check_input(q_code, "q_code", 3)
-    _check_rows(dist_scratch, "dist_scratch")
-    q_heads = _query_heads(q, k, "decode_step")
-    _require(tuple(q.shape) == tuple(o.shape) and k.size(0) == 1, "q, o must be [1, Hq, D], k, v [1, H, D]")
-    _require(q_code.element_size() == 2 and q_code.numel() == q_heads * head_dim // 8, "q_code must be [1, Hq, D/8] 16-bit")
-    _require(dist_scratch.element_size() == 2 and dist_scratch.size(0) == q_heads, "dist_scratch must be 16-bit [Hq, n]")
-    out_stride = 0
-    if indices_out is not None:
-        _check_rows(indices_out, "indices_out")
-        _require(indices_out.dtype == torch.int32 and indices_out.size(0) == q_heads
-                 and indices_out.size(1) >= budget - 1, "indices_out must be int32 [Hq, >=budget-1]")
-        out_stride = indices_out.stride(0)
-    s = 1.0 / math.sqrt(head_dim) if scale is None else float(scale)
-    rs, rt, inv_freq, mscale = _rope_args(rope)
-    _lib.check(lib.adamas_decode_step(
-        _ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(lse), _ptr(q_code),
-        _ptr(kv_data), _ptr(kv_indices), kv_indices.numel(), int(kv_last_page_len), int(kv_last_page_idx),
-        _ptr(hadamard_data), _ptr(hadamard_indices), hadamard_indices.numel(), int(hadamard_last_page_len),
-        num_heads, q_heads, head_dim, page_size, _dtype_code(k.dtype, "decode_step"), int(budget),
-        _ptr(dist_scratch), dist_scratch.stride(0), _ptr(_check_hist(hist, q_heads)), _ptr(indices_out), out_stride, s,
-        _lib.thresholds_arg(thresholds), rs, rt, _ptr(inv_freq), mscale, 1.0 / math.sqrt(head_dim), _stream()),
-        "decode_step")
+    _native.decode_step(q, k, v, o, q_code, kv_data, kv_indices, kv_last_page_len, kv_last_page_idx, hadamard_data,
+                        hadamard_indices, hadamard_last_page_len, budget, dist_scratch, hist, indices_out, lse, scale,
+                        thresholds, rope)
 
 
 def _rope_args(rope):
@@ -632,34 +504,8 @@ def decode_step_dev(q, k, v, o, q_code, kv_data, kv_indices, hadamard_data, hada
     memory: the launches depend on max_seq_len only, so a CUDA graph captured once serves every token
     (advance `seq_len` with seq_len_advance at the end of each token's work).  kv_indices /
     hadamard_indices: the page tables, with an entry for every page the current length needs."""
-    num_heads, head_dim, page_size = _check_append(k, v, kv_data, kv_indices, hadamard_data, hadamard_indices, NHD)
-    _check_input(q, "q", 3)
-    _check_input(o, "o", 3)
-    _check_input(q_code, "q_code", 3)
-    _check_rows(dist_scratch, "dist_scratch")
-    _check_seq_len(seq_len)
-    q_heads = _query_heads(q, k, "decode_step_dev")
-    _require(tuple(q.shape) == tuple(o.shape) and k.size(0) == 1, "q, o must be [1, Hq, D], k, v [1, H, D]")
-    _require(q_code.element_size() == 2 and q_code.numel() == q_heads * head_dim // 8, "q_code must be [1, Hq, D/8] 16-bit")
-    _require(dist_scratch.element_size() == 2 and dist_scratch.size(0) == q_heads
-             and dist_scratch.size(1) >= max_seq_len - 1, "dist_scratch must be 16-bit [Hq, >= max_seq_len - 1]")
-    _require(kv_indices.numel() * page_size >= max_seq_len and hadamard_indices.numel() * page_size >= max_seq_len,
-             "the page tables must have room for max_seq_len tokens")
-    out_stride = 0
-    if indices_out is not None:
-        _check_rows(indices_out, "indices_out")
-        _require(indices_out.dtype == torch.int32 and indices_out.size(0) == q_heads
-                 and indices_out.size(1) >= budget - 1, "indices_out must be int32 [Hq, >=budget-1]")
-        out_stride = indices_out.stride(0)
-    s = 1.0 / math.sqrt(head_dim) if scale is None else float(scale)
-    rs, rt, inv_freq, mscale = _rope_args(rope)
-    _lib.check(lib.adamas_decode_step_dev(
-        _ptr(q), _ptr(k), _ptr(v), _ptr(o), _ptr(lse), _ptr(q_code), _ptr(kv_data), _ptr(kv_indices),
-        _ptr(hadamard_data), _ptr(hadamard_indices), _ptr(seq_len), int(max_seq_len), num_heads, q_heads, head_dim,
-        page_size, _dtype_code(k.dtype, "decode_step_dev"), int(budget), _ptr(dist_scratch),
-        dist_scratch.stride(0), _ptr(_check_hist(hist, q_heads)), _ptr(indices_out), out_stride, s,
-        _lib.thresholds_arg(thresholds), rs, rt, _ptr(inv_freq), mscale, 1.0 / math.sqrt(head_dim), _stream()),
-        "decode_step_dev")
+    _native.decode_step_dev(q, k, v, o, q_code, kv_data, kv_indices, hadamard_data, hadamard_indices, seq_len, max_seq_len,
+                            budget, dist_scratch, hist, indices_out, lse, scale, thresholds, rope)
 
 
 def seq_len_advance(seq_len: torch.Tensor, delta: int = 1) -> None:

@@ -137,7 +137,7 @@ def decode_step(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, iController: 
     _kernels.decode_step(
         q, k, v, o, c.q_code_scratch(k.dtype), c.kv_cache.buf_layer(layer_idx), c.kv_indices_with_last,
         c.kv_cache.last_page_len, c.kv_last_page_idx, c.hadamard_cache.buf_layer(layer_idx), c.hadamard_indices,
-        c.hadamard_cache.last_page_len, c.inference_token_budget, c.distance_scratch(n), c.hist_scratch,
+        c.hadamard_cache.last_page_len, c.inference_token_budget, c.distance_store(n), c.hist_scratch,
         indices_out=c.topk_dindices_buffer if record_indices else None, scale=scale, rope=rope)
     return o
 
@@ -166,7 +166,7 @@ def decode_step_dev(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, iControll
         return o
     _kernels.decode_step_dev(q, k, v, o, c.q_code_scratch(k.dtype), c.kv_cache.buf_layer(layer_idx), kv_table,
                              c.hadamard_cache.buf_layer(layer_idx), code_table, c.seq_len_dev, c.max_seq_len,
-                             c.token_budget(), c.distance_scratch(c.max_seq_len - 1), c.hist_scratch,
+                             c.token_budget(), c.distance_store(c.max_seq_len - 1), c.hist_scratch,
                              scale=scale, rope=rope)
     return o
 

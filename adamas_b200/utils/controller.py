@@ -50,7 +50,7 @@ class InferenceController:
         self._decode_handler = BatchDecodeWithPagedKVCacheWrapper(kv_layout="NHD")
 
         self.kv_indices_with_last = None
-        self.kv_indices_without_last = None
+        self._without_last = None        # (pages, view): kv_indices_without_last, made when it is asked for
         self.hadamard_indices = None
         self.kv_last_page_idx = None
         self.hadamard_last_page_idx = None
@@ -65,7 +65,9 @@ class InferenceController:
         self.topk_dindices_buffer = None
         self.topk_buf = None
         self._topk_store = None
+        self._topk_k = -1                # columns of the current top-k views
         self._estimate_store = None
+        self._estimate_view = None
 
         self.max_seq_len = self.kv_cache.pool.capacity * page_size
         self._hist = None
@@ -87,6 +89,16 @@ class InferenceController:
         if self._indptr_vals.get(name) != vals:
             self._indptr_vals[name] = vals
             self._indptr_cache.pop(name, None)
+
+    @property
+    def kv_indices_without_last(self):
+        """[Hq, pages - 1] view of the page table (a shared row), made on the first use in a forward."""
+        w = self._without_last
+        if w is None:
+            return None
+        if w[1] is None:
+            w[1] = self.kv_indices_with_last[:w[0]].unsqueeze(0).expand(self.num_q_heads, w[0])
+        return w[1]
 
     kv_indptr_for_append = property(lambda self: self._indptr("kv_append"))
     hadamard_indptr_for_append = property(lambda self: self._indptr("code_append"))
@@ -117,8 +129,8 @@ class InferenceController:
         cur_page_nums = len(self.kv_cache.indicies)
         assert cur_page_nums > 1 or self.page_size > 1   # the newest token is always kept apart
         if updateTensor:
-            n = cur_page_nums - 1
-            self.kv_indices_without_last = self.kv_indices_with_last[:n].unsqueeze(0).expand(self.num_q_heads, n)
+            if self._without_last is None or self._without_last[0] != cur_page_nums - 1:
+                self._without_last = [cur_page_nums - 1, None]
 
         if self.page_size == 1:
             self.inference_page_budget = min(self._page_budget, cur_page_nums)
@@ -137,16 +149,18 @@ class InferenceController:
             vals = torch.zeros((self.num_q_heads, cap), dtype=torch.int16, device=self.device)
             idx = torch.zeros((self.num_q_heads, cap), dtype=torch.int32, device=self.device)
             self._topk_store = (vals, idx)
-        vdtype = self.dtype if self.dtype == torch.float16 else torch.int16
-        self.topk_dout_buffer = self._topk_store[0].view(vdtype)[:, :k]
-        self.topk_dindices_buffer = self._topk_store[1][:, :k]
+            self._topk_k = -1
+        if self._topk_k != k:
+            vdtype = self.dtype if self.dtype == torch.float16 else torch.int16
+            self.topk_dout_buffer = self._topk_store[0].view(vdtype)[:, :k]
+            self.topk_dindices_buffer = self._topk_store[1][:, :k]
+            self._topk_k = k
         if self.topk_buf is None:
             # the reference's radix-select scratch (controller.py:122); unused here, kept for callers
             self.topk_buf = torch.zeros((self.num_q_heads, 8192 * 2 * (2 + 4) // 2 // 48), dtype=self.dtype,
                                         device=self.device)
 
-        self._decode_handler.begin_forward(torch.tensor([0, k], dtype=torch.int32), self.num_q_heads,
-                                           self.num_heads, self.head_dim, self.page_size, self.dtype)
+        self._decode_handler.begin_forward(None, self.num_q_heads, self.num_heads, self.head_dim, self.page_size, self.dtype)
 
     def end_forward(self):
         self._decode_handler.end_forward()
@@ -160,18 +174,26 @@ class InferenceController:
 
     def estimate_buffer(self, n: int) -> torch.Tensor:
         """[H, n] distance buffer (fp16 for fp16 models as in the reference, else int16), reused."""
-        vdtype = self.dtype if self.dtype == torch.float16 else torch.int16
-        if self._estimate_store is None or self._estimate_store.size(1) < n:
-            cap = max(n, 1) if self._estimate_store is None else max(n, 2 * self._estimate_store.size(1))
+        store = self.distance_store(n)
+        view = self._estimate_view
+        if view is None or view.size(1) != n:      # (the layers of a token share one length)
+            view = self._estimate_view = store.view(self.dtype if self.dtype == torch.float16 else torch.int16)[:, :n]
+        return view
+
+    def distance_store(self, n: int) -> torch.Tensor:
+        """The [H, >= n] int16 buffer behind estimate_buffer, rows on 16-byte boundaries (the fused step's scratch)."""
+        store = self._estimate_store
+        if store is None or store.size(1) < n:
+            cap = max(n, 1) if store is None else max(n, 2 * store.size(1))
             cap = max(min(cap, self.kv_cache.pool.capacity * self.page_size), n)
             cap = (cap + 7) // 8 * 8     # rows start on 16-byte boundaries (the top-k kernel's fast layout)
-            self._estimate_store = torch.empty((self.num_q_heads, cap), dtype=torch.int16, device=self.device)
-        return self._estimate_store.view(vdtype)[:, :n]
+            store = self._estimate_store = torch.empty((self.num_q_heads, cap), dtype=torch.int16, device=self.device)
+            self._estimate_view = None
+        return store
 
     def distance_scratch(self, n: int) -> torch.Tensor:
-        """[H, n] int16 view of the same buffer, rows on 16-byte boundaries (fused decode step)."""
-        self.estimate_buffer(n)
-        return self._estimate_store[:, :n]
+        """[H, n] int16 view of the same buffer."""
+        return self.distance_store(n)[:, :n]
 
     # ---- state of the fused / graph-replayable decode step ------------------------------------
     @property

@@ -20,6 +20,7 @@ class KvPool:
         self._layout = TensorLayout.NHD
         self._buf = torch.empty((num_layers, capacity, items, block_len, num_heads, head_dim),
                                 dtype=dtype, device=device)
+        self._layers = self._buf.unbind(0)     # one view per layer, handed out by buf_layer
         self._free = list(range(capacity))
         heapq.heapify(self._free)
         self._in_use = set()
@@ -65,6 +66,7 @@ class KvCache:
         if self._table.is_cuda:
             self._host_table = self._host_table.pin_memory()
         self._uploaded = 0
+        self._table_view = None      # table_device()'s view of the current pages
 
     pool = property(lambda self: self._pool)
     seqlen = property(lambda self: self._seqlen)
@@ -75,8 +77,8 @@ class KvCache:
         return (self._seqlen - 1) % self._pool.block_len + 1
 
     def buf_layer(self, layer_idx: int) -> torch.Tensor:
-        assert layer_idx < self._pool.num_layers
-        return self._pool.buf[layer_idx]
+        assert layer_idx < len(self._pool._layers)
+        return self._pool._layers[layer_idx]
 
     def append_seq(self, seq_len: int) -> int:
         """Reserve room for seq_len more tokens; returns the number of pages added."""
@@ -99,7 +101,9 @@ class KvCache:
             self._host_table[self._uploaded:n] = torch.tensor(self._indicies[self._uploaded:n], dtype=torch.int32)
             self._table[self._uploaded:n].copy_(self._host_table[self._uploaded:n], non_blocking=True)
             self._uploaded = n
-        return self._table[:n]
+        if self._table_view is None or self._table_view.size(0) != n:
+            self._table_view = self._table[:n]
+        return self._table_view
 
     def table_all(self) -> torch.Tensor:
         """The whole persistent table buffer (capacity entries; entries beyond the current page count
