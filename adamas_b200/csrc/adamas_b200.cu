@@ -86,6 +86,8 @@ constexpr int kEstAppendStatic = 1792;   // static shared memory of estimate_app
 constexpr int kEstPagesStatic = 8448;    // static shared memory of estimate_pages_kernel, rounded up
 constexpr int kSaMaxDynSmem = 160 * 1024;   // dynamic shared memory select_attend may ask for (a long winner list)
 
+constexpr int kDecSmem = kDecWarps * kDecStages * kDecTileBytes;
+
 // Per-device facts and one-time kernel attributes.
 struct DeviceInfo {
   bool ready = false;
@@ -142,8 +144,8 @@ int get_device_info(const DeviceInfo** out) {
     ESTA_ATTR_ALL(__nv_bfloat16);
 #undef ESTA_ATTR_ALL
 #undef ESTA_ATTR
-    ADAMAS_CUDA(cudaFuncSetAttribute(sparse_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kDecStageBytes));
-    ADAMAS_CUDA(cudaFuncSetAttribute(sparse_decode_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kDecStageBytes));
+    ADAMAS_CUDA(cudaFuncSetAttribute(paged_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem));
+    ADAMAS_CUDA(cudaFuncSetAttribute(paged_decode_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem));
     // One shared-memory carve-out for every kernel of the decode step: a kernel that asks for a
     // different L1 / shared split than its predecessor cannot start until the SMs have drained.
 #define SET_CARVEOUT(kern) \
@@ -168,8 +170,8 @@ int get_device_info(const DeviceInfo** out) {
     SET_CARVEOUT((topk_cluster_kernel<1, 1, 256>));
     SET_CARVEOUT((topk_cluster_kernel<1, 2, 256>));
     SET_CARVEOUT((topk_cluster_kernel<1, 4, 256>));
-    SET_CARVEOUT((sparse_decode_kernel<__half>));
-    SET_CARVEOUT((sparse_decode_kernel<__nv_bfloat16>));
+    SET_CARVEOUT((paged_decode_kernel<__half>));
+    SET_CARVEOUT((paged_decode_kernel<__nv_bfloat16>));
 #undef SET_CARVEOUT
     // select+attend: large dynamic shared memory
 #define SA_ATTR(T, I)                                                                                          \
@@ -807,7 +809,7 @@ int adamas_topk(const void* values, int value_format, int64_t value_stride, int 
 struct adamas_decode_handler {
   void* scratch = nullptr;        // partial_o | partial_ml | counters
   size_t scratch_bytes = 0;
-  int64_t cap_units = 0;          // H * max_splits the scratch was sized for
+  int64_t cap_units = 0;          // results (128 floats each) the scratch was sized for
   int cap_heads = 0;
   int num_sms = 0;
   int device = -1;
@@ -819,26 +821,49 @@ struct adamas_decode_handler {
 
 namespace {
 
-struct SplitPlan {
-  int tiles_per_block;
-  int num_splits;
+// Shape of a paged_decode launch over `batch` sequences of (up to) n_tokens tokens.  shared_list: all query heads
+// of a cache head attend to the same tokens (the dense layers), so they go through the tiles together.
+struct DecPlan {
+  int row_heads, row_to_kv, group, subs, gs, splits;
+  unsigned blocks;
 };
 
-// One wave of resident blocks: up to 4 single-tile blocks per SM (34 KB of shared memory each) or 3
-// double-buffered multi-tile blocks (68 KB each), over all heads; never more splits than tiles.
-SplitPlan plan_splits(int64_t n_tokens, int num_heads, int num_sms) {
+// query heads of a cache head that go through the tiles together (at most kDecMaxGroup, in equal parts)
+int dec_group_part(int group) {
+  const int subs = (group + kDecMaxGroup - 1) / kDecMaxGroup;
+  return (group + subs - 1) / subs;
+}
+
+DecPlan plan_decode(int64_t n_tokens, int batch, int kv_heads, int q_heads, bool shared_list, int num_sms) {
+  DecPlan d;
+  const int g = q_heads / kv_heads;
+  d.row_heads = shared_list ? kv_heads : q_heads;
+  d.row_to_kv = shared_list ? 1 : g;
+  d.group = shared_list ? g : 1;
+  d.gs = dec_group_part(d.group);
+  d.subs = (d.group + d.gs - 1) / d.gs;
   const int64_t tiles = (n_tokens + kDecTile - 1) / kDecTile;
-  const int64_t cap1 = std::max<int64_t>(1, (static_cast<int64_t>(num_sms) * 4 + num_heads - 1) / num_heads);
-  SplitPlan p;
-  if (tiles <= cap1) {
-    p.tiles_per_block = 1;
-    p.num_splits = static_cast<int>(tiles);
-    return p;
+  const int64_t rows = static_cast<int64_t>(batch) * d.row_heads * d.subs;
+  d.splits = 0;
+  const int64_t slots = static_cast<int64_t>(kDecBlocksPerSm) * num_sms;
+  if (rows <= slots && rows * tiles < slots * kDecWarps * 4) {
+    // little work: latency counts, so a block gets a share of ONE row (a second row in a block would be a second
+    // pass through index list, rows and merge)
+    // (a group of query heads has as many results to merge per part: half as many parts; measured at 28 query heads
+    // over 4 x 2001 tokens: 11.9 us with 6 tiles per block, 10.7 with 12; one query head per row, 512 tokens: 7.4 / 8.3)
+    const int min_tiles = d.gs > 1 ? 2 * kDecMinTiles : kDecMinTiles;
+    d.splits = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(slots / rows, (tiles + min_tiles - 1) / min_tiles)));
+    d.blocks = static_cast<unsigned>(rows * d.splits);
+    return d;
   }
-  const int64_t cap2 = std::max<int64_t>(1, static_cast<int64_t>(num_sms) * 3 / num_heads);
-  p.tiles_per_block = static_cast<int>((tiles + cap2 - 1) / cap2);
-  p.num_splits = static_cast<int>((tiles + p.tiles_per_block - 1) / p.tiles_per_block);
-  return p;
+  d.blocks = static_cast<unsigned>(kDecBlocksPerSm * num_sms);
+  return d;
+}
+
+// Results a launch over `rows` query rows (`group` per cache head) may park in the scratch: a block writes one unit of
+// gs results per row group it touches, and the units along the line number fewer than blocks + row groups.
+int64_t dec_scratch_units(int64_t rows, int group, int num_sms) {
+  return static_cast<int64_t>(dec_group_part(group)) * kDecBlocksPerSm * num_sms + 2 * rows;
 }
 
 size_t scratch_layout(int64_t units, int heads, size_t* off_ml, size_t* off_cnt) {
@@ -876,7 +901,7 @@ int adamas_decode_begin_forward(adamas_decode_handler_t* handler, int64_t max_to
   if (int rc = check_q_heads(num_heads, num_q_heads)) return rc;
   const int kv_heads = num_heads;
   num_heads = num_q_heads;   // from here on: the rows of the launch
-  ADAMAS_REQUIRE(max_tokens >= 1 && max_tokens < (int64_t(1) << 31) - kDecTile, "max_tokens out of range");
+  ADAMAS_REQUIRE(max_tokens >= 1 && max_tokens < (int64_t(1) << 31) - 64, "max_tokens out of range");
   int dev = 0;
   ADAMAS_CUDA(cudaGetDevice(&dev));
   const DeviceInfo* di = nullptr;
@@ -886,11 +911,10 @@ int adamas_decode_begin_forward(adamas_decode_handler_t* handler, int64_t max_to
     handler->num_sms = di->num_sms;
     handler->device = dev;
   }
-  // The planner never gives a head more than ceil(4 * SMs / H) splits, so H * splits <= 4 * SMs + H
-  // whatever the length: sized once for that bound, the scratch never has to grow while the head count
-  // stays (a regrow costs a stream synchronisation and a cudaFree / cudaMalloc pair).
+  // The bound does not depend on the length: sized once for it, the scratch never has to grow while the head
+  // count and the batch stay (a regrow costs a stream synchronisation and a cudaFree / cudaMalloc pair).
   const int rows = num_heads * batch;
-  const int64_t units = static_cast<int64_t>(4) * handler->num_sms + rows;
+  const int64_t units = dec_scratch_units(rows, num_heads / kv_heads, handler->num_sms);
   if (units > handler->cap_units || rows > handler->cap_heads) {
     size_t off_ml, off_cnt;
     const int64_t new_units = units > handler->cap_units ? units : handler->cap_units;
@@ -925,6 +949,47 @@ int adamas_decode_end_forward(adamas_decode_handler_t* handler) {
   return ADAMAS_OK;
 }
 
+static int launch_decode(const DecPlan& d, const void* q, void* o, float* o_f32, float* lse, const void* kv_data,
+                         const int32_t* indices, int64_t idx_stride, int n_idx, int idx_unit, int page_size, int kv_heads,
+                         int q_heads, unsigned tail_slot0, int64_t n_tokens, float sm_scale, int dtype, void* partial_o,
+                         void* partial_ml, void* counters, const int32_t* seq_len_dev, const SeqDesc* seqs, int batch,
+                         adamas_stream_t stream) {
+  DecodeParams prm;
+  prm.q = q;
+  prm.o = o;
+  prm.o_f32 = o_f32;
+  prm.lse = lse;
+  prm.kv = kv_data;
+  prm.indices = indices ? indices : reinterpret_cast<const int32_t*>(kv_data);
+  prm.idx_stride = idx_stride;
+  prm.n_listed = n_idx * idx_unit;
+  prm.idx_unit = idx_unit;
+  prm.page_size = page_size;
+  prm.ps_shift = log2_exact(page_size);
+  prm.H = kv_heads;
+  prm.q_heads = q_heads;
+  prm.row_heads = d.row_heads;
+  prm.row_to_kv = d.row_to_kv;
+  prm.group = d.group;
+  prm.subs = d.subs;
+  prm.gs = d.gs;
+  prm.batch = batch;
+  prm.tail_slot0 = tail_slot0;
+  prm.n_tokens = static_cast<int>(n_tokens);
+  prm.splits = d.splits;
+  prm.partial_o = static_cast<float*>(partial_o);
+  prm.partial_ml = static_cast<float*>(partial_ml);
+  prm.counters = static_cast<unsigned*>(counters);
+  prm.scale_log2 = sm_scale * 1.4426950408889634f;
+  prm.seq_len_dev = seq_len_dev;
+  prm.seqs = seqs;
+  if (dtype == ADAMAS_F16)
+    ADAMAS_LAUNCH("paged_decode_kernel", paged_decode_kernel<__half>, dim3(d.blocks), dim3(kDecThreads), kDecSmem, to_stream(stream), 1, prm);
+  else
+    ADAMAS_LAUNCH("paged_decode_kernel", paged_decode_kernel<__nv_bfloat16>, dim3(d.blocks), dim3(kDecThreads), kDecSmem, to_stream(stream), 1, prm);
+  return check_launch("paged_decode_kernel");
+}
+
 // seq_len_dev (optional): attend to every token of a sequence whose length lives on the device; indices
 // is then the page table, n_idx / tail_len describe the LONGEST sequence (they size the grid), and the
 // kernel derives the actual lists from the device value.
@@ -949,58 +1014,22 @@ static int decode_forward_impl(adamas_decode_handler_t* handler, const void* q, 
   ADAMAS_REQUIRE(last_page_idx >= 0, "last_page_idx must be >= 0");
   const int64_t n_tokens = static_cast<int64_t>(n_idx) * idx_unit + tail_len;
   ADAMAS_REQUIRE(n_tokens >= 1, "nothing to attend to");
-  ADAMAS_REQUIRE(n_tokens < (int64_t(1) << 31) - kDecTile, "too many tokens");
+  ADAMAS_REQUIRE(n_tokens < (int64_t(1) << 31) - 64, "too many tokens");
   ADAMAS_REQUIRE(idx_stride == 0 || idx_stride >= n_idx || handler->num_heads == 1,
                  "idx_stride must be 0 (shared row) or >= n_idx");
-  const int H = handler->num_heads;
-  const SplitPlan p = plan_splits(n_tokens, H * batch, handler->num_sms);
-  if (static_cast<int64_t>(H) * batch * p.num_splits > handler->cap_units)
-    return fail(ADAMAS_ERR_STATE,
-                "decode forward needs %d splits per head but begin_forward planned for fewer tokens",
-                p.num_splits);
-  size_t off_ml, off_cnt;
-  scratch_layout(handler->cap_units, handler->cap_heads, &off_ml, &off_cnt);
-  DecodeParams prm;
-  prm.q = q;
-  prm.o = o;
-  prm.o_f32 = o_f32;
-  prm.lse = lse;
-  prm.kv = kv_data;
-  prm.indices = indices ? indices : reinterpret_cast<const int32_t*>(kv_data);
-  prm.seqs = seqs;
-  prm.idx_stride = idx_stride;
-  prm.n_idx = n_idx;
-  prm.idx_unit = idx_unit;
-  prm.page_size = ps;
-  prm.H = handler->kv_heads;
-  prm.q_group = H / handler->kv_heads;
   const int64_t tail0 = static_cast<int64_t>(last_page_idx) * ps + (last_page_len - tail_len);
   ADAMAS_REQUIRE(tail0 + tail_len < (int64_t(1) << 31), "token slots must be below 2^31");
-  prm.tail_slot0 = static_cast<unsigned>(tail0);
-  prm.ps_shift = -1;
-  if ((ps & (ps - 1)) == 0) {
-    prm.ps_shift = 0;
-    while ((1 << prm.ps_shift) < ps) ++prm.ps_shift;
-  }
-  prm.n_tokens = static_cast<int>(n_tokens);
-  prm.tiles_per_block = p.tiles_per_block;
-  prm.num_splits = p.num_splits;
+  const int H = handler->num_heads;
+  // (a list row shared by all heads: the query heads of a cache head go through the tiles together)
+  const DecPlan d = plan_decode(n_tokens, batch, handler->kv_heads, H, idx_stride == 0, handler->num_sms);
+  if (dec_scratch_units(static_cast<int64_t>(H) * batch, H / handler->kv_heads, handler->num_sms) > handler->cap_units || H * batch > handler->cap_heads)
+    return fail(ADAMAS_ERR_STATE, "begin_forward planned for fewer heads than decode forward needs");
+  size_t off_ml, off_cnt;
+  scratch_layout(handler->cap_units, handler->cap_heads, &off_ml, &off_cnt);
   uint8_t* base = static_cast<uint8_t*>(handler->scratch);
-  prm.partial_o = reinterpret_cast<float*>(base);
-  prm.partial_ml = reinterpret_cast<float*>(base + off_ml);
-  prm.counters = reinterpret_cast<unsigned*>(base + off_cnt);
-  prm.scale_log2 = sm_scale * 1.4426950408889634f;
-  prm.seq_len_dev = seq_len_dev;
-  // (with the length on the device a block may get more than one tile later on: two stages)
-  const size_t smem = static_cast<size_t>(p.tiles_per_block > 1 || seq_len_dev ? 2 : 1) * kDecStageBytes;
-  dim3 grid(p.num_splits, H, batch);
-  if (handler->dtype == ADAMAS_F16)
-    ADAMAS_LAUNCH("sparse_decode_kernel", sparse_decode_kernel<__half>, grid, dim3(kDecThreads), smem,
-                  to_stream(stream), 1, prm);
-  else
-    ADAMAS_LAUNCH("sparse_decode_kernel", sparse_decode_kernel<__nv_bfloat16>, grid, dim3(kDecThreads), smem,
-                  to_stream(stream), 1, prm);
-  return check_launch("sparse_decode_kernel");
+  return launch_decode(d, q, o, o_f32, lse, kv_data, indices, idx_stride, n_idx, idx_unit, ps, handler->kv_heads, H,
+                       static_cast<unsigned>(tail0), n_tokens, sm_scale, handler->dtype, base, base + off_ml, base + off_cnt,
+                       seq_len_dev, seqs, batch, stream);
 }
 
 int adamas_decode_forward(adamas_decode_handler_t* handler, const void* q, void* o, float* lse,
@@ -1025,7 +1054,7 @@ int adamas_decode_forward_partial(adamas_decode_handler_t* handler, const void* 
 // max / sum pairs and the per-head arrival counters) lives in the fixed array below instead of a
 // handler-owned cudaMalloc buffer.  Every device that loads this library keeps the array until
 // the process exits; all calls on a device share it.
-constexpr int kStaticMaxUnits = 2048;   // heads x splits
+constexpr int kStaticMaxUnits = 2048;   // results parked by blocks (dec_scratch_units)
 constexpr int kStaticMaxHeads = 256;
 constexpr size_t kStaticOffMl = static_cast<size_t>(kStaticMaxUnits) * kHeadDim * sizeof(float);
 constexpr size_t kStaticOffCnt = kStaticOffMl + static_cast<size_t>(kStaticMaxUnits) * 2 * sizeof(float);
@@ -1046,7 +1075,7 @@ int adamas_decode_forward_static(const void* q, void* o, float* lse, const void*
   ADAMAS_REQUIRE(last_page_idx >= 0, "last_page_idx must be >= 0");
   const int64_t n_tokens = static_cast<int64_t>(n_idx) * idx_unit + tail_len;
   ADAMAS_REQUIRE(n_tokens >= 1, "nothing to attend to");
-  ADAMAS_REQUIRE(n_tokens < (int64_t(1) << 31) - kDecTile, "too many tokens");
+  ADAMAS_REQUIRE(n_tokens < (int64_t(1) << 31) - 64, "too many tokens");
   ADAMAS_REQUIRE(idx_stride == 0 || idx_stride >= n_idx || num_heads == 1,
                  "idx_stride must be 0 (shared row) or >= n_idx");
 
@@ -1067,57 +1096,22 @@ int adamas_decode_forward_static(const void* q, void* o, float* lse, const void*
   }
   init_lock.unlock();
 
-  const SplitPlan p = plan_splits(n_tokens, num_heads, di->num_sms);
   ADAMAS_REQUIRE(num_heads <= kStaticMaxHeads,
                  "adamas_decode_forward_static supports at most %d heads (got %d)", kStaticMaxHeads,
                  num_heads);
-  ADAMAS_REQUIRE(static_cast<int64_t>(num_heads) * p.num_splits <= kStaticMaxUnits,
-                 "adamas_decode_forward_static: %d heads x %d splits exceeds the fixed scratch of %d "
-                 "(head, split) units; use the handler-based adamas_decode_forward",
-                 num_heads, p.num_splits, kStaticMaxUnits);
-
-  uint8_t* base = static_cast<uint8_t*>(scratch_ptr[dev]);
-  cudaStream_t st = to_stream(stream);
-  // the arrival counters must start at zero whatever an earlier (possibly failed) call left behind
-  ADAMAS_CUDA(cudaMemsetAsync(base + kStaticOffCnt, 0, static_cast<size_t>(num_heads) * sizeof(unsigned), st));
-
-  DecodeParams prm;
-  prm.q = q;
-  prm.o = o;
-  prm.o_f32 = nullptr;
-  prm.lse = lse;
-  prm.kv = kv_data;
-  prm.indices = indices ? indices : reinterpret_cast<const int32_t*>(kv_data);
-  prm.idx_stride = idx_stride;
-  prm.n_idx = n_idx;
-  prm.idx_unit = idx_unit;
-  prm.page_size = page_size;
-  prm.H = num_heads;
-  prm.q_group = 1;
-  prm.seqs = nullptr;
+  const DecPlan d = plan_decode(n_tokens, 1, num_heads, num_heads, idx_stride == 0, di->num_sms);
+  ADAMAS_REQUIRE(dec_scratch_units(num_heads, 1, di->num_sms) <= kStaticMaxUnits,
+                 "adamas_decode_forward_static: the fixed scratch of %d results is too small for this device; use the "
+                 "handler-based adamas_decode_forward", kStaticMaxUnits);
   const int64_t tail0 = static_cast<int64_t>(last_page_idx) * page_size + (last_page_len - tail_len);
   ADAMAS_REQUIRE(tail0 + tail_len < (int64_t(1) << 31), "token slots must be below 2^31");
-  prm.tail_slot0 = static_cast<unsigned>(tail0);
-  prm.ps_shift = -1;
-  if ((page_size & (page_size - 1)) == 0) {
-    prm.ps_shift = 0;
-    while ((1 << prm.ps_shift) < page_size) ++prm.ps_shift;
-  }
-  prm.n_tokens = static_cast<int>(n_tokens);
-  prm.tiles_per_block = p.tiles_per_block;
-  prm.num_splits = p.num_splits;
-  prm.partial_o = reinterpret_cast<float*>(base);
-  prm.partial_ml = reinterpret_cast<float*>(base + kStaticOffMl);
-  prm.counters = reinterpret_cast<unsigned*>(base + kStaticOffCnt);
-  prm.scale_log2 = sm_scale * 1.4426950408889634f;
-  prm.seq_len_dev = nullptr;
-  const size_t smem = static_cast<size_t>(p.tiles_per_block > 1 ? 2 : 1) * kDecStageBytes;
-  dim3 grid(p.num_splits, num_heads);
-  if (dtype == ADAMAS_F16)
-    sparse_decode_kernel<__half><<<grid, kDecThreads, smem, st>>>(prm);
-  else
-    sparse_decode_kernel<__nv_bfloat16><<<grid, kDecThreads, smem, st>>>(prm);
-  return check_launch("sparse_decode_kernel (static scratch)");
+
+  uint8_t* base = static_cast<uint8_t*>(scratch_ptr[dev]);
+  // the arrival counters must start at zero whatever an earlier (possibly failed) call left behind
+  ADAMAS_CUDA(cudaMemsetAsync(base + kStaticOffCnt, 0, static_cast<size_t>(num_heads) * sizeof(unsigned), to_stream(stream)));
+  return launch_decode(d, q, o, nullptr, lse, kv_data, indices, idx_stride, n_idx, idx_unit, page_size, num_heads, num_heads,
+                       static_cast<unsigned>(tail0), n_tokens, sm_scale, dtype, base, base + kStaticOffMl, base + kStaticOffCnt,
+                       nullptr, nullptr, 1, stream);
 }
 
 }  // extern "C"

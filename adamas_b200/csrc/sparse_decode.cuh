@@ -1,337 +1,517 @@
-// Stage 4 of the decode path: decode attention of one query row per head over a per-head list of
-// selected token slots (plus an always-attended tail) in the paged KV cache.
+// Stage 4 of the decode path: decode attention of one query row per head over a list of token slots in the
+// paged KV cache: a per-head list of selected slots (plus an always-attended tail), or, in the dense layers,
+// every token of the sequence through its page table.
 //
-// grid = (num_splits, H).  A thread block walks its share of the head's token list in tiles of
-// kDecTile tokens.  For each tile it resolves the token slots from the index list, gathers the
-// 256-byte K and V rows into shared memory with one bulk (TMA) copy per row (double buffered across
-// tiles, one mbarrier per stage counting the bytes; waits are bounded), computes the logits with two
-// threads per token, runs an online softmax in base 2, and accumulates P.V with one thread per (token
-// group, 8-dim chunk).  Rows are padded to 272 bytes so that both access patterns are bank-conflict
-// free.
-//
-// With more than one split per head each block writes an unnormalised partial (o, m, l) to global
-// scratch, and the block that arrives last at the head's counter merges the partials and writes the
-// output (no block ever waits for another).  The counter is left at zero for the next launch.
+// Bound: HBM (512 bytes of K and V per attended token and cache head; the contraction is one to a few query
+// rows deep).  What the kernel is built around is therefore bytes in flight and few instructions per byte:
+//   * A warp works alone on tiles of 16 tokens of one cache head, gathered by its own 16-byte asynchronous copies
+//     into a ring of kDecStages tiles (8 KB each) in shared memory: no block barrier, and 16 KB on their way per
+//     warp whatever the warp is doing.  (The same tiles loaded straight into registers measured 160-185 us instead
+//     of 126: the loads shared scoreboards with the softmax's shuffles, which then waited for memory.)
+//   * q.K and P.V run on the tensor cores (mma.sync m16n8k16, fp32 accumulation) for up to 8 query heads that
+//     share the cache head (grouped queries), so a K/V row is read once per group and not once per query head.
+//     Even for a single query head the matrix form needs about half of the instructions of a multiply-add form.
+//     The order of the 128 dimensions is free in q.K, and of the output rows in P.V, so every lane reads whole
+//     16-byte chunks: chunk 4j + t of K rows g and g + 8, chunks g and 8 + g of V rows 2t, 2t + 1, 2t + 8, 2t + 9
+//     (g = lane / 4, t = lane % 4).  Chunk c of row r is stored at c ^ dec_swizzle(r), which makes both patterns
+//     free of bank conflicts.
+//   * P enters P.V as the sum of two 16-bit numbers (its rounding and the remainder), so that it keeps more than
+//     16 bits for fp16 rows and 16 for bf16.
+// A block is 4 warps that deal out the tiles of one row group (a cache head and its query heads), two blocks per SM.
+// The work of a launch is a line of tiles, row group after row group; each block takes an equal piece of it (so that
+// sequences of different lengths and head counts that do not divide the chip leave nothing idle), or, for small
+// launches where the latency of a second row group would count, an equal share of one.  A row group cut over several
+// blocks is merged by the block that arrives last at its counter (no block ever waits for another).
+// Measured, attention over all tokens of a layer: 32 heads x 32768 tokens, fp16: 125 -> 87 us (6.2 TB/s; 96 % of the
+// copy rate); 21 sequences x 64 query heads over 8 x 7366 tokens: 1097 -> 118 us.  One block of 8 warps per SM: 91 us
+// (the end of a piece leaves the SM idle); three blocks of 4 with two ring slots: 93 us.  Blocks that take four
+// neighbouring heads of a token (1 KB in a row) measured no better than one head per block.
 #pragma once
 #include "common.cuh"
 
 namespace adamas {
 
-constexpr int kDecTile = 64;       // tokens per tile
-constexpr int kDecThreads = 128;
-constexpr int kDecRowBytes = kHeadDim * 2 + 16;             // a row plus 16 bytes of padding
-constexpr int kDecStageBytes = 2 * kDecTile * kDecRowBytes;  // K + V rows of one tile (34 KB)
+constexpr int kDecTile = 16;        // tokens per warp tile
+constexpr int kDecWarps = 4;
+constexpr int kDecBlocksPerSm = 2;
+constexpr int kDecThreads = kDecWarps * 32;
+constexpr int kDecStages = 3;
+constexpr int kDecTileBytes = 2 * kDecTile * kHeadDim * 2;   // 16 K rows, 16 V rows
+constexpr int kDecMaxGroup = 8;     // query heads per matrix instruction; larger groups are split
+constexpr int kDecMaxBatch = 1024;
+constexpr int kDecMinTiles = 6;     // tiles a block is worth starting for
 
 struct DecodeParams {
-  const void* q;          // [H, 128]
-  void* o;                // [H, 128] in the cache's element type, or null
-  float* o_f32;           // [H, 128] fp32 output (partial results of a sequence shard), or null
-  float* lse;             // [H] or null (base-2 log-sum-exp of the scaled logits)
+  const void* q;          // [rows, 128]
+  void* o;                // [rows, 128] in the cache's element type, or null
+  float* o_f32;           // [rows, 128] fp32 output (partial results of a sequence shard), or null
+  float* lse;             // [rows] or null (base-2 log-sum-exp of the scaled logits)
   const void* kv;         // [pages, 2, page_size, H, 128]
-  const int32_t* indices; // [H, idx_stride]
+  const int32_t* indices; // [q heads, idx_stride], or one row for all heads (idx_stride 0)
   int64_t idx_stride;
-  int n_idx;              // indices used per head
+  int n_listed;           // tokens the index list stands for
   int idx_unit;           // token slots covered by one index
   int page_size;
-  int H;                  // heads of the KV cache
-  int q_group;            // query heads per cache head (1: multi-head attention); the grid has H * q_group rows
-  unsigned tail_slot0;    // physical token slot of the first tail token
   int ps_shift;           // log2(page_size) or -1
-  int n_tokens;           // n_idx * idx_unit + tail_len
-  int tiles_per_block;
-  int num_splits;
-  float* partial_o;       // [H, num_splits, 128]
-  float* partial_ml;      // [H, num_splits, 2]
-  unsigned* counters;     // [H], zero on entry and on exit
+  int H;                  // heads of the KV cache
+  int q_heads;
+  // row heads: what a tile belongs to.  One list for all heads: the cache heads, each with `group` query heads in
+  // `subs` parts of at most `gs`.  A list per query head: the query heads, group 1 (row_to_kv of them share a cache head).
+  int row_heads, row_to_kv, group, subs, gs;
+  int batch;
+  unsigned tail_slot0;    // physical token slot of the first tail token (tokens n_listed ..)
+  int n_tokens;
+  int splits;             // > 0: blocks per row group; 0: the line of all tiles is cut evenly over the grid
+  float* partial_o;       // [units * gs, 128]
+  float* partial_ml;      // [units * gs, 2]
+  unsigned* counters;     // [row groups], zero on entry and on exit
   float scale_log2;       // sm_scale * log2(e)
-  // optional: attend to EVERY token of a sequence whose length lives on the device (the dense layers
-  // of a graph-captured decode step): `indices` is then the page table (idx_stride 0, idx_unit =
-  // page_size) and n_idx, n_tokens, tail_slot0 and tiles_per_block are derived from *seq_len_dev here;
-  // num_splits (the grid) was sized for the longest sequence.
+  // optional: attend to EVERY token of a sequence whose length lives on the device (the dense layers of a
+  // graph-captured decode step): `indices` is then the page table
   const int32_t* seq_len_dev;
-  // optional (needs seq_len_dev): a batch of sequences, grid.z = sequence.  q, o, o_f32, lse and the
-  // scratch have one row per (sequence, head); the cache, its page table and the length are the sequence's.
+  // optional (needs seq_len_dev): a batch of sequences.  q, o, o_f32 and lse have one row per (sequence, head); the
+  // cache, its page table and the length are the sequence's.
   const SeqDesc* seqs;
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kDecThreads, 4) sparse_decode_kernel(DecodeParams prm) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ float s_logit[kDecTile];
-  __shared__ unsigned char s_skip[2][kDecTile];   // per stage: token masked out (negative index)
-  __shared__ float s_p[kDecTile];
-  __shared__ float s_red[4];
-  __shared__ float s_sum[4];
-  __shared__ float s_o[8][kHeadDim];
-  __shared__ unsigned s_last;
-  __shared__ __align__(8) uint64_t full_bar[2];
-
-  const int split = blockIdx.x;
-  const int head = blockIdx.z * gridDim.y + blockIdx.y;   // row of q, o, lse and the scratch: (sequence, query head)
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-  const int H = prm.H;
-  const int head_kv = prm.q_group == 1 ? blockIdx.y : blockIdx.y / prm.q_group;
-
-  const T* kvp = static_cast<const T*>(prm.kv);
-  const int32_t* idx_row = prm.indices + static_cast<int64_t>(head) * prm.idx_stride;
-  const int32_t* seq_len_dev = prm.seq_len_dev;
-  if (prm.seqs) {   // (the table of sequences is set up once, long before this launch)
-    kvp = static_cast<const T*>(prm.seqs[blockIdx.z].kv_data);
-    idx_row = prm.seqs[blockIdx.z].kv_table;
-    seq_len_dev += blockIdx.z;
+struct Mma;
+template <>
+struct Mma<__half> {
+  static __device__ __forceinline__ void run(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
   }
-  const int64_t v_delta = static_cast<int64_t>(prm.page_size) * H * kHeadDim;
+};
+template <>
+struct Mma<__nv_bfloat16> {
+  static __device__ __forceinline__ void run(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+};
 
-  // ---- gather one tile into a stage --------------------------------------------------------------
-  // thread -> (token tl = tid / 2, K or V row): one 256-byte bulk copy each.  Every thread arrives at
-  // the stage's barrier once, with the bytes it has asked for (none for a skipped or absent token).
-  // Slots are < 2^31 (checked on the host), so the index arithmetic is 32-bit; only the final element
-  // offset is 64-bit.
-  if (tid == 0) {
-    mbar_init(&full_bar[0], kDecThreads);
-    mbar_init(&full_bar[1], kDecThreads);
-    mbar_fence_init();
+// The token list of one row.
+struct DecRow {
+  const int32_t* idx;
+  int n_listed, n_tokens;
+  unsigned tail_slot0;
+};
+
+// The list entry token j is looked up by (a page number or a slot; requested well before it is needed) ...
+__device__ __forceinline__ int dec_list_entry(const DecodeParams& p, const DecRow& r, int j) {
+  if (j >= min(r.n_listed, r.n_tokens)) return 0;
+  const unsigned uj = static_cast<unsigned>(j);
+  const unsigned item = p.idx_unit == 1 ? uj : p.ps_shift >= 0 ? uj >> p.ps_shift : uj / static_cast<unsigned>(p.page_size);
+  return __ldg(r.idx + item);
+}
+// ... and the row of the cache (in units of H * 128 elements, K part) it stands for, or -1: absent, or a hole in the list.
+__device__ __forceinline__ int dec_cache_row(const DecodeParams& p, const DecRow& r, int j, int entry) {
+  if (j >= r.n_tokens) return -1;
+  const unsigned ps = static_cast<unsigned>(p.page_size), uj = static_cast<unsigned>(j);
+  unsigned page, off;
+  if (j < r.n_listed && p.idx_unit != 1) {   // whole pages: idx_unit == page_size
+    page = static_cast<unsigned>(entry);
+    off = p.ps_shift >= 0 ? uj & (ps - 1) : uj % ps;
+  } else {
+    if (j < r.n_listed && entry < 0) return -1;
+    const unsigned slot = j < r.n_listed ? static_cast<unsigned>(entry) : r.tail_slot0 + static_cast<unsigned>(j - r.n_listed);
+    page = p.ps_shift >= 0 ? slot >> p.ps_shift : slot / ps;
+    off = slot - page * ps;
+  }
+  return static_cast<int>(page * (2 * ps) + off);
+}
+
+// State of a warp over the tiles it has seen: head g = lane / 4 in m, l (l: this lane's tokens only);
+// o[j]: output dims (8g' + j, 64 + 8g' + j) of heads 2t, 2t + 1 with g' = lane / 4 (the C fragment of P.V).
+struct DecState {
+  float m, l;
+  float o[8][4];
+};
+
+__device__ __forceinline__ int dec_swizzle(int r) { return (r & 6) ^ ((r & 1) << 2); }
+
+// Requests tile `tile` (16 K rows, 16 V rows) into a ring slot and returns the mask of its tokens that exist.  An
+// absent token counts with weight 0, but its values still go through P.V and have to be finite: it borrows the row
+// of one that exists (a tile without any is skipped by its consumer).
+template <typename T>
+__device__ __forceinline__ unsigned dec_request(const DecodeParams& p, const DecRow& r, int tile, int entry, const T* kbase,
+                                                int64_t row_elems, uint8_t* slot, int lane) {
+  int row = dec_cache_row(p, r, tile * kDecTile + (lane & 15), entry);
+  const unsigned mask = __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
+  const int safe = __shfl_sync(0xffffffffu, row, mask ? __ffs(mask) - 1 : 0);
+  row = max(row >= 0 ? row : safe, 0);
+  const int half = lane >> 4, c = lane & 15;
+  const int64_t v_delta = p.page_size * row_elems;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {   // a half-warp per row
+    const int rr = 2 * i + half;
+    const T* src = kbase + __shfl_sync(0xffffffffu, row, rr) * row_elems + c * 8;
+    uint8_t* dst = slot + rr * 256 + ((c ^ dec_swizzle(rr)) << 4);
+    cp_async_16(dst, src);
+    cp_async_16(dst + kDecTile * 256, src + v_delta);
+  }
+  return mask;
+}
+
+__device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// One tile: logits (S[head g][tokens 2t, 2t + 1, 2t + 8, 2t + 9] in this lane), softmax in base 2, P.V.
+template <typename T>
+__device__ __forceinline__ void dec_tile(DecState& st, const uint8_t* slot, const uint4 (&q)[4], unsigned mask, float scale_log2,
+                                         int lane) {
+  if (mask == 0) return;
+  const int g = lane >> 2, t = lane & 3;
+  float c[2][2][4] = {};   // [rows g, g + 8][two accumulators: shorter chains]
+  const uint8_t* krow = slot + g * 256;
+  const int ksw = dec_swizzle(g);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint4 k = *reinterpret_cast<const uint4*>(krow + u * 2048 + (((4 * j + t) ^ ksw) << 4));
+      Mma<T>::run(c[u][0], q[j].x, 0u, q[j].y, 0u, k.x, k.y);
+      Mma<T>::run(c[u][1], q[j].z, 0u, q[j].w, 0u, k.z, k.w);
+    }
+  }
+  uint4 v[4][2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int rr = 2 * t + (u & 1) + 8 * (u >> 1);
+    const uint8_t* vrow = slot + kDecTile * 256 + rr * 256;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) v[u][h] = *reinterpret_cast<const uint4*>(vrow + (((g + 8 * h) ^ dec_swizzle(rr)) << 4));
+  }
+  float s[4] = {c[0][0][0] + c[0][1][0], c[0][0][1] + c[0][1][1], c[1][0][0] + c[1][1][0], c[1][0][1] + c[1][1][1]};
+#pragma unroll
+  for (int u = 0; u < 4; ++u) s[u] = (mask >> (2 * t + (u & 1) + 8 * (u >> 1))) & 1u ? s[u] * scale_log2 : -INFINITY;
+  float m_new = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+  m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
+  m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
+  m_new = fmaxf(m_new, st.m);
+  if (__any_sync(0xffffffffu, m_new > st.m)) {
+    const float r = (st.m == -INFINITY) ? 0.f : exp2f(st.m - m_new);
+    st.l *= r;
+    st.m = m_new;
+    const float r0 = __shfl_sync(0xffffffffu, r, 8 * t), r1 = __shfl_sync(0xffffffffu, r, 8 * t + 4);   // heads 2t, 2t + 1
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      st.o[j][0] *= r0;
+      st.o[j][1] *= r1;
+      st.o[j][2] *= r0;
+      st.o[j][3] *= r1;
+    }
+  }
+  float pr[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) pr[u] = exp2f(s[u] - st.m);   // (a masked token: exp2(-inf) = 0; st.m is finite)
+  st.l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
+  // B fragments of P.V: tokens 2t, 2t + 1 and 2t + 8, 2t + 9 of head g
+  const uint32_t hi0 = Elem<T>::from_f2(pr[0], pr[1]), hi1 = Elem<T>::from_f2(pr[2], pr[3]);
+  const float2 f0 = Elem<T>::to_f2(hi0), f1 = Elem<T>::to_f2(hi1);
+  const uint32_t lo0 = Elem<T>::from_f2(pr[0] - f0.x, pr[1] - f0.y), lo1 = Elem<T>::from_f2(pr[2] - f1.x, pr[3] - f1.y);
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    uint32_t a[2][4];   // [even / odd dimension of the word][a0 .. a3]
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {   // rows g (dims 8g ..) and g + 8 (dims 64 + 8g ..)
+      const uint32_t v0 = word_of(v[0][h], w), v1 = word_of(v[1][h], w);
+      const uint32_t v2 = word_of(v[2][h], w), v3 = word_of(v[3][h], w);
+      a[0][h] = __byte_perm(v0, v1, 0x5410);
+      a[1][h] = __byte_perm(v0, v1, 0x7632);
+      a[0][2 + h] = __byte_perm(v2, v3, 0x5410);
+      a[1][2 + h] = __byte_perm(v2, v3, 0x7632);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) Mma<T>::run(st.o[2 * w + e], a[e][0], a[e][1], a[e][2], a[e][3], hi0, hi1);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) Mma<T>::run(st.o[2 * w + e], a[e][0], a[e][1], a[e][2], a[e][3], lo0, lo1);
+  }
+}
+
+struct DecShared {
+  float ml[kDecWarps][kDecMaxGroup][2];
+  int cum[kDecMaxBatch + 1];     // tiles of the sequences before (batched launches)
+  unsigned last;
+};
+
+// Dynamic shared memory: the rings, [4 warps][kDecStages][16 K rows, 16 V rows]; a warp parks its results in its own ring.
+template <typename T>
+__global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_kernel(const DecodeParams p) {
+  extern __shared__ __align__(128) uint8_t dec_smem[];
+  __shared__ DecShared sh;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  // The index list and the query are the preceding kernels' output (a RoPE-fused append rotates q in place), so
+  // nothing of them is touched before the dependency has resolved.  A dense step over a device-resident length is
+  // different: the length, the page tables and every cached row but the newest token's were final before the
+  // preceding kernel, the append, started, so the first tiles are requested while that one still runs.
+  bool waited = p.seq_len_dev == nullptr;
+  if (waited) grid_dependency_wait();
+  grid_launch_dependents();
+
+  const int rps = p.row_heads * p.subs;   // row groups per sequence
+  if (p.seqs) {
+    if (warp == 0) {
+      int base = 0;
+      for (int s0 = 0; s0 < p.batch; s0 += 32) {
+        int v = s0 + lane < p.batch ? (__ldg(p.seq_len_dev + s0 + lane) + kDecTile - 1) / kDecTile : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, v, o);
+          if (lane >= o) v += u;
+        }
+        if (s0 + lane < p.batch) sh.cum[s0 + lane + 1] = base + v;
+        base += __shfl_sync(0xffffffffu, v, 31);
+      }
+      if (lane == 0) sh.cum[0] = 0;
+    }
+  } else if (tid == 0) {
+    sh.cum[0] = 0;
+    sh.cum[1] = ((p.seq_len_dev ? __ldg(p.seq_len_dev) : p.n_tokens) + kDecTile - 1) / kDecTile;
   }
   __syncthreads();
-  // The index list, the query and a device-resident length are the preceding kernels' output (a
-  // RoPE-fused append rotates q in place), so nothing of them is touched before the dependency has
-  // resolved.
-  grid_dependency_wait();
-  grid_launch_dependents();
-  int n_tokens = prm.n_tokens, tiles_per_block = prm.tiles_per_block, n_listed = prm.n_idx * prm.idx_unit;
-  unsigned tail_slot0 = prm.tail_slot0;
-  if (seq_len_dev) {
-    const int len = __ldg(seq_len_dev);
-    const int pages = (len + prm.page_size - 1) / prm.page_size;
-    n_listed = (pages - 1) * prm.page_size;
-    n_tokens = len;
-    tail_slot0 = static_cast<unsigned>(__ldg(idx_row + pages - 1)) * static_cast<unsigned>(prm.page_size);
-    const int tiles = (len + kDecTile - 1) / kDecTile;
-    tiles_per_block = (tiles + prm.num_splits - 1) / prm.num_splits;
-  }
-  const int tok_begin = split * tiles_per_block * kDecTile;
-  const int tok_end = min(n_tokens, tok_begin + tiles_per_block * kDecTile);
-  const int n_tiles = max(0, (tok_end - tok_begin + kDecTile - 1) / kDecTile);
-  auto issue_tile = [&](int tile, int stage) {
-    uint8_t* sk = smem + stage * kDecStageBytes;
-    uint8_t* sv = sk + kDecTile * kDecRowBytes;
-    const int tl = tid >> 1;
-    const int is_v = tid & 1;
-    const int j = tok_begin + tile * kDecTile + tl;
-    const unsigned ps = static_cast<unsigned>(prm.page_size);
-    bool ok = j < tok_end;
-    unsigned slot = 0;
-    if (ok) {
-      if (j < n_listed) {
-        if (prm.idx_unit == 1) {
-          const int32_t id = __ldg(idx_row + j);
-          ok = id >= 0;   // a negative entry is a hole in the list: the token is skipped
-          slot = static_cast<unsigned>(id);
-        } else {  // page-granular list: idx_unit == page_size
-          unsigned item, off;
-          if (prm.ps_shift >= 0) {
-            item = static_cast<unsigned>(j) >> prm.ps_shift;
-            off = static_cast<unsigned>(j) & (ps - 1);
-          } else {
-            item = static_cast<unsigned>(j) / ps;
-            off = static_cast<unsigned>(j) - item * ps;
-          }
-          slot = static_cast<unsigned>(__ldg(idx_row + item)) * ps + off;
-        }
-      } else {
-        slot = tail_slot0 + static_cast<unsigned>(j - n_listed);
-      }
-    }
-    if (is_v == 0) s_skip[stage][tl] = ok ? 0 : 1;
-    if (ok) {
-      unsigned page, e;
-      if (prm.ps_shift >= 0) {
-        page = slot >> prm.ps_shift;
-        e = slot & (ps - 1);
-      } else {
-        page = slot / ps;
-        e = slot - page * ps;
-      }
-      const int64_t row = static_cast<int64_t>(page) * (2 * ps) + e;
-      const T* src = kvp + (row * H + head_kv) * kHeadDim + (is_v ? v_delta : 0);
-      mbar_arrive_expect_tx(&full_bar[stage], kHeadDim * 2);
-      bulk_copy_g2s((is_v ? sv : sk) + tl * kDecRowBytes, src, kHeadDim * 2, &full_bar[stage]);
-    } else {
-      mbar_arrive(&full_bar[stage]);
-    }
+
+  const int total = sh.cum[p.batch] * rps;
+  // (with the lengths on the device the work may be far less than the grid was sized for: every piece has tiles)
+  const int b = blockIdx.x, B = max(1, min(static_cast<int>(gridDim.x), total / kDecMinTiles));
+  auto line_start = [&](int blk) { return static_cast<int>(static_cast<int64_t>(blk) * total / B); };
+  auto block_of = [&](int tile) {   // the block whose piece of the line holds `tile`
+    int k = static_cast<int>((static_cast<int64_t>(tile) * B) / total);
+    while (k + 1 < B && line_start(k + 1) <= tile) ++k;
+    return k;
   };
 
-  issue_tile(0, 0);
-
-  // ---- query: 64 dims per thread, in the order the thread walks its chunks ---------------------
-  // thread pair (tl = tid / 2, half = tid % 2); step i reads logical chunk half*8 + (i ^ half*4)
-  const int qk_tl = tid >> 1;
-  const int half = tid & 1;
-  float qreg[8][8];
-  {
-    const T* qp = static_cast<const T*>(prm.q) + static_cast<int64_t>(head) * kHeadDim;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int lc = half * 8 + (i ^ (half * 4));
-      unpack8<T>(ld_16(qp + lc * 8), qreg[i]);
-#pragma unroll
-      for (int d = 0; d < 8; ++d) qreg[i][d] *= prm.scale_log2;
+  if (p.splits == 0 && b >= B) return;
+  int pos = p.splits > 0 ? 0 : line_start(b);
+  const int line_end = p.splits > 0 ? 1 : line_start(b + 1);
+  while (pos < line_end) {
+    // ---- this block's next piece: tiles [a, e) of row group x of sequence s ------------------------------
+    int s, x, a, e, nparts, part, unit;
+    if (p.splits > 0) {
+      const int r = b / p.splits;
+      part = b - r * p.splits;
+      s = r / rps;
+      x = r - s * rps;
+      const int nt = sh.cum[s + 1] - sh.cum[s];
+      a = static_cast<int>(static_cast<int64_t>(nt) * part / p.splits);
+      e = static_cast<int>(static_cast<int64_t>(nt) * (part + 1) / p.splits);
+      nparts = p.splits;
+      unit = b;
+      pos = line_end;
+    } else {
+      int lo = 0, hi = p.batch - 1;
+      while (lo < hi) {   // the last sequence that starts at or before pos
+        const int mid = (lo + hi + 1) >> 1;
+        if (sh.cum[mid] * rps <= pos) lo = mid; else hi = mid - 1;
+      }
+      s = lo;
+      const int nt = sh.cum[s + 1] - sh.cum[s], seq0 = sh.cum[s] * rps;
+      x = (pos - seq0) / nt;
+      a = pos - seq0 - x * nt;
+      e = min(nt, a + line_end - pos);
+      const int row0 = seq0 + x * nt;
+      const int first = block_of(row0), last = block_of(row0 + nt - 1);
+      nparts = last - first + 1;
+      part = b - first;
+      unit = b + s * rps + x;   // strictly increasing along the line
+      pos += e - a;
     }
-  }
+    const int rh = x / p.subs, sub = x - rh * p.subs;         // row head
+    const int gsub = min(p.gs, p.group - sub * p.gs);         // query heads of this part
+    const int kv_head = rh / p.row_to_kv;
+    const int q_row0 = s * p.q_heads + rh * p.group + sub * p.gs;
 
+    const T* kvp = static_cast<const T*>(p.kv);
+    DecRow row;
+    row.idx = p.indices + (p.idx_stride ? static_cast<int64_t>(rh * p.group) * p.idx_stride : 0);
+    row.n_listed = p.n_listed;
+    row.n_tokens = p.n_tokens;
+    row.tail_slot0 = p.tail_slot0;
+    if (p.seqs) {
+      kvp = static_cast<const T*>(p.seqs[s].kv_data);
+      row.idx = p.seqs[s].kv_table;
+    }
+    if (p.seq_len_dev) row.n_tokens = row.n_listed = __ldg(p.seq_len_dev + s);
+    const int64_t row_elems = static_cast<int64_t>(p.H) * kHeadDim;
+    const T* kbase = kvp + kv_head * kHeadDim;
 
-  float m_run = -INFINITY, l_run = 0.f;
-  float o_acc[8];
+    DecState st;
+    st.m = -INFINITY;
+    st.l = 0.f;
 #pragma unroll
-  for (int d = 0; d < 8; ++d) o_acc[d] = 0.f;
-  const int pv_g = tid >> 4;   // token group: tokens pv_g*8 .. pv_g*8+7 of the tile
-  const int pv_c = tid & 15;   // 8-dim chunk
-
-  for (int tile = 0; tile < n_tiles; ++tile) {
-    const int stage = tile & 1;
-    if (tile + 1 < n_tiles) issue_tile(tile + 1, stage ^ 1);
-    // bounded wait for this tile's bytes (a stage is used every other tile: its phase parity follows)
-    if (!mbar_wait_bounded(&full_bar[stage], (tile >> 1) & 1, 1u << 20)) atomicOr(&g_adamas_error, kErrDecodeTimeout);
-    __syncthreads();   // s_skip of this stage is visible to all threads
-    const uint8_t* sk = smem + stage * kDecStageBytes;
-    const uint8_t* sv = sk + kDecTile * kDecRowBytes;
-    const int tile_tokens = min(kDecTile, tok_end - (tok_begin + tile * kDecTile));
-
-    // logits
-    float acc = 0.f;
-    const bool qk_live = qk_tl < tile_tokens && s_skip[stage][qk_tl] == 0;
-    if (qk_live) {
+    for (int j = 0; j < 8; ++j)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int lc = half * 8 + (i ^ (half * 4));
-        float kf[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(sk + qk_tl * kDecRowBytes + lc * 16), kf);
+      for (int i = 0; i < 4; ++i) st.o[j][i] = 0.f;
+
+    uint8_t* ring = dec_smem + warp * kDecStages * kDecTileBytes;
+    {
+      // tiles a + warp, + kDecWarps, ...: the list entries of a tile are fetched a round before its rows are requested, its
+      // rows kDecStages - 1 rounds before they are used
+      const int lane_tok = lane & 15;
+      int req = a + warp, entry = req < e ? dec_list_entry(p, row, req * kDecTile + lane_tok) : 0;
+      unsigned masks[kDecStages - 1];
 #pragma unroll
-        for (int d = 0; d < 8; ++d) acc = fmaf(qreg[i][d], kf[d], acc);
+      for (int i = 0; i < kDecStages - 1; ++i) {
+        masks[i] = 0;
+        if (req < e) {
+          const int cur = entry, nxt = req + kDecWarps;
+          entry = nxt < e ? dec_list_entry(p, row, nxt * kDecTile + lane_tok) : 0;
+          if (!waited && (req + 1) * kDecTile >= row.n_tokens) {   // (the newest token's tile)
+            grid_dependency_wait();
+            waited = true;
+          }
+          masks[i] = dec_request<T>(p, row, req, cur, kbase, row_elems, ring + i * kDecTileBytes, lane);
+          req = nxt;
+        }
+        cp_async_commit();
+      }
+      if (!waited) {
+        grid_dependency_wait();
+        waited = true;
+      }
+      // query fragments: head g, dims 32j + 8t .. + 7 (zeros for heads beyond the group)
+      uint4 q[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        q[j] = g < gsub ? ld_16(static_cast<const T*>(p.q) + static_cast<int64_t>(q_row0 + g) * kHeadDim + j * 32 + t * 8)
+                        : make_uint4(0, 0, 0, 0);
+      int use = 0, fill = kDecStages - 1;
+      for (int tile = a + warp; tile < e; tile += kDecWarps) {
+        unsigned mask_new = 0;
+        if (req < e) {
+          const int cur = entry, nxt = req + kDecWarps;
+          entry = nxt < e ? dec_list_entry(p, row, nxt * kDecTile + lane_tok) : 0;
+          mask_new = dec_request<T>(p, row, req, cur, kbase, row_elems, ring + fill * kDecTileBytes, lane);
+          req = nxt;
+        }
+        cp_async_commit();
+        cp_async_wait<kDecStages - 1>();
+        __syncwarp();
+        dec_tile<T>(st, ring + use * kDecTileBytes, q, masks[0], p.scale_log2, lane);
+        __syncwarp();   // the slot may be filled again
+#pragma unroll
+        for (int i = 0; i + 1 < kDecStages - 1; ++i) masks[i] = masks[i + 1];
+        masks[kDecStages - 2] = mask_new;
+        use = use + 1 == kDecStages ? 0 : use + 1;
+        fill = fill + 1 == kDecStages ? 0 : fill + 1;
+      }
+      cp_async_wait<0>();
+      __syncwarp();
+    }
+    // ---- the warps of a head -> one result per query head ---------------------------------------------------
+    st.l += __shfl_xor_sync(0xffffffffu, st.l, 1);
+    st.l += __shfl_xor_sync(0xffffffffu, st.l, 2);
+    if (t == 0) {
+      sh.ml[warp][g][0] = st.m;
+      sh.ml[warp][g][1] = st.l;
+    }
+    {
+      float* mine = reinterpret_cast<float*>(ring);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int h = 2 * t + i;
+        if (h < gsub) {
+#pragma unroll
+          for (int j = 0; j < 8; j += 4) {
+            *reinterpret_cast<float4*>(mine + h * kHeadDim + g * 8 + j) =
+                make_float4(st.o[j][i], st.o[j + 1][i], st.o[j + 2][i], st.o[j + 3][i]);
+            *reinterpret_cast<float4*>(mine + h * kHeadDim + 64 + g * 8 + j) =
+                make_float4(st.o[j][2 + i], st.o[j + 1][2 + i], st.o[j + 2][2 + i], st.o[j + 3][2 + i]);
+          }
+        }
       }
     }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    const float logit = qk_live ? acc : -INFINITY;
-    if (half == 0) s_logit[qk_tl] = logit;
-    float wmax = logit;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, o));
-    if (lane == 0) s_red[warp] = wmax;
     __syncthreads();
-
-    const float m_tile = fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3]));
-    const float m_new = fmaxf(m_run, m_tile);
-    const float rescale = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_new);
-    float psum = 0.f;
-    if (tid < kDecTile) {
-      const float lg = s_logit[tid];
-      const float p = (lg == -INFINITY) ? 0.f : exp2f(lg - m_new);   // masked tokens weigh nothing
-      s_p[tid] = p;
-      psum = p;
-    }
+    // a warp takes a query head: four dims per lane
+    auto finish = [&](int h, float M, float L, float4 acc) {
+      const int out = q_row0 + h;
+      const float inv = L > 0.f ? 1.f / L : 0.f;   // nothing attended: zeros and lse = -inf
+      acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
+      if (p.o_f32) reinterpret_cast<float4*>(p.o_f32 + static_cast<int64_t>(out) * kHeadDim)[lane] = acc;
+      if (p.o)
+        reinterpret_cast<uint2*>(static_cast<T*>(p.o) + static_cast<int64_t>(out) * kHeadDim)[lane] =
+            make_uint2(Elem<T>::from_f2(acc.x, acc.y), Elem<T>::from_f2(acc.z, acc.w));
+      if (lane == 0 && p.lse) p.lse[out] = L > 0.f ? M + log2f(L) : -INFINITY;
+    };
+    for (int h = warp; h < gsub; h += kDecWarps) {
+      float M = -INFINITY, L = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
-    if (lane == 0) s_sum[warp] = psum;
-    __syncthreads();
-    l_run = l_run * rescale + (s_sum[0] + s_sum[1]);
-    m_run = m_new;
-
-    // P.V for this thread's token group and chunk
+      for (int w = 0; w < kDecWarps; ++w) M = fmaxf(M, sh.ml[w][h][0]);
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int d = 0; d < 8; ++d) o_acc[d] *= rescale;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int tl = pv_g * 8 + i;
-      const float p = s_p[tl];
-      if (p != 0.f) {   // masked or absent tokens: their rows in shared memory are stale
-        float vf[8];
-        unpack8<T>(*reinterpret_cast<const uint4*>(sv + tl * kDecRowBytes + pv_c * 16), vf);
-#pragma unroll
-        for (int d = 0; d < 8; ++d) o_acc[d] = fmaf(p, vf[d], o_acc[d]);
+      for (int w = 0; w < kDecWarps; ++w) {
+        const float m = sh.ml[w][h][0];
+        const float wt = m == -INFINITY ? 0.f : exp2f(m - M);
+        const float4 v = reinterpret_cast<const float4*>(dec_smem + w * kDecStages * kDecTileBytes + h * kHeadDim * 4)[lane];
+        L += wt * sh.ml[w][h][1];
+        acc.x = fmaf(wt, v.x, acc.x);
+        acc.y = fmaf(wt, v.y, acc.y);
+        acc.z = fmaf(wt, v.z, acc.z);
+        acc.w = fmaf(wt, v.w, acc.w);
+      }
+      if (nparts > 1) {
+        const int64_t at = static_cast<int64_t>(unit) * p.gs + h;
+        __stcg(reinterpret_cast<float4*>(p.partial_o + at * kHeadDim) + lane, acc);
+        if (lane == 0) __stcg(reinterpret_cast<float2*>(p.partial_ml) + at, make_float2(M, L));
+      } else {
+        finish(h, M, L, acc);
       }
     }
-    __syncthreads();  // the stage is free for the tile after next; s_logit / s_p reusable
-  }
-
-  // ---- reduce the 8 token groups ----------------------------------------------------------------
+    __syncthreads();   // the parked results are read (the rings are free for the next piece), the parts are stored
+    if (nparts > 1) {
+      unsigned* counter = p.counters + s * rps + x;
+      if (tid == 0) {
+        unsigned ticket;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
+        sh.last = ticket == static_cast<unsigned>(nparts - 1);
+      }
+      __syncthreads();
+      if (sh.last) {
+        if (tid == 0) *counter = 0u;
+        for (int h = warp; h < gsub; h += kDecWarps) {
+          const int64_t at0 = static_cast<int64_t>(unit - part) * p.gs + h;
+          float M = -INFINITY, L = 0.f;
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int p0 = 0; p0 < nparts; p0 += 8) {   // eight parts' loads in flight
+            float2 ml[8];
+            float4 v[8];
 #pragma unroll
-  for (int d = 0; d < 8; ++d) s_o[pv_g][pv_c * 8 + d] = o_acc[d];
-  __syncthreads();
-  float od = 0.f;
+            for (int u = 0; u < 8; ++u) {
+              ml[u] = make_float2(-INFINITY, 0.f);
+              v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (p0 + u < nparts) {
+                ml[u] = __ldcg(reinterpret_cast<const float2*>(p.partial_ml) + at0 + (p0 + u) * p.gs);
+                v[u] = __ldcg(reinterpret_cast<const float4*>(p.partial_o + (at0 + (p0 + u) * p.gs) * kHeadDim) + lane);
+              }
+            }
+            float m_new = M;
 #pragma unroll
-  for (int g = 0; g < 8; ++g) od += s_o[g][tid];
-
-  T* op = static_cast<T*>(prm.o) + static_cast<int64_t>(head) * kHeadDim;
-  if (prm.num_splits == 1) {
-    const float r = l_run > 0.f ? od / l_run : 0.f;   // nothing attended: zeros and lse = -inf
-    // pairs of threads share a 32-bit store
-    const float r1 = __shfl_down_sync(0xffffffffu, r, 1);
-    if (prm.o_f32) prm.o_f32[static_cast<int64_t>(head) * kHeadDim + tid] = r;
-    if (prm.o && (tid & 1) == 0) reinterpret_cast<uint32_t*>(op)[tid >> 1] = Elem<T>::from_f2(r, r1);
-    if (tid == 0 && prm.lse) prm.lse[head] = l_run > 0.f ? m_run + log2f(l_run) : -INFINITY;
-    return;
-  }
-
-  const int64_t pidx = static_cast<int64_t>(head) * prm.num_splits + split;
-  prm.partial_o[pidx * kHeadDim + tid] = od;
-  if (tid == 0) {
-    prm.partial_ml[pidx * 2] = m_run;
-    prm.partial_ml[pidx * 2 + 1] = l_run;
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    const unsigned ticket = atomicAdd(prm.counters + head, 1u);
-    s_last = (ticket == static_cast<unsigned>(prm.num_splits - 1));
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-
-  // ---- merge by the last block of the head ---------------------------------------------------
-  // (m, l) of every split -> shared memory (the stage buffers are free now), then one pass per dim.
-  const int64_t p0 = static_cast<int64_t>(head) * prm.num_splits;
-  float* s_w = reinterpret_cast<float*>(smem);       // num_splits weights (fits: checked on the host)
-  float mloc = -INFINITY;
-  for (int s = tid; s < prm.num_splits; s += kDecThreads)
-    mloc = fmaxf(mloc, __ldcg(prm.partial_ml + (p0 + s) * 2));
+            for (int u = 0; u < 8; ++u) m_new = fmaxf(m_new, ml[u].x);
+            const float r = M == -INFINITY ? 0.f : exp2f(M - m_new);
+            L *= r;
+            acc.x *= r; acc.y *= r; acc.z *= r; acc.w *= r;
+            M = m_new;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mloc = fmaxf(mloc, __shfl_xor_sync(0xffffffffu, mloc, o));
-  if (lane == 0) s_red[warp] = mloc;
-  __syncthreads();
-  const float M = fmaxf(fmaxf(s_red[0], s_red[1]), fmaxf(s_red[2], s_red[3]));
-  float lloc = 0.f;
-  for (int s = tid; s < prm.num_splits; s += kDecThreads) {
-    const float2 ml = __ldcg(reinterpret_cast<const float2*>(prm.partial_ml + (p0 + s) * 2));
-    const float w = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M);
-    s_w[s] = w;
-    lloc += w * ml.y;
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) lloc += __shfl_xor_sync(0xffffffffu, lloc, o);
-  if (lane == 0) s_sum[warp] = lloc;
-  __syncthreads();
-  const float Lsum = (s_sum[0] + s_sum[1]) + (s_sum[2] + s_sum[3]);
-  float accd = 0.f;
-  const float* po = prm.partial_o + p0 * kHeadDim + tid;
-  int s = 0;
-  for (; s + 8 <= prm.num_splits; s += 8) {
-    float t[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) t[u] = __ldcg(po + static_cast<int64_t>(s + u) * kHeadDim);
-#pragma unroll
-    for (int u = 0; u < 8; ++u) accd = fmaf(s_w[s + u], t[u], accd);
-  }
-  for (; s < prm.num_splits; ++s) accd = fmaf(s_w[s], __ldcg(po + static_cast<int64_t>(s) * kHeadDim), accd);
-  const float r = Lsum > 0.f ? accd / Lsum : 0.f;
-  const float r1 = __shfl_down_sync(0xffffffffu, r, 1);
-  if (prm.o_f32) prm.o_f32[static_cast<int64_t>(head) * kHeadDim + tid] = r;
-  if (prm.o && (tid & 1) == 0) reinterpret_cast<uint32_t*>(op)[tid >> 1] = Elem<T>::from_f2(r, r1);
-  if (tid == 0) {
-    if (prm.lse) prm.lse[head] = Lsum > 0.f ? M + log2f(Lsum) : -INFINITY;
-    prm.counters[head] = 0;
+            for (int u = 0; u < 8; ++u) {
+              const float wt = ml[u].x == -INFINITY ? 0.f : exp2f(ml[u].x - M);
+              L += wt * ml[u].y;
+              acc.x = fmaf(wt, v[u].x, acc.x);
+              acc.y = fmaf(wt, v[u].y, acc.y);
+              acc.z = fmaf(wt, v[u].z, acc.z);
+              acc.w = fmaf(wt, v[u].w, acc.w);
+            }
+          }
+          finish(h, M, L, acc);
+        }
+      }
+    }
   }
 }
 

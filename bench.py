@@ -571,7 +571,7 @@ def run_ours(args):
         for stage in ("append", "estimate", "topk", "attention"):
             stage_us[stage] = stage_time(stage)
         kernels = {"append": "append_decode_kernel", "estimate": "estimate_kernel", "topk": "topk_cluster_kernel",
-                   "attention": "sparse_decode_kernel"}
+                   "attention": "paged_decode_kernel"}
         kbytes = lambda by: {"append": 0, "estimate": by["estimate"], "topk": by["topk"], "attention": by["attention"]}
     else:
         first = "append_estimate" if two_launch_step(args) else "estimate"

@@ -20,3 +20,56 @@ def test_rope_token_groups(seq, hq, hk):
     # the reference's tolerance for this operator (adamas/tests/test_rope.py:10-15)
     torch.testing.assert_close(qd.cpu().float(), ref.rope(q, 100, 8.0).float(), rtol=5e-3, atol=5e-3)
     torch.testing.assert_close(kd.cpu().float(), ref.rope(k, 100, 8.0).float(), rtol=5e-3, atol=5e-3)
+
+
+@pytest.mark.parametrize("hq,hkv,L,ps", [
+    (32, 32, 1, 16), (32, 32, 17, 16), (4, 4, 63, 1),     # single tile, tile remainders
+    (8, 8, 700, 7),                                       # blocks share a row evenly
+    (32, 32, 2500, 16),                                   # the line of tiles is cut over the grid
+    (32, 8, 9473, 16), (28, 4, 16001, 32),                # grouped queries in one part, line cut inside rows
+    (12, 1, 333, 16), (32, 2, 5000, 16), (9, 1, 20000, 1),   # groups of more than 8: several parts
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_dense_decode_shapes(hq, hkv, L, ps, dtype):
+    """Attention over every token (one page list for all heads) at the edges of the tiles and of the two ways
+    in which the work is cut, all query heads of a cache head together."""
+    _, K, _ = _mods()
+    pages = (L + ps - 1) // ps
+    perm = torch.randperm(pages, generator=torch.Generator().manual_seed(L))
+    kv = _randn((pages, 2, ps, hkv, 128), 7 + L, dtype)
+    q = _randn((1, hq, 128), 8 + L, dtype)
+    last = L - (pages - 1) * ps
+    w = K.BatchDecodeWithPagedKVCachePyTorchWrapper(0)
+    w.begin_forward(torch.tensor([0, pages], dtype=torch.int32), hq, hkv, 128, ps, torch.empty(0, dtype=dtype))
+    table = perm.to(torch.int32).to(DEV)
+    o, lse = torch.empty_like(q.to(DEV)), torch.zeros(hq, dtype=torch.float32, device=DEV)
+    for _ in range(2):      # (the counters are back at zero after a launch)
+        w.forward(q.to(DEV), o, kv.to(DEV), table[: pages - 1].unsqueeze(0).expand(hq, pages - 1), None, last, int(perm[-1]), lse=lse)
+    t = torch.arange(L)
+    k_all, v_all = (ref.repeat_kv(kv[perm[t // ps], i, t % ps], hq // hkv) for i in (0, 1))
+    want = ref.sparse_attention(q[0], k_all, v_all, np.tile(np.arange(L), (hq, 1)))
+    _assert_attn_close(o[0], want)
+    s = torch.einsum("hd,lhd->hl", q[0].float(), k_all.float()) / np.sqrt(128.0)
+    torch.testing.assert_close(lse.cpu(), torch.logsumexp(s, 1) / np.log(2.0), rtol=1e-4, atol=1e-3)
+
+
+def test_sparse_decode_list_with_holes():
+    """Negative list entries are skipped: whole tiles of them, single ones, and a list of nothing else."""
+    _, K, _ = _mods()
+    H, L, ps, n = 4, 900, 16, 130
+    pages = (L + ps - 1) // ps
+    kv = _randn((pages, 2, ps, H, 128), 3, torch.float16)
+    q = _randn((1, H, 128), 4, torch.float16)
+    idx = torch.stack([torch.randperm(L - 1, generator=torch.Generator().manual_seed(h))[:n] for h in range(H)]).to(torch.int32)
+    idx[0, 16:64] = -1
+    idx[1, ::3] = -1
+    idx[2, :] = -1
+    w = K.BatchDecodeWithPagedKVCachePyTorchWrapper(0)
+    w.begin_forward(torch.tensor([0, n], dtype=torch.int32), H, H, 128, ps, torch.empty(0, dtype=torch.float16))
+    o = torch.empty_like(q.to(DEV))
+    w.forward(q.to(DEV), o, kv.to(DEV), idx.to(DEV), None, (L - 1) % ps + 1, pages - 1, token_granular=True)
+    flat = kv.permute(0, 2, 1, 3, 4).reshape(pages * ps, 2, H, 128)
+    for h in range(H):
+        sel = np.append(idx[h][idx[h] >= 0].numpy(), L - 1)
+        want = ref.sparse_attention(q[0, h:h + 1], flat[:, 0, h:h + 1], flat[:, 1, h:h + 1], sel[None])
+        _assert_attn_close(o[0, h:h + 1], want)
