@@ -403,8 +403,8 @@ def set_estimate_blocks_per_sm(blocks: int) -> None:
 
 
 def set_fused_append(enable: bool) -> None:
-    """decode_step with the append folded into the estimate launch (two launches, the default for 16,
-    32 or 64 heads) or as three launches; the results are identical."""
+    """decode_step with the append folded into the estimate launch (two launches, the default) or as
+    three launches; the results are identical."""
     _lib.check(lib.adamas_set_fused_append(int(bool(enable))), "set_fused_append")
 
 
@@ -468,8 +468,8 @@ def decode_step(q, k, v, o, q_code, kv_data, kv_indices, kv_last_page_len, kv_la
                 hist: torch.Tensor, indices_out: Optional[torch.Tensor] = None,
                 lse: Optional[torch.Tensor] = None, scale: Optional[float] = None, thresholds=None,
                 rope=None) -> None:
-    """One layer's decode step in one call: append + estimate, select + attend (two launches for 16, 32
-    or 64 heads, else three, for what adamas/models/Adamas.py:145-200 does with seven).  Needs context > budget.  `hist`: a histogram_scratch(H), all zero between steps.  With
+    """One layer's decode step in one call: append + estimate, select + attend (two launches,
+    for what adamas/models/Adamas.py:145-200 does with seven).  Needs context > budget.  `hist`: a histogram_scratch(H), all zero between steps.  With
     rope=(rope_scale, rope_theta) or {"inv_freq": tensor[64], "mscale": float} q and k arrive un-rotated
     and are rotated in place first.  q, o may have a multiple of k's heads (grouped-query attention)."""
     _native.decode_step(q, k, v, o, q_code, kv_data, kv_indices, kv_last_page_len, kv_last_page_idx, hadamard_data,
@@ -613,7 +613,7 @@ def apply_rope_table_in_place(q: torch.Tensor, k: torch.Tensor, past_kv_len: int
 def append_estimate(q, k, v, q_code, kv_data, kv_indices, kv_last_page_len, hadamard_data, hadamard_indices,
                     hadamard_last_page_len, dist: torch.Tensor, scale: Optional[float] = None,
                     thresholds=None, hist: Optional[torch.Tensor] = None, hist_slices: int = 0) -> None:
-    """Decode append and distance estimate in one launch (16, 32 or 64 heads; q and k after RoPE): what
+    """Decode append and distance estimate in one launch (q and k after RoPE): what
     append_kv_cache_decode_fused followed by estimate_attn_score do, with integer (16-bit) distances
     in `dist` [H, >= context-1]."""
     num_heads, head_dim, page_size = _check_append(k, v, kv_data, kv_indices, hadamard_data, hadamard_indices, NHD)

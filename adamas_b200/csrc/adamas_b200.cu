@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "estimate.cuh"
+#include "estimate_items.cuh"
 #include "hadamard_append.cuh"
 #include "select_attend.cuh"
 #include "sparse_decode.cuh"
@@ -82,8 +83,7 @@ int check_q_heads(int num_heads, int num_q_heads) {
   return ADAMAS_OK;
 }
 
-constexpr int kEstAppendStatic = 1792;   // static shared memory of estimate_append_kernel (with the cos / sin table), rounded up
-constexpr int kEstPagesStatic = 8448;    // static shared memory of estimate_pages_kernel, rounded up
+constexpr int kEstStatic = 6144;   // static shared memory of the estimate kernels, rounded up
 constexpr int kSaMaxDynSmem = 160 * 1024;   // dynamic shared memory select_attend may ask for (a long winner list)
 
 constexpr int kDecSmem = kDecWarps * kDecStages * kDecTileBytes;
@@ -113,37 +113,31 @@ int get_device_info(const DeviceInfo** out) {
     d.topk_dyn_smem = d.max_smem_optin - static_cast<int>(sizeof(TopkShared)) - 1024;
     ADAMAS_CUDA(cudaFuncSetAttribute(topk_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.topk_dyn_smem));
     ADAMAS_CUDA(cudaFuncSetAttribute(topk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.topk_dyn_smem));
-    const int est_max = d.max_smem_optin - 1024;
-#define EST_ATTR(M, OT, HPW)                                                                       \
-  ADAMAS_CUDA(cudaFuncSetAttribute(estimate_kernel<M, OT, HPW>,                                    \
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, est_max))
-#define EST_ATTR_ALL(M, OT) \
-  EST_ATTR(M, OT, 0);       \
-  EST_ATTR(M, OT, 1);       \
-  EST_ATTR(M, OT, 2);       \
-  EST_ATTR(M, OT, 4)
-    EST_ATTR_ALL(0, __half);
-    EST_ATTR_ALL(0, uint16_t);
-    EST_ATTR_ALL(1, __half);
-    EST_ATTR_ALL(1, uint16_t);
-#undef EST_ATTR_ALL
+#define EST_ATTR(...)                                                                                                   \
+  ADAMAS_CUDA(cudaFuncSetAttribute((__VA_ARGS__), cudaFuncAttributeMaxDynamicSharedMemorySize, d.max_smem_optin - kEstStatic)); \
+  ADAMAS_CUDA(cudaFuncSetAttribute((__VA_ARGS__), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared))
+#define EST_ATTR_HPW(HPW)                                       \
+  EST_ATTR(estimate_kernel<0, __half, HPW>);                    \
+  EST_ATTR(estimate_kernel<0, uint16_t, HPW>);                  \
+  EST_ATTR(estimate_kernel<1, __half, HPW>);                    \
+  EST_ATTR(estimate_kernel<1, uint16_t, HPW>);                  \
+  EST_ATTR(estimate_append_kernel<__half, HPW, false>);         \
+  EST_ATTR(estimate_append_kernel<__half, HPW, true>);          \
+  EST_ATTR(estimate_append_kernel<__nv_bfloat16, HPW, false>);  \
+  EST_ATTR(estimate_append_kernel<__nv_bfloat16, HPW, true>)
+    EST_ATTR_HPW(1);
+    EST_ATTR_HPW(2);
+    EST_ATTR_HPW(4);
+#undef EST_ATTR_HPW
+#define EST_ATTR_HP(HP)                                \
+  EST_ATTR(estimate_items_kernel<__half, 0, HP>);      \
+  EST_ATTR(estimate_items_kernel<__half, 1, HP>);      \
+  EST_ATTR(estimate_items_kernel<__nv_bfloat16, 0, HP>)
+    EST_ATTR_HP(1);
+    EST_ATTR_HP(2);
+    EST_ATTR_HP(4);
+#undef EST_ATTR_HP
 #undef EST_ATTR
-#define ESTA_ATTR(T, HPW, R)                                                                           \
-  ADAMAS_CUDA(cudaFuncSetAttribute((estimate_append_kernel<T, HPW, R>),                                \
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, est_max - kEstAppendStatic)); \
-  ADAMAS_CUDA(cudaFuncSetAttribute((estimate_append_kernel<T, HPW, R>),                                \
-                                   cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared))
-#define ESTA_ATTR_ALL(T)    \
-  ESTA_ATTR(T, 1, false);   \
-  ESTA_ATTR(T, 2, false);   \
-  ESTA_ATTR(T, 4, false);   \
-  ESTA_ATTR(T, 1, true);    \
-  ESTA_ATTR(T, 2, true);    \
-  ESTA_ATTR(T, 4, true)
-    ESTA_ATTR_ALL(__half);
-    ESTA_ATTR_ALL(__nv_bfloat16);
-#undef ESTA_ATTR_ALL
-#undef ESTA_ATTR
     ADAMAS_CUDA(cudaFuncSetAttribute(paged_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem));
     ADAMAS_CUDA(cudaFuncSetAttribute(paged_decode_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem));
     // One shared-memory carve-out for every kernel of the decode step: a kernel that asks for a
@@ -156,14 +150,6 @@ int get_device_info(const DeviceInfo** out) {
     SET_CARVEOUT((append_decode_kernel<__nv_bfloat16, false, false>));
     SET_CARVEOUT((append_decode_kernel<__half, true, true>));
     SET_CARVEOUT((append_decode_kernel<__nv_bfloat16, true, true>));
-    SET_CARVEOUT((estimate_kernel<0, __half, 0>));
-    SET_CARVEOUT((estimate_kernel<0, __half, 1>));
-    SET_CARVEOUT((estimate_kernel<0, __half, 2>));
-    SET_CARVEOUT((estimate_kernel<0, __half, 4>));
-    SET_CARVEOUT((estimate_kernel<0, uint16_t, 0>));
-    SET_CARVEOUT((estimate_kernel<0, uint16_t, 1>));
-    SET_CARVEOUT((estimate_kernel<0, uint16_t, 2>));
-    SET_CARVEOUT((estimate_kernel<0, uint16_t, 4>));
     SET_CARVEOUT((topk_cluster_kernel<0, 1, 256>));
     SET_CARVEOUT((topk_cluster_kernel<0, 2, 256>));
     SET_CARVEOUT((topk_cluster_kernel<0, 4, 256>));
@@ -188,16 +174,6 @@ int get_device_info(const DeviceInfo** out) {
     SA_ATTR_ALL(__nv_bfloat16);
 #undef SA_ATTR_ALL
 #undef SA_ATTR
-#define ESTP_ATTR(M, OT)                                                                                      \
-  ADAMAS_CUDA(cudaFuncSetAttribute(estimate_pages_kernel<M, OT>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                   d.max_smem_optin - 1024 - kEstPagesStatic));                               \
-  ADAMAS_CUDA(cudaFuncSetAttribute(estimate_pages_kernel<M, OT>, cudaFuncAttributePreferredSharedMemoryCarveout, \
-                                   cudaSharedmemCarveoutMaxShared))
-    ESTP_ATTR(0, __half);
-    ESTP_ATTR(0, uint16_t);
-    ESTP_ATTR(1, __half);
-    ESTP_ATTR(1, uint16_t);
-#undef ESTP_ATTR
     d.ready = true;
   }
   *out = &d;
@@ -561,18 +537,21 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 }
 
 // ---------------------------------------------------------------------------------------------
-// n: distances per head (host mode), or their upper bound when seq_len_dev gives the length on the
-// device (the grid is then sized for n and each block derives its share from the device value).
-// num_heads: heads of the code cache; q_heads: rows of q_code / out / hist (a multiple of num_heads).
-static int estimate_impl(const void* q_code, const void* code_data, const int32_t* code_page_table, int n,
-                         int page_size, int num_heads, int q_heads, void* out, int64_t out_stride, int out_format,
-                         int metric, const int32_t* seq_len_dev, uint32_t* hist, int hist_cl, adamas_stream_t stream,
-                         const SeqDesc* seqs = nullptr, int batch = 1) {
+static bool estimate_by_tiles(int num_heads, int q_heads) {
+  return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64);
+}
+
+// Launches the estimate.  n: distances per row, or their upper bound when seq_len_dev gives the length on the device
+// (it sizes the grid; each block derives its share from the device value).  num_heads: heads of the code cache; q_heads:
+// query rows per sequence (a multiple of num_heads).  ap.q set: with the append inside (dtype of q, k, v); else q_code is given.
+static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, const void* code_data,
+                           const int32_t* code_page_table, int n, int page_size, int num_heads, int q_heads, void* out,
+                           int64_t out_stride, int out_format, int metric, const int32_t* seq_len_dev, uint32_t* hist,
+                           int hist_cl, adamas_stream_t stream, const SeqDesc* seqs, int batch) {
   if (int rc = check_q_heads(num_heads, q_heads)) return rc;
   if (!seqs) batch = 1;
-  const int q_group = q_heads / num_heads;
-  ADAMAS_REQUIRE(q_code && out && (seqs || (code_data && code_page_table)), "null pointer");
-  ADAMAS_REQUIRE(!seqs || seq_len_dev, "a batched estimate needs device lengths");
+  ADAMAS_REQUIRE((q_code || ap.q) && out && (seqs || (code_data && code_page_table)), "null pointer");
+  ADAMAS_REQUIRE(!seqs || (seq_len_dev && batch <= kEstMaxBatch), "a batched estimate needs device lengths");
   ADAMAS_REQUIRE(out_stride >= n, "out_stride (%lld) smaller than the row length (%d)",
                  static_cast<long long>(out_stride), n);
   ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(q_code) & 15) == 0 &&
@@ -581,101 +560,86 @@ static int estimate_impl(const void* q_code, const void* code_data, const int32_
   ADAMAS_REQUIRE(!hist || (hist_cl >= 1 && hist_cl <= kSaMaxSlices), "histogram slices out of range (%d)", hist_cl);
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
-  cudaStream_t st = to_stream(stream);
-  // (8 and 16 heads with histograms go token by token: in the page-copy kernel the 16 lanes of a count
-  // instruction hit the tables of different heads, one L2 transaction each, where a warp of the token-copy
-  // kernel counts 32 tokens of ONE head into a few neighbouring bins.  Measured at 32K with the counts: 16
-  // heads 13.9 us by pages, 6.0 by tokens; 8 heads 7.9 / 6.6; 4 heads 4.7 / 7.7)
-  constexpr int kPagesMaxHeadsWithHist = 4;
-  if (q_group == 1 && num_heads <= 16 && !(hist && num_heads > kPagesMaxHeadsWithHist) && 32 % (2 * num_heads) == 0 &&
-      page_size * num_heads * 32 >= 512) {
-    // few heads (a head-sharded model): whole pages per copy, one chunk per lane
-    const int page_bytes = page_size * num_heads * 32;
-    const int ppt = std::max(1, std::min(32, 32768 / page_bytes));
-    const int pages = (n + page_size - 1) / page_size;
-    const int num_tiles = (pages + ppt - 1) / ppt;
-    // spare bytes: a partial last unit reads up to 8 tokens past the valid ones
-    const size_t smem = static_cast<size_t>(kEstStages) * ppt * page_bytes + 4096 + 512;
-    ADAMAS_REQUIRE(smem <= static_cast<size_t>(di->max_smem_optin - 1024 - kEstPagesStatic),
-                   "page too large for the estimate kernel");
-    const int per_sm = std::min(est_blocks_per_sm(),
-                                (smem + 1024 + kEstPagesStatic) * 2 <= static_cast<size_t>(di->max_smem_optin) ? 2 : 1);
-    const unsigned blocks = static_cast<unsigned>(std::min(num_tiles, std::max(1, di->num_sms * per_sm / batch)));
-    EstimatePagesParams pp;
-    pp.codes = static_cast<const uint4*>(code_data);
-    pp.page_table = code_page_table;
-    pp.q_code = static_cast<const uint4*>(q_code);
-    pp.out = out;
-    pp.out_stride = out_stride;
-    pp.n_tokens = n;
-    pp.H = num_heads;
-    pp.page_size = page_size;
-    pp.pages_per_tile = ppt;
-    pp.num_tiles = num_tiles;
-    pp.stage_out = num_heads >= 16 ? 1 : 0;
-    pp.seq_len_dev = seq_len_dev;
-    pp.hist = hist;
-    pp.hist_cl = hist_cl;
-    pp.seqs = seqs;
-#define LAUNCH_ESTP(M, OT) \
-  ADAMAS_LAUNCH("estimate_pages_kernel", (estimate_pages_kernel<M, OT>), dim3(blocks, batch), dim3(kEstPagesThreads), smem, st, 1, pp)
-    if (metric == ADAMAS_METRIC_L1) {
-      if (out_format == ADAMAS_VAL_F16) LAUNCH_ESTP(0, __half); else LAUNCH_ESTP(0, uint16_t);
-    } else {
-      if (out_format == ADAMAS_VAL_F16) LAUNCH_ESTP(1, __half); else LAUNCH_ESTP(1, uint16_t);
-    }
-#undef LAUNCH_ESTP
-    return check_launch("estimate_pages_kernel");
-  }
-  const int hpw = (num_heads % kEstConsumerWarps == 0) ? num_heads / kEstConsumerWarps : 0;
-  const bool in_regs = q_group == 1 && (hpw == 1 || hpw == 2 || hpw == 4);   // grouped queries: the generic kernel
-  // fewer than 16 heads: a tile holds 32 / H groups of 32 tokens, so that all 16 consumer warps work,
-  // each on one head of two token groups
-  const int groups = (q_group == 1 && num_heads < kEstConsumerWarps && kEstConsumerWarps % num_heads == 0)
-                         ? 2 * kEstConsumerWarps / num_heads : 1;
-  const int tile_span = kEstTile * groups;
-  const int num_tiles = (n + tile_span - 1) / tile_span;
-  const size_t smem = static_cast<size_t>(kEstStages) * tile_span * (2 * num_heads + 1) * 16 +
-                      (in_regs ? 0 : static_cast<size_t>(2 * q_heads) * sizeof(QPlanes));
-  ADAMAS_REQUIRE(smem <= static_cast<size_t>(di->max_smem_optin - 1024),
-                 "num_heads (%d) too large for the estimate kernel", num_heads);
-  const int per_sm = std::min(est_blocks_per_sm(), (smem + 1024) * 2 <= static_cast<size_t>(di->max_smem_optin) ? 2 : 1);
-  const unsigned blocks = static_cast<unsigned>(std::min(num_tiles, std::max(1, di->num_sms * per_sm / batch)));
+  const size_t most = static_cast<size_t>(di->max_smem_optin - kEstStatic);
   EstimateParams prm;
-  prm.seqs = seqs;
   prm.codes = static_cast<const uint4*>(code_data);
   prm.page_table = code_page_table;
   prm.q_code = static_cast<const uint4*>(q_code);
   prm.out = out;
   prm.out_stride = out_stride;
+  prm.out_half = out_format == ADAMAS_VAL_F16 ? 1 : 0;
   prm.n_tokens = n;
   prm.H = num_heads;
-  prm.q_group = q_group;
+  prm.q_group = q_heads / num_heads;
   prm.page_size = page_size;
   prm.ps_shift = log2_exact(page_size);
-  prm.groups = groups;
-  prm.num_tiles = num_tiles;
+  prm.batch = batch;
   prm.seq_len_dev = seq_len_dev;
   prm.hist = hist;
   prm.hist_cl = hist_cl;
-#define LAUNCH_EST(M, OT)                                                                      \
-  do {                                                                                         \
-    if (in_regs && hpw == 1)                                                                   \
-      ADAMAS_LAUNCH("estimate_kernel", estimate_kernel<M, OT, 1>, dim3(blocks, batch), dim3(kEstThreads), smem, st, 1, prm);                       \
-    else if (in_regs && hpw == 2)                                                              \
-      ADAMAS_LAUNCH("estimate_kernel", estimate_kernel<M, OT, 2>, dim3(blocks, batch), dim3(kEstThreads), smem, st, 1, prm);                       \
-    else if (in_regs && hpw == 4)                                                              \
-      ADAMAS_LAUNCH("estimate_kernel", estimate_kernel<M, OT, 4>, dim3(blocks, batch), dim3(kEstThreads), smem, st, 1, prm);                       \
-    else                                                                                       \
-      ADAMAS_LAUNCH("estimate_kernel", estimate_kernel<M, OT, 0>, dim3(blocks, batch), dim3(kEstThreads), smem, st, 1, prm);                       \
+  prm.count_local = 0;
+  prm.seqs = seqs;
+  prm.ap = ap;
+  cudaStream_t st = to_stream(stream);
+  if (estimate_by_tiles(num_heads, q_heads)) {
+    const int num_tiles = (n + kEstTile - 1) / kEstTile;
+    const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
+    ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
+    const int per_sm = std::min(est_blocks_per_sm(), (smem + 1024 + 2048) * 2 <= static_cast<size_t>(di->max_smem_optin) ? 2 : 1);
+    const dim3 grid(static_cast<unsigned>(std::min(num_tiles, std::max(1, di->num_sms * per_sm / batch))), batch);
+#define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_kernel", (__VA_ARGS__), grid, dim3(kEstThreads), smem, st, 1, prm)
+#define LAUNCH_EST_HPW(HPW)                                                                     \
+  do {                                                                                          \
+    if (ap.q) {                                                                                 \
+      if (dtype == ADAMAS_F16) {                                                                \
+        if (ap.rope_on) LAUNCH_EST(estimate_append_kernel<__half, HPW, true>);                  \
+        else LAUNCH_EST(estimate_append_kernel<__half, HPW, false>);                            \
+      } else {                                                                                  \
+        if (ap.rope_on) LAUNCH_EST(estimate_append_kernel<__nv_bfloat16, HPW, true>);           \
+        else LAUNCH_EST(estimate_append_kernel<__nv_bfloat16, HPW, false>);                     \
+      }                                                                                         \
+    } else if (metric == ADAMAS_METRIC_L1) {                                                    \
+      if (prm.out_half) LAUNCH_EST(estimate_kernel<0, __half, HPW>);                            \
+      else LAUNCH_EST(estimate_kernel<0, uint16_t, HPW>);                                       \
+    } else {                                                                                    \
+      if (prm.out_half) LAUNCH_EST(estimate_kernel<1, __half, HPW>);                            \
+      else LAUNCH_EST(estimate_kernel<1, uint16_t, HPW>);                                       \
+    }                                                                                           \
   } while (0)
-  if (metric == ADAMAS_METRIC_L1) {
-    if (out_format == ADAMAS_VAL_F16) LAUNCH_EST(0, __half); else LAUNCH_EST(0, uint16_t);
-  } else {
-    if (out_format == ADAMAS_VAL_F16) LAUNCH_EST(1, __half); else LAUNCH_EST(1, uint16_t);
-  }
+    if (num_heads == 16) LAUNCH_EST_HPW(1);
+    else if (num_heads == 32) LAUNCH_EST_HPW(2);
+    else LAUNCH_EST_HPW(4);
+#undef LAUNCH_EST_HPW
 #undef LAUNCH_EST
-  return check_launch("estimate_kernel");
+    return check_launch("estimate_kernel");
+  }
+  const int hp = num_heads % 4 == 0 ? 4 : num_heads % 2 == 0 ? 2 : 1;   // heads per item: as long a run of a token's codes as divides
+  const int64_t items = static_cast<int64_t>((n + 128 / hp - 1) / (128 / hp)) * (num_heads / hp) * batch;
+  ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
+  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(di->num_sms, items)));
+  const size_t slot = static_cast<size_t>(kItemWarps) * kItemBytes, counts = static_cast<size_t>(q_heads) * kItemCountWords * sizeof(uint32_t);
+  // The counts in shared memory where they fit beside two ring slots per warp and where there are enough distances to be
+  // worth clearing and adding up a table per block (12K tokens x 40 heads: 6.4 us with an L2 atomic each, 7.5 with tables;
+  // 30K x 32: 8.8 / 8.7; 64K x 64: 26.9 / 21.1); a third slot where it fits beside them.
+  size_t smem = static_cast<size_t>(q_heads) * 2 * sizeof(QPlanes);
+  prm.count_local = hist && static_cast<int64_t>(q_heads) * n * batch >= (int64_t(1) << 20) && smem + 2 * slot + counts <= most ? 1 : 0;
+  if (prm.count_local) smem += counts;
+  const int slots = smem + 3 * slot <= most ? 3 : 2;
+  smem += slots * slot;
+  ADAMAS_REQUIRE(smem <= most, "num_q_heads (%d) too large for the estimate kernel", q_heads);
+#define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_items_kernel", (__VA_ARGS__), grid, dim3(kItemThreads), smem, st, 1, prm, slots)
+#define LAUNCH_EST_HP(HP)                                                                                 \
+  do {                                                                                                    \
+    if (metric != ADAMAS_METRIC_L1) LAUNCH_EST(estimate_items_kernel<__half, 1, HP>);   /* (no append) */ \
+    else if (dtype == ADAMAS_F16) LAUNCH_EST(estimate_items_kernel<__half, 0, HP>);                       \
+    else LAUNCH_EST(estimate_items_kernel<__nv_bfloat16, 0, HP>);                                         \
+  } while (0)
+  if (hp == 4) LAUNCH_EST_HP(4);
+  else if (hp == 2) LAUNCH_EST_HP(2);
+  else LAUNCH_EST_HP(1);
+#undef LAUNCH_EST_HP
+#undef LAUNCH_EST
+  return check_launch("estimate_items_kernel");
 }
 
 int adamas_estimate(const void* q_code, const void* code_data, const int32_t* code_page_table,
@@ -692,10 +656,11 @@ int adamas_estimate(const void* q_code, const void* code_data, const int32_t* co
   ADAMAS_REQUIRE(exclude_last == 0 || exclude_last == 1, "exclude_last must be 0 or 1");
   const int64_t n64 =
       static_cast<int64_t>(code_num_pages - 1) * page_size + code_last_page_len - exclude_last;
-  ADAMAS_REQUIRE(n64 < (int64_t(1) << 31) - kEstTile * kEstConsumerWarps * 2, "sequence too long");
+  ADAMAS_REQUIRE(n64 < (int64_t(1) << 31) - 1024, "sequence too long");
   if (n64 == 0) return ADAMAS_OK;
-  return estimate_impl(q_code, code_data, code_page_table, static_cast<int>(n64), page_size, num_heads, num_q_heads,
-                       out, out_stride, out_format, metric, nullptr, hist, hist_slices, stream);
+  return launch_estimate(q_code, StepAppend{}, ADAMAS_F16, code_data, code_page_table, static_cast<int>(n64), page_size,
+                         num_heads, num_q_heads, out, out_stride, out_format, metric, nullptr, hist, hist_slices, stream,
+                         nullptr, 1);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1362,52 +1327,20 @@ int adamas_seq_len_advance(int32_t* seq_len_dev, int count, int delta, adamas_st
   return check_launch("seq_len_advance_kernel");
 }
 
-// Stages 1 + 2 of a decode step in one launch (estimate_append_kernel); the caller has checked that
-// num_heads is 16, 32 or 64.  n: distances per head (host mode) or their upper bound (seq_len_dev).
-static int estimate_append_launch(const void* q, const void* k, const void* v, void* q_code, void* kv_data,
+// Stages 1 + 2 of a decode step in one launch.  n: distances per row (host mode) or their upper bound (seq_len_dev).
+static int estimate_append_launch(const void* q, void* k, const void* v, void* q_code, void* kv_data,
                                   const int32_t* kv_page_table, int kv_num_pages, int kv_last_page_len,
                                   void* code_data, const int32_t* code_page_table, int code_num_pages,
-                                  int code_last_page_len, int n, int num_heads, int page_size, int dtype, void* dist,
+                                  int code_last_page_len, int n, int num_heads, int q_heads, int page_size, int dtype, void* dist,
                                   int64_t dist_stride, float hadamard_scale, const float* thresholds3_host,
                                   const int32_t* seq_len_dev, uint32_t* hist, int hist_cl, adamas_stream_t stream,
                                   const SeqDesc* seqs = nullptr, int batch = 1, const RopeSpec& rope = RopeSpec()) {
   ADAMAS_REQUIRE(q && k && v && q_code && dist && (seqs || (kv_data && code_data && kv_page_table && code_page_table)),
                  "null pointer");
-  if (!seqs) batch = 1;
-  ADAMAS_REQUIRE(n >= 1 && n < 2147483647 - kEstTile, "sequence length out of range");
-  ADAMAS_REQUIRE(dist_stride >= n, "dist_stride (%lld) smaller than the row length (%d)",
-                 static_cast<long long>(dist_stride), n);
-  ADAMAS_REQUIRE((seqs || (reinterpret_cast<uintptr_t>(code_data) & 15) == 0) && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
-                     (reinterpret_cast<uintptr_t>(k) & 15) == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0,
-                 "q, k, v and code_data must be 16-byte aligned");
-  ADAMAS_REQUIRE(!hist || (hist_cl >= 1 && hist_cl <= kSaMaxSlices), "histogram slices out of range (%d)", hist_cl);
-  const DeviceInfo* di = nullptr;
-  if (int rc = get_device_info(&di)) return rc;
-  const int num_tiles = (n + kEstTile - 1) / kEstTile;
-  const int hpw = num_heads / kEstConsumerWarps;
-  const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
-  ADAMAS_REQUIRE(smem <= static_cast<size_t>(di->max_smem_optin - 1024 - kEstAppendStatic),
-                 "num_heads (%d) too large", num_heads);
-  const int per_sm = std::min(est_blocks_per_sm(),
-                              (smem + 1024 + kEstAppendStatic) * 2 <= static_cast<size_t>(di->max_smem_optin) ? 2 : 1);
-  const unsigned blocks = static_cast<unsigned>(std::min(num_tiles, std::max(1, di->num_sms * per_sm / batch)));
-  EstimateParams prm;
-  prm.seqs = seqs;
-  prm.codes = static_cast<const uint4*>(code_data);
-  prm.page_table = code_page_table;
-  prm.q_code = nullptr;
-  prm.out = dist;
-  prm.out_stride = dist_stride;
-  prm.n_tokens = n;
-  prm.H = num_heads;
-  prm.q_group = 1;
-  prm.page_size = page_size;
-  prm.ps_shift = log2_exact(page_size);
-  prm.groups = 1;
-  prm.num_tiles = num_tiles;
-  prm.seq_len_dev = seq_len_dev;
-  prm.hist = hist;
-  prm.hist_cl = hist_cl;
+  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(q) & 15) == 0 && (reinterpret_cast<uintptr_t>(k) & 15) == 0 &&
+                     (reinterpret_cast<uintptr_t>(v) & 15) == 0, "q, k and v must be 16-byte aligned");
+  ADAMAS_REQUIRE(!rope.on || rope.inv_freq || (rope.scale > 0.f && rope.theta > 0.f),
+                 "rope_scale and rope_theta must be positive");
   StepAppend ap;
   ap.q = q;
   ap.k = k;
@@ -1421,27 +1354,10 @@ static int estimate_append_launch(const void* q, const void* k, const void* v, v
   ap.code_entry = code_last_page_len - 1;
   ap.scale = hadamard_scale;
   ap.th = make_thresholds(thresholds3_host);
+  ap.rope_on = rope.on ? 1 : 0;
   ap.rp = RopeParams{rope.scale > 0.f ? 1.0f / rope.scale : 1.f, rope.theta, rope.inv_freq, rope.mscale};
-  cudaStream_t st = to_stream(stream);
-#define LAUNCH_ESTA(T, HPW, R)                                                                        \
-  ADAMAS_LAUNCH("estimate_append_kernel", (estimate_append_kernel<T, HPW, R>), dim3(blocks, batch),   \
-                dim3(kEstThreads), smem, st, 1, prm, ap)
-#define LAUNCH_ESTA_T(T)                                                        \
-  do {                                                                          \
-    if (rope.on) {                                                              \
-      if (hpw == 1) LAUNCH_ESTA(T, 1, true);                                    \
-      else if (hpw == 2) LAUNCH_ESTA(T, 2, true);                               \
-      else LAUNCH_ESTA(T, 4, true);                                             \
-    } else {                                                                    \
-      if (hpw == 1) LAUNCH_ESTA(T, 1, false);                                   \
-      else if (hpw == 2) LAUNCH_ESTA(T, 2, false);                              \
-      else LAUNCH_ESTA(T, 4, false);                                            \
-    }                                                                           \
-  } while (0)
-  if (dtype == ADAMAS_F16) LAUNCH_ESTA_T(__half); else LAUNCH_ESTA_T(__nv_bfloat16);
-#undef LAUNCH_ESTA_T
-#undef LAUNCH_ESTA
-  return check_launch("estimate_append_kernel");
+  return launch_estimate(nullptr, ap, dtype, code_data, code_page_table, n, page_size, num_heads, q_heads, dist, dist_stride,
+                         ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, hist, hist_cl, stream, seqs, batch);
 }
 
 int adamas_append_estimate(const void* q, const void* k, const void* v, void* q_code, void* kv_data,
@@ -1452,18 +1368,15 @@ int adamas_append_estimate(const void* q, const void* k, const void* v, void* q_
                            const float* thresholds3_host, uint32_t* hist, int hist_slices,
                            adamas_stream_t stream) {
   if (int rc = check_common(num_heads, head_dim, page_size, dtype)) return rc;
-  ADAMAS_REQUIRE(num_heads == 16 || num_heads == 32 || num_heads == 64,
-                 "adamas_append_estimate supports 16, 32 or 64 heads (got %d); use adamas_append_decode_fused "
-                 "and adamas_estimate", num_heads);
   ADAMAS_REQUIRE(kv_num_pages >= 1 && code_num_pages >= 1, "page tables must not be empty");
   ADAMAS_REQUIRE(kv_last_page_len >= 1 && kv_last_page_len <= page_size, "kv_last_page_len out of range");
   ADAMAS_REQUIRE(code_last_page_len >= 1 && code_last_page_len <= page_size,
                  "code_last_page_len out of range");
   const int64_t n64 = static_cast<int64_t>(code_num_pages - 1) * page_size + code_last_page_len - 1;
-  ADAMAS_REQUIRE(n64 >= 1 && n64 < (int64_t(1) << 31) - kEstTile, "sequence length out of range");
-  return estimate_append_launch(q, k, v, q_code, kv_data, kv_page_table, kv_num_pages, kv_last_page_len,
+  ADAMAS_REQUIRE(n64 >= 1 && n64 < (int64_t(1) << 31) - 1024, "sequence length out of range");
+  return estimate_append_launch(q, const_cast<void*>(k), v, q_code, kv_data, kv_page_table, kv_num_pages, kv_last_page_len,
                                 code_data, code_page_table, code_num_pages, code_last_page_len,
-                                static_cast<int>(n64), num_heads, page_size, dtype, dist, dist_stride,
+                                static_cast<int>(n64), num_heads, num_heads, page_size, dtype, dist, dist_stride,
                                 hadamard_scale, thresholds3_host, nullptr, hist, hist_slices, stream);
 }
 
@@ -1487,7 +1400,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
                  "a decode step needs budget >= 2 and a context longer than the budget (%lld vs %d); "
                  "shorter contexts attend to every page through adamas_decode_forward",
                  static_cast<long long>(seq_len), budget);
-  ADAMAS_REQUIRE(seq_len - 1 < (int64_t(1) << 31) - kEstTile * kEstConsumerWarps * 2, "sequence too long");
+  ADAMAS_REQUIRE(seq_len - 1 < (int64_t(1) << 31) - 1024, "sequence too long");
   ADAMAS_REQUIRE(q && o && dist_scratch && q_code && hist, "null pointer");
   ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(dist_scratch) & 15) == 0 && (dist_stride * 2) % 16 == 0,
                  "distance rows must start on 16-byte boundaries");
@@ -1500,18 +1413,16 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   SaPlan pl;
   if (int rc = sa_plan(n, budget - 1, q_heads * batch, di, &pl)) return rc;
   int rc;
-  // The histogram counts: one L2 atomic per distance from inside the estimate, or, for launches with 3 M
-  // distances and more (a 128K context of 32 heads, three 32K sequences), a launch of their own that
-  // counts in shared memory (measured: the estimate of one 128K sequence 31.7 us with the counts, 23.7
-  // without).  Few heads per GPU keep the counts inside (the extra launch costs more than it saves).
-  const bool count_apart = static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20) && q_heads >= 16;
+  // The histogram counts.  Tile pipeline: one L2 atomic per distance from inside the estimate, or, for launches with 3 M
+  // distances and more (a 128K context of 32 heads, three 32K sequences), a launch of their own that counts in shared
+  // memory (measured: the estimate of one 128K sequence 31.7 us with the counts, 23.7 without).
+  const bool count_apart = estimate_by_tiles(num_heads, q_heads) && static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20);
   uint32_t* est_hist = count_apart ? nullptr : hist;
-  const bool two_launches = fused_append_enabled() && q_heads == num_heads &&
-                            (num_heads == 16 || num_heads == 32 || num_heads == 64);
+  const bool two_launches = fused_append_enabled();
   if (two_launches) {
     // two launches: the estimate with the append (and, with RoPE, the rotation) inside, then select + attend
     rc = estimate_append_launch(q, k, v, q_code, kv_data, kv_page_table, pages, last_len, code_data,
-                                code_page_table, pages, last_len, n, num_heads, page_size, dtype, dist_scratch,
+                                code_page_table, pages, last_len, n, num_heads, q_heads, page_size, dtype, dist_scratch,
                                 dist_stride, hadamard_scale, thresholds3_host, seq_len_dev, est_hist, pl.cl, stream, seqs,
                                 batch, rope);
     if (rc) return rc;
@@ -1520,8 +1431,8 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
                             code_page_table, pages, last_len, num_heads, head_dim, page_size, hadamard_scale,
                             thresholds3_host, dtype, stream, rope, seq_len_dev, q_heads, seqs, batch);
     if (rc) return rc;
-    rc = estimate_impl(q_code, code_data, code_page_table, n, page_size, num_heads, q_heads, dist_scratch,
-                       dist_stride, ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, est_hist, pl.cl, stream, seqs, batch);
+    rc = launch_estimate(q_code, StepAppend{}, dtype, code_data, code_page_table, n, page_size, num_heads, q_heads, dist_scratch,
+                         dist_stride, ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, est_hist, pl.cl, stream, seqs, batch);
     if (rc) return rc;
   }
   if (count_apart) {

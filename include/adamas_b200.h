@@ -85,11 +85,10 @@ int adamas_device_error(unsigned* flags, int clear);
  * reference launches everything on the legacy default stream (e.g. adamas/ops/csrc/page.cu:99). */
 int adamas_set_pdl(int enable);
 
-/* Chooses how the decode-step entry points launch a step of 16, 32 or 64 heads (multi-head attention):
+/* Chooses how the decode-step entry points launch a step:
  * with the append, and the rotary embedding if one is asked for, folded into the estimate launch (two
  * launches; the default) or as three launches (append, estimate, select+attend;
- * ADAMAS_FUSED_APPEND=0 in the environment selects it).  Other head counts and grouped queries always
- * take three.  Results are identical.  No counterpart in the reference. */
+ * ADAMAS_FUSED_APPEND=0 in the environment selects it).  Results are identical.  No counterpart in the reference. */
 int adamas_set_fused_append(int enable);
 
 /* How many blocks of the estimate kernel may be resident per SM: 2 (default; fastest for one sequence)
@@ -342,7 +341,7 @@ int adamas_hist_rowsum(const uint32_t* hist, int num_heads, int slices, uint32_t
 int adamas_global_cut(const uint32_t* all_hists, int num_shards, int shard, int num_heads, int k, int32_t* ext_cut,
                       adamas_stream_t stream);
 
-/* Stages 1 and 2 of a decode step in one launch, for 16, 32 or 64 heads: the append of
+/* Stages 1 and 2 of a decode step in one launch: the append of
  * adamas_append_decode_fused (new token's K, V and code into the caches, query code to q_code; q and k
  * already rotated) and the estimate of adamas_estimate with ADAMAS_VAL_U16 output, the L1 metric and
  * exclude_last = 1 (dist [H, dist_stride], rows on 16-byte boundaries, dist_stride >= context - 1).
@@ -425,7 +424,7 @@ int adamas_seq_len_advance(int32_t* seq_len_dev, int count, int delta, adamas_st
 /* ---- several sequences in one launch ------------------------------------------------------------
  * The reference decodes one sequence per call (adamas/models/Adamas.py:83 asserts batch size 1, and an
  * InferenceController holds one sequence); a server loops over its sequences.
- * Here `batch` sequences of one cache geometry go through the SAME two or three launches of a step:
+ * Here `batch` sequences of one cache geometry go through the SAME launches of a step:
  * every kernel's grid gets a sequence coordinate.  Each sequence keeps its own caches and page
  * tables, described by one adamas_seq_desc_t in a device array; everything else is one contiguous
  * array over (sequence, head) rows: q, o [batch, Hq, D]; k, v [batch, H, D]; q_code [batch, Hq, D/8];

@@ -73,3 +73,42 @@ def test_sparse_decode_list_with_holes():
         sel = np.append(idx[h][idx[h] >= 0].numpy(), L - 1)
         want = ref.sparse_attention(q[0, h:h + 1], flat[:, 0, h:h + 1], flat[:, 1, h:h + 1], sel[None])
         _assert_attn_close(o[0, h:h + 1], want)
+
+
+@pytest.mark.parametrize("H,Hq", [(1, 1), (2, 2), (3, 9), (4, 4), (5, 5), (8, 64), (12, 12), (28, 28), (40, 40), (6, 48), (96, 96)])
+@pytest.mark.parametrize("L,ps", [(2, 16), (33, 1), (130, 16), (257, 7), (5000, 32), (40001, 16)])
+def test_estimate_items_shapes(H, Hq, L, ps):
+    """The estimate for any head count: remainders of its items, one item, several per warp, and (from 1 M distances
+    on) the counts in shared memory; distances and per-slice counts exact, grouped queries included."""
+    _, K, _ = _mods()
+    if Hq * L > 1 << 22:
+        pytest.skip("larger than the range this is about")
+    g = torch.Generator().manual_seed(L + H)
+    pages = (L + ps - 1) // ps
+    perm = torch.randperm(pages, generator=g)
+    codes = torch.randint(-32768, 32768, (pages, 1, ps, H, 16), generator=g, dtype=torch.int32).to(torch.int16)
+    q = torch.randint(-32768, 32768, (1, Hq, 16), generator=g, dtype=torch.int32).to(torch.int16)
+    n = L - 1
+    slices = 5
+    store = torch.zeros(Hq, (n + 7) // 8 * 8, dtype=torch.int16, device=DEV)
+    hist = K.histogram_scratch(Hq, DEV)
+    K.estimate_attn_score(q.to(DEV), store[:, :n], codes.to(DEV), perm.to(torch.int32).to(DEV), None, L - (pages - 1) * ps, 0, 0,
+                          hist=hist, hist_slices=slices)
+    t = torch.arange(n)
+    kc = codes[perm[t // ps], 0, t % ps]                                  # [n, H, 16]
+    want = torch.empty(Hq, n, dtype=torch.int64)
+    def bits(x):
+        x = x.to(torch.int32) & 0xffff
+        return torch.stack([(x >> (2 * i)) & 3 for i in range(8)], -1).flatten(-2).to(torch.int8)
+    qb, group = bits(q[0]), Hq // H
+    for h in range(H):
+        kb = bits(kc[:, h])
+        for r in range(h * group, (h + 1) * group):
+            want[r] = (kb - qb[r]).abs().sum(1, dtype=torch.int64)
+    got = store[:, :n].cpu().to(torch.int64)
+    assert torch.equal(got, want)
+    per = ((((n + 7) // 8 + slices - 1) // slices + 3) // 4 * 4) * 8      # tokens per slice
+    counts = K.histogram_counts(hist).cpu()
+    for r in (0, Hq // 2, Hq - 1):
+        for sl in range(slices):
+            assert torch.equal(counts[r, sl].to(torch.int64), torch.bincount(want[r, sl * per:(sl + 1) * per], minlength=512))
