@@ -160,19 +160,13 @@ int get_device_info(const DeviceInfo** out) {
     SET_CARVEOUT((paged_decode_kernel<__nv_bfloat16>));
 #undef SET_CARVEOUT
     // select+attend: large dynamic shared memory
-#define SA_ATTR(T, I)                                                                                          \
-  ADAMAS_CUDA(cudaFuncSetAttribute(select_attend_kernel<T, I>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
+#define SA_ATTR(T)                                                                                             \
+  ADAMAS_CUDA(cudaFuncSetAttribute(select_attend_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
                                    kSaMaxDynSmem));                                                            \
-  ADAMAS_CUDA(cudaFuncSetAttribute(select_attend_kernel<T, I>, cudaFuncAttributePreferredSharedMemoryCarveout, \
+  ADAMAS_CUDA(cudaFuncSetAttribute(select_attend_kernel<T>, cudaFuncAttributePreferredSharedMemoryCarveout,    \
                                    cudaSharedmemCarveoutMaxShared))
-#define SA_ATTR_ALL(T) \
-  SA_ATTR(T, 1);       \
-  SA_ATTR(T, 2);       \
-  SA_ATTR(T, 4);       \
-  SA_ATTR(T, 8)
-    SA_ATTR_ALL(__half);
-    SA_ATTR_ALL(__nv_bfloat16);
-#undef SA_ATTR_ALL
+    SA_ATTR(__half);
+    SA_ATTR(__nv_bfloat16);
 #undef SA_ATTR
     d.ready = true;
   }
@@ -204,11 +198,12 @@ bool fused_append_enabled() { return setting(g_fused_append, "ADAMAS_FUSED_APPEN
 // ADAMAS_EST_BLOCKS_PER_SM): 2 by default, 1 leaves half of every SM to kernels of other streams.
 std::atomic<int> g_est_blocks_per_sm{-1};
 int est_blocks_per_sm() { return setting(g_est_blocks_per_sm, "ADAMAS_EST_BLOCKS_PER_SM", 2, 1, 2); }
-// Upper bound on the cluster size of select_attend (adamas_set_max_cluster / ADAMAS_MAX_CLUSTER).
+// Upper bound on the blocks per head of select_attend (adamas_set_max_cluster / ADAMAS_MAX_CLUSTER); while neither has
+// been given, what the histogram table has room for.
 std::atomic<int> g_max_cluster{-1};
 int max_cluster() {
-  const int v = setting(g_max_cluster, "ADAMAS_MAX_CLUSTER", kSaMaxCluster, 1, kSaMaxCluster);
-  return (v & (v - 1)) == 0 ? v : kSaMaxCluster;
+  const int v = setting(g_max_cluster, "ADAMAS_MAX_CLUSTER", kSaMaxSlices, 1, kSaMaxCluster);
+  return (v & (v - 1)) == 0 ? v : kSaMaxSlices;
 }
 
 template <typename... KArgs, typename... Args>
@@ -1084,89 +1079,38 @@ int adamas_decode_forward_static(const void* q, void* o, float* lse, const void*
 // ---------------------------------------------------------------------------------------------
 namespace {
 
-template <typename T, int I>
-int launch_select_attend_one(const SelectAttendParams& prm, int cl, int num_heads, int batch, size_t smem,
-                             cudaStream_t st) {
+template <typename T>
+int launch_select_attend(const SelectAttendParams& prm, int cl, int num_heads, int batch, size_t smem, cudaStream_t st) {
   const dim3 grid(static_cast<unsigned>(cl), static_cast<unsigned>(num_heads), static_cast<unsigned>(batch));
-  ADAMAS_LAUNCH("select_attend_kernel", (select_attend_kernel<T, I>), grid, dim3(kSaThreads), smem, st, 1, prm);
+  ADAMAS_LAUNCH("select_attend_kernel", (select_attend_kernel<T>), grid, dim3(kSaThreads), smem, st, 1, prm);
   return check_launch("select_attend_kernel");
 }
 
-template <typename T>
-int launch_select_attend(const SelectAttendParams& prm, int items, int cl, int num_heads, int batch, size_t smem,
-                         cudaStream_t st) {
-  switch (items) {
-    case 1: return launch_select_attend_one<T, 1>(prm, cl, num_heads, batch, smem, st);
-    case 2: return launch_select_attend_one<T, 2>(prm, cl, num_heads, batch, smem, st);
-    case 4: return launch_select_attend_one<T, 4>(prm, cl, num_heads, batch, smem, st);
-    case 8: return launch_select_attend_one<T, 8>(prm, cl, num_heads, batch, smem, st);
-    default: break;
-  }
-  return fail(ADAMAS_ERR_INVALID, "unsupported row length for select_attend");
-}
-
-// Shape of a select_attend launch: blocks per head (= histogram slices), granules per thread, winner
-// list and dynamic shared memory (the tile | winner list).  Planned for rows of up to n distances; shorter rows run in the same shape.
+// Shape of a select_attend launch: blocks per head (= histogram slices), winner list and dynamic shared memory (the tiles |
+// winner list).  Planned for rows of up to n distances; shorter rows run in the same shape.
 struct SaPlan {
-  int cl, items, list_capacity;
+  int cl, list_capacity;
   size_t smem;
 };
 
-void sa_shape(int n, int k, int cl, SaPlan* pl) {
-  const int slice_tokens = std::min(n, sa_granules_per_block(n, cl) * 8);
-  const int max_loc = std::min(k, slice_tokens) + 1;   // winners of one block at most, plus the newest token
-  pl->list_capacity = max_loc;
-  pl->smem = static_cast<size_t>(kSaWarps) * 2 * kSaWarpRows * 256 +
-             ((static_cast<size_t>(pl->list_capacity) * 4 + 15) & ~static_cast<size_t>(15));
-}
-
 int sa_plan(int n, int k, int num_heads, const DeviceInfo* di, SaPlan* pl) {
+  // Blocks per head: any number up to 16 (the blocks of a head do not wait for one another).  num_heads counts the rows of
+  // the launch (query heads x sequences).  A block's work is a chain of short dependent steps, so what counts is that
+  // a block's winners fit the tiles of its warps, that a thread has a granule or two, and that the whole launch is
+  // resident at once: as many blocks as the first two ask for if they are resident, else as many as are (but never more
+  // tokens per block than its 16-bit counts can hold).
   const int g_total = (n + 7) / 8;
-  // Blocks per head: any number up to 16 (the blocks of a head do not wait for one another).  num_heads
-  // counts the rows of the launch (query heads x sequences).  By default up to 8 blocks, or more as long as
-  // every block of the launch is resident at once (a row a little beyond 8 * 512 granules then takes 9
-  // blocks instead of two granules per thread, which would double the selection's work);
-  // adamas_set_max_cluster lowers the bound.
-  const int user_limit = max_cluster();
-  const int resident_blocks = 2 * di->num_sms;
-  const int resident = std::max(1, resident_blocks / num_heads);
-  const int cl_limit = user_limit < kSaMaxCluster ? user_limit
-                                                  : std::min(kSaBigCluster, std::max(kSaMaxCluster, resident));
-  // As few granules per thread as possible while the whole launch is resident at once: a block's work is a
-  // chain of short dependent steps that leaves the SM mostly idle, so a second wave of blocks costs a whole
-  // chain again, while more granules per thread only lengthen the first steps (many rows, i.e. a batch of
-  // sequences: 128 rows of 32K distances run as 2 blocks x 4 granules, not 8 x 1 in four waves).  If no
-  // shape is resident at once, the one with the fewest blocks.
-  int cl = 0, items = 0, fewest_cl = 0, fewest_items = 0;
-  for (int it = 1; it <= 8 && cl == 0; it *= 2) {
-    const int need = std::max(1, (g_total + it * kSaThreads - 1) / (it * kSaThreads));
-    if (need > cl_limit) continue;
-    fewest_cl = need;
-    fewest_items = it;
-    if (need * num_heads <= resident_blocks) {
-      cl = need;
-      items = it;
-    }
-  }
-  if (cl == 0) {
-    cl = fewest_cl;
-    items = fewest_items;
-  }
-  ADAMAS_REQUIRE(cl > 0, "select_attend supports at most %d distances per head with %d blocks per head (got %d)",
-                 cl_limit * 8 * kSaThreads * 8, cl_limit, n);
-  // with several granules per thread, rather twice the blocks with half-filled threads than the fewest
-  // blocks that cover the row, if they are still resident at once
-  if (items >= 2) {
-    const int twice = std::min(cl_limit, std::max(cl, (g_total + items * kSaThreads / 2 - 1) / (items * kSaThreads / 2)));
-    if (twice * num_heads <= resident_blocks) cl = twice;
-  }
-  // a large budget on a short row: more blocks per head than the scan needs, so that each block
-  // attends to about one tile of winners, as long as all blocks stay resident at once
-  while (cl < std::min(cl_limit, kSaMaxCluster) && k > cl * kSaTile && 2 * cl * num_heads <= resident_blocks) cl *= 2;
-  cl = std::min(cl, cl_limit);
-  pl->cl = cl;
-  pl->items = items;
-  sa_shape(n, k, cl, pl);
+  const int cl_limit = max_cluster();
+  const int least = (n + kSaMaxBlockTokens - 1) / kSaMaxBlockTokens;
+  ADAMAS_REQUIRE(least <= cl_limit, "select_attend supports at most %d distances per head with %d blocks per head (got %d)",
+                 cl_limit * kSaMaxBlockTokens, cl_limit, n);
+  const int winners = kSaWarps * kSaSlots * kTileRows * 3 / 4;
+  const int wanted = std::max((g_total + 2 * kSaThreads - 1) / (2 * kSaThreads), (k + winners - 1) / winners);
+  const int resident = std::max(1, kSaBlocksPerSm * di->num_sms / num_heads);
+  pl->cl = std::min(std::max(std::min(wanted, resident), least), cl_limit);
+  const int slice_tokens = std::min(n, sa_granules_per_block(n, pl->cl) * 8);
+  pl->list_capacity = std::min(k, slice_tokens) + 1;   // winners of one block at most, plus the newest token
+  pl->smem = static_cast<size_t>(kSaTileBytes) + ((static_cast<size_t>(pl->list_capacity) * 4 + 15) & ~static_cast<size_t>(15));
   ADAMAS_REQUIRE(pl->smem <= static_cast<size_t>(kSaMaxDynSmem), "winner list too long for select_attend (k=%d)", k);
   return ADAMAS_OK;
 }
@@ -1210,8 +1154,8 @@ int select_attend_impl(const void* dist, int64_t dist_stride, int n, int k, cons
   prm.list_capacity = pl.list_capacity;
   prm.scale_log2 = sm_scale * 1.4426950408889634f;
   if (dtype == ADAMAS_F16)
-    return launch_select_attend<__half>(prm, pl.items, pl.cl, q_heads, batch, pl.smem, to_stream(stream));
-  return launch_select_attend<__nv_bfloat16>(prm, pl.items, pl.cl, q_heads, batch, pl.smem, to_stream(stream));
+    return launch_select_attend<__half>(prm, pl.cl, q_heads, batch, pl.smem, to_stream(stream));
+  return launch_select_attend<__nv_bfloat16>(prm, pl.cl, q_heads, batch, pl.smem, to_stream(stream));
 }
 
 static_assert(ADAMAS_HIST_WORDS_PER_HEAD == kSaScratchWordsPerHead, "scratch layout of select_attend");
@@ -1272,7 +1216,7 @@ int adamas_select_attend(const void* dist, int64_t dist_stride, int n, int k, co
     hp.n = n;
     hp.cl = pl.cl;
     hp.seq_len_dev = nullptr;
-    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.cl, num_heads), dim3(kSaThreads), 0,
+    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.cl, num_heads), dim3(kSaBins), 0,
                   to_stream(stream), 1, hp);
   }
   return select_attend_impl(dist, dist_stride, n, k, q, o, o_f32, lse, kv_data, kv_page_table, page_size, kv_heads,
@@ -1294,7 +1238,7 @@ int adamas_dist_histograms(const void* dist, int64_t dist_stride, int n, int num
   hp.n = n;
   hp.cl = slices;
   hp.seq_len_dev = nullptr;
-  ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(slices, num_heads), dim3(kSaThreads), 0,
+  ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(slices, num_heads), dim3(kSaBins), 0,
                 to_stream(stream), 1, hp);
   return check_launch("dist_histogram_kernel");
 }
@@ -1443,7 +1387,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
     hp.n = n;
     hp.cl = pl.cl;
     hp.seq_len_dev = seq_len_dev;
-    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.cl, q_heads, batch), dim3(kSaThreads), 0,
+    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.cl, q_heads, batch), dim3(kSaBins), 0,
                   to_stream(stream), 1, hp);
     if (int rc2 = check_launch("dist_histogram_kernel")) return rc2;
   }

@@ -1,0 +1,149 @@
+// A warp's attention over a tile of 16 gathered K and V rows, on the tensor cores (mma.sync m16n8k16, fp32
+// accumulation): up to 8 query rows at once.  Used by the decode attention (all query heads of a cache head) and by
+// select+attend (one query row, an eighth of the instruction's width: still about half of the instructions of a
+// multiply-add form).
+//
+// The order of the 128 dimensions is free in q.K, and of the output rows in P.V, so every lane reads whole 16-byte
+// chunks: chunk 4j + t of K rows g and g + 8, chunks g and 8 + g of V rows 2t, 2t + 1, 2t + 8, 2t + 9 (g = lane / 4,
+// t = lane % 4).  Chunk c of row r is stored at c ^ tile_swizzle(r), which makes both patterns free of bank conflicts.
+// P enters P.V as the sum of two 16-bit numbers (its rounding and the remainder), so that it keeps more than 16 bits
+// for fp16 rows and 16 for bf16.
+#pragma once
+#include "common.cuh"
+
+namespace adamas {
+
+constexpr int kTileRows = 16;
+constexpr int kTileBytes = 2 * kTileRows * kHeadDim * 2;   // 16 K rows, 16 V rows
+
+template <typename T>
+struct Mma;
+template <>
+struct Mma<__half> {
+  static __device__ __forceinline__ void run(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+};
+template <>
+struct Mma<__nv_bfloat16> {
+  static __device__ __forceinline__ void run(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                             uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+};
+
+// State of a warp over the tiles it has seen: head g = lane / 4 in m, l (l: this lane's tokens only);
+// o[j]: output dims (8g' + j, 64 + 8g' + j) of heads 2t, 2t + 1 with g' = lane / 4 (the C fragment of P.V).
+struct TileState {
+  float m, l;
+  float o[8][4];
+};
+
+__device__ __forceinline__ int tile_swizzle(int r) { return (r & 6) ^ ((r & 1) << 2); }
+
+__device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// Requests the tile's K and / or V rows with 16-byte asynchronous copies: lane l (and l + 16) holds the cache row of token
+// l, in units of row_elems elements behind kbase; its V row lies v_delta elements behind its K row.
+template <typename T, bool K, bool V>
+__device__ __forceinline__ void tile_copy(const T* kbase, int64_t v_delta, int64_t row_elems, int row, uint8_t* slot, int lane) {
+  const int half = lane >> 4, c = lane & 15;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {   // a half-warp per row
+    const int rr = 2 * i + half;
+    const T* src = kbase + __shfl_sync(0xffffffffu, row, rr) * row_elems + c * 8;
+    uint8_t* dst = slot + rr * 256 + ((c ^ tile_swizzle(rr)) << 4);
+    if (K) cp_async_16(dst, src);
+    if (V) cp_async_16(dst + kTileRows * 256, src + v_delta);
+  }
+}
+
+// Scaled logits of the tile: S[head g][tokens 2t, 2t + 1, 2t + 8, 2t + 9] in this lane; -inf for tokens outside `mask`.
+template <typename T>
+__device__ __forceinline__ void tile_logits(const uint8_t* slot, const uint4 (&q)[4], unsigned mask, float scale_log2, int lane,
+                                            float (&s)[4]) {
+  const int g = lane >> 2, t = lane & 3;
+  float c[2][2][4] = {};   // [rows g, g + 8][two accumulators: shorter chains]
+  const uint8_t* krow = slot + g * 256;
+  const int ksw = tile_swizzle(g);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const uint4 k = *reinterpret_cast<const uint4*>(krow + u * 2048 + (((4 * j + t) ^ ksw) << 4));
+      Mma<T>::run(c[u][0], q[j].x, 0u, q[j].y, 0u, k.x, k.y);
+      Mma<T>::run(c[u][1], q[j].z, 0u, q[j].w, 0u, k.z, k.w);
+    }
+  }
+  s[0] = c[0][0][0] + c[0][1][0];
+  s[1] = c[0][0][1] + c[0][1][1];
+  s[2] = c[1][0][0] + c[1][1][0];
+  s[3] = c[1][0][1] + c[1][1][1];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) s[u] = (mask >> (2 * t + (u & 1) + 8 * (u >> 1))) & 1u ? s[u] * scale_log2 : -INFINITY;
+}
+
+// Softmax in base 2 and P.V over the tile; at least one token must exist, and rows of absent ones must hold finite values.
+template <typename T>
+__device__ __forceinline__ void tile_softmax_pv(TileState& st, const uint8_t* slot, const float (&s)[4], int lane) {
+  const int g = lane >> 2, t = lane & 3;
+  uint4 v[4][2];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int rr = 2 * t + (u & 1) + 8 * (u >> 1);
+    const uint8_t* vrow = slot + kTileRows * 256 + rr * 256;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) v[u][h] = *reinterpret_cast<const uint4*>(vrow + (((g + 8 * h) ^ tile_swizzle(rr)) << 4));
+  }
+  float m_new = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+  m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
+  m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
+  m_new = fmaxf(m_new, st.m);
+  if (__any_sync(0xffffffffu, m_new > st.m)) {
+    const float r = (st.m == -INFINITY) ? 0.f : exp2f(st.m - m_new);
+    st.l *= r;
+    st.m = m_new;
+    const float r0 = __shfl_sync(0xffffffffu, r, 8 * t), r1 = __shfl_sync(0xffffffffu, r, 8 * t + 4);   // heads 2t, 2t + 1
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      st.o[j][0] *= r0;
+      st.o[j][1] *= r1;
+      st.o[j][2] *= r0;
+      st.o[j][3] *= r1;
+    }
+  }
+  float pr[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) pr[u] = exp2f(s[u] - st.m);   // (a masked token: exp2(-inf) = 0; st.m is finite)
+  st.l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
+  // B fragments of P.V: tokens 2t, 2t + 1 and 2t + 8, 2t + 9 of head g
+  const uint32_t hi0 = Elem<T>::from_f2(pr[0], pr[1]), hi1 = Elem<T>::from_f2(pr[2], pr[3]);
+  const float2 f0 = Elem<T>::to_f2(hi0), f1 = Elem<T>::to_f2(hi1);
+  const uint32_t lo0 = Elem<T>::from_f2(pr[0] - f0.x, pr[1] - f0.y), lo1 = Elem<T>::from_f2(pr[2] - f1.x, pr[3] - f1.y);
+#pragma unroll
+  for (int w = 0; w < 4; ++w) {
+    uint32_t a[2][4];   // [even / odd dimension of the word][a0 .. a3]
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {   // rows g (dims 8g ..) and g + 8 (dims 64 + 8g ..)
+      const uint32_t v0 = word_of(v[0][h], w), v1 = word_of(v[1][h], w);
+      const uint32_t v2 = word_of(v[2][h], w), v3 = word_of(v[3][h], w);
+      a[0][h] = __byte_perm(v0, v1, 0x5410);
+      a[1][h] = __byte_perm(v0, v1, 0x7632);
+      a[0][2 + h] = __byte_perm(v2, v3, 0x5410);
+      a[1][2 + h] = __byte_perm(v2, v3, 0x7632);
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) Mma<T>::run(st.o[2 * w + e], a[e][0], a[e][1], a[e][2], a[e][3], hi0, hi1);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) Mma<T>::run(st.o[2 * w + e], a[e][0], a[e][1], a[e][2], a[e][3], lo0, lo1);
+  }
+}
+
+}  // namespace adamas

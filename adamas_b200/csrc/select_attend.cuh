@@ -8,40 +8,47 @@
 // in a global table [H][kSaMaxSlices][512] u32: slice r covers the granules (8 distances) that block
 // r of the head's cluster owns.  A distance is at most 3 * 128 = 384; larger values count as 511.
 //
-// CL <= 16 blocks x 512 threads per head (grid (CL, H)); the blocks of a head never wait for one another.
+// CL <= 16 blocks x 128 threads per head (grid (CL, H)); the blocks of a head never wait for one another.
 // Block `cr`:
-//   load   its slice of the distance row (registers), the head's CL histograms (one bin per thread)
-//          and the query chunks, all in flight together;
+//   load   its slice of the distance row (asynchronous copies into the shared memory that later holds K and V rows), the
+//          head's CL histograms (four bins per thread) and the query, all in flight together;
 //   cut    block-wide scan of the summed histogram: the cut distance, how many cut-valued elements
 //          are taken in all, how many of them and how many smaller elements lie in lower-ranked
 //          slices (= this slice's tie quota and its offset in the output list).  Every block
 //          derives this by itself from the same table: no exchange between blocks;
 //   pick   ordered compaction of the block's winners into a list in shared memory;
-//   attend the rows of the list are dealt out evenly to the 16 warps; a warp gathers the K and V rows of
-//          its tokens itself (16-byte asynchronous copies, a half-warp per 256-byte row, into its own
-//          part of the tile; K rows as one group, V rows as a second), computes q.K with four lanes per token, a
-//          softmax in base 2 over its tokens and P.V with four dimensions per lane: no block barrier
-//          inside the attention;
-//   merge  the 16 warps' partial (o, m, l) are merged in shared memory and the block's partial goes to
+//   attend the rows of the list are dealt out evenly to the 4 warps; a warp gathers the K and V rows of
+//          its tokens itself, 16 at a time (16-byte asynchronous copies into its own tile), and works on
+//          them alone (q.K on the tensor cores, attend_tile.cuh): no block barrier inside the attention;
+//   merge  the 4 warps' partial (o, m, l) are merged in shared memory and the block's partial goes to
 //          the head's slot table in global scratch; the block that arrives LAST at the head's counter
 //          merges the CL partials, writes the head's output, clears the head's histogram rows and the
-//          counter.  Every other block is gone by then: its SM is free for the next kernel's blocks
-//          while the slowest block of the head still works (with a cluster barrier at this point all
-//          blocks of a head stayed resident until the slowest had finished, 2 us at 32K / 1024).
+//          counter.  Every other block is gone by then.
+// BOUNDTEXT
 #pragma once
+#include "attend_tile.cuh"
 #include "common.cuh"
 #include "hadamard_append.cuh"
 
 namespace adamas {
 
-constexpr int kSaThreads = 512;
+#ifndef SB
+#define SB 4
+#endif
+#ifndef SS
+#define SS 1
+#endif
+constexpr int kSaThreads = 128;
 constexpr int kSaWarps = kSaThreads / 32;
+constexpr int kSaBlocksPerSm = SB;
 constexpr int kSaBins = 512;
-constexpr int kSaMaxSlices = 16;      // histogram rows per head = largest cluster
-constexpr int kSaTile = 128;          // planning unit of the host (winners per block it aims for)
-constexpr int kSaWarpRows = 12;       // rows a warp gathers per round (its part of the tile: 12 K + 12 V rows)
-constexpr int kSaMaxCluster = 8;      // blocks per head by default (more, up to 16, while all blocks are resident at once)
-constexpr int kSaBigCluster = 16;     // long rows of few heads (see the host code)
+constexpr int kSaMaxSlices = 16;      // histogram rows per head = largest number of blocks per head
+constexpr int kSaSlots = SS;          // tiles per warp
+constexpr int kSaTileBytes = kSaWarps * kSaSlots * kTileBytes;
+constexpr int kSaStaged = kSaTileBytes / 16 * 8 / 9 - 8;   // granules of a slice that are staged in the tiles' memory
+constexpr int kSaMaxBlockTokens = 32768;
+constexpr int kSaMaxCluster = 8;      // upper bound of adamas_set_max_cluster
+
 // Scratch words (32 bit) per head: kSaMaxSlices histogram rows of 512 counts, then kSaMaxSlices slots of
 // kSaSlotWords floats for the blocks' partial results (128 outputs, running max, running sum; word 130
 // of slot 0 is the head's arrival counter).
@@ -93,21 +100,41 @@ struct SelectAttendParams {
 
 struct SaShared {
   float ml[kSaWarps][2];
-  unsigned warp_a[kSaWarps];
-  unsigned warp_b[kSaWarps];
+  uint2 warp_sum[kSaWarps];
   unsigned cut, need_eq, lt_before, eq_before;
   unsigned last;   // this block arrived last at the head's counter
   uint4 q[16];     // the head's query row
   float2 cs[kHeadDim / 2];   // rope_on: (cos, sin) of the position
 };
 
-// Dynamic shared memory: the tile (16 warps x (12 K rows + 12 V rows) x 256 B; a warp parks its partial
-// output in its own K rows at the end) | winner list (list_capacity * 4 B).
-template <typename T, int ITEMS>
-__global__ void __launch_bounds__(kSaThreads, 2) select_attend_kernel(const SelectAttendParams p) {
-  constexpr int NT = kSaThreads;
-  static_assert(NT >= kSaBins, "one histogram bin per thread");
-  extern __shared__ __align__(16) uint8_t sa_smem[];
+// The 8 values of a granule against two thresholds, halfword-parallel: bit w (element 2w) or 16 + w (element 2w + 1) of the
+// result is set where the value, at most 511 after clamping, reaches threshold c with k = (0x8000 - c) in both halves.
+__device__ __forceinline__ void sa_compare(uint4 v, unsigned k_ge, unsigned k_gt, unsigned* ge, unsigned* gt) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  unsigned a = 0, b = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const unsigned x = __vminu2(w[i], 0x01ff01ffu);
+    a |= (((x + k_ge) >> 15) & 0x00010001u) << i;
+    b |= (((x + k_gt) >> 15) & 0x00010001u) << i;
+  }
+  *ge = a;
+  *gt = b;
+}
+// bits w / 16 + w -> bit = element
+__device__ __forceinline__ unsigned sa_in_order(unsigned m) {
+  unsigned x = (m & 0xfu) | ((m >> 8) & 0xf00u);
+  x = (x | (x << 2)) & 0x3333u;
+  x = (x | (x << 1)) & 0x5555u;
+  return (x & 0xffu) | ((x >> 7) & 0xaau);
+}
+
+// Dynamic shared memory: the warps' tiles (8 KB each; first the staged distances, at the end a warp parks its partial
+// output in its first tile) | winner list (list_capacity * 4 B).
+template <typename T>
+__global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kernel(const SelectAttendParams p) {
+  static_assert(4 * kSaThreads == kSaBins && kSaThreads == kHeadDim, "four histogram bins and one output per thread");
+  extern __shared__ __align__(128) uint8_t sa_smem[];
   __shared__ __align__(16) SaShared sh;
 
   const unsigned CL = gridDim.x;
@@ -127,78 +154,60 @@ __global__ void __launch_bounds__(kSaThreads, 2) select_attend_kernel(const Sele
     seq_len_dev += blockIdx.z;
   }
 
-  uint8_t* sa_tile = sa_smem;                                                         // [16 warps][K rows | V rows]
-  int32_t* s_list = reinterpret_cast<int32_t*>(sa_smem + kSaWarps * 2 * kSaWarpRows * 256);   // the block's winners, in position order
+  int32_t* s_list = reinterpret_cast<int32_t*>(sa_smem + kSaTileBytes);               // the block's winners, in position order
   uint32_t* head_scratch = p.hist + static_cast<size_t>(head) * kSaScratchWordsPerHead;
   float* slots = reinterpret_cast<float*>(head_scratch + kSaMaxSlices * kSaBins);     // [CL][kSaSlotWords]
-  uint4* s_q = sh.q;
 
   // ---- set-up that needs no input (overlaps the tail of the preceding kernel) -----------------------
   if (tid == 0) sh.cut = 0xffffffffu;
-  __syncthreads();
   grid_dependency_wait();
   grid_launch_dependents();
 
-  // ---- loads: distances, histograms, query, page numbers --------------------------------------------
+  // ---- loads: distances, histograms, query ------------------------------------------------------------
   const int n = seq_len_dev ? (__ldg(seq_len_dev) - 1) : p.n;
   const int G = (n + 7) >> 3;
   const int gpb = sa_granules_per_block(n, static_cast<int>(CL));
   const int blk_first = cr * gpb;
-  // (rope_on: warps 2 and 3 form the position's cos / sin pairs; the block barriers of the cut phase order
-  // them before the query is rotated)
-  const bool rope_thread = p.rope_on && tid >= kHeadDim / 2 && tid < kHeadDim;
-  const int blk_end = min(G, blk_first + gpb);
-  const int g0 = blk_first + tid * ITEMS;
-  const uint4* gbase = reinterpret_cast<const uint4*>(p.dist + static_cast<int64_t>(head) * p.dist_stride);
-  uint32_t raw[ITEMS][4];
-  unsigned vmask[ITEMS];
-#pragma unroll
-  for (int i = 0; i < ITEMS; ++i) {
-    uint4 v = make_uint4(0, 0, 0, 0);
-    unsigned m = 0;
-    const int g = g0 + i;
-    if (g < blk_end) {
-      v = ld_16(gbase + g);
-      m = 0xffu;
-      if (g * 8 + 8 > n) m = 0xffu >> (g * 8 + 8 - n);
-    }
-    raw[i][0] = v.x; raw[i][1] = v.y; raw[i][2] = v.z; raw[i][3] = v.w;
-    vmask[i] = m;
-  }
-  // (all loads are issued before the first count is used: one trip to L2, not one per slice)
-  unsigned hcnt[kSaMaxSlices];
+  const int blk_count = max(0, min(G - blk_first, gpb));
+  const uint4* gbase = reinterpret_cast<const uint4*>(p.dist + static_cast<int64_t>(head) * p.dist_stride) + blk_first;
+  uint4* staged = reinterpret_cast<uint4*>(sa_smem);   // granule g at g + g / 8: reads of neighbouring threads' runs do not conflict
+  uint4 tot = make_uint4(0u, 0u, 0u, 0u), low = tot;   // bins 4 * tid ..: the whole row; lower-ranked slices
+  uint4 qraw = tot;                                    // the query row, 16 lanes x 16 bytes
   {
-    const uint32_t* hrow = head_scratch + tid;
+    const uint4* hrow = reinterpret_cast<const uint4*>(head_scratch) + tid;
+    for (int g = tid; g < min(blk_count, kSaStaged); g += kSaThreads) cp_async_16(staged + g + (g >> 3), gbase + g);
+    cp_async_commit();
+    if (tid < 16) qraw = ld_16(static_cast<const T*>(p.q) + static_cast<int64_t>(head) * kHeadDim + tid * 8);
+#pragma unroll 1
+    for (unsigned r0 = 0; r0 < CL; r0 += 8) {
+      uint4 c[8];   // (eight loads in flight)
 #pragma unroll
-    for (unsigned r = 0; r < kSaMaxSlices; ++r) hcnt[r] = r < CL ? __ldcg(hrow + r * kSaBins) : 0u;
-  }
-  // With pages of 8 tokens or more (a power of two) a granule lies inside one page: fetch its
-  // physical page number now, long before the winners are known.
-  const bool page_per_granule = p.ps_shift >= 3;
-  int granule_page[ITEMS];
+      for (unsigned u = 0; u < 8; ++u) c[u] = r0 + u < CL ? __ldcg(hrow + (r0 + u) * (kSaBins / 4)) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-  for (int i = 0; i < ITEMS; ++i) {
-    granule_page[i] = 0;
-    if (page_per_granule && g0 + i < blk_end) granule_page[i] = __ldg(kv_table + (((g0 + i) * 8) >> p.ps_shift));
+      for (unsigned u = 0; u < 8; ++u) {
+        tot.x += c[u].x; tot.y += c[u].y; tot.z += c[u].z; tot.w += c[u].w;
+        if (r0 + u < cr) { low.x += c[u].x; low.y += c[u].y; low.z += c[u].z; low.w += c[u].w; }
+      }
+    }
   }
+  // (rope_on: the last two warps form the position's cos / sin pairs; the block barriers of the cut phase order them before
+  // the query is rotated)
+  if (p.rope_on && tid >= kHeadDim / 2)
+    sh.cs[tid - kHeadDim / 2] = rope_cos_sin(tid - kHeadDim / 2, static_cast<float>(n), p.rope);
   // the newest token rides with the last slice
   const bool tail_here = p.tail_mode != 0 && cr == CL - 1;
+  const unsigned ps = static_cast<unsigned>(p.page_size);
   unsigned tail_slot = p.tail_slot;
   if (tail_here && tid == 0 && p.tail_mode == 2) {
-    const unsigned un = static_cast<unsigned>(n), ps = static_cast<unsigned>(p.page_size);
+    const unsigned un = static_cast<unsigned>(n);
     const unsigned pg = p.ps_shift >= 0 ? (un >> p.ps_shift) : (un / ps);
     tail_slot = static_cast<unsigned>(__ldg(kv_table + pg)) * ps + (un - pg * ps);
   }
-  if (rope_thread) sh.cs[tid - kHeadDim / 2] = rope_cos_sin(tid - kHeadDim / 2, static_cast<float>(n), p.rope);
-  // ---- cut: one bin per thread ------------------------------------------------------------------------
-  unsigned tot = 0, low = 0;
-#pragma unroll
-  for (unsigned r = 0; r < kSaMaxSlices; ++r) {
-    tot += hcnt[r];
-    low += r < cr ? hcnt[r] : 0u;
-  }
+
+  // ---- cut ----------------------------------------------------------------------------------------------
   {
-    unsigned it = tot, il = low;
+    const unsigned t4 = (tot.x + tot.y) + (tot.z + tot.w), l4 = (low.x + low.y) + (low.z + low.w);
+    unsigned it = t4, il = l4;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned t = __shfl_up_sync(0xffffffffu, it, o);
@@ -208,112 +217,128 @@ __global__ void __launch_bounds__(kSaThreads, 2) select_attend_kernel(const Sele
         il += u;
       }
     }
-    if (lane == 31) {
-      sh.warp_a[warp] = it;
-      sh.warp_b[warp] = il;
-    }
+    if (lane == 31) sh.warp_sum[warp] = make_uint2(it, il);
     __syncthreads();
-    unsigned wa = 0, wb = 0;
+    unsigned below = it - t4, below_low = il - l4;   // elements below this thread's first bin: whole row, lower-ranked slices
 #pragma unroll
-    for (int w2 = 0; w2 < kSaWarps; ++w2) {
-      wa += (w2 < warp) ? sh.warp_a[w2] : 0u;
-      wb += (w2 < warp) ? sh.warp_b[w2] : 0u;
+    for (int w2 = 0; w2 < kSaWarps - 1; ++w2) {
+      const uint2 v = sh.warp_sum[w2];
+      below += w2 < warp ? v.x : 0u;
+      below_low += w2 < warp ? v.y : 0u;
     }
-    const unsigned excl = wa + it - tot;        // elements of smaller value, whole row
-    const unsigned excl_low = wb + il - low;    // ... in lower-ranked slices
-    bool mine, all_win = false;
-    unsigned need = 0;
+    const unsigned tb[4] = {tot.x, tot.y, tot.z, tot.w}, lb[4] = {low.x, low.y, low.z, low.w};
     if (p.ext_cut) {
-      // (a cut of 512, beyond every bin: the whole row wins; thread 511 stands in, there are no ties)
+      // (a cut of 512, beyond every bin: the whole row wins; the last thread stands in, there are no ties)
       const int2 e = __ldg(p.ext_cut + head);
-      all_win = e.x >= kSaBins;
-      mine = tid == min(e.x, kSaBins - 1);
-      need = all_win ? 0u : static_cast<unsigned>(e.y);
+      const bool all_win = e.x >= kSaBins;
+      const int bin = min(e.x, kSaBins - 1);
+      if (tid == bin >> 2) {
+        unsigned lt = below_low;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (i < (bin & 3) || all_win) lt += lb[i];
+          if (i == (bin & 3)) sh.eq_before = all_win ? 0u : lb[i];
+        }
+        sh.cut = all_win ? static_cast<unsigned>(kSaBins) : static_cast<unsigned>(bin);
+        sh.need_eq = all_win ? 0u : static_cast<unsigned>(e.y);
+        sh.lt_before = lt;
+      }
     } else {
       const unsigned want = static_cast<unsigned>(p.k);
-      mine = excl < want && excl + tot >= want;   // exactly one thread
-      need = want - excl;
+      if (below < want && below + t4 >= want) {   // exactly one thread
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (below < want && below + tb[i] >= want) {
+            sh.cut = 4 * tid + i;
+            sh.need_eq = want - below;     // cut-valued winners in all
+            sh.lt_before = below_low;      // smaller-valued elements in lower-ranked slices
+            sh.eq_before = lb[i];          // cut-valued elements in lower-ranked slices
+          }
+          below += tb[i];
+          below_low += lb[i];
+        }
+      }
     }
-    if (mine) {
-      sh.cut = all_win ? static_cast<unsigned>(kSaBins) : static_cast<unsigned>(tid);
-      sh.need_eq = need;                                  // cut-valued winners in all
-      sh.lt_before = excl_low + (all_win ? low : 0u);     // smaller-valued elements in lower-ranked slices
-      sh.eq_before = all_win ? 0u : low;                  // cut-valued elements in lower-ranked slices
-    }
-    __syncthreads();
+    cp_async_wait<0>();
+    __syncthreads();   // the cut is known, the staged distances are visible
   }
   unsigned cut = sh.cut;
-  unsigned need_eq = sh.need_eq;
+  unsigned need_eq = sh.need_eq, lt_before = sh.lt_before, eq_before = sh.eq_before;
   if (cut == 0xffffffffu) {
     // the table does not describe this row (fewer than k entries): take nothing but the newest token
     if (tid == 0) atomicOr(&g_adamas_error, kErrHistogram);
-    cut = 0;
-    need_eq = 0;
+    cut = need_eq = lt_before = eq_before = 0;
   }
-  const unsigned eq_before = (sh.cut == 0xffffffffu) ? 0u : sh.eq_before;
   const unsigned take_eq = need_eq > eq_before ? need_eq - eq_before : 0u;   // this slice's tie quota
-  const unsigned out_base = ((sh.cut == 0xffffffffu) ? 0u : sh.lt_before) + min(eq_before, need_eq);
+  const unsigned out_base = lt_before + min(eq_before, need_eq);
 
   // ---- pick: ordered compaction of this block's winners -----------------------------------------------
-  // Two halfword-parallel compares per register give, per granule, the 8-bit masks of the elements below
-  // the cut and at the cut (values of 511 and more count as 511).
-  const unsigned cut2 = min(cut, 0xffffu) * 0x00010001u;
-  unsigned m_lt[ITEMS], m_eq[ITEMS];
-  unsigned c_lt = 0, c_eq = 0;
-#pragma unroll
-  for (int i = 0; i < ITEMS; ++i) {
-    unsigned lt = 0, eq = 0;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const unsigned x = __vminu2(raw[i][w], 0x01ff01ffu);
-      const unsigned l = __vcmpltu2(x, cut2);   // 0xffff per halfword that is below the cut
-      const unsigned e = __vcmpeq2(x, cut2);
-      lt |= ((l & 1u) | ((l >> 15) & 2u)) << (2 * w);
-      eq |= ((e & 1u) | ((e >> 15) & 2u)) << (2 * w);
-    }
-    m_lt[i] = lt & vmask[i];
-    m_eq[i] = eq & vmask[i];
-    c_lt += __popc(m_lt[i]);
-    c_eq += __popc(m_eq[i]);
+  // A thread owns `run` consecutive granules; it counts its elements below and at the cut, a block scan gives it its place
+  // in the list, and a second look at the granules that hold any writes the winners.
+  const unsigned k_ge = (0x8000u - cut) * 0x00010001u, k_gt = (0x7fffu - cut) * 0x00010001u;
+  const int run = (blk_count + kSaThreads - 1) / kSaThreads;
+  const int g_first = tid * run, g_end = min(blk_count, g_first + run);
+  auto masks = [&](int g, unsigned* lt, unsigned* eq) {
+    const uint4 v = g < kSaStaged ? staged[g + (g >> 3)] : ld_16(gbase + g);
+    unsigned ge, gt;
+    sa_compare(v, k_ge, k_gt, &ge, &gt);
+    unsigned valid = 0x000f000fu;
+    const int left = n - (blk_first + g) * 8;
+    if (left < 8) valid = ((1u << ((left + 1) >> 1)) - 1u) | (((1u << (left >> 1)) - 1u) << 16);
+    *lt = ~ge & valid;
+    *eq = ge & ~gt & valid;
+  };
+  unsigned packed = 0;   // elements below the cut | elements at the cut << 16 (a block holds at most 32768)
+#pragma unroll 2
+  for (int g = g_first; g < g_end; ++g) {
+    unsigned lt, eq;
+    masks(g, &lt, &eq);
+    packed += __popc(lt) + (__popc(eq) << 16);
   }
-  const unsigned packed = c_lt | (c_eq << 16);
   unsigned incl = packed;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  if (lane == 31) sh.warp_a[warp] = incl;   // (its readers of the cut phase are past a block barrier)
+  if (lane == 31) sh.warp_sum[warp].x = incl;   // (its readers of the cut phase are past a block barrier)
+  if (warp == 0) {
+    if (p.rope_on) {   // (dimension pairs sit in lanes l and l ^ 8)
+      float x[8];
+      unpack8<T>(qraw, x);
+      rope_halfwarp_cs<T>(x, lane & 15, sh.cs, p.rope.inv_freq != nullptr, p.rope.mscale);
+      qraw = pack8<T>(x);
+    }
+    if (lane < 16) sh.q[lane] = qraw;
+  }
   __syncthreads();
-  unsigned wbase = 0, blk_tot = 0;
+  unsigned before = incl - packed, blk_tot = 0;
 #pragma unroll
   for (int w2 = 0; w2 < kSaWarps; ++w2) {
-    const unsigned a = sh.warp_a[w2];
-    wbase += (w2 < warp) ? a : 0u;
+    const unsigned a = sh.warp_sum[w2].x;
+    before += (w2 < warp) ? a : 0u;
     blk_tot += a;
   }
-  const unsigned excl = wbase + incl - packed;
-  unsigned run_lt = excl & 0xffffu, run_eq = excl >> 16;
-  const unsigned blk_lt = blk_tot & 0xffffu, blk_eq = blk_tot >> 16;
-  const int n_win = static_cast<int>(blk_lt + min(blk_eq, take_eq));
+  unsigned run_lt = before & 0xffffu, run_eq = before >> 16;
+  const int n_win = static_cast<int>((blk_tot & 0xffffu) + min(blk_tot >> 16, take_eq));
   const int n_loc = min(n_win + (tail_here ? 1 : 0), p.list_capacity);
-
-  const T* kvp = static_cast<const T*>(kv_base);
-  const unsigned ps = static_cast<unsigned>(p.page_size);
-  const int64_t v_delta = static_cast<int64_t>(p.page_size) * H * kHeadDim;
-  // The winners go to a list in shared memory (a few instructions on a divergent path).
+  // The winners go to a list in shared memory.
   int32_t* oi = p.out_idx ? p.out_idx + static_cast<int64_t>(head) * p.out_stride + out_base : nullptr;
-  if (c_lt | c_eq) {
-#pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-      // only the elements at or below the cut are visited, in position order (a warp takes as many turns
-      // as its busiest lane has candidates: one or two at the usual budgets)
-      unsigned cand = m_lt[i] | m_eq[i];
-      while (cand) {
+  if (packed) {
+    for (int g = g_first; g < g_end; ++g) {
+      unsigned lt, eq;
+      masks(g, &lt, &eq);
+      if (!(lt | eq)) continue;
+      lt = sa_in_order(lt);
+      unsigned cand = lt | sa_in_order(eq);
+      const unsigned t0 = static_cast<unsigned>(blk_first + g) * 8;
+      unsigned page = 0;   // (with pages of 8 tokens or more, a power of two, a granule lies inside one page)
+      if (p.ps_shift >= 3) page = static_cast<unsigned>(__ldg(kv_table + (t0 >> p.ps_shift)));
+      while (cand) {   // in position order
         const int j = __ffs(cand) - 1;
         cand &= cand - 1;
         int pos = -1;
-        if ((m_lt[i] >> j) & 1u) {
+        if ((lt >> j) & 1u) {
           pos = static_cast<int>(run_lt + min(run_eq, take_eq));
           ++run_lt;
         } else {
@@ -321,20 +346,13 @@ __global__ void __launch_bounds__(kSaThreads, 2) select_attend_kernel(const Sele
           ++run_eq;
         }
         if (pos >= 0) {
-          const unsigned t = static_cast<unsigned>((g0 + i) * 8 + j);   // logical token position
+          const unsigned t = t0 + j;   // logical token position
           unsigned slot;
-          if (page_per_granule) {
-            slot = static_cast<unsigned>(granule_page[i]) * ps + (t & (ps - 1));
+          if (p.ps_shift >= 3) {
+            slot = page * ps + (t & (ps - 1));
           } else {
-            unsigned pg, e;
-            if (p.ps_shift >= 0) {
-              pg = t >> p.ps_shift;
-              e = t & (ps - 1);
-            } else {
-              pg = t / ps;
-              e = t - pg * ps;
-            }
-            slot = static_cast<unsigned>(__ldg(kv_table + pg)) * ps + e;
+            const unsigned pg = p.ps_shift >= 0 ? t >> p.ps_shift : t / ps;
+            slot = static_cast<unsigned>(__ldg(kv_table + pg)) * ps + (t - pg * ps);
           }
           if (pos < p.list_capacity) s_list[pos] = static_cast<int32_t>(slot);
           if (oi) oi[pos] = static_cast<int32_t>(slot);
@@ -343,222 +361,148 @@ __global__ void __launch_bounds__(kSaThreads, 2) select_attend_kernel(const Sele
     }
   }
   if (tail_here && tid == 0 && n_win < p.list_capacity) s_list[n_win] = static_cast<int32_t>(tail_slot);
-  if (warp == 0) {
-    // the query row: 16 lanes x 16 bytes (with rope_on rotated first: dimension pairs sit in lanes l and l ^ 8)
-    uint4 raw = make_uint4(0, 0, 0, 0);
-    if (lane < 16) raw = ld_16(static_cast<const T*>(p.q) + static_cast<int64_t>(head) * kHeadDim + lane * 8);
-    if (p.rope_on) {
-      float x[8];
-      unpack8<T>(raw, x);
-      rope_halfwarp_cs<T>(x, lane & 15, sh.cs, p.rope.inv_freq != nullptr, p.rope.mscale);
-      raw = pack8<T>(x);
-    }
-    if (lane < 16) s_q[lane] = raw;
-  }
+  __syncthreads();   // the list and the query are complete, the staged distances are read
 
-  // ---- attend: every warp over its own rows --------------------------------------------------------------
-  // The rows are dealt out evenly: warp w owns rows w*rpw .. of the list.  It gathers them itself, kSaWarpRows
-  // at a time, with 16-byte asynchronous copies (cp.async), a half-warp per 256-byte row, into the warp's own
-  // part of the tile: first all K rows (one commit group), then all V rows (a second group); then q.K with
-  // four lanes per token as soon as the K group has landed, a softmax in base 2 over its tokens and, after
-  // the V group, P.V with four dimensions per lane.  Nothing in here is shared between warps: no block
-  // barrier inside the attention.
-  // Measured alternatives for the gather (select+attend alone, 32K / 1024): one 256-byte bulk (TMA) copy
-  // per row with an mbarrier per warp 12.4-12.5 us against 12.2 with the 16-byte copies (a bulk copy with
-  // a different address in every lane is issued lane after lane, about 45 ns each: 0.7 us for the 16 rows
-  // of a warp); all bulk copies issued by the first n_loc / 16 warps 1.9 us instead of 0.7; plain vector
-  // loads into registers instead of the tile (all rows cannot be in flight at once in 64 registers: the
-  // second round of a warp pays the memory latency again) 4.5 us in this phase.
-  __syncthreads();   // the list and the query are complete
-  float m_run = -INFINITY, l_run = 0.f;   // l_run is kept by the lanes with quarter == 0
-  float o_acc[4] = {0.f, 0.f, 0.f, 0.f};  // dimensions 4*lane .. 4*lane+3
+  // ---- attend: warp w takes rows w*rpw .. of the list, 16 at a time --------------------------------------
+  uint8_t* tiles = sa_smem + warp * (kSaSlots * kTileBytes);
+  float m_run = -INFINITY, l_run = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);   // dimensions 4 * lane ..
   const int rpw = (n_loc + kSaWarps - 1) / kSaWarps;
   const int my_first = warp * rpw;
   const int my_total = max(0, min(rpw, n_loc - my_first));
-  uint8_t* wk = sa_tile + warp * (2 * kSaWarpRows * 256);   // this warp's K rows, then its V rows
-  uint8_t* wv = wk + kSaWarpRows * 256;
-  // q.K mapping: four lanes per token (tq = lane / 4, quarter = lane % 4); step i of a lane reads chunk
-  // 4*quarter + ((i + quarter + tq) & 3).  A quarter-warp covers an even and an odd token; the rows are
-  // 256 bytes apart (the same banks), and with this order the two tokens' four chunks fall on
-  // complementary 16-byte bank groups, so the 8 lanes hit 8 different ones.
-  const int tq = lane >> 2;
-  const int quarter = lane & 3;
-  uint4 qpk[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) qpk[i] = s_q[4 * quarter + ((i + quarter + tq) & 3)];
-  constexpr int kGroups = (kSaWarpRows + 7) / 8;   // groups of 8 rows per round
-  for (int done = 0; done < my_total; done += kSaWarpRows) {
-    const int my_rows = min(kSaWarpRows, my_total - done);
-    if (done > 0) __syncwarp();   // every lane has read the rows of the round before
-    // 16-byte asynchronous copies, a half-warp per 256-byte row: all K rows of the round as one group, then
-    // all V rows as a second one, so that the logits are formed while the V rows are still on their way.
-    {
-      const int half = lane >> 4, l16 = lane & 15;
-#pragma unroll
-      for (int kv = 0; kv < 2; ++kv) {
-        for (int r = half; r < my_rows; r += 2) {
-          const unsigned slot = static_cast<unsigned>(s_list[my_first + done + r]);
-          unsigned page, e;
-          if (p.ps_shift >= 0) {
-            page = slot >> p.ps_shift;
-            e = slot & (ps - 1);
-          } else {
-            page = slot / ps;
-            e = slot - page * ps;
-          }
-          const T* src = kvp + (static_cast<int64_t>(page * (2 * ps) + e) * H + head_kv) * kHeadDim + (kv ? v_delta : 0);
-          cp_async_16((kv ? wv : wk) + r * 256 + l16 * 16, src + l16 * 8);
-        }
+  if (my_total > 0) {
+    const int64_t row_elems = static_cast<int64_t>(H) * kHeadDim, v_delta = p.page_size * row_elems;
+    const T* kbase = static_cast<const T*>(kv_base) + head_kv * kHeadDim;
+    // K rows as one commit group, V rows as a second: the logits are formed while the V rows are still on their way
+    auto request = [&](int done, uint8_t* tile) {
+      if (done < my_total) {
+        // (lanes beyond the rows borrow the last one)
+        const unsigned slot = static_cast<unsigned>(s_list[my_first + min(done + (lane & 15), my_total - 1)]);
+        const unsigned page = p.ps_shift >= 0 ? slot >> p.ps_shift : slot / ps;
+        const int row = static_cast<int>(slot + page * ps);   // page * 2 ps + entry
+        tile_copy<T, true, false>(kbase, v_delta, row_elems, row, tile, lane);
+        cp_async_commit();
+        tile_copy<T, false, true>(kbase, v_delta, row_elems, row, tile, lane);
+      } else {
         cp_async_commit();
       }
-    }
-    cp_async_wait<1>();
-    __syncwarp();
-    float logit[kGroups];
+      cp_async_commit();
+    };
 #pragma unroll
-    for (int g = 0; g < kGroups; ++g) {
-      const int row = g * 8 + tq;
-      const bool live = row < my_rows;
-      float acc = 0.f;
-      if (live) {
+    for (int i = 0; i < kSaSlots; ++i) request(i * kTileRows, tiles + i * kTileBytes);
+    uint4 q[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int lc = 4 * quarter + ((i + quarter + tq) & 3);
-          const uint4 kk = *reinterpret_cast<const uint4*>(wk + row * 256 + lc * 16);
-          acc = Elem<T>::dot2(qpk[i].x, kk.x, acc);
-          acc = Elem<T>::dot2(qpk[i].y, kk.y, acc);
-          acc = Elem<T>::dot2(qpk[i].z, kk.z, acc);
-          acc = Elem<T>::dot2(qpk[i].w, kk.w, acc);
-        }
+    for (int j = 0; j < 4; ++j) q[j] = lane < 4 ? sh.q[4 * j + lane] : make_uint4(0, 0, 0, 0);
+    int use = 0;
+    for (int done = 0; done < my_total; done += kTileRows) {
+      uint8_t* tile = tiles + use * kTileBytes;
+      float sc[4];
+      cp_async_wait<2 * kSaSlots - 1>();
+      __syncwarp();
+      tile_logits<T>(tile, q, (1u << min(kTileRows, my_total - done)) - 1u, p.scale_log2, lane, sc);
+      cp_async_wait<2 * kSaSlots - 2>();
+      __syncwarp();
+      // softmax in base 2 (the head's logits are in lanes 0 .. 3: tokens 2t, 2t + 1, 2t + 8, 2t + 9) and P.V with four
+      // dimensions per lane: one query row leaves the matrix form an eighth used and its accumulators cost 28 registers
+      float m_new = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
+      m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
+      m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
+      m_new = fmaxf(m_run, __shfl_sync(0xffffffffu, m_new, 0));   // finite: the tile's first token exists
+      const float rescale = exp2f(m_run - m_new);
+      m_run = m_new;
+      l_run *= rescale;
+      acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
+      float pr[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) pr[u] = exp2f(sc[u] - m_new);
+      l_run += (pr[0] + pr[1]) + (pr[2] + pr[3]);
+      const uint8_t* vbase = tile + kTileRows * 256 + (lane & 1) * 8;
+#pragma unroll
+      for (int j = 0; j < kTileRows; ++j) {
+        const float pj = __shfl_sync(0xffffffffu, pr[(j & 1) + 2 * (j >> 3)], (j & 7) >> 1);
+        const uint2 vv = *reinterpret_cast<const uint2*>(vbase + j * 256 + (((lane >> 1) ^ tile_swizzle(j)) << 4));
+        const float2 a = Elem<T>::to_f2(vv.x), b = Elem<T>::to_f2(vv.y);
+        acc.x = fmaf(pj, a.x, acc.x);
+        acc.y = fmaf(pj, a.y, acc.y);
+        acc.z = fmaf(pj, b.x, acc.z);
+        acc.w = fmaf(pj, b.y, acc.w);
       }
-      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-      logit[g] = live ? acc * p.scale_log2 : -INFINITY;
+      __syncwarp();   // the tile may be filled again
+      request(done + kSaSlots * kTileRows, tile);
+      use = use + 1 == kSaSlots ? 0 : use + 1;
     }
     cp_async_wait<0>();
-    __syncwarp();
-#pragma unroll
-    for (int g = 0; g < kGroups; ++g) {
-      const int base = g * 8;
-      if (base >= my_rows) break;   // warp-uniform
-      const bool live = base + tq < my_rows;
-      float m_new = logit[g];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
-      m_new = fmaxf(m_new, m_run);      // finite: the first row of a group is live
-      const float rescale = (m_run == -INFINITY) ? 0.f : exp2f(m_run - m_new);
-      const float pr = live ? exp2f(logit[g] - m_new) : 0.f;
-      float psum = quarter == 0 ? pr : 0.f;
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, o);
-      l_run = l_run * rescale + psum;
-      m_run = m_new;
-#pragma unroll
-      for (int d = 0; d < 4; ++d) o_acc[d] *= rescale;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, pr, 4 * j);
-        if (pj != 0.f) {   // warp-uniform; rows past the end are stale
-          const uint2 vv = *reinterpret_cast<const uint2*>(wv + (base + j) * 256 + lane * 8);
-          const float2 a = Elem<T>::to_f2(vv.x), b = Elem<T>::to_f2(vv.y);
-          o_acc[0] = fmaf(pj, a.x, o_acc[0]);
-          o_acc[1] = fmaf(pj, a.y, o_acc[1]);
-          o_acc[2] = fmaf(pj, b.x, o_acc[2]);
-          o_acc[3] = fmaf(pj, b.y, o_acc[3]);
-        }
-      }
-    }
   }
 
   // ---- merge: warps -> block -> head ----------------------------------------------------------------------
-  // a warp parks its partial output in its own K rows, which nobody else touches
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);   // (lanes 0 .. 3)
+  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   __syncwarp();
-  reinterpret_cast<float4*>(wk)[lane] = make_float4(o_acc[0], o_acc[1], o_acc[2], o_acc[3]);
+  reinterpret_cast<float4*>(tiles)[lane] = acc;
   if (lane == 0) {
     sh.ml[warp][0] = m_run;
     sh.ml[warp][1] = l_run;
   }
   __syncthreads();
-  {
-    // all 512 threads: thread (part = tid / 128, d = tid % 128) folds the partials of warps 4*part .. 4*part+3
-    // for output d; the four parts are added by the first 128 threads
-    float M = -INFINITY;
+  float od = 0.f, L = 0.f, M = -INFINITY;
 #pragma unroll
-    for (int w2 = 0; w2 < kSaWarps; ++w2) M = fmaxf(M, sh.ml[w2][0]);
-    const int d = tid & (kHeadDim - 1), part = tid >> 7;
-    float od = 0.f, L = 0.f;
+  for (int w2 = 0; w2 < kSaWarps; ++w2) M = fmaxf(M, sh.ml[w2][0]);
 #pragma unroll
-    for (int j = 0; j < kSaWarps / 4; ++j) {
-      const int w2 = part * (kSaWarps / 4) + j;
-      const float m = sh.ml[w2][0];
-      const float w = (m == -INFINITY) ? 0.f : exp2f(m - M);
-      L += w * sh.ml[w2][1];
-      if (w != 0.f) od += w * reinterpret_cast<const float*>(sa_tile + w2 * (2 * kSaWarpRows * 256))[d];
-    }
-    float* fold = reinterpret_cast<float*>(sa_tile + kSaWarpRows * 256);   // [4][130], in warp 0's V rows (free by now)
-    fold[part * 130 + d] = od;
-    if (d == 0) fold[part * 130 + kHeadDim] = L;
-    __syncthreads();
-    if (tid < kHeadDim) {
-      float* slot = slots + cr * kSaSlotWords;
-      __stcg(slot + tid, (fold[tid] + fold[130 + tid]) + (fold[260 + tid] + fold[390 + tid]));
-      if (tid == 0) {
-        __stcg(slot + kHeadDim, M);
-        __stcg(slot + kHeadDim + 1, (fold[kHeadDim] + fold[130 + kHeadDim]) + (fold[260 + kHeadDim] + fold[390 + kHeadDim]));
-      }
-    }
+  for (int w2 = 0; w2 < kSaWarps; ++w2) {
+    const float m = sh.ml[w2][0];
+    const float w = (m == -INFINITY) ? 0.f : exp2f(m - M);
+    L += w * sh.ml[w2][1];
+    od += w * reinterpret_cast<const float*>(sa_smem + w2 * (kSaSlots * kTileBytes))[tid];
   }
-  // the block that arrives last at the head's counter merges; nobody waits.  The block barrier orders
-  // the slot stores of all threads before thread 0's release at the counter; the last block's acquire
-  // there, followed by the second barrier, orders its loads of the slots after every block's stores.
   unsigned* counter = head_scratch + kSaMaxSlices * kSaBins + kHeadDim + 2;   // word 130 of slot 0
-  __syncthreads();
-  if (tid == 0) {
-    unsigned ticket;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
-    sh.last = (ticket == CL - 1) ? 1u : 0u;
-  }
-  __syncthreads();
-  if (!sh.last) return;
-  // every block of the head has read the histograms long ago: clear them and the counter for the next launch
-#pragma unroll
-  for (unsigned r = 0; r < kSaMaxSlices; ++r)
-    if (r < CL) head_scratch[r * kSaBins + tid] = 0u;
-  if (tid == 0) *counter = 0u;
-  // (every block of the head has read the un-rotated query long ago)
-  if (p.rope_on && tid < 16)
-    st_16(static_cast<T*>(const_cast<void*>(p.q)) + static_cast<int64_t>(head) * kHeadDim + tid * 8, s_q[tid]);
-  if (tid >= kHeadDim) return;
-  // all loads of the CL partials are issued before the first is used: one trip to L2
-  float pm[kSaMaxSlices], pl[kSaMaxSlices], po[kSaMaxSlices];
-#pragma unroll
-  for (unsigned r = 0; r < kSaMaxSlices; ++r) {
-    pm[r] = -INFINITY;
-    pl[r] = 0.f;
-    po[r] = 0.f;
-    if (r < CL) {
-      pm[r] = __ldcg(slots + r * kSaSlotWords + kHeadDim);
-      pl[r] = __ldcg(slots + r * kSaSlotWords + kHeadDim + 1);
-      po[r] = __ldcg(slots + r * kSaSlotWords + tid);
+  if (CL > 1) {
+    float* slot = slots + cr * kSaSlotWords;
+    __stcg(slot + tid, od);
+    if (tid == 0) __stcg(reinterpret_cast<float2*>(slot + kHeadDim), make_float2(M, L));
+    // the block that arrives last at the head's counter merges; nobody waits.  The block barrier orders
+    // the slot stores of all threads before thread 0's release at the counter; the last block's acquire
+    // there, followed by the second barrier, orders its loads of the slots after every block's stores.
+    __syncthreads();
+    if (tid == 0) {
+      unsigned ticket;
+      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
+      sh.last = (ticket == CL - 1) ? 1u : 0u;
     }
-  }
-  float M = -INFINITY;
+    __syncthreads();
+    if (!sh.last) return;
+    // lane r of every warp takes block r's (max, sum); all loads of the partials are issued before the first is used
+    float2 ml = make_float2(-INFINITY, 0.f);
+    if (lane < static_cast<int>(CL)) ml = __ldcg(reinterpret_cast<const float2*>(slots + lane * kSaSlotWords + kHeadDim));
+    float po[kSaMaxSlices];
 #pragma unroll
-  for (unsigned r = 0; r < kSaMaxSlices; ++r) M = fmaxf(M, pm[r]);
-  float accd = 0.f, L = 0.f;
+    for (unsigned r = 0; r < kSaMaxSlices; ++r) po[r] = r < CL ? __ldcg(slots + r * kSaSlotWords + tid) : 0.f;
+    M = ml.x;
 #pragma unroll
-  for (unsigned r = 0; r < kSaMaxSlices; ++r) {
-    const float w = (pm[r] == -INFINITY) ? 0.f : exp2f(pm[r] - M);
-    L += w * pl[r];
-    if (w != 0.f) accd += w * po[r];
+    for (int o = 1; o < kSaMaxSlices; o <<= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+    const float w = (ml.x == -INFINITY) ? 0.f : exp2f(ml.x - M);
+    L = w * ml.y;
+#pragma unroll
+    for (int o = 1; o < kSaMaxSlices; o <<= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+    // (lanes 16 .. 31 hold no block)
+    M = __shfl_sync(0xffffffffu, M, 0);
+    L = __shfl_sync(0xffffffffu, L, 0);
+    od = 0.f;
+#pragma unroll
+    for (unsigned r = 0; r < kSaMaxSlices; ++r) od = fmaf(__shfl_sync(0xffffffffu, w, r), po[r], od);
   }
-  const float res = L > 0.f ? accd / L : 0.f;
+  const float res = L > 0.f ? od / L : 0.f;
   const float res1 = __shfl_down_sync(0xffffffffu, res, 1);
   if (p.o_f32) p.o_f32[static_cast<int64_t>(head) * kHeadDim + tid] = res;
   if (p.o && (tid & 1) == 0)
     reinterpret_cast<uint32_t*>(static_cast<T*>(p.o) + static_cast<int64_t>(head) * kHeadDim)[tid >> 1] =
         Elem<T>::from_f2(res, res1);
   if (tid == 0 && p.lse) p.lse[head] = L > 0.f ? M + log2f(L) : -INFINITY;
+  // every block of the head has read the histograms and the un-rotated query long ago: clear the table and the counter
+  // for the next launch
+  for (unsigned r = 0; r < CL; ++r) reinterpret_cast<uint4*>(head_scratch)[r * (kSaBins / 4) + tid] = make_uint4(0u, 0u, 0u, 0u);
+  if (tid == 0) *counter = 0u;
+  if (p.rope_on && tid < 16)
+    st_16(static_cast<T*>(const_cast<void*>(p.q)) + static_cast<int64_t>(head) * kHeadDim + tid * 8, sh.q[tid]);
 }
 
 // Per-slice histograms of distance rows, for callers of select_attend that did not get them from an
@@ -577,7 +521,7 @@ struct DistHistogramParams {
 // already (the stand-alone select_attend call) and, in the fused step, for launches with so many distances
 // that one L2 atomic per distance from inside the estimate would bound it (3 M and more per launch): a
 // block counts its slice in shared memory and stores 512 totals.
-__global__ void __launch_bounds__(kSaThreads) dist_histogram_kernel(const DistHistogramParams p) {
+__global__ void __launch_bounds__(kSaBins) dist_histogram_kernel(const DistHistogramParams p) {
   __shared__ unsigned h_local[kSaBins];
   const int tid = threadIdx.x;
   const int r = blockIdx.x;
@@ -591,7 +535,7 @@ __global__ void __launch_bounds__(kSaThreads) dist_histogram_kernel(const DistHi
   const int gpb = sa_granules_per_block(n, p.cl);
   const int g_end = min(G, (r + 1) * gpb);
   const uint4* gbase = reinterpret_cast<const uint4*>(p.dist + static_cast<int64_t>(head) * p.dist_stride);
-  for (int g = r * gpb + tid; g < g_end; g += kSaThreads) {
+  for (int g = r * gpb + tid; g < g_end; g += kSaBins) {
     const uint4 v = ld_16(gbase + g);
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     const int valid = min(8, n - g * 8);
