@@ -84,6 +84,8 @@ int check_q_heads(int num_heads, int num_q_heads) {
 }
 
 constexpr int kEstStatic = 6144;   // static shared memory of the estimate kernels, rounded up
+constexpr int kSaStatic = 1024;             // static shared memory of select_attend_kernel, rounded up
+constexpr int kSaMaxPageBytes = 4096;       // page numbers of a block that are staged in shared memory at most
 constexpr int kSaMaxDynSmem = 160 * 1024;   // dynamic shared memory select_attend may ask for (a long winner list)
 
 constexpr int kDecSmem = kDecWarps * kDecStages * kDecTileBytes;
@@ -784,7 +786,7 @@ namespace {
 // Shape of a paged_decode launch over `batch` sequences of (up to) n_tokens tokens.  shared_list: all query heads
 // of a cache head attend to the same tokens (the dense layers), so they go through the tiles together.
 struct DecPlan {
-  int row_heads, row_to_kv, group, subs, gs, splits;
+  int row_heads, row_to_kv, group, subs, gs, splits, slots;
   unsigned blocks;
 };
 
@@ -802,21 +804,10 @@ DecPlan plan_decode(int64_t n_tokens, int batch, int kv_heads, int q_heads, bool
   d.group = shared_list ? g : 1;
   d.gs = dec_group_part(d.group);
   d.subs = (d.group + d.gs - 1) / d.gs;
-  const int64_t tiles = (n_tokens + kDecTile - 1) / kDecTile;
-  const int64_t rows = static_cast<int64_t>(batch) * d.row_heads * d.subs;
-  d.splits = 0;
-  const int64_t slots = static_cast<int64_t>(kDecBlocksPerSm) * num_sms;
-  if (rows <= slots && rows * tiles < slots * kDecWarps * 4) {
-    // little work: latency counts, so a block gets a share of ONE row (a second row in a block would be a second
-    // pass through index list, rows and merge)
-    // (a group of query heads has as many results to merge per part: half as many parts; measured at 28 query heads
-    // over 4 x 2001 tokens: 11.9 us with 6 tiles per block, 10.7 with 12; one query head per row, 512 tokens: 7.4 / 8.3)
-    const int min_tiles = d.gs > 1 ? 2 * kDecMinTiles : kDecMinTiles;
-    d.splits = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(slots / rows, (tiles + min_tiles - 1) / min_tiles)));
-    d.blocks = static_cast<unsigned>(rows * d.splits);
-    return d;
-  }
-  d.blocks = static_cast<unsigned>(kDecBlocksPerSm * num_sms);
+  const int rows = batch * d.row_heads * d.subs, tiles = static_cast<int>((n_tokens + kDecTile - 1) / kDecTile);
+  d.slots = kDecBlocksPerSm * num_sms;
+  d.splits = dec_splits(rows, tiles, d.gs, d.slots);
+  d.blocks = static_cast<unsigned>(d.splits > 0 ? rows * d.splits : d.slots);
   return d;
 }
 
@@ -937,6 +928,7 @@ static int launch_decode(const DecPlan& d, const void* q, void* o, float* o_f32,
   prm.tail_slot0 = tail_slot0;
   prm.n_tokens = static_cast<int>(n_tokens);
   prm.splits = d.splits;
+  prm.slots = d.slots;
   prm.partial_o = static_cast<float*>(partial_o);
   prm.partial_ml = static_cast<float*>(partial_ml);
   prm.counters = static_cast<unsigned*>(counters);
@@ -1086,14 +1078,33 @@ int launch_select_attend(const SelectAttendParams& prm, int cl, int num_heads, i
   return check_launch("select_attend_kernel");
 }
 
-// Shape of a select_attend launch: blocks per head (= histogram slices), winner list and dynamic shared memory (the tiles |
-// winner list).  Planned for rows of up to n distances; shorter rows run in the same shape.
+// Shape of a select_attend launch: blocks per head, histogram slices, and dynamic shared memory (the tiles | winner list |
+// page numbers).  Planned for rows of up to n distances; shorter rows run in the same shape.
 struct SaPlan {
-  int cl, list_capacity;
+  int cl, slices, tokens, list_capacity, staged_granules, pages_at;   // tokens: of a block at most
   size_t smem;
 };
 
-int sa_plan(int n, int k, int num_heads, const DeviceInfo* di, SaPlan* pl) {
+// For `cl` blocks per head: everything but the staged page numbers.
+void sa_shape(int n, int k, int cl, SaPlan* pl) {
+  pl->cl = cl;
+  // Every block reads every histogram slice of its head, 2 KB each: with 16 blocks and slices of 32 heads 17 MB from L2, 1.8 us.
+  // Two blocks share a slice where the second one can count what lies in front of it in a few instructions.
+  pl->slices = cl >= 8 && cl % 2 == 0 && sa_granules_per_block(n, cl / 2) <= 4 * kSaThreads ? cl / 2 : cl;
+  const int granules = sa_granules_per_block(n, pl->slices), sharing = cl / pl->slices;
+  pl->tokens = std::min(n, (granules + sharing - 1) / sharing * 8);
+  pl->list_capacity = std::min(k, pl->tokens) + 1;   // winners of one block at most, plus the newest token
+  pl->staged_granules = std::min(granules, kSaTileBytes / 16 / 9 * 8);   // (one in nine places is padding)
+  pl->smem = static_cast<size_t>(kSaTileBytes + ((pl->list_capacity * 2 + 15) & ~15));
+  pl->pages_at = 0;
+}
+
+int sa_resident(size_t smem, const DeviceInfo* di) {   // blocks per SM
+  return std::min<int>(kSaBlocksPerSm, static_cast<int>(di->smem_per_sm / (smem + 1024 + kSaStatic)));
+}
+
+// (page_size plays no part in the number of blocks and slices: adamas_select_attend_slices does not know it)
+int sa_plan(int n, int k, int num_heads, int page_size, const DeviceInfo* di, SaPlan* pl) {
   // Blocks per head: any number up to 16 (the blocks of a head do not wait for one another).  num_heads counts the rows of
   // the launch (query heads x sequences).  A block's work is a chain of short dependent steps, so what counts is that
   // a block's winners fit the tiles of its warps, that a thread has a granule or two, and that the whole launch is
@@ -1104,13 +1115,18 @@ int sa_plan(int n, int k, int num_heads, const DeviceInfo* di, SaPlan* pl) {
   const int least = (n + kSaMaxBlockTokens - 1) / kSaMaxBlockTokens;
   ADAMAS_REQUIRE(least <= cl_limit, "select_attend supports at most %d distances per head with %d blocks per head (got %d)",
                  cl_limit * kSaMaxBlockTokens, cl_limit, n);
-  const int winners = kSaWarps * kSaSlots * kTileRows * 3 / 4;
-  const int wanted = std::max((g_total + 2 * kSaThreads - 1) / (2 * kSaThreads), (k + winners - 1) / winners);
-  const int resident = std::max(1, kSaBlocksPerSm * di->num_sms / num_heads);
-  pl->cl = std::min(std::max(std::min(wanted, resident), least), cl_limit);
-  const int slice_tokens = std::min(n, sa_granules_per_block(n, pl->cl) * 8);
-  pl->list_capacity = std::min(k, slice_tokens) + 1;   // winners of one block at most, plus the newest token
-  pl->smem = static_cast<size_t>(kSaTileBytes) + ((static_cast<size_t>(pl->list_capacity) * 4 + 15) & ~static_cast<size_t>(15));
+  const int winners = kSaWarps * kSaRows * 3 / 4;   // (the slices' shares differ)
+  int wanted = std::max((g_total + 2 * kSaThreads - 1) / (2 * kSaThreads), (k + winners - 1) / winners);
+  if (wanted >= 8) wanted = (wanted + 1) & ~1;   // (two blocks then share a slice)
+  for (int cl = std::min(std::max(wanted, least), cl_limit);; --cl) {
+    sa_shape(n, k, cl, pl);
+    if (cl == std::max(least, 1) || cl * num_heads <= sa_resident(pl->smem, di) * di->num_sms) break;
+  }
+  const int page_bytes = ((pl->tokens / page_size + 2) * 4 + 15) & ~15;
+  if (page_bytes <= kSaMaxPageBytes && sa_resident(pl->smem + page_bytes, di) == sa_resident(pl->smem, di)) {
+    pl->pages_at = static_cast<int>(pl->smem);
+    pl->smem += page_bytes;
+  }
   ADAMAS_REQUIRE(pl->smem <= static_cast<size_t>(kSaMaxDynSmem), "winner list too long for select_attend (k=%d)", k);
   return ADAMAS_OK;
 }
@@ -1122,7 +1138,7 @@ int select_attend_impl(const void* dist, int64_t dist_stride, int n, int k, cons
                        int q_heads, int dtype, int tail_mode, unsigned tail_slot, uint32_t* hist, const int32_t* ext_cut,
                        const int32_t* seq_len_dev, int32_t* out_idx, int64_t out_stride, float sm_scale,
                        const SaPlan& pl, adamas_stream_t stream, const SeqDesc* seqs = nullptr, int batch = 1,
-                       const RopeSpec* rope_q = nullptr) {
+                       const RopeSpec* rope_q = nullptr, int dist_bins = kSaBins) {
   SelectAttendParams prm;
   prm.rope_on = rope_q != nullptr && rope_q->on;
   prm.rope = RopeParams{1.f, 1e4f, nullptr, 1.f};
@@ -1152,6 +1168,10 @@ int select_attend_impl(const void* dist, int64_t dist_stride, int n, int k, cons
   prm.out_idx = out_idx;
   prm.out_stride = out_stride;
   prm.list_capacity = pl.list_capacity;
+  prm.slices = pl.slices;
+  prm.staged_granules = pl.staged_granules;
+  prm.pages_at = pl.pages_at;
+  prm.bin_threads = dist_bins > 3 * kHeadDim ? kSaThreads : (3 * kHeadDim + 4) / 4;
   prm.scale_log2 = sm_scale * 1.4426950408889634f;
   if (dtype == ADAMAS_F16)
     return launch_select_attend<__half>(prm, pl.cl, q_heads, batch, pl.smem, to_stream(stream));
@@ -1177,8 +1197,8 @@ int adamas_select_attend_slices(int n, int k, int num_heads, int* slices) {
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
   SaPlan pl;
-  if (int rc = sa_plan(n, k, num_heads, di, &pl)) return rc;
-  *slices = pl.cl;
+  if (int rc = sa_plan(n, k, num_heads, 16, di, &pl)) return rc;
+  *slices = pl.slices;
   return ADAMAS_OK;
 }
 
@@ -1207,16 +1227,16 @@ int adamas_select_attend(const void* dist, int64_t dist_stride, int n, int k, co
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
   SaPlan pl;
-  if (int rc = sa_plan(n, k, num_heads, di, &pl)) return rc;
+  if (int rc = sa_plan(n, k, num_heads, page_size, di, &pl)) return rc;
   if (!hist_ready) {
     DistHistogramParams hp;
     hp.dist = static_cast<const uint16_t*>(dist);
     hp.dist_stride = dist_stride;
     hp.hist = hist;
     hp.n = n;
-    hp.cl = pl.cl;
+    hp.cl = pl.slices;
     hp.seq_len_dev = nullptr;
-    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.cl, num_heads), dim3(kSaBins), 0,
+    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.slices, num_heads), dim3(kSaBins), 0,
                   to_stream(stream), 1, hp);
   }
   return select_attend_impl(dist, dist_stride, n, k, q, o, o_f32, lse, kv_data, kv_page_table, page_size, kv_heads,
@@ -1355,7 +1375,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
   SaPlan pl;
-  if (int rc = sa_plan(n, budget - 1, q_heads * batch, di, &pl)) return rc;
+  if (int rc = sa_plan(n, budget - 1, q_heads * batch, page_size, di, &pl)) return rc;
   int rc;
   // The histogram counts.  Tile pipeline: one L2 atomic per distance from inside the estimate, or, for launches with 3 M
   // distances and more (a 128K context of 32 heads, three 32K sequences), a launch of their own that counts in shared
@@ -1367,7 +1387,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
     // two launches: the estimate with the append (and, with RoPE, the rotation) inside, then select + attend
     rc = estimate_append_launch(q, k, v, q_code, kv_data, kv_page_table, pages, last_len, code_data,
                                 code_page_table, pages, last_len, n, num_heads, q_heads, page_size, dtype, dist_scratch,
-                                dist_stride, hadamard_scale, thresholds3_host, seq_len_dev, est_hist, pl.cl, stream, seqs,
+                                dist_stride, hadamard_scale, thresholds3_host, seq_len_dev, est_hist, pl.slices, stream, seqs,
                                 batch, rope);
     if (rc) return rc;
   } else {
@@ -1376,7 +1396,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
                             thresholds3_host, dtype, stream, rope, seq_len_dev, q_heads, seqs, batch);
     if (rc) return rc;
     rc = launch_estimate(q_code, StepAppend{}, dtype, code_data, code_page_table, n, page_size, num_heads, q_heads, dist_scratch,
-                         dist_stride, ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, est_hist, pl.cl, stream, seqs, batch);
+                         dist_stride, ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, est_hist, pl.slices, stream, seqs, batch);
     if (rc) return rc;
   }
   if (count_apart) {
@@ -1385,9 +1405,9 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
     hp.dist_stride = dist_stride;
     hp.hist = hist;
     hp.n = n;
-    hp.cl = pl.cl;
+    hp.cl = pl.slices;
     hp.seq_len_dev = seq_len_dev;
-    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.cl, q_heads, batch), dim3(kSaBins), 0,
+    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.slices, q_heads, batch), dim3(kSaBins), 0,
                   to_stream(stream), 1, hp);
     if (int rc2 = check_launch("dist_histogram_kernel")) return rc2;
   }
@@ -1395,7 +1415,8 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   rc = select_attend_impl(dist_scratch, dist_stride, n, budget - 1, q, o, nullptr, lse, kv_data, kv_page_table,
                           page_size, num_heads, q_heads, dtype, seq_len_dev ? 2 : 1, static_cast<unsigned>(tail), hist, nullptr,
                           seq_len_dev, out_idx, out_stride, sm_scale, pl, stream, seqs, batch,
-                          two_launches ? &rope : nullptr);   // (after a separate append q is rotated already)
+                          two_launches ? &rope : nullptr,    // (after a separate append q is rotated already)
+                          3 * kHeadDim);   // (an estimate's distances are at most 384)
   if (rc) {
     // the estimate has filled the histogram table and nothing will clear it: restore the all-zero state
     cudaMemsetAsync(hist, 0, hist_bytes(q_heads * batch), to_stream(stream));

@@ -1,7 +1,6 @@
-// A warp's attention over a tile of 16 gathered K and V rows, on the tensor cores (mma.sync m16n8k16, fp32
+// A warp's attention over a tile of 16 (or 24) gathered K and V rows, on the tensor cores (mma.sync m16n8k16, fp32
 // accumulation): up to 8 query rows at once.  Used by the decode attention (all query heads of a cache head) and by
-// select+attend (one query row, an eighth of the instruction's width: still about half of the instructions of a
-// multiply-add form).
+// select+attend (one query row: q.K only).
 //
 // The order of the 128 dimensions is free in q.K, and of the output rows in P.V, so every lane reads whole 16-byte
 // chunks: chunk 4j + t of K rows g and g + 8, chunks g and 8 + g of V rows 2t, 2t + 1, 2t + 8, 2t + 9 (g = lane / 4,
@@ -50,47 +49,47 @@ __device__ __forceinline__ int tile_swizzle(int r) { return (r & 6) ^ ((r & 1) <
 
 __device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// Requests the tile's K and / or V rows with 16-byte asynchronous copies: lane l (and l + 16) holds the cache row of token
-// l, in units of row_elems elements behind kbase; its V row lies v_delta elements behind its K row.
-template <typename T, bool K, bool V>
+// Requests a tile's K and / or V rows with 16-byte asynchronous copies: lane l holds the cache row of token l (of 16 tokens:
+// lanes l and l + 16), in units of row_elems elements behind kbase; its V row lies v_delta elements behind its K row.
+template <typename T, int ROWS, bool K, bool V>
 __device__ __forceinline__ void tile_copy(const T* kbase, int64_t v_delta, int64_t row_elems, int row, uint8_t* slot, int lane) {
   const int half = lane >> 4, c = lane & 15;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {   // a half-warp per row
+  for (int i = 0; i < ROWS / 2; ++i) {   // a half-warp per row
     const int rr = 2 * i + half;
     const T* src = kbase + __shfl_sync(0xffffffffu, row, rr) * row_elems + c * 8;
     uint8_t* dst = slot + rr * 256 + ((c ^ tile_swizzle(rr)) << 4);
     if (K) cp_async_16(dst, src);
-    if (V) cp_async_16(dst + kTileRows * 256, src + v_delta);
+    if (V) cp_async_16(dst + ROWS * 256, src + v_delta);
   }
 }
 
-// Scaled logits of the tile: S[head g][tokens 2t, 2t + 1, 2t + 8, 2t + 9] in this lane; -inf for tokens outside `mask`.
-template <typename T>
+// Scaled logits of a tile of ROWS tokens: s[2u], s[2u + 1] are head g's for tokens 8u + 2t, 8u + 2t + 1; -inf for tokens
+// outside `mask`.
+template <typename T, int ROWS>
 __device__ __forceinline__ void tile_logits(const uint8_t* slot, const uint4 (&q)[4], unsigned mask, float scale_log2, int lane,
-                                            float (&s)[4]) {
+                                            float (&s)[ROWS / 4]) {
   const int g = lane >> 2, t = lane & 3;
-  float c[2][2][4] = {};   // [rows g, g + 8][two accumulators: shorter chains]
+  float c[ROWS / 8][2][4] = {};   // (two accumulators per 8 rows: shorter chains)
   const uint8_t* krow = slot + g * 256;
   const int ksw = tile_swizzle(g);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < ROWS / 8; ++u) {
       const uint4 k = *reinterpret_cast<const uint4*>(krow + u * 2048 + (((4 * j + t) ^ ksw) << 4));
       Mma<T>::run(c[u][0], q[j].x, 0u, q[j].y, 0u, k.x, k.y);
       Mma<T>::run(c[u][1], q[j].z, 0u, q[j].w, 0u, k.z, k.w);
     }
   }
-  s[0] = c[0][0][0] + c[0][1][0];
-  s[1] = c[0][0][1] + c[0][1][1];
-  s[2] = c[1][0][0] + c[1][1][0];
-  s[3] = c[1][0][1] + c[1][1][1];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) s[u] = (mask >> (2 * t + (u & 1) + 8 * (u >> 1))) & 1u ? s[u] * scale_log2 : -INFINITY;
+  for (int u = 0; u < ROWS / 4; ++u) {
+    const int tok = 8 * (u >> 1) + 2 * t + (u & 1);
+    s[u] = (mask >> tok) & 1u ? (c[u >> 1][0][u & 1] + c[u >> 1][1][u & 1]) * scale_log2 : -INFINITY;
+  }
 }
 
-// Softmax in base 2 and P.V over the tile; at least one token must exist, and rows of absent ones must hold finite values.
+// Softmax in base 2 and P.V over a tile of 16 tokens; at least one token must exist, and rows of absent ones must hold finite values.
 template <typename T>
 __device__ __forceinline__ void tile_softmax_pv(TileState& st, const uint8_t* slot, const float (&s)[4], int lane) {
   const int g = lane >> 2, t = lane & 3;

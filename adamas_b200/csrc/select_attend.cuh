@@ -18,13 +18,19 @@
 //          derives this by itself from the same table: no exchange between blocks;
 //   pick   ordered compaction of the block's winners into a list in shared memory;
 //   attend the rows of the list are dealt out evenly to the 4 warps; a warp gathers the K and V rows of
-//          its tokens itself, 16 at a time (16-byte asynchronous copies into its own tile), and works on
+//          its tokens itself, 24 at a time (16-byte asynchronous copies into its own tile), and works on
 //          them alone (q.K on the tensor cores, attend_tile.cuh): no block barrier inside the attention;
 //   merge  the 4 warps' partial (o, m, l) are merged in shared memory and the block's partial goes to
 //          the head's slot table in global scratch; the block that arrives LAST at the head's counter
 //          merges the CL partials, writes the head's output, clears the head's histogram rows and the
 //          counter.  Every other block is gone by then.
-// BOUNDTEXT
+// Bound: a chain of short dependent phases for one sequence, HBM (the gathered rows) for the longest of them; latency times
+// rows in flight for batches.  Blocks are therefore small: four to an SM, so that the chains of different rows overlap, and
+// up to 16 to a row, so that a block's winners fit its warps' tiles in one round and a thread has a granule or two.  What
+// does not depend on the preceding kernel (length, page numbers, rotation table) is done before its completion.
+// Measured, the whole step: blocks of 512 threads with the distances in registers, two to an SM, took 22.7 us per layer for
+// one sequence (32 heads, 32K tokens, budget 1024), 103 us for 8 x 32K and 125 us for 32 x 4-8K; this form 20.7, 79 and 81.
+// (Blocks of 256 threads, three to an SM: 26.0 / - / 122.  16 rows per tile: a second round for half of the warps.)
 #pragma once
 #include "attend_tile.cuh"
 #include "common.cuh"
@@ -32,20 +38,14 @@
 
 namespace adamas {
 
-#ifndef SB
-#define SB 4
-#endif
-#ifndef SS
-#define SS 1
-#endif
 constexpr int kSaThreads = 128;
 constexpr int kSaWarps = kSaThreads / 32;
-constexpr int kSaBlocksPerSm = SB;
+constexpr int kSaBlocksPerSm = 4;
 constexpr int kSaBins = 512;
 constexpr int kSaMaxSlices = 16;      // histogram rows per head = largest number of blocks per head
-constexpr int kSaSlots = SS;          // tiles per warp
-constexpr int kSaTileBytes = kSaWarps * kSaSlots * kTileBytes;
-constexpr int kSaStaged = kSaTileBytes / 16 * 8 / 9 - 8;   // granules of a slice that are staged in the tiles' memory
+constexpr int kSaRows = 24;           // rows of a warp's tile
+constexpr int kSaWarpBytes = 2 * kSaRows * kHeadDim * 2;
+constexpr int kSaTileBytes = kSaWarps * kSaWarpBytes;
 constexpr int kSaMaxBlockTokens = 32768;
 constexpr int kSaMaxCluster = 8;      // upper bound of adamas_set_max_cluster
 
@@ -89,6 +89,10 @@ struct SelectAttendParams {
   unsigned tail_slot;       // physical slot of the newest token (tail_mode 1)
   int32_t* out_idx;         // optional [H, out_stride]: physical slots of the winners, ascending position
   int64_t out_stride;
+  int slices;               // histogram rows per head; gridDim.x / slices (1 or 2) blocks share one
+  int staged_granules;      // granules of a slice staged in the tiles' memory
+  int pages_at;             // where in shared memory the block's page numbers go; 0: they are not staged
+  int bin_threads;          // threads that read histogram bins (four each): the bins that can be in use
   int list_capacity;        // entries of the shared-memory winner list (a block's winners at most, plus the newest token)
   float scale_log2;
   // q arrives un-rotated (the append-fused estimate in front of this launch has coded the rotated query but left
@@ -102,6 +106,7 @@ struct SaShared {
   float ml[kSaWarps][2];
   uint2 warp_sum[kSaWarps];
   unsigned cut, need_eq, lt_before, eq_before;
+  unsigned tail_slot;
   unsigned last;   // this block arrived last at the head's counter
   uint4 q[16];     // the head's query row
   float2 cs[kHeadDim / 2];   // rope_on: (cos, sin) of the position
@@ -129,8 +134,8 @@ __device__ __forceinline__ unsigned sa_in_order(unsigned m) {
   return (x & 0xffu) | ((x >> 7) & 0xaau);
 }
 
-// Dynamic shared memory: the warps' tiles (8 KB each; first the staged distances, at the end a warp parks its partial
-// output in its first tile) | winner list (list_capacity * 4 B).
+// Dynamic shared memory: the warps' tiles (12 KB each; first the staged distances, at the end a warp parks
+// its partial output in its tile) | winner list (list_capacity * 2 B) | page numbers.
 template <typename T>
 __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kernel(const SelectAttendParams p) {
   static_assert(4 * kSaThreads == kSaBins && kSaThreads == kHeadDim, "four histogram bins and one output per thread");
@@ -154,54 +159,62 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     seq_len_dev += blockIdx.z;
   }
 
-  int32_t* s_list = reinterpret_cast<int32_t*>(sa_smem + kSaTileBytes);               // the block's winners, in position order
+  uint16_t* s_list = reinterpret_cast<uint16_t*>(sa_smem + kSaTileBytes);             // the block's winners in position order: tokens behind its first
   uint32_t* head_scratch = p.hist + static_cast<size_t>(head) * kSaScratchWordsPerHead;
   float* slots = reinterpret_cast<float*>(head_scratch + kSaMaxSlices * kSaBins);     // [CL][kSaSlotWords]
 
-  // ---- set-up that needs no input (overlaps the tail of the preceding kernel) -----------------------
+  // ---- set-up that does not depend on the preceding kernel (overlaps its tail) ------------------------
+  // (a device-resident length and the page tables are final before the kernel in front of this one starts)
   if (tid == 0) sh.cut = 0xffffffffu;
+  const int n = seq_len_dev ? (__ldg(seq_len_dev) - 1) : p.n;
+  const int G = (n + 7) >> 3;
+  // slice of the histograms, and this block's part of it (one or two blocks share a slice; the second one counts what lies
+  // in front of it in the first part by itself)
+  const int per_slice = sa_granules_per_block(n, p.slices), sharing = static_cast<int>(CL) / p.slices;
+  const int slice = cr / sharing, part = cr - slice * sharing, per_part = (per_slice + sharing - 1) / sharing;
+  const int seg_first = slice * per_slice, seg_end = min(G, seg_first + per_slice);
+  const int pre = max(0, min(part * per_part, seg_end - seg_first));            // granules of the slice in front of this block's
+  const int blk_first = seg_first + pre, blk_count = max(0, min(per_part, seg_end - blk_first));
+  // the page numbers of the block's tokens, where they fit
+  const unsigned ps = static_cast<unsigned>(p.page_size);
+  auto page_of = [&](unsigned t) { return p.ps_shift >= 0 ? t >> p.ps_shift : t / ps; };
+  int32_t* pages = reinterpret_cast<int32_t*>(sa_smem + p.pages_at);   // (behind the list)
+  const unsigned page0 = page_of(static_cast<unsigned>(blk_first) * 8);
+  const int n_pages = p.pages_at && blk_count > 0 ? static_cast<int>(page_of(min(static_cast<unsigned>(blk_first + blk_count) * 8, static_cast<unsigned>(n)) - 1) - page0) + 1 : 0;
+  for (int i = tid; i < n_pages; i += kSaThreads) pages[i] = __ldg(kv_table + page0 + i);
+  // (rope_on: the position's cos / sin pairs)
+  if (p.rope_on && tid < kHeadDim / 2) sh.cs[tid] = rope_cos_sin(tid, static_cast<float>(n), p.rope);
+  // the newest token rides with the last slice
+  const bool tail_here = p.tail_mode != 0 && cr == CL - 1;
+  if (tail_here && tid == 0) {
+    sh.tail_slot = p.tail_slot;
+    if (p.tail_mode == 2) {
+      const unsigned un = static_cast<unsigned>(n), pg = page_of(un);
+      sh.tail_slot = static_cast<unsigned>(__ldg(kv_table + pg)) * ps + (un - pg * ps);
+    }
+  }
   grid_dependency_wait();
   grid_launch_dependents();
 
-  // ---- loads: distances, histograms, query ------------------------------------------------------------
-  const int n = seq_len_dev ? (__ldg(seq_len_dev) - 1) : p.n;
-  const int G = (n + 7) >> 3;
-  const int gpb = sa_granules_per_block(n, static_cast<int>(CL));
-  const int blk_first = cr * gpb;
-  const int blk_count = max(0, min(G - blk_first, gpb));
-  const uint4* gbase = reinterpret_cast<const uint4*>(p.dist + static_cast<int64_t>(head) * p.dist_stride) + blk_first;
-  uint4* staged = reinterpret_cast<uint4*>(sa_smem);   // granule g at g + g / 8: reads of neighbouring threads' runs do not conflict
+  // ---- loads: histograms, query, distances, all in flight together ------------------------------------
+  const uint4* gbase = reinterpret_cast<const uint4*>(p.dist + static_cast<int64_t>(head) * p.dist_stride) + seg_first;
+  uint4* staged = reinterpret_cast<uint4*>(sa_smem);   // granule g of the slice at g + g / 8: reads of neighbouring threads' runs do not conflict
+  const int n_staged = min(pre + blk_count, p.staged_granules);
   uint4 tot = make_uint4(0u, 0u, 0u, 0u), low = tot;   // bins 4 * tid ..: the whole row; lower-ranked slices
   uint4 qraw = tot;                                    // the query row, 16 lanes x 16 bytes
   {
     const uint4* hrow = reinterpret_cast<const uint4*>(head_scratch) + tid;
-    for (int g = tid; g < min(blk_count, kSaStaged); g += kSaThreads) cp_async_16(staged + g + (g >> 3), gbase + g);
-    cp_async_commit();
+    uint4 c[kSaMaxSlices];
+#pragma unroll
+    for (unsigned r = 0; r < kSaMaxSlices; ++r) c[r] = r < static_cast<unsigned>(p.slices) && tid < p.bin_threads ? __ldcg(hrow + r * (kSaBins / 4)) : make_uint4(0u, 0u, 0u, 0u);
     if (tid < 16) qraw = ld_16(static_cast<const T*>(p.q) + static_cast<int64_t>(head) * kHeadDim + tid * 8);
-#pragma unroll 1
-    for (unsigned r0 = 0; r0 < CL; r0 += 8) {
-      uint4 c[8];   // (eight loads in flight)
+    for (int g = tid; g < n_staged; g += kSaThreads) cp_async_16(staged + g + (g >> 3), gbase + g);
+    cp_async_commit();
 #pragma unroll
-      for (unsigned u = 0; u < 8; ++u) c[u] = r0 + u < CL ? __ldcg(hrow + (r0 + u) * (kSaBins / 4)) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-      for (unsigned u = 0; u < 8; ++u) {
-        tot.x += c[u].x; tot.y += c[u].y; tot.z += c[u].z; tot.w += c[u].w;
-        if (r0 + u < cr) { low.x += c[u].x; low.y += c[u].y; low.z += c[u].z; low.w += c[u].w; }
-      }
+    for (unsigned r = 0; r < kSaMaxSlices; ++r) {
+      tot.x += c[r].x; tot.y += c[r].y; tot.z += c[r].z; tot.w += c[r].w;
+      if (r < static_cast<unsigned>(slice)) { low.x += c[r].x; low.y += c[r].y; low.z += c[r].z; low.w += c[r].w; }
     }
-  }
-  // (rope_on: the last two warps form the position's cos / sin pairs; the block barriers of the cut phase order them before
-  // the query is rotated)
-  if (p.rope_on && tid >= kHeadDim / 2)
-    sh.cs[tid - kHeadDim / 2] = rope_cos_sin(tid - kHeadDim / 2, static_cast<float>(n), p.rope);
-  // the newest token rides with the last slice
-  const bool tail_here = p.tail_mode != 0 && cr == CL - 1;
-  const unsigned ps = static_cast<unsigned>(p.page_size);
-  unsigned tail_slot = p.tail_slot;
-  if (tail_here && tid == 0 && p.tail_mode == 2) {
-    const unsigned un = static_cast<unsigned>(n);
-    const unsigned pg = p.ps_shift >= 0 ? (un >> p.ps_shift) : (un / ps);
-    tail_slot = static_cast<unsigned>(__ldg(kv_table + pg)) * ps + (un - pg * ps);
   }
 
   // ---- cut ----------------------------------------------------------------------------------------------
@@ -269,39 +282,41 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     if (tid == 0) atomicOr(&g_adamas_error, kErrHistogram);
     cut = need_eq = lt_before = eq_before = 0;
   }
-  const unsigned take_eq = need_eq > eq_before ? need_eq - eq_before : 0u;   // this slice's tie quota
-  const unsigned out_base = lt_before + min(eq_before, need_eq);
 
   // ---- pick: ordered compaction of this block's winners -----------------------------------------------
-  // A thread owns `run` consecutive granules; it counts its elements below and at the cut, a block scan gives it its place
-  // in the list, and a second look at the granules that hold any writes the winners.
+  // A thread owns `run` consecutive granules; it counts its elements below and at the cut and leaves their masks in the
+  // first word of the staged granule; a block scan gives it its place in the list, and a second look at the granules that
+  // hold any writes the winners.
   const unsigned k_ge = (0x8000u - cut) * 0x00010001u, k_gt = (0x7fffu - cut) * 0x00010001u;
   const int run = (blk_count + kSaThreads - 1) / kSaThreads;
-  const int g_first = tid * run, g_end = min(blk_count, g_first + run);
-  auto masks = [&](int g, unsigned* lt, unsigned* eq) {
-    const uint4 v = g < kSaStaged ? staged[g + (g >> 3)] : ld_16(gbase + g);
+  const int g_first = pre + tid * run, g_end = min(pre + blk_count, g_first + run);
+  auto masks = [&](int g) {   // below the cut in bits w / 16 + w, at the cut in bits 4 + w / 20 + w
+    const uint4 v = g < n_staged ? staged[g + (g >> 3)] : ld_16(gbase + g);
     unsigned ge, gt;
     sa_compare(v, k_ge, k_gt, &ge, &gt);
     unsigned valid = 0x000f000fu;
-    const int left = n - (blk_first + g) * 8;
+    const int left = n - (seg_first + g) * 8;
     if (left < 8) valid = ((1u << ((left + 1) >> 1)) - 1u) | (((1u << (left >> 1)) - 1u) << 16);
-    *lt = ~ge & valid;
-    *eq = ge & ~gt & valid;
+    return (~ge & valid) | ((ge & ~gt & valid) << 4);
   };
-  unsigned packed = 0;   // elements below the cut | elements at the cut << 16 (a block holds at most 32768)
+  auto counts_of = [](unsigned m) { return static_cast<unsigned>(__popc(m & 0x000f000fu) + (__popc(m & 0x00f000f0u) << 16)); };
+  unsigned packed = 0, ahead = 0;   // elements below the cut | elements at the cut << 16 (a block holds at most 32768)
 #pragma unroll 2
   for (int g = g_first; g < g_end; ++g) {
-    unsigned lt, eq;
-    masks(g, &lt, &eq);
-    packed += __popc(lt) + (__popc(eq) << 16);
+    const unsigned m = masks(g);
+    if (g < n_staged) reinterpret_cast<unsigned*>(staged + g + (g >> 3))[0] = m;
+    packed += counts_of(m);
   }
+#pragma unroll 2
+  for (int g = tid; g < pre; g += kSaThreads) ahead += counts_of(masks(g));
   unsigned incl = packed;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  if (lane == 31) sh.warp_sum[warp].x = incl;   // (its readers of the cut phase are past a block barrier)
+  if (sharing > 1) ahead = __reduce_add_sync(0xffffffffu, ahead);
+  if (lane == 31) sh.warp_sum[warp] = make_uint2(incl, ahead);   // (the readers of the cut phase are past a block barrier)
   if (warp == 0) {
     if (p.rope_on) {   // (dimension pairs sit in lanes l and l ^ 8)
       float x[8];
@@ -315,56 +330,44 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   unsigned before = incl - packed, blk_tot = 0;
 #pragma unroll
   for (int w2 = 0; w2 < kSaWarps; ++w2) {
-    const unsigned a = sh.warp_sum[w2].x;
-    before += (w2 < warp) ? a : 0u;
-    blk_tot += a;
+    const uint2 a = sh.warp_sum[w2];
+    before += (w2 < warp) ? a.x : 0u;
+    blk_tot += a.x;
+    lt_before += a.y & 0xffffu;
+    eq_before += a.y >> 16;
   }
-  unsigned run_lt = before & 0xffffu, run_eq = before >> 16;
+  const unsigned take_eq = need_eq > eq_before ? need_eq - eq_before : 0u;   // this block's tie quota
   const int n_win = static_cast<int>((blk_tot & 0xffffu) + min(blk_tot >> 16, take_eq));
   const int n_loc = min(n_win + (tail_here ? 1 : 0), p.list_capacity);
-  // The winners go to a list in shared memory.
-  int32_t* oi = p.out_idx ? p.out_idx + static_cast<int64_t>(head) * p.out_stride + out_base : nullptr;
-  if (packed) {
+  // of a thread's cut-valued elements the first `quota` win; its winners are neighbours in the list
+  unsigned quota = take_eq > (before >> 16) ? min(take_eq - (before >> 16), packed >> 16) : 0u;
+  unsigned pos = (before & 0xffffu) + min(before >> 16, take_eq);
+  if ((packed & 0xffffu) + quota) {
+    const bool all_eq = quota == packed >> 16;
     for (int g = g_first; g < g_end; ++g) {
-      unsigned lt, eq;
-      masks(g, &lt, &eq);
-      if (!(lt | eq)) continue;
-      lt = sa_in_order(lt);
-      unsigned cand = lt | sa_in_order(eq);
-      const unsigned t0 = static_cast<unsigned>(blk_first + g) * 8;
-      unsigned page = 0;   // (with pages of 8 tokens or more, a power of two, a granule lies inside one page)
-      if (p.ps_shift >= 3) page = static_cast<unsigned>(__ldg(kv_table + (t0 >> p.ps_shift)));
-      while (cand) {   // in position order
-        const int j = __ffs(cand) - 1;
-        cand &= cand - 1;
-        int pos = -1;
-        if ((lt >> j) & 1u) {
-          pos = static_cast<int>(run_lt + min(run_eq, take_eq));
-          ++run_lt;
-        } else {
-          if (run_eq < take_eq) pos = static_cast<int>(run_lt + run_eq);
-          ++run_eq;
+      const unsigned m = g < n_staged ? reinterpret_cast<const unsigned*>(staged + g + (g >> 3))[0] : masks(g);
+      if (!m) continue;
+      unsigned win = sa_in_order(m & 0x000f000fu), eq = sa_in_order((m >> 4) & 0x000f000fu);
+      if (all_eq) {
+        win |= eq;
+      } else {
+        for (; eq && quota; --quota) {
+          win |= eq & -eq;
+          eq &= eq - 1;
         }
-        if (pos >= 0) {
-          const unsigned t = t0 + j;   // logical token position
-          unsigned slot;
-          if (p.ps_shift >= 3) {
-            slot = page * ps + (t & (ps - 1));
-          } else {
-            const unsigned pg = p.ps_shift >= 0 ? t >> p.ps_shift : t / ps;
-            slot = static_cast<unsigned>(__ldg(kv_table + pg)) * ps + (t - pg * ps);
-          }
-          if (pos < p.list_capacity) s_list[pos] = static_cast<int32_t>(slot);
-          if (oi) oi[pos] = static_cast<int32_t>(slot);
-        }
+      }
+      const unsigned t0 = static_cast<unsigned>(g - pre) * 8;
+      while (win) {
+        if (pos < static_cast<unsigned>(p.list_capacity)) s_list[pos] = static_cast<uint16_t>(t0 + __ffs(win) - 1);
+        win &= win - 1;
+        ++pos;
       }
     }
   }
-  if (tail_here && tid == 0 && n_win < p.list_capacity) s_list[n_win] = static_cast<int32_t>(tail_slot);
   __syncthreads();   // the list and the query are complete, the staged distances are read
 
-  // ---- attend: warp w takes rows w*rpw .. of the list, 16 at a time --------------------------------------
-  uint8_t* tiles = sa_smem + warp * (kSaSlots * kTileBytes);
+  // ---- attend: warp w takes rows w*rpw .. of the list, 24 at a time --------------------------------------
+  uint8_t* tile = sa_smem + warp * kSaWarpBytes;
   float m_run = -INFINITY, l_run = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);   // dimensions 4 * lane ..
   const int rpw = (n_loc + kSaWarps - 1) / kSaWarps;
@@ -373,38 +376,39 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   if (my_total > 0) {
     const int64_t row_elems = static_cast<int64_t>(H) * kHeadDim, v_delta = p.page_size * row_elems;
     const T* kbase = static_cast<const T*>(kv_base) + head_kv * kHeadDim;
+    int32_t* oi = p.out_idx ? p.out_idx + static_cast<int64_t>(head) * p.out_stride + lt_before + min(eq_before, need_eq) : nullptr;
     // K rows as one commit group, V rows as a second: the logits are formed while the V rows are still on their way
-    auto request = [&](int done, uint8_t* tile) {
-      if (done < my_total) {
-        // (lanes beyond the rows borrow the last one)
-        const unsigned slot = static_cast<unsigned>(s_list[my_first + min(done + (lane & 15), my_total - 1)]);
-        const unsigned page = p.ps_shift >= 0 ? slot >> p.ps_shift : slot / ps;
-        const int row = static_cast<int>(slot + page * ps);   // page * 2 ps + entry
-        tile_copy<T, true, false>(kbase, v_delta, row_elems, row, tile, lane);
-        cp_async_commit();
-        tile_copy<T, false, true>(kbase, v_delta, row_elems, row, tile, lane);
-      } else {
-        cp_async_commit();
-      }
-      cp_async_commit();
-    };
-#pragma unroll
-    for (int i = 0; i < kSaSlots; ++i) request(i * kTileRows, tiles + i * kTileBytes);
     uint4 q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j] = lane < 4 ? sh.q[4 * j + lane] : make_uint4(0, 0, 0, 0);
-    int use = 0;
-    for (int done = 0; done < my_total; done += kTileRows) {
-      uint8_t* tile = tiles + use * kTileBytes;
-      float sc[4];
-      cp_async_wait<2 * kSaSlots - 1>();
+    for (int done = 0; done < my_total; done += kSaRows) {
+      // K rows as one commit group, V rows as a second: the logits are formed while the V rows are still on their way
+      // (lanes beyond the rows borrow the last one)
+      const int at = my_first + min(done + lane, my_total - 1);
+      unsigned slot;
+      if (at < n_win) {
+        const unsigned t = static_cast<unsigned>(blk_first) * 8 + s_list[at], pg = page_of(t);   // logical token position
+        slot = static_cast<unsigned>(n_pages ? pages[pg - page0] : __ldg(kv_table + pg)) * ps + (t - pg * ps);
+        if (oi && done + lane < my_total && lane < kSaRows) oi[at] = static_cast<int32_t>(slot);
+      } else {
+        slot = sh.tail_slot;
+      }
+      const int row = static_cast<int>(slot + page_of(slot) * ps);   // page * 2 ps + entry
+      tile_copy<T, kSaRows, true, false>(kbase, v_delta, row_elems, row, tile, lane);
+      cp_async_commit();
+      tile_copy<T, kSaRows, false, true>(kbase, v_delta, row_elems, row, tile, lane);
+      cp_async_commit();
+      float sc[kSaRows / 4];
+      cp_async_wait<1>();
       __syncwarp();
-      tile_logits<T>(tile, q, (1u << min(kTileRows, my_total - done)) - 1u, p.scale_log2, lane, sc);
-      cp_async_wait<2 * kSaSlots - 2>();
+      tile_logits<T, kSaRows>(tile, q, my_total - done >= kSaRows ? (1u << kSaRows) - 1u : (1u << (my_total - done)) - 1u, p.scale_log2, lane, sc);
+      cp_async_wait<0>();
       __syncwarp();
-      // softmax in base 2 (the head's logits are in lanes 0 .. 3: tokens 2t, 2t + 1, 2t + 8, 2t + 9) and P.V with four
+      // softmax in base 2 (the head's logits are in lanes 0 .. 3) and P.V with four
       // dimensions per lane: one query row leaves the matrix form an eighth used and its accumulators cost 28 registers
-      float m_new = fmaxf(fmaxf(sc[0], sc[1]), fmaxf(sc[2], sc[3]));
+      float m_new = sc[0];
+#pragma unroll
+      for (int u = 1; u < kSaRows / 4; ++u) m_new = fmaxf(m_new, sc[u]);
       m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
       m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
       m_new = fmaxf(m_run, __shfl_sync(0xffffffffu, m_new, 0));   // finite: the tile's first token exists
@@ -412,14 +416,15 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
       m_run = m_new;
       l_run *= rescale;
       acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
-      float pr[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) pr[u] = exp2f(sc[u] - m_new);
-      l_run += (pr[0] + pr[1]) + (pr[2] + pr[3]);
-      const uint8_t* vbase = tile + kTileRows * 256 + (lane & 1) * 8;
+      for (int u = 0; u < kSaRows / 4; ++u) {
+        sc[u] = exp2f(sc[u] - m_new);
+        l_run += sc[u];
+      }
+      const uint8_t* vbase = tile + kSaRows * 256 + (lane & 1) * 8;
 #pragma unroll
-      for (int j = 0; j < kTileRows; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, pr[(j & 1) + 2 * (j >> 3)], (j & 7) >> 1);
+      for (int j = 0; j < kSaRows; ++j) {
+        const float pj = __shfl_sync(0xffffffffu, sc[(j & 1) + 2 * (j >> 3)], (j & 7) >> 1);
         const uint2 vv = *reinterpret_cast<const uint2*>(vbase + j * 256 + (((lane >> 1) ^ tile_swizzle(j)) << 4));
         const float2 a = Elem<T>::to_f2(vv.x), b = Elem<T>::to_f2(vv.y);
         acc.x = fmaf(pj, a.x, acc.x);
@@ -428,17 +433,14 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
         acc.w = fmaf(pj, b.y, acc.w);
       }
       __syncwarp();   // the tile may be filled again
-      request(done + kSaSlots * kTileRows, tile);
-      use = use + 1 == kSaSlots ? 0 : use + 1;
     }
-    cp_async_wait<0>();
   }
 
   // ---- merge: warps -> block -> head ----------------------------------------------------------------------
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);   // (lanes 0 .. 3)
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   __syncwarp();
-  reinterpret_cast<float4*>(tiles)[lane] = acc;
+  reinterpret_cast<float4*>(tile)[lane] = acc;
   if (lane == 0) {
     sh.ml[warp][0] = m_run;
     sh.ml[warp][1] = l_run;
@@ -452,7 +454,7 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     const float m = sh.ml[w2][0];
     const float w = (m == -INFINITY) ? 0.f : exp2f(m - M);
     L += w * sh.ml[w2][1];
-    od += w * reinterpret_cast<const float*>(sa_smem + w2 * (kSaSlots * kTileBytes))[tid];
+    od += w * reinterpret_cast<const float*>(sa_smem + w2 * kSaWarpBytes)[tid];
   }
   unsigned* counter = head_scratch + kSaMaxSlices * kSaBins + kHeadDim + 2;   // word 130 of slot 0
   if (CL > 1) {

@@ -36,6 +36,18 @@ constexpr int kDecMaxGroup = 8;     // query heads per matrix instruction; large
 constexpr int kDecMaxBatch = 1024;
 constexpr int kDecMinTiles = 6;     // tiles a block is worth starting for
 
+// Blocks per row group for `rows` row groups of `tiles` tiles each, or 0: cut the line of all tiles evenly.  With little
+// work latency counts, so a block gets a share of ONE row group (a second one would be a second pass through index
+// list, rows and merge).  A group of query heads (gs > 1) has as many results to merge per part: half as many parts;
+// measured at 28 query heads over 4 x 2001 tokens: 11.9 us with 6 tiles per block, 10.7 with 12; one query head per
+// row, 512 tokens: 7.4 / 8.3.
+__host__ __device__ __forceinline__ int dec_splits(int rows, int tiles, int gs, int slots) {
+  if (rows > slots || static_cast<int64_t>(rows) * tiles >= static_cast<int64_t>(slots) * kDecWarps * 4) return 0;
+  const int min_tiles = gs > 1 ? 2 * kDecMinTiles : kDecMinTiles;
+  const int most = slots / rows, wanted = (tiles + min_tiles - 1) / min_tiles;
+  return wanted < 1 ? 1 : wanted < most ? wanted : most;
+}
+
 struct DecodeParams {
   const void* q;          // [rows, 128]
   void* o;                // [rows, 128] in the cache's element type, or null
@@ -57,6 +69,7 @@ struct DecodeParams {
   unsigned tail_slot0;    // physical token slot of the first tail token (tokens n_listed ..)
   int n_tokens;
   int splits;             // > 0: blocks per row group; 0: the line of all tiles is cut evenly over the grid
+  int slots;              // blocks resident at once on the device
   float* partial_o;       // [units * gs, 128]
   float* partial_ml;      // [units * gs, 2]
   unsigned* counters;     // [row groups], zero on entry and on exit
@@ -110,7 +123,7 @@ __device__ __forceinline__ unsigned dec_request(const DecodeParams& p, const Dec
   const unsigned mask = __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
   const int safe = __shfl_sync(0xffffffffu, row, mask ? __ffs(mask) - 1 : 0);
   row = max(row >= 0 ? row : safe, 0);
-  tile_copy<T, true, true>(kbase, p.page_size * row_elems, row_elems, row, slot, lane);
+  tile_copy<T, kDecTile, true, true>(kbase, p.page_size * row_elems, row_elems, row, slot, lane);
   return mask;
 }
 
@@ -167,21 +180,24 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
     return k;
   };
 
-  if (p.splits == 0 && b >= B) return;
-  int pos = p.splits > 0 ? 0 : line_start(b);
-  const int line_end = p.splits > 0 ? 1 : line_start(b + 1);
+  // (one sequence with its length on the device is cut as the host cuts one whose length it knows, so that the result does
+  // not depend on the capacity)
+  const int splits = p.seq_len_dev && !p.seqs ? dec_splits(rps, sh.cum[1], p.gs, p.slots) : p.splits;
+  if (splits == 0 ? b >= B : b >= p.batch * rps * splits) return;
+  int pos = splits > 0 ? 0 : line_start(b);
+  const int line_end = splits > 0 ? 1 : line_start(b + 1);
   while (pos < line_end) {
     // ---- this block's next piece: tiles [a, e) of row group x of sequence s ------------------------------
     int s, x, a, e, nparts, part, unit;
-    if (p.splits > 0) {
-      const int r = b / p.splits;
-      part = b - r * p.splits;
+    if (splits > 0) {
+      const int r = b / splits;
+      part = b - r * splits;
       s = r / rps;
       x = r - s * rps;
       const int nt = sh.cum[s + 1] - sh.cum[s];
-      a = static_cast<int>(static_cast<int64_t>(nt) * part / p.splits);
-      e = static_cast<int>(static_cast<int64_t>(nt) * (part + 1) / p.splits);
-      nparts = p.splits;
+      a = static_cast<int>(static_cast<int64_t>(nt) * part / splits);
+      e = static_cast<int>(static_cast<int64_t>(nt) * (part + 1) / splits);
+      nparts = splits;
       unit = b;
       pos = line_end;
     } else {
@@ -275,7 +291,7 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
         __syncwarp();
         if (masks[0]) {
           float sc[4];
-          tile_logits<T>(ring + use * kDecTileBytes, q, masks[0], p.scale_log2, lane, sc);
+          tile_logits<T, kDecTile>(ring + use * kDecTileBytes, q, masks[0], p.scale_log2, lane, sc);
           tile_softmax_pv<T>(st, ring + use * kDecTileBytes, sc, lane);
         }
         __syncwarp();   // the slot may be filled again

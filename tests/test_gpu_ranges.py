@@ -112,3 +112,38 @@ def test_estimate_items_shapes(H, Hq, L, ps):
     for r in (0, Hq // 2, Hq - 1):
         for sl in range(slices):
             assert torch.equal(counts[r, sl].to(torch.int64), torch.bincount(want[r, sl * per:(sl + 1) * per], minlength=512))
+
+
+@pytest.mark.parametrize("n,k,H,ps", [
+    (1, 1, 3, 16), (9, 9, 4, 1),                       # fewer granules than threads; everything wins
+    (2047, 96, 32, 16), (2049, 97, 32, 16),            # one block per head / two; winners around one tile per warp
+    (30000, 1023, 32, 16), (32768, 2047, 8, 1),        # two blocks share a histogram slice; page numbers not staged (page size 1)
+    (40001, 4000, 4, 7),                               # several rounds per warp, a page size that is no power of two
+    (100000, 63, 100, 32),                             # few blocks per row: distances beyond the staged ones
+])
+@pytest.mark.parametrize("ties", [False, True])
+def test_select_attend_shapes(n, k, H, ps, ties):
+    """Selection (exact, ties to the lower position) and attention at the edges of the launch shapes."""
+    _, K, _ = _mods()
+    g = torch.Generator().manual_seed(n + k)
+    dist = torch.randint(180, 183, (H, n), generator=g) if ties else (torch.randn(H, n, generator=g) * 12 + 190).round().clamp(0, 384).long()
+    store = torch.zeros(H, (n + 7) // 8 * 8, dtype=torch.int16, device=DEV)
+    store[:, :n] = dist.to(torch.int16).to(DEV)
+    pages = (n + ps - 1) // ps
+    perm = torch.randperm(pages, generator=g)
+    kv = torch.empty(pages, 2, ps, 1, 128, dtype=torch.float16, device=DEV).normal_(generator=torch.Generator(device=DEV).manual_seed(n))
+    q = _randn((1, H, 128), 5, torch.float16)
+    idx = torch.full((H, k), -1, dtype=torch.int32, device=DEV)
+    o = torch.empty_like(q.to(DEV))
+    hist = K.histogram_scratch(H, DEV)
+    for _ in range(2):
+        K.select_attend(store[:, :n], k, q.to(DEV), o, kv, perm.to(torch.int32).to(DEV), 0, 0, indices_out=idx, hist=hist)
+    order = torch.argsort(dist * (n + 1) + torch.arange(n), 1)[:, :k].sort(1).values          # ascending positions of the winners
+    slots = (perm[order // ps] * ps + order % ps).to(torch.int32)
+    assert torch.equal(idx.cpu(), slots)
+    assert int(K.histogram_counts(hist).abs().sum().item()) == 0
+    flat = kv.permute(0, 2, 1, 3, 4).reshape(pages * ps, 2, 128).cpu()
+    for h in (0, H // 2, H - 1):
+        rows = flat[slots[h].long()]
+        want = ref.sparse_attention(q[0, h:h + 1], rows[:, 0:1], rows[:, 1:2], np.arange(k)[None])
+        _assert_attn_close(o[0, h:h + 1], want)
