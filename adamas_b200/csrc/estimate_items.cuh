@@ -29,7 +29,6 @@ constexpr int kItemWarps = 16;
 constexpr int kItemThreads = kItemWarps * 32;
 constexpr int kItemBytes = 4096;
 constexpr int kItemCountWords = 196;     // per query row: 392 16-bit counts (a distance is at most 384)
-constexpr int kEstMaxBatch = 1024;
 
 // 128-point transform of a row spread over 8 lanes, 16 elements each: the butterflies of wht128_halfwarp in the
 // same order, so the same bits.
@@ -118,20 +117,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
   const int pieces = p.H / HP;
   int tiles_all;
   if (p.seqs) {
-    if (warp == 0) {
-      int base = 0;
-      for (int s0 = 0; s0 < p.batch; s0 += 32) {
-        int v = s0 + lane < p.batch ? (__ldg(p.seq_len_dev + s0 + lane) - 1 + TT - 1) / TT : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, v, o);
-          if (lane >= o) v += u;
-        }
-        if (s0 + lane < p.batch) sh.cum[s0 + lane + 1] = base + v;
-        base += __shfl_sync(0xffffffffu, v, 31);
-      }
-      if (lane == 0) sh.cum[0] = 0;
-    }
+    if (warp == 0) est_line(p, TT, lane, sh.cum);
     __syncthreads();
     tiles_all = sh.cum[p.batch];
   } else {
