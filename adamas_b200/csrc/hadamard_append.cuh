@@ -101,11 +101,13 @@ __device__ __forceinline__ void rope_halfwarp_cs(float (&x)[8], unsigned l16, co
 // Bound: HBM (q and k are read and written once).  A block takes kRopeTokens consecutive tokens (one for short
 // calls, so that the grid still covers the chip): its 64 (cos, sin) pairs per token are formed once, one pair
 // per thread, and shared by all rows of the token.  A power and a sine/cosine per ELEMENT, as the kernel before
-// this one had it, was bound by those: 32768 tokens x (32 + 32) heads took 1220 us against 166 us of traffic.
+// this one had it, was bound by those: 32768 tokens x (32 + 32) heads took 1220 us against 166 us of traffic; 212 us
+// with two rows in flight per thread and the pairs of a lane 64 bytes apart in shared memory (bank conflicts), 178 us now.
 // Eight lanes per row, each with 8 dimensions of the lower half and their 8 partners of the upper half: no
 // exchange between lanes, and every access is a full 128-byte line.
 constexpr int kRopeThreads = 256;
 constexpr int kRopeTokens = 4;
+constexpr int kRopeRows = 4;      // rows in flight per thread
 
 template <typename T>
 __device__ __forceinline__ T* rope_row(T* q, T* k, int64_t tok, int r, int hq, int hk) {
@@ -115,70 +117,63 @@ __device__ __forceinline__ T* rope_row(T* q, T* k, int64_t tok, int r, int hq, i
 template <typename T>
 __global__ void __launch_bounds__(kRopeThreads) rope_kernel(T* __restrict__ q, T* __restrict__ k, int seq, int hq, int hk,
                                                             int past_len, int tokens_per_block, RopeParams rp) {
-  constexpr int kRows = kRopeThreads / 8;   // rows in flight per pass of the block
-  __shared__ __align__(16) float2 s_cs[kRopeTokens][kHeadDim / 2];
+  constexpr int kRows = kRopeThreads / 8;   // rows per pass of the block
+  __shared__ float2 s_cs[kRopeTokens][8][8];   // [token][i][l8]: the pair of element i of lane l8 (no bank conflicts)
   const int tid = threadIdx.x;
   const int l8 = tid & 7;
-  const int slot = tid >> 3;
   const int rows = hq + hk;
   const int64_t tok0 = static_cast<int64_t>(blockIdx.x) * tokens_per_block;
   const int nt = min(tokens_per_block, static_cast<int>(seq - tok0));
-  // the first rows do not depend on the table: have them on their way while it is formed
-  uint4 lo[2], hi[2];
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int r = slot + u * kRows;
-    if (r < rows) {
-      const T* p = rope_row(q, k, tok0, r, hq, hk) + l8 * 8;
-      lo[u] = ld_16(p);
-      hi[u] = ld_16(p + kHeadDim / 2);
-    }
-  }
-  for (int i = tid; i < nt * (kHeadDim / 2); i += kRopeThreads)
-    s_cs[i >> 6][i & 63] = rope_cos_sin(i & 63, static_cast<float>(past_len + tok0 + (i >> 6)), rp);
-  __syncthreads();
+  const int all = nt * rows;   // rows of the block: token after token
   const bool scaled = rp.inv_freq != nullptr;
-  for (int t = 0; t < nt; ++t) {
-    float2 cs[8];
+  // kRopeRows rows in flight per thread, the first ones while the table is formed
+  T* at[kRopeRows];
+  int t[kRopeRows];
+  uint4 lo[kRopeRows], hi[kRopeRows];
+  auto load = [&](int r0) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) cs[i] = s_cs[t][l8 * 8 + i];
-    for (int r0 = slot; r0 < rows; r0 += 2 * kRows) {
-      if (t > 0 || r0 != slot) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int r = r0 + u * kRows;
-          if (r < rows) {
-            const T* p = rope_row(q, k, tok0 + t, r, hq, hk) + l8 * 8;
-            lo[u] = ld_16(p);
-            hi[u] = ld_16(p + kHeadDim / 2);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int r = r0 + u * kRows;
-        if (r < rows) {
-          float a[8], b[8];
-          unpack8<T>(lo[u], a);
-          unpack8<T>(hi[u], b);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            // lower half: x*cos - partner*sin; upper half: x*cos + partner*sin
-            float x = fmaf(-b[i], cs[i].y, a[i] * cs[i].x);
-            float y = fmaf(a[i], cs[i].y, b[i] * cs[i].x);
-            if (scaled) {
-              x *= rp.mscale;
-              y *= rp.mscale;
-            }
-            a[i] = x;
-            b[i] = y;
-          }
-          T* p = rope_row(q, k, tok0 + t, r, hq, hk) + l8 * 8;
-          st_16(p, pack8<T>(a));
-          st_16(p + kHeadDim / 2, pack8<T>(b));
-        }
+    for (int u = 0; u < kRopeRows; ++u) {
+      const int r = r0 + u * kRows;
+      t[u] = r / rows;
+      if (r < all) {
+        at[u] = rope_row(q, k, tok0 + t[u], r - t[u] * rows, hq, hk) + l8 * 8;
+        lo[u] = ld_16(at[u]);
+        hi[u] = ld_16(at[u] + kHeadDim / 2);
       }
     }
+  };
+  int r0 = tid >> 3;
+  load(r0);
+  for (int i = tid; i < nt * (kHeadDim / 2); i += kRopeThreads)
+    s_cs[i >> 6][i & 7][(i & 63) >> 3] = rope_cos_sin(i & 63, static_cast<float>(past_len + tok0 + (i >> 6)), rp);
+  __syncthreads();
+  while (true) {
+#pragma unroll
+    for (int u = 0; u < kRopeRows; ++u) {
+      if (r0 + u * kRows < all) {
+        float a[8], b[8];
+        unpack8<T>(lo[u], a);
+        unpack8<T>(hi[u], b);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float2 cs = s_cs[t[u]][i][l8];
+          // lower half: x*cos - partner*sin; upper half: x*cos + partner*sin
+          float x = fmaf(-b[i], cs.y, a[i] * cs.x);
+          float y = fmaf(a[i], cs.y, b[i] * cs.x);
+          if (scaled) {
+            x *= rp.mscale;
+            y *= rp.mscale;
+          }
+          a[i] = x;
+          b[i] = y;
+        }
+        st_16(at[u], pack8<T>(a));
+        st_16(at[u] + kHeadDim / 2, pack8<T>(b));
+      }
+    }
+    r0 += kRopeRows * kRows;
+    if (r0 >= all) break;
+    load(r0);
   }
 }
 
@@ -323,7 +318,8 @@ append_decode_kernel(const T* __restrict__ k, const T* __restrict__ v, const T* 
   }
 }
 
-// Prefill append: one half-warp per (token, head) row; token n sits at position start_pos + n.
+// Prefill append: one half-warp per (token, head) row; token n sits at position start_pos + n.  Bound: HBM (K and V read once
+// and written once, and the codes).  (Two or four rows per half-warp in flight, and streaming stores, measured no better.)
 template <typename T, bool FUSED>
 __global__ void __launch_bounds__(256)
 append_prefill_kernel(const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ h,
@@ -333,15 +329,15 @@ append_prefill_kernel(const T* __restrict__ k, const T* __restrict__ v, const T*
   const bool valid = row < rows;
   const int64_t r = valid ? row : 0;
   const int H = tgt.num_heads;
-  const int64_t n = r / H;
-  const int head = static_cast<int>(r - n * H);
-  const int64_t pos = start_pos + n;
-  const int64_t lp = pos / tgt.page_size;
-  const int e = static_cast<int>(pos - lp * tgt.page_size);
   const int64_t in_off = r * kHeadDim + l16 * 8;
-
   uint4 kraw = ld_stream_16(k + in_off);
   uint4 vraw = ld_stream_16(v + in_off);
+  // (32-bit divisions wherever they hold the numbers: positions are below 2^31)
+  const int64_t n = rows <= 0x7fffffff ? static_cast<int64_t>(static_cast<unsigned>(r) / static_cast<unsigned>(H)) : r / H;
+  const int head = static_cast<int>(r - n * H);
+  const unsigned pos = static_cast<unsigned>(start_pos + n), lp = pos / static_cast<unsigned>(tgt.page_size);
+  const int e = static_cast<int>(pos - lp * static_cast<unsigned>(tgt.page_size));
+
   const int64_t kv_page = tgt.kv_table[lp];
   T* kv = static_cast<T*>(tgt.kv_data);
   const int64_t k_off = ((kv_page * 2 * tgt.page_size + e) * H + head) * kHeadDim + l16 * 8;
