@@ -108,7 +108,7 @@ struct SaShared {
   unsigned cut, need_eq, lt_before, eq_before;
   unsigned tail_slot;
   unsigned last;   // this block arrived last at the head's counter
-  uint4 q[16];     // the head's query row
+  alignas(16) uint16_t q[kHeadDim];   // the head's query row, rotated
   float2 cs[kHeadDim / 2];   // rope_on: (cos, sin) of the position
 };
 
@@ -201,13 +201,15 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   uint4* staged = reinterpret_cast<uint4*>(sa_smem);   // granule g of the slice at g + g / 8: reads of neighbouring threads' runs do not conflict
   const int n_staged = min(pre + blk_count, p.staged_granules);
   uint4 tot = make_uint4(0u, 0u, 0u, 0u), low = tot;   // bins 4 * tid ..: the whole row; lower-ranked slices
-  uint4 qraw = tot;                                    // the query row, 16 lanes x 16 bytes
+  const T* q_row = static_cast<const T*>(p.q) + static_cast<int64_t>(head) * kHeadDim;
+  uint16_t q_own, q_pair = 0;                          // the query's element tid, and the one it rotates with
   {
     const uint4* hrow = reinterpret_cast<const uint4*>(head_scratch) + tid;
     uint4 c[kSaMaxSlices];
 #pragma unroll
     for (unsigned r = 0; r < kSaMaxSlices; ++r) c[r] = r < static_cast<unsigned>(p.slices) && tid < p.bin_threads ? __ldcg(hrow + r * (kSaBins / 4)) : make_uint4(0u, 0u, 0u, 0u);
-    if (tid < 16) qraw = ld_16(static_cast<const T*>(p.q) + static_cast<int64_t>(head) * kHeadDim + tid * 8);
+    q_own = reinterpret_cast<const uint16_t*>(q_row)[tid];
+    if (p.rope_on) q_pair = reinterpret_cast<const uint16_t*>(q_row)[tid ^ (kHeadDim / 2)];
     for (int g = tid; g < n_staged; g += kSaThreads) cp_async_16(staged + g + (g >> 3), gbase + g);
     cp_async_commit();
 #pragma unroll
@@ -317,15 +319,14 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   }
   if (sharing > 1) ahead = __reduce_add_sync(0xffffffffu, ahead);
   if (lane == 31) sh.warp_sum[warp] = make_uint2(incl, ahead);   // (the readers of the cut phase are past a block barrier)
-  if (warp == 0) {
-    if (p.rope_on) {   // (dimension pairs sit in lanes l and l ^ 8)
-      float x[8];
-      unpack8<T>(qraw, x);
-      rope_halfwarp_cs<T>(x, lane & 15, sh.cs, p.rope.inv_freq != nullptr, p.rope.mscale);
-      qraw = pack8<T>(x);
-    }
-    if (lane < 16) sh.q[lane] = qraw;
+  if (p.rope_on) {   // (rope_halfwarp_cs, one element per thread)
+    const float2 cs = sh.cs[tid & (kHeadDim / 2 - 1)];
+    const float x = Elem<T>::to_f2(q_own).x, other = Elem<T>::to_f2(q_pair).x;
+    float r = tid >= kHeadDim / 2 ? fmaf(other, cs.y, x * cs.x) : fmaf(-other, cs.y, x * cs.x);
+    if (p.rope.inv_freq) r *= p.rope.mscale;
+    q_own = static_cast<uint16_t>(Elem<T>::from_f2(r, 0.f));
   }
+  sh.q[tid] = q_own;
   __syncthreads();
   unsigned before = incl - packed, blk_tot = 0;
 #pragma unroll
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     // K rows as one commit group, V rows as a second: the logits are formed while the V rows are still on their way
     uint4 q[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) q[j] = lane < 4 ? sh.q[4 * j + lane] : make_uint4(0, 0, 0, 0);
+    for (int j = 0; j < 4; ++j) q[j] = lane < 4 ? reinterpret_cast<const uint4*>(sh.q)[4 * j + lane] : make_uint4(0, 0, 0, 0);
     for (int done = 0; done < my_total; done += kSaRows) {
       // K rows as one commit group, V rows as a second: the logits are formed while the V rows are still on their way
       // (lanes beyond the rows borrow the last one)
@@ -501,10 +502,10 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   if (tid == 0 && p.lse) p.lse[head] = L > 0.f ? M + log2f(L) : -INFINITY;
   // every block of the head has read the histograms and the un-rotated query long ago: clear the table and the counter
   // for the next launch
-  for (unsigned r = 0; r < CL; ++r) reinterpret_cast<uint4*>(head_scratch)[r * (kSaBins / 4) + tid] = make_uint4(0u, 0u, 0u, 0u);
+  for (int r = 0; r < p.slices; ++r) reinterpret_cast<uint4*>(head_scratch)[r * (kSaBins / 4) + tid] = make_uint4(0u, 0u, 0u, 0u);
   if (tid == 0) *counter = 0u;
   if (p.rope_on && tid < 16)
-    st_16(static_cast<T*>(const_cast<void*>(p.q)) + static_cast<int64_t>(head) * kHeadDim + tid * 8, sh.q[tid]);
+    st_16(const_cast<T*>(q_row) + tid * 8, reinterpret_cast<const uint4*>(sh.q)[tid]);
 }
 
 // Per-slice histograms of distance rows, for callers of select_attend that did not get them from an
