@@ -583,8 +583,8 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
     const int per_sm = std::min(est_blocks_per_sm(), (smem + 1024 + 2048) * 2 <= static_cast<size_t>(di->max_smem_optin) ? 2 : 1);
-    // (a batch: one block per sequence at least)
-    const dim3 grid(static_cast<unsigned>(std::max<int64_t>(batch, std::min<int64_t>(static_cast<int64_t>(num_tiles) * batch, di->num_sms * per_sm))));
+    // (a batch: one block per sequence at least; with an append, one per sequence that has nothing else to do where there is room)
+    const dim3 grid(static_cast<unsigned>(std::max<int64_t>(batch, std::min<int64_t>(static_cast<int64_t>(num_tiles + (ap.q ? 1 : 0)) * batch, di->num_sms * per_sm))));
 #define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_kernel", (__VA_ARGS__), grid, dim3(kEstThreads), smem, st, 1, prm)
 #define LAUNCH_EST_HPW(HPW)                                                                     \
   do {                                                                                          \

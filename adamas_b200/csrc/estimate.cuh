@@ -91,7 +91,7 @@ __device__ __forceinline__ __half dist_to_out<__half>(unsigned d) {
 
 // The decode append inside the estimate.  Every block codes all query heads of the sequences it works on by itself
 // (the rows come from L2), so no block waits for another.  The new token's K and V rows, the key's code and the query
-// codes are stored by one block (estimate_append_kernel) or dealt out over the sequence's blocks by cache head
+// codes are stored by one block each (estimate_append_kernel) or dealt out over the sequence's blocks by cache head
 // (estimate_items_kernel); none of this is read by the scan, which leaves the newest token out, and the kernel after
 // this one finds all of it complete.
 // rope_on: q and k arrive un-rotated.  The position's 64 (cos, sin) pairs are formed once per block and sequence, the
@@ -155,7 +155,7 @@ __device__ __forceinline__ void est_line(const EstimateParams& p, int tile_token
   if (lane == 0) cum[0] = 0;
 }
 
-// What a block works on: tiles rank, rank + blocks, ... of one sequence.
+// What a block works on: tiles rank, rank + blocks, ... of one sequence; nothing to scan where rank == blocks.
 struct EstGeom {
   int n_tokens;
   int num_tiles;
@@ -164,6 +164,7 @@ struct EstGeom {
   const int32_t* page_table;
   int seq;
   int rank, blocks;
+  bool appends;       // stores the sequence's new token
   int row0;           // first row of this sequence in q_code, out and hist
 };
 // Called by all threads of the block.  A batch's sequences get one block each and the other blocks in proportion to their
@@ -180,7 +181,7 @@ __device__ __forceinline__ EstGeom est_geom(const EstimateParams& p, int* cum) {
   if (p.seqs) {   // (the table of sequences is set up once, long before this launch)
     if (threadIdx.x < 32) est_line(p, kEstTile, threadIdx.x, cum);
     __syncthreads();
-    const int64_t total = cum[p.batch], spare = static_cast<int>(gridDim.x) - p.batch;
+    const int64_t total = max(cum[p.batch], 1), spare = static_cast<int>(gridDim.x) - p.batch;
     auto first_block = [&](int s) { return s + static_cast<int>(cum[s] * spare / total); };
     int lo = 0, hi = p.batch - 1;
     while (lo < hi) {   // the last sequence that starts at or before this block
@@ -199,6 +200,11 @@ __device__ __forceinline__ EstGeom est_geom(const EstimateParams& p, int* cum) {
   }
   g.row0 = g.seq * p.H;
   g.num_tiles = (g.n_tokens + kEstTile - 1) / kEstTile;
+  // The sequence's last block appends.  It scans nothing where that gives no other block a tile more: with tiles to scan
+  // as well it finished 1 to 2 us after all the others (one sequence, 4K to 128K tokens x 32 heads).  Where every block
+  // has many tiles it scans its own after the append (appending after them: 80.0 us a layer for 8 x 32K, before 79.5).
+  g.appends = g.rank == g.blocks - 1;
+  if (p.ap.q && g.blocks > 1 && (g.num_tiles + g.blocks - 1) / g.blocks == (g.num_tiles + g.blocks - 2) / (g.blocks - 1)) --g.blocks;
   g.slice_tokens = p.hist ? 8 * sa_granules_per_block(g.n_tokens, p.hist_cl) : 1;
   return g;
 }
@@ -220,7 +226,7 @@ struct EstRing {
   int stage_chunks;   // chunks per ring slot
 };
 
-__device__ __forceinline__ int est_tiles_of_block(const EstGeom& g) { return max(0, (g.num_tiles - g.rank + g.blocks - 1) / g.blocks); }
+__device__ __forceinline__ int est_tiles_of_block(const EstGeom& g) { return g.rank < g.blocks ? max(0, (g.num_tiles - g.rank + g.blocks - 1) / g.blocks) : 0; }
 
 // Producer warps: one bulk copy per token (its H codes) into the padded ring slot.
 // A bulk copy with a different address in every lane is issued lane after lane, about 45 ns each
@@ -379,7 +385,7 @@ __global__ void __launch_bounds__(kEstThreads) estimate_kernel(const EstimatePar
 
 // ---- estimate with the decode append inside: the same pipeline; warp w loads the query rows of its HPW heads (one
 // half-warp per row), transforms, buckets and packs them, and spreads the 16 code words of each head over the warp
-// through shared memory.  The last block (it has the fewest tiles) appends.
+// through shared memory.
 template <typename T, int HPW, bool ROPE>
 __global__ void __launch_bounds__(kEstThreads) estimate_append_kernel(const EstimateParams p) {
   static_assert(HPW == 1 || HPW == 2 || HPW == 4, "heads per warp");
@@ -412,39 +418,68 @@ __global__ void __launch_bounds__(kEstThreads) estimate_append_kernel(const Esti
   grid_dependency_wait();
   grid_launch_dependents();
 
-  const bool appender = geom.rank == geom.blocks - 1;
-  // slot of the new token: from the host, or from the device-resident sequence length (position n)
-  int kv_last_page = a.kv_last_page, kv_entry = a.kv_entry, code_last_page = a.code_last_page, code_entry = a.code_entry;
-  if (p.seq_len_dev) {
-    kv_last_page = code_last_page = geom.n_tokens / p.page_size;
-    kv_entry = code_entry = geom.n_tokens - kv_last_page * p.page_size;
-  }
   const unsigned l16 = lane & 15;
   const int half = lane >> 4;
-  const int H = p.H;
-  PagedTarget tgt = a.tgt;
-  if (p.seqs) {
-    const SeqDesc sd = p.seqs[geom.seq];
-    tgt.kv_data = sd.kv_data;
-    tgt.kv_table = sd.kv_table;
-    tgt.code_data = static_cast<uint16_t*>(sd.code_data);
-    tgt.code_table = sd.code_table;
+  constexpr int kPasses = (HPW + 1) / 2;
+  // row of a pass for this half-warp: head warp*HPW + 2*pass + half (HPW == 1: both halves take the one head, half 0 stores)
+  const int head0 = warp * HPW + (HPW == 1 ? 0 : half);
+  const bool writer = HPW > 1 || half == 0;
+  const int64_t in_off0 = static_cast<int64_t>(geom.row0 + head0) * kHeadDim + l16 * 8;   // rows of q, k, v: (sequence, head)
+  if (geom.appends) {   // block-uniform
+    // slot of the new token: from the host, or from the device-resident sequence length (position n)
+    int kv_last_page = a.kv_last_page, kv_entry = a.kv_entry, code_last_page = a.code_last_page, code_entry = a.code_entry;
+    if (p.seq_len_dev) {
+      kv_last_page = code_last_page = geom.n_tokens / p.page_size;
+      kv_entry = code_entry = geom.n_tokens - kv_last_page * p.page_size;
+    }
+    PagedTarget tgt = a.tgt;
+    if (p.seqs) {
+      const SeqDesc sd = p.seqs[geom.seq];
+      tgt.kv_data = sd.kv_data;
+      tgt.kv_table = sd.kv_table;
+      tgt.code_data = static_cast<uint16_t*>(sd.code_data);
+      tgt.code_table = sd.code_table;
+    }
+    uint4 kraw[kPasses], vraw[kPasses];
+#pragma unroll
+    for (int pass = 0; pass < kPasses; ++pass) {
+      kraw[pass] = ld_16(static_cast<const T*>(a.k) + in_off0 + 2 * pass * kHeadDim);
+      vraw[pass] = ld_16(static_cast<const T*>(a.v) + in_off0 + 2 * pass * kHeadDim);
+    }
+    const int64_t kv_page = __ldg(tgt.kv_table + kv_last_page), code_page = __ldg(tgt.code_table + code_last_page);
+    const int64_t v_delta = static_cast<int64_t>(p.page_size) * p.H * kHeadDim;
+#pragma unroll
+    for (int pass = 0; pass < kPasses; ++pass) {
+      const int head = head0 + 2 * pass;
+      T* slot = static_cast<T*>(tgt.kv_data) + ((kv_page * 2 * p.page_size + kv_entry) * p.H + head) * kHeadDim + l16 * 8;
+      float x[8];
+      unpack8<T>(kraw[pass], x);
+      if (ROPE) {
+        rope_halfwarp_cs<T>(x, l16, s_cs, a.rp.inv_freq != nullptr, a.rp.mscale);
+        kraw[pass] = pack8<T>(x);
+        if (writer) st_16(static_cast<T*>(a.k) + in_off0 + 2 * pass * kHeadDim, kraw[pass]);
+        unpack8<T>(kraw[pass], x);
+      }
+      if (writer) {
+        st_16(slot, kraw[pass]);
+        st_16(slot + v_delta, vraw[pass]);
+      }
+      wht128_halfwarp(x, l16);
+      scale_round<T>(x, a.scale);
+      if (writer) tgt.code_data[((code_page * p.page_size + code_entry) * p.H + head) * kCodeWords + l16] = bucketize_pack8(x, a.th);
+    }
   }
+  if (geom.rank >= geom.blocks) return;
   QPlanes qp[HPW][2];
 #pragma unroll
-  for (int pass = 0; pass < (HPW + 1) / 2; ++pass) {
-    // this half-warp's row: head warp*HPW + 2*pass + half (HPW == 1: both halves take the one head)
-    const int hh_mine = (HPW == 1) ? 0 : 2 * pass + half;
-    const int head = warp * HPW + hh_mine;
-    const int64_t in_off = static_cast<int64_t>(geom.row0 + head) * kHeadDim + l16 * 8;   // rows of q, k, v: (sequence, head)
-    const bool writer = appender && (HPW > 1 || half == 0);
+  for (int pass = 0; pass < kPasses; ++pass) {
     float x[8];
-    unpack8<T>(ld_16(static_cast<const T*>(a.q) + in_off), x);
+    unpack8<T>(ld_16(static_cast<const T*>(a.q) + in_off0 + 2 * pass * kHeadDim), x);
     if (ROPE) rope_halfwarp_cs<T>(x, l16, s_cs, a.rp.inv_freq != nullptr, a.rp.mscale);
     wht128_halfwarp(x, l16);
     scale_round<T>(x, a.scale);
-    const unsigned word = bucketize_pack8(x, a.th);   // code word l16 of `head`
-    if (writer) a.q_code_out[(geom.row0 + head) * kCodeWords + l16] = static_cast<uint16_t>(word);
+    const unsigned word = bucketize_pack8(x, a.th);   // code word l16 of the row
+    if (geom.rank == 0 && writer) a.q_code_out[(geom.row0 + head0 + 2 * pass) * kCodeWords + l16] = static_cast<uint16_t>(word);
     // spread the 16 code words of each row over the warp: through shared memory (one 2-byte store per
     // lane, two 16-byte broadcast loads per head)
     __syncwarp();
@@ -456,35 +491,6 @@ __global__ void __launch_bounds__(kEstThreads) estimate_append_kernel(const Esti
       const int hh = (HPW == 1) ? 0 : 2 * pass + s;
       qp[hh][0] = make_qplanes(cw[0]);
       qp[hh][1] = make_qplanes(cw[1]);
-    }
-    if (appender) {   // block-uniform
-      const int kv_page = __ldg(tgt.kv_table + kv_last_page);
-      const int code_page = __ldg(tgt.code_table + code_last_page);
-      const int ps = tgt.page_size;
-      T* kv = static_cast<T*>(tgt.kv_data);
-      const int64_t k_off =
-          ((static_cast<int64_t>(kv_page) * 2 * ps + kv_entry) * H + head) * kHeadDim + l16 * 8;
-      const int64_t v_delta = static_cast<int64_t>(ps) * H * kHeadDim;
-      uint4 kraw = ld_16(static_cast<const T*>(a.k) + in_off);
-      const uint4 vraw = ld_16(static_cast<const T*>(a.v) + in_off);
-      float b[8];
-      unpack8<T>(kraw, b);
-      if (ROPE) {
-        rope_halfwarp_cs<T>(b, l16, s_cs, a.rp.inv_freq != nullptr, a.rp.mscale);
-        kraw = pack8<T>(b);
-        if (writer) st_16(static_cast<T*>(a.k) + in_off, kraw);
-      }
-      if (writer) {
-        st_16(kv + k_off, kraw);
-        st_16(kv + k_off + v_delta, vraw);
-      }
-      wht128_halfwarp(b, l16);
-      scale_round<T>(b, a.scale);
-      if (writer) {
-        const int64_t c_off =
-            ((static_cast<int64_t>(code_page) * ps + code_entry) * H + head) * kCodeWords + l16;
-        tgt.code_data[c_off] = bucketize_pack8(b, a.th);
-      }
     }
   }
   est_consume<0, uint16_t, HPW>(p, geom, ring, my_tiles, lane, warp, qp);
