@@ -167,8 +167,8 @@ def run_reference_arm(args):
 
 
 def two_launch_step(args) -> bool:
-    """decode_step folds the append (and a rotation) into the estimate launch for 16, 32 or 64 heads."""
-    return (not args.unfused) and args.heads in (16, 32, 64) and os.environ.get("ADAMAS_FUSED_APPEND", "1") != "0"
+    """decode_step folds the append (and a rotation) into the estimate launch."""
+    return (not args.unfused) and os.environ.get("ADAMAS_FUSED_APPEND", "1") != "0"
 
 
 def launches_per_layer(args) -> int:
@@ -583,7 +583,8 @@ def run_ours(args):
         both = stage_time("select_attend", pre="estimate")
         stage_us["estimate_then_select_attend"] = both
         stage_us["select_attend"] = both - stage_us["estimate"]
-        kernels = {first: "estimate_append_kernel" if first == "append_estimate" else "estimate_kernel",
+        by_tiles = args.heads in (16, 32, 64)
+        kernels = {first: "estimate_items_kernel" if not by_tiles else "estimate_append_kernel" if first == "append_estimate" else "estimate_kernel",
                    "select_attend": "select_attend_kernel"}
         if first == "estimate":
             kernels["append"] = "append_decode_kernel"

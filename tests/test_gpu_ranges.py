@@ -147,3 +147,32 @@ def test_select_attend_shapes(n, k, H, ps, ties):
         rows = flat[slots[h].long()]
         want = ref.sparse_attention(q[0, h:h + 1], rows[:, 0:1], rows[:, 1:2], np.arange(k)[None])
         _assert_attn_close(o[0, h:h + 1], want)
+
+
+@pytest.mark.parametrize("H", [16, 32, 64])
+@pytest.mark.parametrize("L", [2, 33, 34, 148 * 32 + 1, 295 * 32 + 1, 296 * 32 + 1, 297 * 32 + 1, 2 * 296 * 32 + 1, 20001])
+def test_append_estimate_tiles(H, L):
+    """Estimate with the append inside, where the appending block has tiles of its own and where it has none: the
+    same bits as the separate append and estimate."""
+    _, K, _ = _mods()
+    ps, n = 16, L - 1
+    pages = (L + ps - 1) // ps
+    g = torch.Generator().manual_seed(L + H)
+    table = torch.randperm(pages, generator=g).to(torch.int32).to(DEV)
+    codes = torch.randint(-32768, 32768, (pages, 1, ps, H, 16), generator=g, dtype=torch.int32).to(torch.int16)
+    q, k, v = (_randn((1, H, 128), s + L, torch.float16) for s in (1, 2, 3))
+    results = []
+    for inside in (False, True):
+        qd, kd, vd = q.to(DEV), k.to(DEV), v.to(DEV)
+        code_cache, kv_cache = codes.to(DEV), torch.zeros(pages, 2, ps, H, 128, dtype=torch.float16, device=DEV)
+        q_code = torch.zeros(1, H, 16, dtype=torch.int16, device=DEV)
+        dist = torch.zeros(H, (n + 7) // 8 * 8, dtype=torch.int16, device=DEV)
+        last = L - (pages - 1) * ps
+        if inside:
+            K.append_estimate(qd, kd, vd, q_code, kv_cache, table, last, code_cache, table, last, dist[:, :n], scale=1.0)
+        else:
+            K.append_kv_cache_decode_fused(qd, kd, vd, q_code, kv_cache, table, last, code_cache, table, last, 0, scale=1.0)
+            K.estimate_attn_score(q_code, dist[:, :n], code_cache, table, None, last, 0, 0)
+        results.append([t.cpu() for t in (kv_cache, code_cache, q_code, dist)])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
