@@ -153,11 +153,13 @@ struct RopeArg {
 
 inline adamas_stream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-// Runs `f` (a call of the C ABI) without the interpreter lock; a non-zero status becomes RuntimeError.
-template <typename F>
-void call(const char* what, F f) {
+// Calls `f`, a function of the C ABI, without the interpreter lock; a non-zero status becomes RuntimeError.  The arguments
+// (pointers of tensors, the current stream) are formed by the caller, before the lock is given up: forming them may throw,
+// or warn through Python (a tensor without memory of its own, no driver), and both need the lock.
+template <typename... P, typename... A>
+void call(const char* what, int (*f)(P...), A... args) {
   PyThreadState* st = PyEval_SaveThread();
-  const int rc = f();
+  const int rc = f(args...);
   PyEval_RestoreThread(st);
   REQUIRE(rc == ADAMAS_OK, "%s failed: %s", what, adamas_last_error());
 }
@@ -233,7 +235,7 @@ PyObject* py_hadamard_transform(PyObject*, PyObject* const* a, Py_ssize_t n) {  
     const int dt = dtype_code(x, "hadamard_transform");
     at::Tensor y = inplace ? x : at::empty_like(x);
     const int64_t count = x.numel() / 128;
-    call("hadamard_transform", [&] { return adamas_hadamard_transform(ptr(x), ptr(y), count, 128, s, dt, stream()); });
+    call("hadamard_transform", adamas_hadamard_transform, ptr(x), ptr(y), count, 128, s, dt, stream());
     if (inplace) {
       Py_INCREF(a[0]);
       return a[0];
@@ -251,10 +253,8 @@ PyObject* py_apply_rope(PyObject*, PyObject* const* a, Py_ssize_t n) {   // q, k
     const int64_t past = integer(a[2]);
     const float rs = static_cast<float>(real(a[3])), rt = static_cast<float>(real(a[4]));
     const int dt = dtype_code(q, "apply_rope_in_place");
-    call("apply_rope_in_place", [&] {
-      return adamas_apply_rope_in_place(ptr(q), ptr(k), q.size(0), static_cast<int>(q.size(1)), static_cast<int>(k.size(1)),
-                                        128, past, rs, rt, dt, stream());
-    });
+    call("apply_rope_in_place", adamas_apply_rope_in_place, ptr(q), ptr(k), q.size(0), static_cast<int>(q.size(1)),
+         static_cast<int>(k.size(1)), 128, past, rs, rt, dt, stream());
     return none();
   });
 }
@@ -271,12 +271,10 @@ PyObject* py_append_decode(PyObject*, PyObject* const* a, Py_ssize_t n) {
     REQUIRE(o.size(1) == c.heads && o.size(2) == k.size(2) / 8 && o.element_size() == 2, "o must be [1, H, D/8] 16-bit");
     const int kl = int32(a[6]), cl = int32(a[9]), dt = dtype_code(k, "Append_kv_cache_decode");
     const ThresholdsArg th(a[11]);
-    call("Append_kv_cache_decode", [&] {
-      return adamas_append_decode(ptr(k), ptr(v), ptr(h), ptr(o), ptr(*c.kv_data), ptr_as<int32_t>(*c.kv_indices),
-                                  static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data), ptr_as<int32_t>(*c.code_indices),
-                                  static_cast<int>(c.code_indices->numel()), cl, c.heads, static_cast<int>(k.size(2)), c.page_size,
-                                  th.p, dt, stream());
-    });
+    call("Append_kv_cache_decode", adamas_append_decode, ptr(k), ptr(v), ptr(h), ptr(o), ptr(*c.kv_data),
+         ptr_as<int32_t>(*c.kv_indices), static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data),
+         ptr_as<int32_t>(*c.code_indices), static_cast<int>(c.code_indices->numel()), cl, c.heads, static_cast<int>(k.size(2)),
+         c.page_size, th.p, dt, stream());
     return none();
   });
 }
@@ -298,21 +296,16 @@ PyObject* py_append_decode_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const RopeArg rope(a[13]);
     if (rope.on) {
       const int dt = dtype_code(k, "append_kv_cache_decode_rope_fused");
-      call("append_kv_cache_decode_rope_fused", [&] {
-        return adamas_append_decode_rope_fused(
-            ptr(q), ptr(k), ptr(v), ptr(o), ptr(*c.kv_data), ptr_as<int32_t>(*c.kv_indices), static_cast<int>(c.kv_indices->numel()),
-            kl, ptr(*c.code_data), ptr_as<int32_t>(*c.code_indices), static_cast<int>(c.code_indices->numel()), cl, c.heads, hq, d,
-            c.page_size, s, th.p, rope.inv_freq ? 1.f : rope.scale, rope.inv_freq ? 1e4f : rope.theta, rope.inv_freq, rope.mscale, dt,
-            stream());
-      });
+      call("append_kv_cache_decode_rope_fused", adamas_append_decode_rope_fused, ptr(q), ptr(k), ptr(v), ptr(o), ptr(*c.kv_data),
+           ptr_as<int32_t>(*c.kv_indices), static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data),
+           ptr_as<int32_t>(*c.code_indices), static_cast<int>(c.code_indices->numel()), cl, c.heads, hq, d, c.page_size, s, th.p,
+           rope.inv_freq ? 1.f : rope.scale, rope.inv_freq ? 1e4f : rope.theta, rope.inv_freq, rope.mscale, dt, stream());
     } else {
       const int dt = dtype_code(k, "append_kv_cache_decode_fused");
-      call("append_kv_cache_decode_fused", [&] {
-        return adamas_append_decode_fused(ptr(q), ptr(k), ptr(v), ptr(o), ptr(*c.kv_data), ptr_as<int32_t>(*c.kv_indices),
-                                          static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data),
-                                          ptr_as<int32_t>(*c.code_indices), static_cast<int>(c.code_indices->numel()), cl, c.heads, hq,
-                                          d, c.page_size, s, th.p, dt, stream());
-      });
+      call("append_kv_cache_decode_fused", adamas_append_decode_fused, ptr(q), ptr(k), ptr(v), ptr(o), ptr(*c.kv_data),
+           ptr_as<int32_t>(*c.kv_indices), static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data),
+           ptr_as<int32_t>(*c.code_indices), static_cast<int>(c.code_indices->numel()), cl, c.heads, hq, d, c.page_size, s, th.p,
+           dt, stream());
     }
     return none();
   });
@@ -333,12 +326,10 @@ PyObject* py_append_prefill(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int kl = int32(a[5]), cl = int32(a[8]), dt = dtype_code(k, "Append_kv_cache_prefill");
     const float s = scale_or_default(a[10]);
     const ThresholdsArg th(a[11]);
-    call("Append_kv_cache_prefill", [&] {
-      return adamas_append_prefill(ptr(k), ptr(v), h, k.size(0), ptr(*c.kv_data), ptr_as<int32_t>(*c.kv_indices),
-                                   static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data), ptr_as<int32_t>(*c.code_indices),
-                                   static_cast<int>(c.code_indices->numel()), cl, c.heads, static_cast<int>(k.size(2)), c.page_size, s,
-                                   th.p, dt, stream());
-    });
+    call("Append_kv_cache_prefill", adamas_append_prefill, ptr(k), ptr(v), h, k.size(0), ptr(*c.kv_data),
+         ptr_as<int32_t>(*c.kv_indices), static_cast<int>(c.kv_indices->numel()), kl, ptr(*c.code_data),
+         ptr_as<int32_t>(*c.code_indices), static_cast<int>(c.code_indices->numel()), cl, c.heads, static_cast<int>(k.size(2)),
+         c.page_size, s, th.p, dt, stream());
     return none();
   });
 }
@@ -362,11 +353,9 @@ PyObject* py_estimate(PyObject*, PyObject* const* a, Py_ssize_t n) {
     REQUIRE(o.size(0) == hq && o.size(1) == cols, "o must be [%lld, %lld]", static_cast<long long>(hq), static_cast<long long>(cols));
     const int fmt = value_format(o, "Estimate_attn_score"), slices = int32(a[9]);
     uint32_t* hist = histogram(a[8], hq);
-    call("Estimate_attn_score", [&] {
-      return adamas_estimate(ptr(q), ptr(cd), ptr_as<int32_t>(ci), static_cast<int>(ci.numel()), last, static_cast<int>(ps),
-                             static_cast<int>(h), static_cast<int>(hq), 128, ptr(o), o.stride(0), fmt, metric, exclude, hist, slices,
-                             stream());
-    });
+    call("Estimate_attn_score", adamas_estimate, ptr(q), ptr(cd), ptr_as<int32_t>(ci), static_cast<int>(ci.numel()), last,
+         static_cast<int>(ps), static_cast<int>(h), static_cast<int>(hq), 128, ptr(o), o.stride(0), fmt, metric, exclude, hist,
+         slices, stream());
     return none();
   });
 }
@@ -387,10 +376,8 @@ PyObject* py_topk_filtering(PyObject*, PyObject* const* a, Py_ssize_t n) {
     REQUIRE(d.size(0) == count && oi.size(0) == count, "outputs must have one row per head");
     REQUIRE(d.scalar_type() == v.scalar_type(), "d_out must have the dtype of estimated_value");
     const int fmt = value_format(v, "Top-k filtering");
-    call("Top-k filtering", [&] {
-      return adamas_topk(ptr(v), fmt, v.stride(0), static_cast<int>(cols), ptr_as<int32_t>(vi), vi.stride(0), 1,
-                         static_cast<int>(count), static_cast<int>(k), ptr(d), ptr_as<int32_t>(oi), oi.stride(0), stream());
-    });
+    call("Top-k filtering", adamas_topk, ptr(v), fmt, v.stride(0), static_cast<int>(cols), ptr_as<int32_t>(vi), vi.stride(0), 1,
+         static_cast<int>(count), static_cast<int>(k), ptr(d), ptr_as<int32_t>(oi), oi.stride(0), stream());
     return none();
   });
 }
@@ -416,10 +403,8 @@ PyObject* py_topk_select(PyObject*, PyObject* const* a, Py_ssize_t n) {
       table = ptr_as<int32_t>(t);
     }
     const int fmt = value_format(v, "topk_select");
-    call("topk_select", [&] {
-      return adamas_topk(ptr(v), fmt, v.stride(0), static_cast<int>(cols), table, 0, static_cast<int>(ps), static_cast<int>(count),
-                         static_cast<int>(k), vo, ptr_as<int32_t>(oi), oi.stride(0), stream());
-    });
+    call("topk_select", adamas_topk, ptr(v), fmt, v.stride(0), static_cast<int>(cols), table, 0, static_cast<int>(ps),
+         static_cast<int>(count), static_cast<int>(k), vo, ptr_as<int32_t>(oi), oi.stride(0), stream());
     return none();
   });
 }
@@ -454,15 +439,13 @@ PyObject* py_decode_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
       lse = ptr_as<float>(t);
     }
     if (tokens > planned) {
-      call("BatchDecodeWithPagedKVCache",
-           [&] { return adamas_decode_begin_forward(handle, tokens, batch, hkv, hq, d, ps, dt, stream()); });
+      call("BatchDecodeWithPagedKVCache", adamas_decode_begin_forward, handle, tokens, batch, hkv, hq, d, ps, dt, stream());
       planned = tokens;
     }
     const float sm_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(d)));
-    call("BatchDecodeWithPagedKVCache", [&] {
-      return adamas_decode_forward(handle, ptr(q), ptr(o), lse, ptr(kv), ptr_as<int32_t>(idx), idx.stride(0), static_cast<int>(n_idx),
-                                   static_cast<int>(unit), last_idx, last_len, static_cast<int>(tail), sm_scale, stream());
-    });
+    call("BatchDecodeWithPagedKVCache", adamas_decode_forward, handle, ptr(q), ptr(o), lse, ptr(kv), ptr_as<int32_t>(idx),
+         idx.stride(0), static_cast<int>(n_idx), static_cast<int>(unit), last_idx, last_len, static_cast<int>(tail), sm_scale,
+         stream());
     return PyLong_FromLongLong(planned);
   });
 }
@@ -512,13 +495,11 @@ PyObject* py_decode_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const float scale = scale_or_default(a[17]), sm_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(s.d)));
     const ThresholdsArg th(a[18]);
     const RopeArg rope(a[19]);
-    call("decode_step", [&] {
-      return adamas_decode_step(ptr(*s.q), ptr(*s.k), ptr(*s.v), ptr(*s.o), lse, ptr(*s.code), ptr(*s.c.kv_data),
-                                ptr_as<int32_t>(*s.c.kv_indices), static_cast<int>(s.c.kv_indices->numel()), kl, ki, ptr(*s.c.code_data),
-                                ptr_as<int32_t>(*s.c.code_indices), static_cast<int>(s.c.code_indices->numel()), cl, s.c.heads, s.hq, s.d,
-                                s.c.page_size, s.dt, s.budget, ptr(*s.dist), s.dist->stride(0), hist, s.out_idx, s.out_stride, scale,
-                                th.p, rope.scale, rope.theta, rope.inv_freq, rope.mscale, sm_scale, stream());
-    });
+    call("decode_step", adamas_decode_step, ptr(*s.q), ptr(*s.k), ptr(*s.v), ptr(*s.o), lse, ptr(*s.code), ptr(*s.c.kv_data),
+         ptr_as<int32_t>(*s.c.kv_indices), static_cast<int>(s.c.kv_indices->numel()), kl, ki, ptr(*s.c.code_data),
+         ptr_as<int32_t>(*s.c.code_indices), static_cast<int>(s.c.code_indices->numel()), cl, s.c.heads, s.hq, s.d, s.c.page_size,
+         s.dt, s.budget, ptr(*s.dist), s.dist->stride(0), hist, s.out_idx, s.out_stride, scale, th.p, rope.scale, rope.theta,
+         rope.inv_freq, rope.mscale, sm_scale, stream());
     return none();
   });
 }
@@ -540,13 +521,10 @@ PyObject* py_decode_step_dev(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const float scale = scale_or_default(a[16]), sm_scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(s.d)));
     const ThresholdsArg th(a[17]);
     const RopeArg rope(a[18]);
-    call("decode_step_dev", [&] {
-      return adamas_decode_step_dev(ptr(*s.q), ptr(*s.k), ptr(*s.v), ptr(*s.o), lse, ptr(*s.code), ptr(*s.c.kv_data),
-                                    ptr_as<int32_t>(*s.c.kv_indices), ptr(*s.c.code_data), ptr_as<int32_t>(*s.c.code_indices),
-                                    ptr_as<int32_t>(len), max_len, s.c.heads, s.hq, s.d, s.c.page_size, s.dt, s.budget, ptr(*s.dist),
-                                    s.dist->stride(0), hist, s.out_idx, s.out_stride, scale, th.p, rope.scale, rope.theta,
-                                    rope.inv_freq, rope.mscale, sm_scale, stream());
-    });
+    call("decode_step_dev", adamas_decode_step_dev, ptr(*s.q), ptr(*s.k), ptr(*s.v), ptr(*s.o), lse, ptr(*s.code),
+         ptr(*s.c.kv_data), ptr_as<int32_t>(*s.c.kv_indices), ptr(*s.c.code_data), ptr_as<int32_t>(*s.c.code_indices),
+         ptr_as<int32_t>(len), max_len, s.c.heads, s.hq, s.d, s.c.page_size, s.dt, s.budget, ptr(*s.dist), s.dist->stride(0),
+         hist, s.out_idx, s.out_stride, scale, th.p, rope.scale, rope.theta, rope.inv_freq, rope.mscale, sm_scale, stream());
     return none();
   });
 }

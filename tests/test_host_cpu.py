@@ -174,3 +174,25 @@ def test_header_is_plain_c_and_a_c_program_links(tmp_path):
     subprocess.run([gcc, "-std=c99", "-Wall", "-Wextra", "-pedantic", "-Werror", "-I", os.path.join(ROOT, "include"),
                     str(src), "-o", str(exe), "-L", lib_dir, "-ladamas_b200", f"-Wl,-rpath,{lib_dir}"], check=True)
     assert subprocess.run([str(exe)]).returncode == 0
+
+
+def test_tensor_without_memory_is_refused_with_an_exception():
+    """The extension module forms pointers and the stream while it holds the interpreter lock: both may throw or warn
+    through Python (here: a fake tensor, and no driver where there is no GPU).  In a process of its own, because
+    doing so without the lock crashes the interpreter."""
+    import subprocess
+    import sys
+    code = (
+        "import torch\n"
+        "from torch._subclasses.fake_tensor import FakeTensorMode\n"
+        "from adamas_b200 import _kernels as K\n"
+        "with FakeTensorMode():\n"
+        "    x = torch.empty(4, 2, 128, dtype=torch.float16, device='cuda:0')\n"
+        "for f in (lambda: K.hadamard_transform(x, True), lambda: K.apply_rope_in_place(x, x, 0)):\n"
+        "    try:\n"
+        "        f()\n"
+        "    except RuntimeError:\n"
+        "        continue\n"
+        "    raise SystemExit(3)\n")
+    proc = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert proc.returncode == 0, proc.stderr
