@@ -87,6 +87,11 @@ double real(PyObject* o) {
   if (v == -1.0 && PyErr_Occurred()) throw PyFailure{};
   return v;
 }
+bool truth(PyObject* o) {   // (an object may refuse to be a truth value, as a tensor of several elements does)
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw PyFailure{};
+  return v != 0;
+}
 float scale_or_default(PyObject* o) { return static_cast<float>(given(o) ? real(o) : 1.0 / std::sqrt(128.0)); }
 
 int dtype_code(const at::Tensor& t, const char* what) {
@@ -230,7 +235,7 @@ PyObject* py_hadamard_transform(PyObject*, PyObject* const* a, Py_ssize_t n) {  
   return guarded("hadamard_transform", n, 3, [&]() -> PyObject* {
     const at::Tensor& x = input(a[0], "x");
     REQUIRE(x.dim() >= 1 && x.size(-1) == 128, "hadamard_transform supports a last dimension of 128");
-    const int inplace = PyObject_IsTrue(a[1]);
+    const bool inplace = truth(a[1]);
     const float s = scale_or_default(a[2]);
     const int dt = dtype_code(x, "hadamard_transform");
     at::Tensor y = inplace ? x : at::empty_like(x);
@@ -348,7 +353,7 @@ PyObject* py_estimate(PyObject*, PyObject* const* a, Py_ssize_t n) {
     REQUIRE(hq >= h && h >= 1 && hq % h == 0 && cd.size(4) == words && words == 16,
             "hadamard_data must be [pages, 1, page_size, num_heads, 16], q [1, Hq, 16]");
     REQUIRE(q.element_size() == 2 && cd.element_size() == 2, "codes must be 16-bit words");
-    const int last = int32(a[4]), metric = int32(a[6]), exclude = PyObject_IsTrue(a[7]) ? 1 : 0;
+    const int last = int32(a[4]), metric = int32(a[6]), exclude = truth(a[7]) ? 1 : 0;
     const int64_t cols = (ci.numel() - 1) * ps + last - exclude;
     REQUIRE(o.size(0) == hq && o.size(1) == cols, "o must be [%lld, %lld]", static_cast<long long>(hq), static_cast<long long>(cols));
     const int fmt = value_format(o, "Estimate_attn_score"), slices = int32(a[9]);
@@ -418,7 +423,7 @@ PyObject* py_decode_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& o = input(a[2], "o", 3);
     const at::Tensor& kv = input(a[4], "paged_kv_data", 5);
     const at::Tensor& idx = rows(a[5], "paged_kv_indices");
-    const int last_len = int32(a[6]), last_idx = int32(a[7]), token_granular = PyObject_IsTrue(a[8]);
+    const int last_len = int32(a[6]), last_idx = int32(a[7]), token_granular = truth(a[8]);
     const int hq = int32(a[9]), hkv = int32(a[10]), d = int32(a[11]), ps = int32(a[12]), dt = int32(a[13]), batch = int32(a[15]);
     int64_t planned = integer(a[14]);
     REQUIRE(q.size(0) == 1 && q.size(1) == hq && q.size(2) == d, "q must be [1, H, D]");
