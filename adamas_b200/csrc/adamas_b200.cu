@@ -131,13 +131,16 @@ int get_device_info(const DeviceInfo** out) {
     EST_ATTR_HPW(2);
     EST_ATTR_HPW(4);
 #undef EST_ATTR_HPW
-#define EST_ATTR_HP(HP)                                \
-  EST_ATTR(estimate_items_kernel<__half, 0, HP>);      \
-  EST_ATTR(estimate_items_kernel<__half, 1, HP>);      \
-  EST_ATTR(estimate_items_kernel<__nv_bfloat16, 0, HP>)
-    EST_ATTR_HP(1);
-    EST_ATTR_HP(2);
-    EST_ATTR_HP(4);
+#define EST_ATTR_HP(HP, G)                                \
+  EST_ATTR(estimate_items_kernel<__half, 0, HP, G>);      \
+  EST_ATTR(estimate_items_kernel<__half, 1, HP, G>);      \
+  EST_ATTR(estimate_items_kernel<__nv_bfloat16, 0, HP, G>)
+    EST_ATTR_HP(1, false);
+    EST_ATTR_HP(2, false);
+    EST_ATTR_HP(4, false);
+    EST_ATTR_HP(1, true);
+    EST_ATTR_HP(2, true);
+    EST_ATTR_HP(4, true);
 #undef EST_ATTR_HP
 #undef EST_ATTR
     ADAMAS_CUDA(cudaFuncSetAttribute(paged_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDecSmem));
@@ -568,6 +571,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   prm.n_tokens = n;
   prm.H = num_heads;
   prm.q_group = q_heads / num_heads;
+  prm.chip_warps = kItemWarps * di->num_sms;
   prm.page_size = page_size;
   prm.ps_shift = log2_exact(page_size);
   prm.batch = batch;
@@ -612,29 +616,43 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
     return check_launch("estimate_kernel");
   }
   const int hp = num_heads % 4 == 0 ? 4 : num_heads % 2 == 0 ? 2 : 1;   // heads per item: as long a run of a token's codes as divides
-  const int64_t items = static_cast<int64_t>((n + 128 / hp - 1) / (128 / hp)) * (num_heads / hp) * batch;
+  int64_t items = static_cast<int64_t>((n + 128 / hp - 1) / (128 / hp)) * (num_heads / hp) * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
+  const int q_part = item_query_heads(static_cast<int>(items), prm.q_group, prm.chip_warps);
+  items *= (prm.q_group + q_part - 1) / q_part;   // (still below 2^31: only few items are divided)
   const dim3 grid(static_cast<unsigned>(std::min<int64_t>(di->num_sms, items)));
-  const size_t slot = static_cast<size_t>(kItemWarps) * kItemBytes, counts = static_cast<size_t>(q_heads) * kItemCountWords * sizeof(uint32_t);
+  // Little work: blocks of half the size, which leave the other half of the SM's registers to the first blocks of the kernel
+  // behind (whole step, 3000 tokens: 8 heads 12.1 -> 10.7 us, 28 over 4 14.7 -> 14.1; one head, 60K: 14.5 -> 12.4).  They code
+  // 32 query heads in one pass; with 64 the second pass costs what this gains (16.1 / 18.1 us).
+  const int64_t per_block = (items + grid.x - 1) / grid.x;
+  const int warps = per_block <= kItemWarps / 2 && q_heads <= 2 * kItemWarps ? kItemWarps / 2 : kItemWarps;
+  const size_t slot = static_cast<size_t>(warps) * kItemBytes, counts = static_cast<size_t>(q_heads) * kItemCountWords * sizeof(uint32_t);
+  const int wanted = static_cast<int>(std::min<int64_t>(3, (per_block + warps - 1) / warps)), least = std::min(wanted, 2);   // ring slots
   // The counts in shared memory where they fit beside two ring slots per warp and where there are enough distances to be
   // worth clearing and adding up a table per block (12K tokens x 40 heads: 6.4 us with an L2 atomic each, 7.5 with tables;
   // 30K x 32: 8.8 / 8.7; 64K x 64: 26.9 / 21.1); a third slot where it fits beside them.
   size_t smem = static_cast<size_t>(q_heads) * 2 * sizeof(QPlanes);
-  prm.count_local = hist && static_cast<int64_t>(q_heads) * n * batch >= (int64_t(1) << 20) && smem + 2 * slot + counts <= most ? 1 : 0;
+  prm.count_local = hist && static_cast<int64_t>(q_heads) * n * batch >= (int64_t(1) << 20) && smem + least * slot + counts <= most ? 1 : 0;
   if (prm.count_local) smem += counts;
-  const int slots = smem + 3 * slot <= most ? 3 : 2;
+  const int slots = smem + wanted * slot <= most ? wanted : least;
   smem += slots * slot;
   ADAMAS_REQUIRE(smem <= most, "num_q_heads (%d) too large for the estimate kernel", q_heads);
-#define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_items_kernel", (__VA_ARGS__), grid, dim3(kItemThreads), smem, st, 1, prm, slots)
-#define LAUNCH_EST_HP(HP)                                                                                 \
-  do {                                                                                                    \
-    if (metric != ADAMAS_METRIC_L1) LAUNCH_EST(estimate_items_kernel<__half, 1, HP>);   /* (no append) */ \
-    else if (dtype == ADAMAS_F16) LAUNCH_EST(estimate_items_kernel<__half, 0, HP>);                       \
-    else LAUNCH_EST(estimate_items_kernel<__nv_bfloat16, 0, HP>);                                         \
+#define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_items_kernel", (__VA_ARGS__), grid, dim3(warps * 32), smem, st, 1, prm, slots)
+#define LAUNCH_EST_HP(HP, G)                                                                                 \
+  do {                                                                                                       \
+    if (metric != ADAMAS_METRIC_L1) LAUNCH_EST(estimate_items_kernel<__half, 1, HP, G>);   /* (no append) */ \
+    else if (dtype == ADAMAS_F16) LAUNCH_EST(estimate_items_kernel<__half, 0, HP, G>);                       \
+    else LAUNCH_EST(estimate_items_kernel<__nv_bfloat16, 0, HP, G>);                                         \
   } while (0)
-  if (hp == 4) LAUNCH_EST_HP(4);
-  else if (hp == 2) LAUNCH_EST_HP(2);
-  else LAUNCH_EST_HP(1);
+#define LAUNCH_EST_G(G)                    \
+  do {                                     \
+    if (hp == 4) LAUNCH_EST_HP(4, G);      \
+    else if (hp == 2) LAUNCH_EST_HP(2, G); \
+    else LAUNCH_EST_HP(1, G);              \
+  } while (0)
+  if (prm.q_group > 1) LAUNCH_EST_G(true);
+  else LAUNCH_EST_G(false);
+#undef LAUNCH_EST_G
 #undef LAUNCH_EST_HP
 #undef LAUNCH_EST
   return check_launch("estimate_items_kernel");

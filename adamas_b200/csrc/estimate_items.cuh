@@ -25,10 +25,19 @@
 
 namespace adamas {
 
-constexpr int kItemWarps = 16;
+constexpr int kItemWarps = 16;           // warps of a block, or half as many (see the host's rule)
 constexpr int kItemThreads = kItemWarps * 32;
 constexpr int kItemBytes = 4096;
 constexpr int kItemCountWords = 196;     // per query row: 392 16-bit counts (a distance is at most 384)
+
+// Query heads of a cache head that a warp takes at a time.  The group of a cache head is halved as long as every part still
+// finds a warp of its own (`warps` on the chip; `items` are those of undivided groups): a second round costs more than it saves
+// (32 query heads over 2, 60K tokens: 14.3 us in two parts, one round; 17.9 in three parts, two rounds).
+__host__ __device__ __forceinline__ int item_query_heads(int items, int q_group, int warps) {
+  int heads = q_group;
+  for (; heads > 1 && items <= warps / 2; items *= 2) heads = (heads + 1) / 2;
+  return heads;
+}
 
 // 128-point transform of a row spread over 8 lanes, 16 elements each: the butterflies of wht128_halfwarp in the
 // same order, so the same bits.
@@ -100,7 +109,8 @@ struct EstShared {
 };
 
 // Dynamic shared memory: rings | planes [rows of a sequence][2] | counts [rows][kItemCountWords] (count_local).
-template <typename T, int METRIC, int HP>
+// GROUPED: several query heads per cache head (q_group > 1).
+template <typename T, int METRIC, int HP, bool GROUPED>
 __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const EstimateParams p, int slots) {
   constexpr int TT = 128 / HP;          // tokens of an item
   constexpr int kGroups = TT / 32;      // ... in groups of 32
@@ -108,13 +118,14 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
   extern __shared__ __align__(128) uint8_t item_smem[];
   __shared__ EstShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int rows = p.H * p.q_group;     // query rows of a sequence
-  QPlanes* planes = reinterpret_cast<QPlanes*>(item_smem + kItemWarps * slots * kItemBytes);
+  const int threads = blockDim.x, warps = threads >> 5;
+  const int q_group = GROUPED ? p.q_group : 1;
+  const int rows = p.H * q_group;       // query rows of a sequence
+  QPlanes* planes = reinterpret_cast<QPlanes*>(item_smem + warps * slots * kItemBytes);
   uint32_t* counts = reinterpret_cast<uint32_t*>(planes + 2 * rows);
   uint4* ring = reinterpret_cast<uint4*>(item_smem + warp * (slots * kItemBytes));
 
-  // ---- the line of items: token tile after token tile, `pieces` of HP heads each -----------------------------
-  const int pieces = p.H / HP;
+  // ---- the line of items: token tile after token tile, `pieces` each: HP heads with a part of their query heads ---
   int tiles_all;
   if (p.seqs) {
     if (warp == 0) est_line(p, TT, lane, sh.cum);
@@ -123,13 +134,40 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
   } else {
     tiles_all = ((p.seq_len_dev ? __ldg(p.seq_len_dev) - 1 : p.n_tokens) + TT - 1) / TT;
   }
+  const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
+  const int q_split = q_part == q_group ? 1 : (q_group + q_part - 1) / q_part, pieces = p.H / HP * q_split;
+  const float split_inv = 1.f / static_cast<float>(q_split);
+  auto heads_of = [&](int piece) { return q_split == 1 ? piece : __float2int_rz((static_cast<float>(piece) + 0.5f) * split_inv); };   // piece / q_split (exact: pieces <= 1024)
   const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
+  if (total == 0) return;
   // (with the lengths on the device there may be fewer items than blocks: every block that takes part has some)
   const int b = blockIdx.x, B = min(static_cast<int>(gridDim.x), total);
   auto line_start = [&](int blk) { return static_cast<int>(static_cast<int64_t>(blk) * total / B); };
-  if (b >= B) return;
-  int pos = line_start(b);
-  const int line_end = line_start(b + 1);
+  int pos, line_end;
+  int nblk = B, my_blk = b;   // blocks that share out the appends of a piece's sequence, and which of them this one is
+  // A batch with little work: every block takes a piece of ONE sequence, the blocks dealt out in proportion to the items.  (A
+  // block that the line takes into a second sequence codes two queries, one after the other, and the launch waits for it:
+  // 2 sequences of 1250 and 2500 tokens, 32 query heads over 8: 15.2 us, 9.2 this way.)
+  const bool apart = p.seqs && p.batch <= static_cast<int>(gridDim.x) && total <= 2 * p.chip_warps;
+  if (apart) {
+    const int spare = gridDim.x - p.batch;
+    auto first_block = [&](int s) { return s + static_cast<int>(static_cast<int64_t>(sh.cum[s]) * spare / tiles_all); };
+    int lo = 0, hi = p.batch - 1;
+    while (lo < hi) {   // the last sequence that starts at or before this block
+      const int mid = (lo + hi + 1) >> 1;
+      if (first_block(mid) <= b) lo = mid; else hi = mid - 1;
+    }
+    const int seq_items = (sh.cum[lo + 1] - sh.cum[lo]) * pieces;
+    nblk = min(first_block(lo + 1) - first_block(lo), seq_items);
+    my_blk = b - first_block(lo);
+    if (my_blk >= nblk) return;
+    pos = sh.cum[lo] * pieces + static_cast<int>(static_cast<int64_t>(seq_items) * my_blk / nblk);
+    line_end = sh.cum[lo] * pieces + static_cast<int>(static_cast<int64_t>(seq_items) * (my_blk + 1) / nblk);
+  } else {
+    if (b >= B) return;
+    pos = line_start(b);
+    line_end = line_start(b + 1);
+  }
   bool waited = false;
 
   while (pos < line_end) {
@@ -158,7 +196,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
     // ---- copies -----------------------------------------------------------------------------------------------
     // the page numbers of an item's tokens (lane = token of each group of 32) are fetched one item ahead of its copies
     int item_q = first + warp, tile_q = item_q / pieces, piece_q = item_q - tile_q * pieces;
-    const int dt = kItemWarps / pieces, dp = kItemWarps - dt * pieces;
+    const int dt = warps / pieces, dp = warps - dt * pieces;
     auto step = [&](int& tile, int& piece) {
       tile += dt;
       piece += dp;
@@ -184,7 +222,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
       }
       constexpr int RPI = 32 / CPR;   // tokens per copy instruction
       const int c = lane & (CPR - 1), r0 = lane / CPR;
-      const uint4* base = codes + piece * CPR + c;
+      const uint4* base = codes + heads_of(piece) * CPR + c;
       const int64_t stride = 2 * p.H;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -198,7 +236,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
       if (item_q < end) {
         request(tile_q, piece_q, ring + slot * (kItemBytes / 16));
         step(tile_q, piece_q);
-        item_q += kItemWarps;
+        item_q += warps;
         if (item_q < end) fetch_entries(tile_q);
       }
       cp_async_commit();
@@ -215,7 +253,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
       if (tid < kHeadDim / 2) sh.cs[tid] = rope_cos_sin(tid, static_cast<float>(n), p.ap.rp);
     }
     if (p.count_local)
-      for (int i = tid; i < rows * (kItemCountWords / 4); i += kItemThreads) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
+      for (int i = tid; i < rows * (kItemCountWords / 4); i += threads) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
     if (p.ap.rope_on) __syncthreads();
     if (!waited) {
       grid_dependency_wait();   // q, k, v or the query codes are the preceding kernel's output
@@ -226,14 +264,17 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
       const StepAppend& ap = p.ap;
       const unsigned l8 = lane & 7;
       const bool scaled = ap.rp.inv_freq != nullptr;
-      // blocks of this sequence, and which of them this one is: they share out the appends
-      auto block_of = [&](int item) {
-        int k = static_cast<int>(static_cast<int64_t>(item) * B / total);
-        while (line_start(k + 1) <= item) ++k;
-        return k;
-      };
-      const int bf = block_of(seq0), nblk = block_of(seq1 - 1) - bf + 1, my_blk = b - bf;
-      for (int r0 = 0; r0 < rows; r0 += kItemThreads / 8) {
+      if (p.seqs && !apart) {
+        auto block_of = [&](int item) {
+          int k = static_cast<int>(static_cast<int64_t>(item) * B / total);
+          while (line_start(k + 1) <= item) ++k;
+          return k;
+        };
+        const int bf = block_of(seq0);
+        nblk = block_of(seq1 - 1) - bf + 1;
+        my_blk = b - bf;
+      }
+      for (int r0 = 0; r0 < rows; r0 += threads / 8) {
         if (r0 + warp * 4 >= rows) break;   // (warp-uniform)
         const int r = r0 + (tid >> 3);
         const bool live = r < rows;
@@ -246,11 +287,11 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
           uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * r + (l8 >> 2)) + (l8 & 3);
           qp[0] = w;
           qp[4] = qplane_d(w);
-          if ((r / p.q_group) % nblk == my_blk)
+          if ((r / q_group) % nblk == my_blk)
             reinterpret_cast<uint32_t*>(ap.q_code_out)[(static_cast<int64_t>(s) * rows + r) * (kCodeWords / 2) + l8] = w;
         }
       }
-      for (int h = my_blk + nblk * (tid >> 3); h - nblk * ((tid >> 3) & 3) < p.H; h += nblk * (kItemThreads / 8)) {
+      for (int h = my_blk + nblk * (tid >> 3); h - nblk * ((tid >> 3) & 3) < p.H; h += nblk * (threads / 8)) {
         // (warp-uniform trip count: the four rows of a warp advance together)
         const bool live = h < p.H;
         const int64_t in_off = (static_cast<int64_t>(s) * p.H + (live ? h : 0)) * kHeadDim + l8 * 16;
@@ -297,7 +338,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
         }
       }
     } else {
-      for (int c = tid; c < 2 * rows; c += kItemThreads) planes[c] = make_qplanes(__ldg(p.q_code + static_cast<int64_t>(s) * 2 * rows + c));
+      for (int c = tid; c < 2 * rows; c += threads) planes[c] = make_qplanes(__ldg(p.q_code + static_cast<int64_t>(s) * 2 * rows + c));
     }
     __syncthreads();   // planes and zeroed counts are visible
 
@@ -315,12 +356,12 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
     auto count_there = [&](int r, int t0, unsigned d) { hist_count(hist, r, t0 / slice_tokens, d); };
     const int f = HP == 4 ? (lane & 7) : HP == 2 ? ((lane >> 1) & 3) : ((lane >> 2) & 1);
     int use = 0;
-    for (int item = first + warp; item < end; item += kItemWarps) {
-      if (slots == 3) cp_async_wait<2>(); else cp_async_wait<1>();
+    for (int item = first + warp; item < end; item += warps) {
+      if (slots == 3) cp_async_wait<2>(); else if (slots == 2) cp_async_wait<1>(); else cp_async_wait<0>();
       __syncwarp();
       const uint4* lrow = ring + use * (kItemBytes / 16) + lane * CPR;
-      const int r_first = piece_u * HP * p.q_group;              // first query row of the item
-      if (p.q_group == 1) {
+      if (!GROUPED) {
+        const int r_first = piece_u * HP;                        // first query row of the item
         const QPlanes* qp0 = planes + 2 * r_first;
 #pragma unroll
         for (int k = 0; k < kGroups; ++k) {
@@ -347,27 +388,35 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
           }
         }
       } else {
-        // grouped queries: a code is read once for the query heads of its cache head
+        // grouped queries: a code is read once for the item's query heads of its cache head
+        auto grouped = [&](int r_first, int heads) {
 #pragma unroll
-        for (int k = 0; k < kGroups; ++k) {
-          const int t0 = tile_u * TT + k * 32, t = t0 + lane;
+          for (int k = 0; k < kGroups; ++k) {
+            const int t0 = tile_u * TT + k * 32, t = t0 + lane;
 #pragma unroll
-          for (int hh = 0; hh < HP; ++hh) {
-            const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
-            const int r1 = r_first + hh * p.q_group;
-            uint16_t* o = out + r1 * p.out_stride + t;
+            for (int hh = 0; hh < HP; ++hh) {
+              const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
+              const int r1 = r_first + hh * q_group;
+              uint16_t* o = out + r1 * p.out_stride + t;
 #pragma unroll 4
-            for (int g = 0; g < p.q_group; ++g) {
-              const int r = r1 + g;
-              const unsigned d = chunk_distance<METRIC>(k0, planes[2 * r]) + chunk_distance<METRIC>(k1, planes[2 * r + 1]);
-              if (t < n) {
-                *o = to_out(d);
-                if (t0 < slice0_end) count_here(r, d);
-                else if (hist) count_there(r, t0, d);
+              for (int g = 0; g < heads; ++g) {
+                const int r = r1 + g;
+                const unsigned d = chunk_distance<METRIC>(k0, planes[2 * r]) + chunk_distance<METRIC>(k1, planes[2 * r + 1]);
+                if (t < n) {
+                  *o = to_out(d);
+                  if (t0 < slice0_end) count_here(r, d);
+                  else if (hist) count_there(r, t0, d);
+                }
+                o += p.out_stride;
               }
-              o += p.out_stride;
             }
           }
+        };
+        if (q_split == 1) {
+          grouped(piece_u * HP * q_group, q_group);   // (a trip count that is the same for all warps)
+        } else {
+          const int heads0 = heads_of(piece_u), g0 = (piece_u - heads0 * q_split) * q_part;
+          grouped(heads0 * HP * q_group + g0, min(q_part, q_group - g0));
         }
       }
       __syncwarp();   // the slot may be filled again
@@ -379,7 +428,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
     if (p.hist || pos < line_end) __syncthreads();
     if (p.count_local) {
       uint32_t* dst = hist + slice0 * kSaBins;
-      for (int i = tid; i < rows * (kItemCountWords / 4); i += kItemThreads) {
+      for (int i = tid; i < rows * (kItemCountWords / 4); i += threads) {
         const uint4 c4 = reinterpret_cast<const uint4*>(counts)[i];
         if (c4.x | c4.y | c4.z | c4.w) {
           const int r = i / (kItemCountWords / 4);

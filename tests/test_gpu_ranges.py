@@ -75,7 +75,7 @@ def test_sparse_decode_list_with_holes():
         _assert_attn_close(o[0, h:h + 1], want)
 
 
-@pytest.mark.parametrize("H,Hq", [(1, 1), (2, 2), (3, 9), (4, 4), (5, 5), (8, 64), (12, 12), (28, 28), (40, 40), (6, 48), (96, 96)])
+@pytest.mark.parametrize("H,Hq", [(1, 1), (2, 2), (3, 9), (4, 4), (5, 5), (8, 64), (4, 28), (2, 32), (12, 12), (28, 28), (40, 40), (6, 48), (96, 96)])
 @pytest.mark.parametrize("L,ps", [(2, 16), (33, 1), (130, 16), (257, 7), (5000, 32), (40001, 16)])
 def test_estimate_items_shapes(H, Hq, L, ps):
     """The estimate for any head count: remainders of its items, one item, several per warp, and (from 1 M distances
