@@ -28,6 +28,7 @@ def test_rope_token_groups(seq, hq, hk):
     (32, 32, 2500, 16),                                   # the line of tiles is cut over the grid
     (32, 8, 9473, 16), (28, 4, 16001, 32),                # grouped queries in one part, line cut inside rows
     (12, 1, 333, 16), (32, 2, 5000, 16), (9, 1, 20000, 1),   # groups of more than 8: several parts
+    (1, 1, 20001, 16), (2, 1, 9000, 16),                  # many parts of one and of two query heads: merged by all warps
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_dense_decode_shapes(hq, hkv, L, ps, dtype):
