@@ -305,6 +305,10 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
       __syncwarp();
     }
     // ---- the warps of a head -> one result per query head ---------------------------------------------------
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) st.o[j][i] *= 1.f / Mma<T>::kScale;
     st.l += __shfl_xor_sync(0xffffffffu, st.l, 1);
     st.l += __shfl_xor_sync(0xffffffffu, st.l, 2);
     if (t == 0) {

@@ -1,4 +1,6 @@
 """Arguments and values at the edge of what the operators take."""
+import math
+
 import pytest
 import torch
 
@@ -13,3 +15,69 @@ def test_flag_that_has_no_truth_value():
     x = torch.zeros(2, 128, dtype=torch.float16, device=DEV)
     with pytest.raises(RuntimeError, match="[Bb]oolean value"):
         K.hadamard_transform(x, inplace=torch.zeros(2))
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float16, 2.0 ** -11), (torch.bfloat16, 2.0 ** -8)])
+def test_many_weights_far_below_the_largest(dtype, tol):
+    """One dominating token over a flat remainder whose weights, 2^-25 of its own, make up 0.4 % of the sum: handler
+    forward, 32-bit partial result and a batched dense step against 64 bits.  The dominating token's V is zero, so the
+    remainder IS the result.  16-bit results may be off by one rounding (and what the partial may be off by, far less); the
+    partial by 1e-5: the logits' difference of 25 is formed in 32 bits (25 * 2^-24 * ln 2 = 1e-6 relative)."""
+    _, K, U = _mods()
+    L, H, ps = 131072, 2, 16
+    q = torch.zeros(1, H, 128, dtype=dtype)
+    k, v = torch.zeros(L, H, 128, dtype=dtype), torch.ones(L, H, 128, dtype=dtype)
+    v += (torch.randn(L, H, 128, generator=torch.Generator().manual_seed(1)) * 0.25).to(dtype)
+    q[..., 0], k[5, :, 0], v[5] = 14.0, 14.0, 0.0      # 196 / sqrt(128) * log2(e) = 25.0
+    s = torch.einsum("hd,lhd->hl", q[0].double(), k.double()) / 128.0 ** 0.5
+    want = torch.einsum("hl,lhd->hd", torch.softmax(s, 1), v.double())
+
+    pages = L // ps
+    kv = torch.stack([k.view(pages, ps, H, 128), v.view(pages, ps, H, 128)], 1).to(DEV)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)[: pages - 1].unsqueeze(0).expand(H, pages - 1)
+    w = K.BatchDecodeWithPagedKVCachePyTorchWrapper(0)
+    w.begin_forward(torch.tensor([0, pages], dtype=torch.int32), H, H, 128, ps, torch.empty(0, dtype=dtype))
+    o, part, lse = torch.empty(1, H, 128, dtype=dtype, device=DEV), torch.empty(H, 128, device=DEV), torch.empty(H, device=DEV)
+    w.forward(q.to(DEV), o, kv, table, None, ps, pages - 1, lse=lse)
+    torch.testing.assert_close(o[0].cpu().double(), want, rtol=tol * 1.05, atol=0)
+    w.forward(q.to(DEV), None, kv, table, None, ps, pages - 1, lse=lse, o_f32=part)
+    torch.testing.assert_close(part.cpu().double(), want, rtol=1e-5, atol=0)
+    torch.testing.assert_close(lse.cpu().double(), torch.logsumexp(s, 1) / math.log(2.0), rtol=1e-6, atol=1e-5)
+
+    controllers = []
+    for n in (L, 4096):
+        c = U.InferenceController(1, H, 128, ps, 4, L, dtype, DEV)
+        c.prepare_hadamard(n - 1)
+        c.begin_forward(n - 1)
+        U.append_kvh(k[: n - 1].to(DEV), v[: n - 1].to(DEV), None, c, 0)
+        c.end_forward()
+        controllers.append(c)
+    batch = U.SequenceBatch(controllers)
+    batch.prepare(1)
+    batch.sync_seq_lens()
+    row = lambda x: torch.stack([x[L - 1], x[4095]]).to(DEV)
+    got = batch.decode_step_dev(q.expand(2, H, 128).contiguous().to(DEV), row(k), row(v), 0, dense=True)
+    torch.testing.assert_close(got[0].cpu().double(), want, rtol=tol * 1.05, atol=0)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_long_sums_are_rounded(dtype):
+    """32768 tokens of nearly equal weight and V = 2 + noise: the 32-bit result keeps to 1e-6.  A warp adds up 55 tiles one after
+    the other, each sum rounded to 2^-24 of itself at most: 55 * 2^-24 = 3e-6 if all went one way, as cutting off
+    would, and sqrt(55) * 2^-24 = 4e-7 as roundings go."""
+    _, K, _ = _mods()
+    L, H, ps = 32768, 32, 16
+    g = torch.Generator(device=DEV).manual_seed(7)
+    kv = torch.randn(L // ps, 2, ps, H, 128, device=DEV, generator=g)
+    kv[:, 1] += 2
+    kv = kv.to(dtype)
+    q = (torch.randn(1, H, 128, device=DEV, generator=g) * 0.1).to(dtype)
+    w = K.BatchDecodeWithPagedKVCachePyTorchWrapper(0)
+    w.begin_forward(torch.tensor([0, L // ps], dtype=torch.int32), H, H, 128, ps, torch.empty(0, dtype=dtype))
+    table = torch.arange(L // ps - 1, dtype=torch.int32, device=DEV).unsqueeze(0).expand(H, L // ps - 1)
+    part, lse = torch.empty(H, 128, device=DEV), torch.empty(H, device=DEV)
+    w.forward(q, None, kv, table, None, ps, L // ps - 1, lse=lse, o_f32=part)
+    k, v = (kv[:, i].reshape(L, H, 128).double() for i in (0, 1))
+    p = torch.softmax(torch.einsum("hd,lhd->hl", q[0].double(), k) / 128.0 ** 0.5, 1)
+    want = torch.einsum("hl,lhd->hd", p, v)
+    assert float((part.double() - want).norm() / want.norm()) < 1e-6
