@@ -391,8 +391,8 @@ class BatchDecodeWithPagedKVCachePyTorchWrapper:
 
 def set_max_cluster(blocks: int) -> None:
     """Upper bound (1, 2, 4, 8) on the thread blocks that share one head in select_attend /
-    decode_step: 8 is fastest for a single sequence, smaller values let calls of several sequences
-    on different streams overlap."""
+    decode_step: 8, the default, chooses by itself (up to sixteen) and is fastest for a single sequence,
+    smaller values let calls of several sequences on different streams overlap."""
     _lib.check(lib.adamas_set_max_cluster(int(blocks)), "set_max_cluster")
 
 

@@ -203,12 +203,12 @@ bool fused_append_enabled() { return setting(g_fused_append, "ADAMAS_FUSED_APPEN
 // ADAMAS_EST_BLOCKS_PER_SM): 2 by default, 1 leaves half of every SM to kernels of other streams.
 std::atomic<int> g_est_blocks_per_sm{-1};
 int est_blocks_per_sm() { return setting(g_est_blocks_per_sm, "ADAMAS_EST_BLOCKS_PER_SM", 2, 1, 2); }
-// Upper bound on the blocks per head of select_attend (adamas_set_max_cluster / ADAMAS_MAX_CLUSTER); while neither has
-// been given, what the histogram table has room for.
+// Upper bound on the blocks per head of select_attend (adamas_set_max_cluster / ADAMAS_MAX_CLUSTER).  The default and largest
+// value means automatic: what the histogram table has room for.
 std::atomic<int> g_max_cluster{-1};
 int max_cluster() {
-  const int v = setting(g_max_cluster, "ADAMAS_MAX_CLUSTER", kSaMaxSlices, 1, kSaMaxCluster);
-  return (v & (v - 1)) == 0 ? v : kSaMaxSlices;
+  const int v = setting(g_max_cluster, "ADAMAS_MAX_CLUSTER", kSaMaxCluster, 1, kSaMaxCluster);
+  return v < kSaMaxCluster && (v & (v - 1)) == 0 ? v : kSaMaxSlices;
 }
 
 template <typename... KArgs, typename... Args>

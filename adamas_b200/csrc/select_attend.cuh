@@ -47,7 +47,7 @@ constexpr int kSaRows = 24;           // rows of a warp's tile
 constexpr int kSaWarpBytes = 2 * kSaRows * kHeadDim * 2;
 constexpr int kSaTileBytes = kSaWarps * kSaWarpBytes;
 constexpr int kSaMaxBlockTokens = 32768;
-constexpr int kSaMaxCluster = 8;      // upper bound of adamas_set_max_cluster
+constexpr int kSaMaxCluster = 8;      // largest value of adamas_set_max_cluster: as many blocks per head as are of use
 
 // Scratch words (32 bit) per head: kSaMaxSlices histogram rows of 512 counts, then kSaMaxSlices slots of
 // kSaSlotWords floats for the blocks' partial results (128 outputs, running max, running sum; word 130

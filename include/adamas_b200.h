@@ -100,10 +100,10 @@ int adamas_set_estimate_blocks_per_sm(int blocks);
 
 /* Upper bound (1, 2, 4 or 8; default 8, or ADAMAS_MAX_CLUSTER in the environment) on the number of
  * thread blocks that share one head in adamas_select_attend / adamas_decode_step.  8 means automatic:
- * eight blocks per head, or up to sixteen while all blocks of the launch are resident at once (the
+ * as many as are of use, up to sixteen, while all blocks of the launch are resident at once (the
  * shortest single call); fewer take longer per call but leave room on the
  * GPU for calls of other sequences running on other streams (a batch of independent sequences).  Rows
- * longer than 32768 x the bound are rejected.  No counterpart in the reference (batch 1 only). */
+ * longer than 32768 x the bound (524288 where it is automatic) are rejected.  No counterpart in the reference (batch 1 only). */
 int adamas_set_max_cluster(int blocks);
 
 /* ---- stage 1: Hadamard transform, bucketize, pack, append -------------------------------- */
@@ -301,7 +301,7 @@ int adamas_decode_forward_static(const void* q, void* o, float* lse, const void*
  * cut-valued elements THIS call takes, per head, decided elsewhere (the global cut of a sequence split
  * over several GPUs); k is then only an upper bound for the winners of this call.
  * Replaces the topk_filtering + BatchDecodeWithPagedKVCachePyTorchWrapper::Forward pair
- * (adamas/models/Adamas.py:185-200) for n up to 262144 (32768 x the adamas_set_max_cluster bound). */
+ * (adamas/models/Adamas.py:185-200) for n up to 524288 (fewer with an adamas_set_max_cluster bound). */
 int adamas_select_attend(const void* dist, int64_t dist_stride, int n, int k, const void* q, void* o,
                          float* o_f32, float* lse, const void* kv_data, const int32_t* kv_page_table,
                          int page_size, int num_heads, int num_q_heads, int head_dim, int dtype,

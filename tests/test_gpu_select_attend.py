@@ -114,6 +114,15 @@ def test_select_attend_sixteen_block_clusters(n, k, H):
     assert _lib.device_error(clear=False) == 0
 
 
+def test_restored_bound_is_the_default():
+    """Setting the bound and restoring 8 leaves launches of the shape they have in a fresh process: more than eight blocks
+    per head, and rows longer than 8 * 32768."""
+    _, K, _ = _mods()
+    K.set_max_cluster(2)
+    K.set_max_cluster(8)
+    assert [K.select_attend_slices(*s) for s in [(140000, 2047, 2), (400000, 100, 1)]] == [16, 16]
+
+
 def test_select_attend_with_prepared_histograms_and_without_newest_token():
     """The two-call form (estimate with hist, select_attend with hist_ready) and last_page_len = 0
     (no newest token: a sequence shard that does not hold it), with an fp32 partial output."""
