@@ -625,16 +625,21 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   // behind (whole step, 3000 tokens: 8 heads 12.1 -> 10.7 us, 28 over 4 14.7 -> 14.1; one head, 60K: 14.5 -> 12.4).  They code
   // 32 query heads in one pass; with 64 the second pass costs what this gains (16.1 / 18.1 us).
   const int64_t per_block = (items + grid.x - 1) / grid.x;
-  const int warps = per_block <= kItemWarps / 2 && q_heads <= 2 * kItemWarps ? kItemWarps / 2 : kItemWarps;
+  // One block per SM as the setting: half a block as well, with no more than half of the SM's shared memory, where the query
+  // planes leave room for two ring slots per warp.
+  const size_t planes = static_cast<size_t>(q_heads) * 2 * sizeof(QPlanes), half_sm = static_cast<size_t>(di->smem_per_sm / 2 - 1024 - kEstStatic);
+  const bool half = est_blocks_per_sm() == 1 && planes + kItemWarps / 2 * 2 * kItemBytes <= half_sm;
+  const int warps = half || (per_block <= kItemWarps / 2 && q_heads <= 2 * kItemWarps) ? kItemWarps / 2 : kItemWarps;
+  const size_t room = half ? half_sm : most;
   const size_t slot = static_cast<size_t>(warps) * kItemBytes, counts = static_cast<size_t>(q_heads) * kItemCountWords * sizeof(uint32_t);
   const int wanted = static_cast<int>(std::min<int64_t>(3, (per_block + warps - 1) / warps)), least = std::min(wanted, 2);   // ring slots
   // The counts in shared memory where they fit beside two ring slots per warp and where there are enough distances to be
   // worth clearing and adding up a table per block (12K tokens x 40 heads: 6.4 us with an L2 atomic each, 7.5 with tables;
   // 30K x 32: 8.8 / 8.7; 64K x 64: 26.9 / 21.1); a third slot where it fits beside them.
-  size_t smem = static_cast<size_t>(q_heads) * 2 * sizeof(QPlanes);
-  prm.count_local = hist && static_cast<int64_t>(q_heads) * n * batch >= (int64_t(1) << 20) && smem + least * slot + counts <= most ? 1 : 0;
+  size_t smem = planes;
+  prm.count_local = hist && static_cast<int64_t>(q_heads) * n * batch >= (int64_t(1) << 20) && smem + least * slot + counts <= room ? 1 : 0;
   if (prm.count_local) smem += counts;
-  const int slots = smem + wanted * slot <= most ? wanted : least;
+  const int slots = smem + wanted * slot <= room ? wanted : least;
   smem += slots * slot;
   ADAMAS_REQUIRE(smem <= most, "num_q_heads (%d) too large for the estimate kernel", q_heads);
 #define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_items_kernel", (__VA_ARGS__), grid, dim3(warps * 32), smem, st, 1, prm, slots)

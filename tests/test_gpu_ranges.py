@@ -115,6 +115,31 @@ def test_estimate_items_shapes(H, Hq, L, ps):
             assert torch.equal(counts[r, sl].to(torch.int64), torch.bincount(want[r, sl * per:(sl + 1) * per], minlength=512))
 
 
+@pytest.mark.parametrize("H,Hq", [(40, 40), (8, 64), (4, 4), (1000, 1000)])   # (1000: too many query planes for half an SM's memory)
+def test_estimate_leaves_half_of_every_sm(H, Hq):
+    """One estimate block per SM as the setting: the same distances and counts, from half of the SM's registers and shared
+    memory."""
+    _, K, _ = _mods()
+    L, ps = 9001 if H < 1000 else 1100, 16
+    g = torch.Generator().manual_seed(H)
+    pages = (L + ps - 1) // ps
+    codes = torch.randint(-32768, 32768, (pages, 1, ps, H, 16), generator=g, dtype=torch.int32).to(torch.int16).to(DEV)
+    q = torch.randint(-32768, 32768, (1, Hq, 16), generator=g, dtype=torch.int32).to(torch.int16).to(DEV)
+    table = torch.randperm(pages, generator=g).to(torch.int32).to(DEV)
+    results = []
+    for blocks in (2, 1):
+        K.set_estimate_blocks_per_sm(blocks)
+        try:
+            out = torch.zeros(Hq, L - 1, dtype=torch.int16, device=DEV)
+            hist = K.histogram_scratch(Hq, DEV)
+            K.estimate_attn_score(q, out, codes, table, None, L - (pages - 1) * ps, 0, 0, hist=hist, hist_slices=4)
+            results.append((out, K.histogram_counts(hist)))
+        finally:
+            K.set_estimate_blocks_per_sm(2)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("n,k,H,ps", [
     (1, 1, 3, 16), (9, 9, 4, 1),                       # fewer granules than threads; everything wins
     (2047, 96, 32, 16), (2049, 97, 32, 16),            # one block per head / two; winners around one tile per warp
