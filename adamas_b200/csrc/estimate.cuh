@@ -140,11 +140,14 @@ struct EstimateParams {
   StepAppend ap;
 };
 
+// Tiles of n tokens.  A sequence whose first token is being appended (n = 0) has an empty one: somebody has to append.
+__device__ __forceinline__ int est_tiles(int n, int tile_tokens) { return n == 0 ? 1 : (n + tile_tokens - 1) / tile_tokens; }
+
 // Tiles of `tile_tokens` tokens of the batch's sequences in front of each one -> cum[0 .. batch]; one warp.
 __device__ __forceinline__ void est_line(const EstimateParams& p, int tile_tokens, int lane, int* cum) {
   int base = 0;
   for (int s0 = 0; s0 < p.batch; s0 += 32) {
-    int v = s0 + lane < p.batch ? (__ldg(p.seq_len_dev + s0 + lane) - 1 + tile_tokens - 1) / tile_tokens : 0;
+    int v = s0 + lane < p.batch ? est_tiles(__ldg(p.seq_len_dev + s0 + lane) - 1, tile_tokens) : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, v, o);

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
     __syncthreads();
     tiles_all = sh.cum[p.batch];
   } else {
-    tiles_all = ((p.seq_len_dev ? __ldg(p.seq_len_dev) - 1 : p.n_tokens) + TT - 1) / TT;
+    tiles_all = est_tiles(p.seq_len_dev ? __ldg(p.seq_len_dev) - 1 : p.n_tokens, TT);
   }
   const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
   const int q_split = q_part == q_group ? 1 : (q_group + q_part - 1) / q_part, pieces = p.H / HP * q_split;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
     auto fetch_entries = [&](int tile) {
 #pragma unroll
       for (int k = 0; k < kGroups; ++k) {
-        const unsigned t = static_cast<unsigned>(min(tile * TT + k * 32 + lane, n - 1));   // (absent tokens: the last one's codes)
+        const unsigned t = static_cast<unsigned>(min(tile * TT + k * 32 + lane, max(n - 1, 0)));   // (absent tokens: the last one's codes)
         entry[k] = __ldg(table + (p.ps_shift >= 0 ? t >> p.ps_shift : t / static_cast<unsigned>(p.page_size)));
       }
     };
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
       int tok[kGroups];
 #pragma unroll
       for (int k = 0; k < kGroups; ++k) {
-        const unsigned t = static_cast<unsigned>(min(tile * TT + k * 32 + lane, n - 1)), ps = static_cast<unsigned>(p.page_size);
+        const unsigned t = static_cast<unsigned>(min(tile * TT + k * 32 + lane, max(n - 1, 0))), ps = static_cast<unsigned>(p.page_size);
         tok[k] = entry[k] * p.page_size + static_cast<int>(p.ps_shift >= 0 ? t & (ps - 1) : t % ps);
       }
       constexpr int RPI = 32 / CPR;   // tokens per copy instruction
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
     __syncthreads();   // planes and zeroed counts are visible
 
     // ---- scan -----------------------------------------------------------------------------------------------------
-    const int slice_tokens = p.hist ? 8 * sa_granules_per_block(n, p.hist_cl) : 1;
+    const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
     // the counts in shared memory are those of the slice in which this piece starts; tokens of later slices (few, unless
     // the sequences are far shorter than a block's share) are counted in global memory one by one
     const int slice0 = p.hist ? first / pieces * TT / slice_tokens : 0;

@@ -200,3 +200,42 @@ def test_merge_states_with_every_part_empty():
     want, _ = ref.merge_states(o_parts[:, keep], lse[:, keep] * float(np.log(2.0)))
     _assert_attn_close(o[keep], want)
     assert torch.isfinite(o.float()).all()
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (40, 40), (8, 2), (32, 32)])
+def test_first_token_of_a_sequence(hq, hkv):
+    """A device length of 1 (nothing to select from, which sets the error flag): the token is still appended and attended to, in
+    two launches as in three, by itself and beside a longer sequence."""
+    from adamas_b200 import _lib
+    _, K, U = _mods()
+    q, k, v = (_randn((2, h, 128), s, torch.float16).to(DEV) for s, h in ((1, hq), (2, hkv), (3, hkv)))
+    results = []
+    for fused in (True, False):
+        K.set_fused_append(fused)
+        try:
+            out = []
+            cs = [U.InferenceController(1, hkv, 128, 16, 4, 1024, torch.float16, DEV, num_q_heads=hq) for _ in range(3)]
+            for c in cs:
+                c.kv_cache.pool.buf.zero_()
+                c.hadamard_cache.pool.buf.zero_()
+            cs[2].prepare_hadamard(699)
+            cs[2].begin_forward(699)
+            U.append_kvh(_randn((699, hkv, 128), 4, torch.float16).to(DEV), _randn((699, hkv, 128), 5, torch.float16).to(DEV), None, cs[2], 0)
+            cs[2].end_forward()
+            cs[0].prepare_hadamard(1)
+            cs[0].sync_seq_len()
+            out.append(U.decode_step_dev(q[:1], k[:1], v[:1], cs[0], 0))
+            batch = U.SequenceBatch(cs[1:])
+            batch.prepare(1)
+            batch.sync_seq_lens()
+            out.append(batch.decode_step_dev(q, k, v, 0))
+            for c in cs:
+                out += [c.kv_cache.pool.buf, c.hadamard_cache.pool.buf.view(torch.int16)]
+            torch.cuda.synchronize()
+        finally:
+            K.set_fused_append(True)
+            _lib.device_error(clear=True)
+        assert torch.equal(out[0][0], v[0].repeat_interleave(hq // hkv, 0)) and torch.equal(out[1][0], out[0][0])
+        results.append(out)
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
