@@ -615,6 +615,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
 #undef LAUNCH_EST
     return check_launch("estimate_kernel");
   }
+  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0, "q_code must be 16-byte aligned");
   const int hp = num_heads % 4 == 0 ? 4 : num_heads % 2 == 0 ? 2 : 1;   // heads per item: as long a run of a token's codes as divides
   int64_t items = static_cast<int64_t>((n + 128 / hp - 1) / (128 / hp)) * (num_heads / hp) * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
@@ -1237,6 +1238,7 @@ int adamas_select_attend(const void* dist, int64_t dist_stride, int n, int k, co
   const int kv_heads = num_heads;
   num_heads = num_q_heads;   // rows of dist, q, o, hist, out_idx
   ADAMAS_REQUIRE(dist && q && (o || o_f32) && kv_data && kv_page_table && hist, "null pointer");
+  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(hist) & 15) == 0, "the histogram scratch must be 16-byte aligned");
   ADAMAS_REQUIRE(!o_f32 || lse, "a partial result (o_f32) needs lse");
   ADAMAS_REQUIRE(n >= 1 && k >= 1 && k <= n, "need 1 <= k <= n (k=%d, n=%d)", k, n);
   ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(dist) & 15) == 0 && (num_heads == 1 || (dist_stride * 2) % 16 == 0),
@@ -1390,6 +1392,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
                  static_cast<long long>(seq_len), budget);
   ADAMAS_REQUIRE(seq_len - 1 < (int64_t(1) << 31) - 1024, "sequence too long");
   ADAMAS_REQUIRE(q && o && dist_scratch && q_code && hist, "null pointer");
+  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(hist) & 15) == 0, "the histogram scratch must be 16-byte aligned");
   ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(dist_scratch) & 15) == 0 && (dist_stride * 2) % 16 == 0,
                  "distance rows must start on 16-byte boundaries");
   ADAMAS_REQUIRE(out_idx == nullptr || out_stride >= budget - 1 || q_heads * batch == 1, "out_stride smaller than budget - 1");

@@ -337,10 +337,24 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
       const int out = q_row0 + h;
       const float inv = L > 0.f ? 1.f / L : 0.f;   // nothing attended: zeros and lse = -inf
       acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
-      if (p.o_f32) reinterpret_cast<float4*>(p.o_f32 + static_cast<int64_t>(out) * kHeadDim)[lane] = acc;
-      if (p.o)
-        reinterpret_cast<uint2*>(static_cast<T*>(p.o) + static_cast<int64_t>(out) * kHeadDim)[lane] =
-            make_uint2(Elem<T>::from_f2(acc.x, acc.y), Elem<T>::from_f2(acc.z, acc.w));
+      // (results need the alignment of a 32-bit word only; whole vectors where the buffers have theirs)
+      if (p.o_f32) {
+        float* dst = p.o_f32 + static_cast<int64_t>(out) * kHeadDim + 4 * lane;
+        if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+          *reinterpret_cast<float4*>(dst) = acc;
+        } else {
+          dst[0] = acc.x; dst[1] = acc.y; dst[2] = acc.z; dst[3] = acc.w;
+        }
+      }
+      if (p.o) {
+        uint32_t* dst = reinterpret_cast<uint32_t*>(static_cast<T*>(p.o) + static_cast<int64_t>(out) * kHeadDim) + 2 * lane;
+        const uint32_t a = Elem<T>::from_f2(acc.x, acc.y), b = Elem<T>::from_f2(acc.z, acc.w);
+        if ((reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+          *reinterpret_cast<uint2*>(dst) = make_uint2(a, b);
+        } else {
+          dst[0] = a; dst[1] = b;
+        }
+      }
       if (lane == 0 && p.lse) p.lse[out] = L > 0.f ? M + log2f(L) : -INFINITY;
     };
     for (int h = warp; h < gsub; h += kDecWarps) {

@@ -81,3 +81,30 @@ def test_long_sums_are_rounded(dtype):
     p = torch.softmax(torch.einsum("hd,lhd->hl", q[0].double(), k) / 128.0 ** 0.5, 1)
     want = torch.einsum("hl,lhd->hd", p, v)
     assert float((part.double() - want).norm() / want.norm()) < 1e-6
+
+
+def test_results_at_the_alignment_of_a_word():
+    """Attention writes to any buffer whose rows start on a 32-bit word; scratch that the kernels read in vectors is checked."""
+    _, K, _ = _mods()
+    H, ps, pages, last = 3, 16, 7, 4
+    g = torch.Generator().manual_seed(1)
+    kv = torch.randn(pages, 2, ps, H, 128, generator=g).half().to(DEV)
+    q = torch.randn(1, H, 128, generator=g).half().to(DEV)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)
+    lists = table[: pages - 1].unsqueeze(0).expand(H, pages - 1)
+    w = K.BatchDecodeWithPagedKVCachePyTorchWrapper(0)
+    w.begin_forward(torch.tensor([0, pages], dtype=torch.int32), H, H, 128, ps, torch.empty(0, dtype=torch.float16))
+    o, part, lse = torch.empty_like(q), torch.empty(H, 128, device=DEV), torch.empty(H, device=DEV)
+    w.forward(q, o, kv, lists, None, last, pages - 1)
+    w.forward(q, None, kv, lists, None, last, pages - 1, lse=lse, o_f32=part)
+    for off in (1, 2, 3):
+        o2 = torch.empty(H * 128 + 8, dtype=torch.float16, device=DEV)[2 * off: 2 * off + H * 128].view(1, H, 128)
+        p2 = torch.empty(H * 128 + 4, device=DEV)[off: off + H * 128].view(H, 128)
+        w.forward(q, o2, kv, lists, None, last, pages - 1)
+        w.forward(q, None, kv, lists, None, last, pages - 1, lse=lse, o_f32=p2)
+        assert torch.equal(o, o2) and torch.equal(part, p2)
+    dist = torch.zeros(H, 104, dtype=torch.int16, device=DEV)[:, :99]
+    words = K.histogram_scratch(H, DEV).numel()
+    hist = torch.zeros(words + 1, dtype=torch.int32, device=DEV)[1:]
+    with pytest.raises(RuntimeError, match="aligned"):
+        K.select_attend(dist, 10, q, o, kv, table, last, pages - 1, hist=hist, hist_ready=True)
