@@ -12,6 +12,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run with -m gpu on a B200)")
 
 
+@pytest.fixture(autouse=True)
+def _default_settings(request):
+    """The library's launch settings are process-wide: every GPU test starts from the defaults, whatever the one before set."""
+    if "gpu" in request.keywords:
+        from adamas_b200 import _kernels as K
+        K.set_max_cluster(int(os.environ.get("ADAMAS_MAX_CLUSTER", 8)))
+        K.set_estimate_blocks_per_sm(int(os.environ.get("ADAMAS_EST_BLOCKS_PER_SM", 2)))
+        K.set_fused_append(os.environ.get("ADAMAS_FUSED_APPEND", "1") != "0")
+
+
 def pytest_collection_modifyitems(config, items):
     import torch
     if torch.cuda.is_available():

@@ -208,3 +208,43 @@ def test_large_launches_count_their_histograms_in_a_launch_of_their_own():
     _assert_attn_close(o[0], r["out"])
     from adamas_b200 import _lib
     assert _lib.device_error(clear=False) == 0
+
+
+@pytest.mark.parametrize("fused_append", [True, False])
+@pytest.mark.parametrize("lengths,Hq,H,budget", [
+    ([90000, 70001, 85000, 77777], 4, 4, 2048),         # blocks take pieces of two sequences
+    ([40000, 9001, 3000, 35000], 32, 8, 512),           # ... of grouped queries
+    ([20000, 9001, 3000, 15000, 600], 32, 8, 512),      # every block a piece of one sequence
+    ([21000] + [300] * 40, 40, 40, 256),                # short sequences: several in a block, several slices in a piece
+])
+def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
+    """From 1 M distances on a batch is counted in shared memory (head counts other than 16, 32 and 64, and grouped queries): the
+    same selection as each sequence by itself, and a table that is zero afterwards."""
+    _, K, U = _mods()
+    B, ps, cap = len(lengths), 16, max(lengths) + 16
+    assert Hq * B * cap >= 1 << 20
+    gen = torch.Generator(device=DEV).manual_seed(B)
+    rand = lambda *shape: torch.randn(*shape, device=DEV, dtype=torch.float16, generator=gen)
+    both = [[U.InferenceController(1, H, 128, ps, budget // ps, cap, torch.float16, DEV, num_q_heads=Hq) for _ in lengths] for _ in range(2)]
+    for i, L in enumerate(lengths):
+        k, v = rand(L - 1, H, 128), rand(L - 1, H, 128)
+        for cs in both:
+            cs[i].prepare_hadamard(L - 1)
+            cs[i].begin_forward(L - 1)
+            U.append_kvh(k, v, None, cs[i], 0)
+            cs[i].end_forward()
+    q, k, v = rand(B, Hq, 128), rand(B, H, 128), rand(B, H, 128)
+    K.set_fused_append(fused_append)
+    batch = U.SequenceBatch(both[0])
+    batch.prepare(1)
+    batch.sync_seq_lens()
+    idx = torch.full((B * Hq, budget - 1), -1, dtype=torch.int32, device=DEV)
+    o = batch.decode_step_dev(q, k, v, 0, indices_out=idx)
+    assert int(K.histogram_counts(batch._hist).abs().sum()) == 0
+    for i, c in enumerate(both[1]):
+        c.prepare_hadamard(1)
+        c.begin_forward(1)
+        want = U.decode_step(q[i:i + 1], k[i:i + 1], v[i:i + 1], c, 0)
+        assert torch.equal(idx[i * Hq:(i + 1) * Hq], c.topk_dindices_buffer), f"sequence {i}"
+        _assert_attn_close(o[i], want[0])
+        c.end_forward()

@@ -140,15 +140,23 @@ def test_estimate_leaves_half_of_every_sm(H, Hq):
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("n,k,H,ps", [
-    (1, 1, 3, 16), (9, 9, 4, 1),                       # fewer granules than threads; everything wins
-    (2047, 96, 32, 16), (2049, 97, 32, 16),            # one block per head / two; winners around one tile per warp
-    (30000, 1023, 32, 16), (32768, 2047, 8, 1),        # two blocks share a histogram slice; page numbers not staged (page size 1)
-    (40001, 4000, 4, 7),                               # several rounds per warp, a page size that is no power of two
-    (100000, 63, 100, 32),                             # few blocks per row: distances beyond the staged ones
+def _blocks_per_head(hist):
+    """Thread blocks per head of the last select_attend launch with this scratch table (zeroed before): the slots of partial
+    results that hold a sum (a single block leaves none)."""
+    slots = hist.view(hist.size(0), -1)[:, 16 * 512:].view(hist.size(0), 16, 132)
+    return max(1, int((slots[:, :, 129] != 0).sum(1).max()))
+
+
+@pytest.mark.parametrize("n,k,H,ps,blocks,slices", [
+    (1, 1, 3, 16, 1, 1), (9, 9, 4, 1, 1, 1),           # fewer granules than threads; everything wins
+    (2047, 72, 32, 16, 1, 1), (2049, 73, 32, 16, 2, 2),   # one block per head / two; winners around the rows of its tiles
+    (2047, 96, 32, 16, 2, 2), (2049, 97, 32, 16, 2, 2),
+    (30000, 1023, 32, 16, 16, 8), (32768, 2047, 8, 1, 16, 8),   # two blocks share a histogram slice; page numbers not staged (page size 1)
+    (40001, 4000, 4, 7, 16, 16),                       # several rounds per warp, a page size that is no power of two
+    (100000, 63, 100, 32, 5, 5),                       # few blocks per row: distances beyond the staged ones
 ])
 @pytest.mark.parametrize("ties", [False, True])
-def test_select_attend_shapes(n, k, H, ps, ties):
+def test_select_attend_shapes(n, k, H, ps, blocks, slices, ties):
     """Selection (exact, ties to the lower position) and attention at the edges of the launch shapes."""
     _, K, _ = _mods()
     g = torch.Generator().manual_seed(n + k)
@@ -164,6 +172,8 @@ def test_select_attend_shapes(n, k, H, ps, ties):
     hist = K.histogram_scratch(H, DEV)
     for _ in range(2):
         K.select_attend(store[:, :n], k, q.to(DEV), o, kv, perm.to(torch.int32).to(DEV), 0, 0, indices_out=idx, hist=hist)
+    # (with ties all winners are at the front: blocks without any leave no sum)
+    assert K.select_attend_slices(n, k, H) == slices and (ties or _blocks_per_head(hist) == blocks)
     order = torch.argsort(dist * (n + 1) + torch.arange(n), 1)[:, :k].sort(1).values          # ascending positions of the winners
     slots = (perm[order // ps] * ps + order % ps).to(torch.int32)
     assert torch.equal(idx.cpu(), slots)
