@@ -54,6 +54,16 @@ struct TileState {
   float o[8][4];
 };
 
+// acc += w v; nothing where w is 0, whatever v is.
+__device__ __forceinline__ void add_weighted(float4& acc, float w, float4 v) {
+  if (w != 0.f) {
+    acc.x = fmaf(w, v.x, acc.x);
+    acc.y = fmaf(w, v.y, acc.y);
+    acc.z = fmaf(w, v.z, acc.z);
+    acc.w = fmaf(w, v.w, acc.w);
+  }
+}
+
 __device__ __forceinline__ int tile_swizzle(int r) { return (r & 6) ^ ((r & 1) << 2); }
 
 __device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
@@ -98,7 +108,9 @@ __device__ __forceinline__ void tile_logits(const uint8_t* slot, const uint4 (&q
   }
 }
 
-// Softmax in base 2 and P.V over a tile of 16 tokens; at least one token must exist, and rows of absent ones must hold finite values.
+// Softmax in base 2 and P.V over a tile of 16 tokens; at least one token must exist, and absent ones must hold the row of one that
+// does.  A V row with an infinity or a NaN ends as a NaN whatever its weight is (the matrix form multiplies it by every part
+// of every weight, zeros and negative ones among them): the caller looks for that at the end.
 template <typename T>
 __device__ __forceinline__ void tile_softmax_pv(TileState& st, const uint8_t* slot, const float (&s)[4], int lane) {
   const int g = lane >> 2, t = lane & 3;
@@ -128,8 +140,9 @@ __device__ __forceinline__ void tile_softmax_pv(TileState& st, const uint8_t* sl
     }
   }
   float pr[4];
+  const float base = st.m == -INFINITY ? 0.f : st.m;   // (no logit above -inf so far: no weight)
 #pragma unroll
-  for (int u = 0; u < 4; ++u) pr[u] = exp2f(s[u] - st.m);   // (a masked token: exp2(-inf) = 0; st.m is finite)
+  for (int u = 0; u < 4; ++u) pr[u] = exp2f(s[u] - base);   // (a masked token: exp2(-inf) = 0)
   st.l += (pr[0] + pr[1]) + (pr[2] + pr[3]);
   // B fragments of P.V: tokens 2t, 2t + 1 and 2t + 8, 2t + 9 of head g
   uint32_t b[Mma<T>::kParts][2];

@@ -412,15 +412,17 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
       for (int u = 1; u < kSaRows / 4; ++u) m_new = fmaxf(m_new, sc[u]);
       m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
       m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
-      m_new = fmaxf(m_run, __shfl_sync(0xffffffffu, m_new, 0));   // finite: the tile's first token exists
-      const float rescale = exp2f(m_run - m_new);
+      m_new = fmaxf(m_run, __shfl_sync(0xffffffffu, m_new, 0));
+      const float base = m_new == -INFINITY ? 0.f : m_new;   // (no logit above -inf so far: no weight)
+      const float rescale = exp2f(m_run - base);
       m_run = m_new;
       l_run *= rescale;
       acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
 #pragma unroll
       for (int u = 0; u < kSaRows / 4; ++u) {
-        sc[u] = exp2f(sc[u] - m_new);
+        sc[u] = exp2f(sc[u] - base);
         l_run += sc[u];
+        sc[u] = fmaxf(sc[u], 1.4e-45f);   // (0 times an infinity, in the row that an absent one borrows, would be a NaN)
       }
       const uint8_t* vbase = tile + kSaRows * 256 + (lane & 1) * 8;
 #pragma unroll
@@ -455,7 +457,8 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     const float m = sh.ml[w2][0];
     const float w = (m == -INFINITY) ? 0.f : exp2f(m - M);
     L += w * sh.ml[w2][1];
-    od += w * reinterpret_cast<const float*>(sa_smem + w2 * kSaWarpBytes)[tid];
+    const float part = reinterpret_cast<const float*>(sa_smem + w2 * kSaWarpBytes)[tid];
+    if (w != 0.f) od += w * part;   // (it may be infinite)
   }
   unsigned* counter = head_scratch + kSaMaxSlices * kSaBins + kHeadDim + 2;   // word 130 of slot 0
   if (CL > 1) {
@@ -491,7 +494,10 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     L = __shfl_sync(0xffffffffu, L, 0);
     od = 0.f;
 #pragma unroll
-    for (unsigned r = 0; r < kSaMaxSlices; ++r) od = fmaf(__shfl_sync(0xffffffffu, w, r), po[r], od);
+    for (unsigned r = 0; r < kSaMaxSlices; ++r) {
+      const float wr = __shfl_sync(0xffffffffu, w, r);
+      if (wr != 0.f) od = fmaf(wr, po[r], od);
+    }
   }
   const float res = L > 0.f ? od / L : 0.f;
   const float res1 = __shfl_down_sync(0xffffffffu, res, 1);

@@ -127,6 +127,49 @@ __device__ __forceinline__ unsigned dec_request(const DecodeParams& p, const Dec
   return mask;
 }
 
+// A warp's piece of a row group once more, token by token with fp32 weights, for pieces whose result is not finite: a V row with
+// an infinity or a NaN then counts as weight times value does, and not at all where its weight is 0.  `at`: the group's results
+// (128 floats each), `ml`: their (max, sum).
+template <typename T>
+__device__ __noinline__ void dec_plain(const DecodeParams& p, DecRow r, const T* kbase, int64_t row_elems, const T* q, int gsub,
+                                       int first, int end, int lane, float* at, float (*ml)[2]) {
+  auto row4 = [&](const T* src) {
+    const uint2 u = *reinterpret_cast<const uint2*>(src + 4 * lane);
+    const float2 a = Elem<T>::to_f2(u.x), b = Elem<T>::to_f2(u.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+  };
+  for (int h = 0; h < gsub; ++h) {
+    const float4 qv = row4(q + h * kHeadDim);
+    float m = -INFINITY, l = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int tile = first; tile < end; tile += kDecWarps) {
+      const int j0 = tile * kDecTile + (lane & 15), rows = dec_cache_row(p, r, j0, dec_list_entry(p, r, j0));
+      for (int j = 0; j < kDecTile; ++j) {
+        const int row = __shfl_sync(0xffffffffu, rows, j);
+        if (row < 0) continue;
+        const T* krow = kbase + row * row_elems;
+        const float4 k = row4(krow), v = row4(krow + p.page_size * row_elems);
+        float s = fmaf(qv.x, k.x, fmaf(qv.y, k.y, fmaf(qv.z, k.z, qv.w * k.w)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        s *= p.scale_log2;
+        const float m_new = fmaxf(m, s), base = m_new == -INFINITY ? 0.f : m_new;
+        const float rescale = exp2f(m - base), w = exp2f(s - base);
+        m = m_new;
+        l = fmaf(l, rescale, w);
+        if (rescale == 0.f) acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
+        add_weighted(acc, w, v);
+      }
+    }
+    reinterpret_cast<float4*>(at + h * kHeadDim)[lane] = acc;
+    if (lane == 0) {
+      ml[h][0] = m;
+      ml[h][1] = l;
+    }
+  }
+}
+
 struct DecShared {
   float ml[kDecWarps][kDecMaxGroup][2];
   int cum[kDecMaxBatch + 1];     // tiles of the sequences before (batched launches)
@@ -135,7 +178,7 @@ struct DecShared {
 
 // Dynamic shared memory: the rings, [4 warps][kDecStages][16 K rows, 16 V rows]; a warp parks its results in its own ring.
 template <typename T>
-__global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_kernel(const DecodeParams p) {
+__global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_kernel(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(128) uint8_t dec_smem[];
   __shared__ DecShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -311,12 +354,20 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
       for (int i = 0; i < 4; ++i) st.o[j][i] *= 1.f / Mma<T>::kScale;
     st.l += __shfl_xor_sync(0xffffffffu, st.l, 1);
     st.l += __shfl_xor_sync(0xffffffffu, st.l, 2);
-    if (t == 0) {
-      sh.ml[warp][g][0] = st.m;
-      sh.ml[warp][g][1] = st.l;
-    }
-    {
-      float* mine = reinterpret_cast<float*>(ring);
+    float* mine = reinterpret_cast<float*>(ring);
+    float z = 0.f;   // NaN where a result is not finite
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z = fmaf(st.o[j][i], 0.f, z);
+    if (__any_sync(0xffffffffu, z != z)) {
+      dec_plain<T>(p, row, kbase, row_elems, static_cast<const T*>(p.q) + static_cast<int64_t>(q_row0) * kHeadDim, gsub, a + warp, e, lane,
+                   mine, sh.ml[warp]);
+    } else {
+      if (t == 0) {
+        sh.ml[warp][g][0] = st.m;
+        sh.ml[warp][g][1] = st.l;
+      }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int h = 2 * t + i;
@@ -368,10 +419,7 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
         const float wt = m == -INFINITY ? 0.f : exp2f(m - M);
         const float4 v = reinterpret_cast<const float4*>(dec_smem + w * kDecStages * kDecTileBytes + h * kHeadDim * 4)[lane];
         L += wt * sh.ml[w][h][1];
-        acc.x = fmaf(wt, v.x, acc.x);
-        acc.y = fmaf(wt, v.y, acc.y);
-        acc.z = fmaf(wt, v.z, acc.z);
-        acc.w = fmaf(wt, v.w, acc.w);
+        add_weighted(acc, wt, v);
       }
       if (nparts > 1) {
         const int64_t at = static_cast<int64_t>(unit) * p.gs + h;
@@ -416,16 +464,14 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
             for (int u = 0; u < 8; ++u) m_new = fmaxf(m_new, ml[u].x);
             const float r = M == -INFINITY ? 0.f : exp2f(M - m_new);
             L *= r;
+            if (r == 0.f) acc = make_float4(0.f, 0.f, 0.f, 0.f);
             acc.x *= r; acc.y *= r; acc.z *= r; acc.w *= r;
             M = m_new;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
               const float wt = ml[u].x == -INFINITY ? 0.f : exp2f(ml[u].x - M);
               L += wt * ml[u].y;
-              acc.x = fmaf(wt, v[u].x, acc.x);
-              acc.y = fmaf(wt, v[u].y, acc.y);
-              acc.z = fmaf(wt, v[u].z, acc.z);
-              acc.w = fmaf(wt, v[u].w, acc.w);
+              add_weighted(acc, wt, v[u]);
             }
           }
           if (sharing == 1) {
@@ -448,10 +494,7 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
               const float m = sh.ml[w][0][0], wt = m == -INFINITY ? 0.f : exp2f(m - M);
               const float4 v = reinterpret_cast<const float4*>(dec_smem + w * kDecStages * kDecTileBytes)[lane];
               L += wt * sh.ml[w][0][1];
-              acc.x = fmaf(wt, v.x, acc.x);
-              acc.y = fmaf(wt, v.y, acc.y);
-              acc.z = fmaf(wt, v.z, acc.z);
-              acc.w = fmaf(wt, v.w, acc.w);
+              add_weighted(acc, wt, v);
             }
             finish(warp / sharing, M, L, acc);
           }

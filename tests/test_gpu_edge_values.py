@@ -108,3 +108,55 @@ def test_results_at_the_alignment_of_a_word():
     hist = torch.zeros(words + 1, dtype=torch.int32, device=DEV)[1:]
     with pytest.raises(RuntimeError, match="aligned"):
         K.select_attend(dist, 10, q, o, kv, table, last, pages - 1, hist=hist, hist_ready=True)
+
+
+def _attend64(q, k, v, scale=128.0 ** -0.5):
+    """Softmax attention of q [H, 128] over k, v [n, H, 128] in 64 bits; a weight of 0 takes no part, whatever its value is."""
+    s = torch.einsum("hd,lhd->hl", q.double(), k.double()) * scale
+    p = torch.softmax(s, 1).T[..., None]
+    return torch.where(p > 0, p * v.double(), torch.zeros(())).sum(0)
+
+
+@pytest.mark.parametrize("case", ["inf", "two infinities", "nan", "weight 0", "logits -inf"])
+@pytest.mark.parametrize("L", [1, 7, 100, 3000])
+def test_values_that_are_not_finite(case, L):
+    """V rows with infinities and NaN count as weight times value does, and not at all where the weight is 0; a logit of -inf
+    is a weight of 0, also where a warp sees nothing else.  Dense, by list, and select+attend (where a weight that
+    underflows counts as the smallest number there is)."""
+    _, K, _ = _mods()
+    H, ps, dtype = 3, 16, torch.bfloat16
+    g = torch.Generator().manual_seed(L)
+    q, k, v = torch.randn(1, H, 128, generator=g), torch.randn(L, H, 128, generator=g), torch.randn(L, H, 128, generator=g)
+    t = L // 2
+    if case == "inf":
+        v[t, 0, 3], v[t, 1, 70] = math.inf, -math.inf
+    elif case == "two infinities":
+        v[0, 0, 3], v[L - 1, 0, 3], v[L - 1, 1, 9] = math.inf, math.inf, math.inf
+    elif case == "nan":
+        v[t, 0, 3] = math.nan
+    elif case == "weight 0":     # (all but the last token: a logit 2000 below)
+        q[..., 0], k[: L - 1, :, 0] = 100.0, -300.0
+        v[: L - 1, 0, 3], v[: L - 1, 1, 5] = math.inf, math.nan
+    else:
+        q[..., 0], k[: L - 1, :, 0] = 1.0, -math.inf
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+    pages = (L + ps - 1) // ps
+    last = L - (pages - 1) * ps
+    kv = torch.zeros(pages * ps, 2, H, 128, dtype=dtype)
+    kv[:L, 0], kv[:L, 1] = k, v
+    kv = kv.view(pages, ps, 2, H, 128).transpose(1, 2).contiguous().to(DEV)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)
+    want = _attend64(q[0], k, v)
+    tol = dict(rtol=2.0 ** -7, atol=2.0 ** -7, equal_nan=True)
+    o = torch.empty(1, H, 128, dtype=dtype, device=DEV)
+    w = K.BatchDecodeWithPagedKVCachePyTorchWrapper(0)
+    w.begin_forward(torch.tensor([0, pages], dtype=torch.int32), H, H, 128, ps, torch.empty(0, dtype=dtype))
+    w.forward(q.to(DEV), o, kv, table[: pages - 1].unsqueeze(0).expand(H, pages - 1), None, last, pages - 1)
+    torch.testing.assert_close(o[0].cpu().double(), want, **tol)
+    idx = torch.arange(L - 1, dtype=torch.int32).repeat(H, 1).to(DEV)
+    w.forward(q.to(DEV), o, kv, idx, None, last, pages - 1, token_granular=True)
+    torch.testing.assert_close(o[0].cpu().double(), want, **tol)
+    if L > 1 and case != "weight 0":
+        dist = torch.zeros(H, (L + 6) // 8 * 8, dtype=torch.int16, device=DEV)
+        K.select_attend(dist[:, : L - 1], L - 1, q.to(DEV), o, kv, table, last, pages - 1)
+        torch.testing.assert_close(o[0].cpu().double(), want, **tol)
