@@ -58,14 +58,6 @@ def _dtype_code(dtype: torch.dtype, what: str) -> int:
     raise RuntimeError(f"{what} failed to dispatch with dtype {dtype}")
 
 
-def _value_format(dtype: torch.dtype, what: str) -> int:
-    if dtype == torch.float16:
-        return _lib.VAL_F16
-    if dtype in (torch.int16, torch.uint16):
-        return _lib.VAL_U16
-    raise RuntimeError(f"{what} failed to dispatch with dtype {dtype}")
-
-
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 

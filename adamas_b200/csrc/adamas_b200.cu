@@ -537,6 +537,11 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 }
 
 // ---------------------------------------------------------------------------------------------
+// Which estimate kernel.  The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of
+// its heads in registers and two blocks per SM overlap; the item kernel takes the rest.  Whole step, us a layer, tiles / items:
+// 16 heads 4K 10.3 / 11.9, 32K 18.3 / 18.5, 128K 35.9 / 30.6; 32 heads 4K 11.3 / 12.8, 16K 17.4 / 19.2, 32K 21.7 / 24.0,
+// 128K 43.6 / 44.8; 64 heads 4K 13.9 / 15.0, 32K 33.1 / 35.0; batches of 32 heads: 8 x 32K 79.3 / 85.5, 32 x 4-8K 74.3 / 79.0.
+// (16 heads over 128K tokens are the exception: there the item kernel's counts in shared memory pay more than the rest costs.)
 static bool estimate_by_tiles(int num_heads, int q_heads) {
   return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64);
 }

@@ -2,23 +2,25 @@
 // for 16, 32 and 64 heads is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (56 instructions, 12 of them population counts at quarter rate, per 32 distances) for grouped
-// queries, HBM for long rows, fill and drain for short ones.  One persistent block of 16 warps per SM; every warp works
-// alone:
+// queries, HBM for long rows, fill and drain for short ones.  One persistent block of 16 warps (8 with little work) per SM;
+// every warp works alone:
 //   * its unit of work is an item of 4 KB of codes: 128 / HP tokens x HP heads (HP = 4, 2 or 1, the largest that divides
 //     the head count).  Its own 16-byte asynchronous copies bring items into its own ring of two or three slots: no
 //     producer warp, no barrier between warps.  (A bulk copy with a different address in every lane is issued lane after
 //     lane, 45 ns each, which bounded small head counts in a pipeline with producer warps.)
 //   * lane = token: a lane reads the two halves of a code (chunk c of row r is stored at c ^ f(r), which makes 32 rows hit
 //     different bank groups) and the query's planes from shared memory (all lanes the same address).  With grouped
-//     queries the code is read once for all query heads of the cache head.  The 32 lanes store 32 consecutive tokens
+//     queries the code is read once for all query heads of the cache head, or, with fewer items than warps, once for each
+//     of the parts in which several warps take them (item_query_heads).  The 32 lanes store 32 consecutive tokens
 //     of one output row.
 //   * the distances are counted in shared memory (16-bit counts, two to a word, one table per query row) and added to
 //     the global per-slice histograms once per block: one L2 atomic per (block, distance value) instead of one per distance.
 // All items of a launch, sequence after sequence, form one line that is cut evenly over the blocks, so sequences of
-// different lengths and any head count load all SMs alike.  The first items are requested before the kernel's dependency
+// different lengths and any head count load all SMs alike (with little work every block keeps to one sequence).  The first items are requested before the kernel's dependency
 // resolves (the cached codes are final).
 // Measured (with counts): 8 cache heads / 64 query heads, 64K tokens: 31 -> 21 us; 4 heads, 128K: 14.4 -> 7.4 us with the
-// append inside; 32 query heads over 8, 30K tokens: 9.8 -> 8.7 us.  Lane = head with four tokens
+// append inside; 32 query heads over 8, 30K tokens: 9.3 -> 9.3 us; over 2, 16K: 6.8 -> 7.3 (17.9 with
+// undivided groups).  Lane = head with four tokens
 // per lane (one 4 KB run of codes per warp) was slower than lane = token: 36.9 us.
 #pragma once
 #include "estimate.cuh"

@@ -5,8 +5,8 @@
 //
 // The kernel does not count anything itself.  The estimate kernels (or dist_histogram_kernel, for a
 // caller that only has a distance row) leave, per head, one 512-bin histogram per SLICE of the row
-// in a global table [H][kSaMaxSlices][512] u32: slice r covers the granules (8 distances) that block
-// r of the head's cluster owns.  A distance is at most 3 * 128 = 384; larger values count as 511.
+// in a global table [H][kSaMaxSlices][512] u32: a slice covers the granules (8 distances) of one block of
+// the head, or of two neighbouring ones.  A distance is at most 3 * 128 = 384; larger values count as 511.
 //
 // CL <= 16 blocks x 128 threads per head (grid (CL, H)); the blocks of a head never wait for one another.
 // Block `cr`:
@@ -378,7 +378,6 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     const int64_t row_elems = static_cast<int64_t>(H) * kHeadDim, v_delta = p.page_size * row_elems;
     const T* kbase = static_cast<const T*>(kv_base) + head_kv * kHeadDim;
     int32_t* oi = p.out_idx ? p.out_idx + static_cast<int64_t>(head) * p.out_stride + lt_before + min(eq_before, need_eq) : nullptr;
-    // K rows as one commit group, V rows as a second: the logits are formed while the V rows are still on their way
     uint4 q[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) q[j] = lane < 4 ? reinterpret_cast<const uint4*>(sh.q)[4 * j + lane] : make_uint4(0, 0, 0, 0);

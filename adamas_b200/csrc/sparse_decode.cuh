@@ -16,9 +16,9 @@
 // sequences of different lengths and head counts that do not divide the chip leave nothing idle), or, for small
 // launches where the latency of a second row group would count, an equal share of one.  A row group cut over several
 // blocks is merged by the block that arrives last at its counter (no block ever waits for another).
-// Measured, attention over all tokens of a layer: 32 heads x 32768 tokens, fp16: 125 -> 87 us (6.2 TB/s; 96 % of the
-// copy rate); 21 sequences x 64 query heads over 8 x 7366 tokens: 1097 -> 118 us.  One block of 8 warps per SM: 91 us
-// (the end of a piece leaves the SM idle); three blocks of 4 with two ring slots: 93 us.  Blocks that take four
+// Measured, append and attention over all tokens of a layer: 32 heads x 32768 tokens, fp16: 128 -> 92 us (537 MB: 5.8 TB/s, 90 %
+// of the copy rate, the append's launch included); 21 sequences x 64 query heads over 8 x 7366 tokens: 1097 -> 118 us.  One block of 8 warps per SM: 4 us
+// more (the end of a piece leaves the SM idle); three blocks of 4 with two ring slots: 6 us more.  Blocks that take four
 // neighbouring heads of a token (1 KB in a row) measured no better than one head per block.
 #pragma once
 #include "attend_tile.cuh"
