@@ -19,7 +19,7 @@
 // different lengths and any head count load all SMs alike (with little work every block keeps to one sequence).  The first items are requested before the kernel's dependency
 // resolves (the cached codes are final).
 // Measured (with counts): 8 cache heads / 64 query heads, 64K tokens: 31 -> 21 us; 4 heads, 128K: 14.4 -> 7.4 us with the
-// append inside; 32 query heads over 8, 30K tokens: 9.3 -> 9.3 us; over 2, 16K: 6.8 -> 7.3 (17.9 with
+// append inside; 32 query heads over 8, 30K tokens: 9.3 us before and now; over 2, 16K: 6.8 -> 7.3 (17.9 with
 // undivided groups).  Lane = head with four tokens
 // per lane (one 4 KB run of codes per warp) was slower than lane = token: 36.9 us.
 #pragma once
