@@ -84,6 +84,7 @@ int check_q_heads(int num_heads, int num_q_heads) {
 }
 
 constexpr int kEstStatic = 6144;   // static shared memory of the estimate kernels, rounded up
+constexpr int kItemStatic = 1024;           // ... of estimate_items_kernel
 constexpr int kSaStatic = 1024;             // static shared memory of select_attend_kernel, rounded up
 constexpr int kSaMaxPageBytes = 4096;       // page numbers of a block that are staged in shared memory at most
 constexpr int kSaMaxDynSmem = 160 * 1024;   // dynamic shared memory select_attend may ask for (a long winner list)
@@ -131,10 +132,11 @@ int get_device_info(const DeviceInfo** out) {
     EST_ATTR_HPW(2);
     EST_ATTR_HPW(4);
 #undef EST_ATTR_HPW
-#define EST_ATTR_HP(HP, G)                                \
-  EST_ATTR(estimate_items_kernel<__half, 0, HP, G>);      \
-  EST_ATTR(estimate_items_kernel<__half, 1, HP, G>);      \
-  EST_ATTR(estimate_items_kernel<__nv_bfloat16, 0, HP, G>)
+#define EST_ATTR_HP(HP, G)                                  \
+  EST_ATTR(estimate_items_kernel<__half, 0, HP, G>);        \
+  EST_ATTR(estimate_items_kernel<__nv_bfloat16, 0, HP, G>); \
+  EST_ATTR(estimate_items_kernel<__half, 1, HP, G>);        \
+  EST_ATTR(estimate_items_kernel<__half, 2, HP, G>)
     EST_ATTR_HP(1, false);
     EST_ATTR_HP(2, false);
     EST_ATTR_HP(4, false);
@@ -537,13 +539,16 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 }
 
 // ---------------------------------------------------------------------------------------------
+// Launches of 3 M distances and more (a 128K context of 32 heads, three 32K sequences): there one L2 atomic per distance from
+// inside the estimate bounds it (the estimate of one 128K sequence: 31.7 us with the counts, 23.7 without).
+static bool many_distances(int q_heads, int batch, int n) {
+  return static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20);
+}
 // Which estimate kernel.  The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of
-// its heads in registers and two blocks per SM overlap; the item kernel takes the rest.  Whole step, us a layer, tiles / items:
-// 16 heads 4K 10.3 / 11.9, 32K 18.3 / 18.5, 128K 35.9 / 30.6; 32 heads 4K 11.3 / 12.8, 16K 17.4 / 19.2, 32K 21.7 / 24.0,
-// 128K 43.6 / 44.8; 64 heads 4K 13.9 / 15.0, 32K 33.1 / 35.0; batches of 32 heads: 8 x 32K 79.3 / 85.5, 32 x 4-8K 74.3 / 79.0.
-// (16 heads over 128K tokens are the exception: there the item kernel's counts in shared memory pay more than the rest costs.)
-static bool estimate_by_tiles(int num_heads, int q_heads) {
-  return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64);
+// its heads in registers; the item kernel takes the rest, and long single sequences, where it counts in shared memory.  Whole step,
+// us a layer, tiles / items: 32 heads 4K 12.0 / 13.1, 32K 20.5 / 21.0, 128K 48.9 / 47.7; 8 x 32K 79.7 / 82.4; 32 x 4-8K 75.0 / 74.7.
+static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n) {
+  return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64) && (batch > 1 || !many_distances(q_heads, 1, n));
 }
 
 // Launches the estimate.  n: distances per row, or their upper bound when seq_len_dev gives the length on the device
@@ -576,18 +581,17 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   prm.n_tokens = n;
   prm.H = num_heads;
   prm.q_group = q_heads / num_heads;
-  prm.chip_warps = kItemWarps * di->num_sms;
+  prm.chip_warps = kItemWarps * kItemBlocksPerSm * di->num_sms;
   prm.page_size = page_size;
   prm.ps_shift = log2_exact(page_size);
   prm.batch = batch;
   prm.seq_len_dev = seq_len_dev;
   prm.hist = hist;
   prm.hist_cl = hist_cl;
-  prm.count_local = 0;
   prm.seqs = seqs;
   prm.ap = ap;
   cudaStream_t st = to_stream(stream);
-  if (estimate_by_tiles(num_heads, q_heads)) {
+  if (estimate_by_tiles(num_heads, q_heads, batch, n)) {
     const int num_tiles = (n + kEstTile - 1) / kEstTile;
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
@@ -621,39 +625,31 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
     return check_launch("estimate_kernel");
   }
   ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0, "q_code must be 16-byte aligned");
-  const int hp = num_heads % 4 == 0 ? 4 : num_heads % 2 == 0 ? 2 : 1;   // heads per item: as long a run of a token's codes as divides
-  int64_t items = static_cast<int64_t>((n + 128 / hp - 1) / (128 / hp)) * (num_heads / hp) * batch;
+  const int hp = item_cache_heads(num_heads, prm.q_group);
+  int64_t items = static_cast<int64_t>(n / (128 / hp) + 1) * (num_heads / hp) * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
   const int q_part = item_query_heads(static_cast<int>(items), prm.q_group, prm.chip_warps);
-  items *= (prm.q_group + q_part - 1) / q_part;   // (still below 2^31: only few items are divided)
-  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(di->num_sms, items)));
-  // Little work: blocks of half the size, which leave the other half of the SM's registers to the first blocks of the kernel
-  // behind (whole step, 3000 tokens: 8 heads 12.1 -> 10.7 us, 28 over 4 14.7 -> 14.1; one head, 60K: 14.5 -> 12.4).  They code
-  // 32 query heads in one pass; with 64 the second pass costs what this gains (16.1 / 18.1 us).
+  items *= (prm.q_group + q_part - 1) / q_part;
+  ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
+  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(static_cast<int64_t>(est_blocks_per_sm()) * di->num_sms, items)));
   const int64_t per_block = (items + grid.x - 1) / grid.x;
-  // One block per SM as the setting: half a block as well, with no more than half of the SM's shared memory, where the query
-  // planes leave room for two ring slots per warp.
-  const size_t planes = static_cast<size_t>(q_heads) * 2 * sizeof(QPlanes), half_sm = static_cast<size_t>(di->smem_per_sm / 2 - 1024 - kEstStatic);
-  const bool half = est_blocks_per_sm() == 1 && planes + kItemWarps / 2 * 2 * kItemBytes <= half_sm;
-  const int warps = half || (per_block <= kItemWarps / 2 && q_heads <= 2 * kItemWarps) ? kItemWarps / 2 : kItemWarps;
-  const size_t room = half ? half_sm : most;
-  const size_t slot = static_cast<size_t>(warps) * kItemBytes, counts = static_cast<size_t>(q_heads) * kItemCountWords * sizeof(uint32_t);
-  const int wanted = static_cast<int>(std::min<int64_t>(3, (per_block + warps - 1) / warps)), least = std::min(wanted, 2);   // ring slots
-  // The counts in shared memory where they fit beside two ring slots per warp and where there are enough distances to be
-  // worth clearing and adding up a table per block (12K tokens x 40 heads: 6.4 us with an L2 atomic each, 7.5 with tables;
-  // 30K x 32: 8.8 / 8.7; 64K x 64: 26.9 / 21.1); a third slot where it fits beside them.
-  size_t smem = planes;
-  prm.count_local = hist && static_cast<int64_t>(q_heads) * n * batch >= (int64_t(1) << 20) && smem + least * slot + counts <= room ? 1 : 0;
-  if (prm.count_local) smem += counts;
-  const int slots = smem + wanted * slot <= room ? wanted : least;
+  // (with the length on the device a shorter sequence's groups may be cut into smaller parts, never into larger ones)
+  const int seg_rows = hp * q_part;
+  const size_t room = static_cast<size_t>(di->smem_per_sm / kItemBlocksPerSm - 1024 - kItemStatic);
+  size_t smem = static_cast<size_t>(seg_rows) * 2 * sizeof(QPlanes);
+  if (hist) smem += static_cast<size_t>(item_tables(hp, prm.q_group > 1)) * seg_rows * kItemCountWords * sizeof(uint32_t);
+  if (seqs) smem += static_cast<size_t>(batch + 1) * sizeof(int);
+  const size_t slot = static_cast<size_t>(kItemWarps) * kItemBytes;
+  int slots = static_cast<int>(std::min<int64_t>(kItemMaxSlots, (per_block + kItemWarps - 1) / kItemWarps));
+  while (slots > 1 && smem + slots * slot > room) --slots;
   smem += slots * slot;
-  ADAMAS_REQUIRE(smem <= most, "num_q_heads (%d) too large for the estimate kernel", q_heads);
-#define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_items_kernel", (__VA_ARGS__), grid, dim3(warps * 32), smem, st, 1, prm, slots)
+#define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_items_kernel", (__VA_ARGS__), grid, dim3(kItemThreads), smem, st, 1, prm, slots, seg_rows)
 #define LAUNCH_EST_HP(HP, G)                                                                                 \
   do {                                                                                                       \
-    if (metric != ADAMAS_METRIC_L1) LAUNCH_EST(estimate_items_kernel<__half, 1, HP, G>);   /* (no append) */ \
-    else if (dtype == ADAMAS_F16) LAUNCH_EST(estimate_items_kernel<__half, 0, HP, G>);                       \
-    else LAUNCH_EST(estimate_items_kernel<__nv_bfloat16, 0, HP, G>);                                         \
+    if (ap.q && dtype == ADAMAS_F16) LAUNCH_EST(estimate_items_kernel<__half, 0, HP, G>);                    \
+    else if (ap.q) LAUNCH_EST(estimate_items_kernel<__nv_bfloat16, 0, HP, G>);                               \
+    else if (metric == ADAMAS_METRIC_L1) LAUNCH_EST(estimate_items_kernel<__half, 1, HP, G>);                \
+    else LAUNCH_EST(estimate_items_kernel<__half, 2, HP, G>);                                                \
   } while (0)
 #define LAUNCH_EST_G(G)                    \
   do {                                     \
@@ -1409,10 +1405,9 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   SaPlan pl;
   if (int rc = sa_plan(n, budget - 1, q_heads * batch, page_size, di, &pl)) return rc;
   int rc;
-  // The histogram counts.  Tile pipeline: one L2 atomic per distance from inside the estimate, or, for launches with 3 M
-  // distances and more (a 128K context of 32 heads, three 32K sequences), a launch of their own that counts in shared
-  // memory (measured: the estimate of one 128K sequence 31.7 us with the counts, 23.7 without).
-  const bool count_apart = estimate_by_tiles(num_heads, q_heads) && static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20);
+  // The histogram counts.  Item kernel: in shared memory.  Tile pipeline: one L2 atomic per distance from inside the estimate, or,
+  // with many distances, a launch of its own that counts in shared memory.
+  const bool count_apart = estimate_by_tiles(num_heads, q_heads, batch, n) && many_distances(q_heads, batch, n);
   uint32_t* est_hist = count_apart ? nullptr : hist;
   const bool two_launches = fused_append_enabled();
   if (two_launches) {

@@ -91,7 +91,7 @@ __device__ __forceinline__ __half dist_to_out<__half>(unsigned d) {
 
 // The decode append inside the estimate.  Every block codes all query heads of the sequences it works on by itself
 // (the rows come from L2), so no block waits for another.  The new token's K and V rows, the key's code and the query
-// codes are stored by one block each (estimate_append_kernel) or dealt out over the sequence's blocks by cache head
+// codes are stored by one block each (estimate_append_kernel) or by the blocks that start a piece of its heads
 // (estimate_items_kernel); none of this is read by the scan, which leaves the newest token out, and the kernel after
 // this one finds all of it complete.
 // rope_on: q and k arrive un-rotated.  The position's 64 (cos, sin) pairs are formed once per block and sequence, the
@@ -133,7 +133,6 @@ struct EstimateParams {
   // scratch table ([rows][kSaScratchWordsPerHead] u32, rows zero on entry); slice = token / (8 * sa_granules_per_block(n_tokens, hist_cl))
   uint32_t* hist;
   int hist_cl;
-  int count_local;   // estimate_items_kernel: count in shared memory (else one L2 atomic per distance)
   // optional (needs seq_len_dev): a batch of sequences.  Everything on the query side has one row per (sequence, query
   // head); codes, page table and length are the sequence's.
   const SeqDesc* seqs;

@@ -2,10 +2,9 @@
 // for 16, 32 and 64 heads is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (56 instructions, 12 of them population counts at quarter rate, per 32 distances) for grouped
-// queries, HBM for long rows, fill and drain for short ones.  One persistent block of 16 warps (8 with little work) per SM;
-// every warp works alone:
-//   * its unit of work is an item of 4 KB of codes: 128 / HP tokens x HP heads (HP = 4, 2 or 1, the largest that divides
-//     the head count).  Its own 16-byte asynchronous copies bring items into its own ring of two or three slots: no
+// queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM; every warp works alone:
+//   * its unit of work is an item of 4 KB of codes: 128 / HP tokens x HP heads (HP = 4, 2 or 1, see item_cache_heads).
+//     Its own 16-byte asynchronous copies bring items into its own ring of two or three slots: no
 //     producer warp, no barrier between warps.  (A bulk copy with a different address in every lane is issued lane after
 //     lane, 45 ns each, which bounded small head counts in a pipeline with producer warps.)
 //   * lane = token: a lane reads the two halves of a code (chunk c of row r is stored at c ^ f(r), which makes 32 rows hit
@@ -13,33 +12,49 @@
 //     queries the code is read once for all query heads of the cache head, or, with fewer items than warps, once for each
 //     of the parts in which several warps take them (item_query_heads).  The 32 lanes store 32 consecutive tokens
 //     of one output row.
-//   * the distances are counted in shared memory (16-bit counts, two to a word, one table per query row) and added to
-//     the global per-slice histograms once per block: one L2 atomic per (block, distance value) instead of one per distance.
-// All items of a launch, sequence after sequence, form one line that is cut evenly over the blocks, so sequences of
-// different lengths and any head count load all SMs alike (with little work every block keeps to one sequence).  The first items are requested before the kernel's dependency
-// resolves (the cached codes are final).
-// Measured (with counts): 8 cache heads / 64 query heads, 64K tokens: 31 -> 21 us; 4 heads, 128K: 14.4 -> 7.4 us with the
-// append inside; 32 query heads over 8, 30K tokens: 9.3 us before and now; over 2, 16K: 6.8 -> 7.3 (17.9 with
-// undivided groups).  Lane = head with four tokens
-// per lane (one 4 KB run of codes per warp) was slower than lane = token: 36.9 us.
+//   * the distances are counted in shared memory, one table of 32-bit counts per query row and slice, and the tables are added to
+//     the global per-slice histograms once per block.  One L2 atomic per distance runs at 90 to 165 per ns on the whole chip, which
+//     made 1 M distances 6 to 8 us; additions of the constant 1 in shared memory take 1 to 2 cycles per warp, those of packed
+//     16-bit counts 4 to 13 (lanes that meet in a word are taken one after the other).
+// All items of a launch form one line: sequence after sequence, in it piece after piece (HP cache heads), in it token after token.
+// So a block works on a few rows over many tokens: it codes 4 to 16 query rows instead of all, its tables are small, and it adds up as
+// many distances as there are before a table goes out.  The line is cut evenly over the blocks, or, with few segments (a piece of a
+// sequence), every block takes a part of one.  The first items are requested before the kernel's dependency resolves (the cached
+// codes are final).
+// Measured, the whole step, us a layer, against token after token with all heads in it and one block of 16 warps per SM: 40 heads,
+// 12K 18.1 -> 16.7; 32 query heads over 8, 30K 24.6 -> 23.7; 4 sequences x 128K x 4 heads 35.6 -> 34.1; 32 heads, 128K 49.1 -> 47.4
+// (tile pipeline and a counting launch).  Lane = head with four tokens per lane (one 4 KB run of codes per warp) was slower than lane = token.
 #pragma once
 #include "estimate.cuh"
 
 namespace adamas {
 
-constexpr int kItemWarps = 16;           // warps of a block, or half as many (see the host's rule)
+constexpr int kItemWarps = 8;
 constexpr int kItemThreads = kItemWarps * 32;
+constexpr int kItemBlocksPerSm = 2;
+constexpr int kItemMaxSlots = 3;         // ring slots per warp at most
 constexpr int kItemBytes = 4096;
-constexpr int kItemCountWords = 196;     // per query row: 392 16-bit counts (a distance is at most 384)
+constexpr int kItemApart = 4;            // items per block that keeping to one segment may cost
+constexpr int kItemCountWords = 388;     // counts per query row and table (a distance is at most 384)
 
-// Query heads of a cache head that a warp takes at a time.  The group of a cache head is halved as long as every part still
-// finds a warp of its own (`warps` on the chip; `items` are those of undivided groups): a second round costs more than it saves
-// (32 query heads over 2, 60K tokens: 14.3 us in two parts, one round; 17.9 in three parts, two rounds).
+// Cache heads of an item, and the query heads of a cache head that a warp takes at a time.  An item has as long a run of a
+// token's codes as divides the cache heads, but not more than kItemRows query rows (every row has count tables in every block
+// that works on it).  The group of a cache head is halved as long as every part still
+// finds a warp of its own (`warps` on the chip; `items` are those of undivided groups): a second round costs more than it saves.
+constexpr int kItemRows = 8;
+__host__ __device__ __forceinline__ int item_cache_heads(int kv_heads, int q_group) {
+  int hp = 4;
+  while (hp > 1 && (kv_heads % hp != 0 || (q_group > 1 && hp * q_group > kItemRows))) hp /= 2;
+  return hp;
+}
 __host__ __device__ __forceinline__ int item_query_heads(int items, int q_group, int warps) {
   int heads = q_group;
+  for (; heads > 2 * kItemRows; items *= 2) heads = (heads + 1) / 2;
   for (; heads > 1 && items <= warps / 2; items *= 2) heads = (heads + 1) / 2;
   return heads;
 }
+// Count tables of a block: the slices that its tokens may fall into.
+__host__ __device__ __forceinline__ constexpr int item_tables(int hp, bool grouped) { return hp == 1 && !grouped ? 4 : 2; }
 
 // 128-point transform of a row spread over 8 lanes, 16 elements each: the butterflies of wht128_halfwarp in the
 // same order, so the same bits.
@@ -107,115 +122,122 @@ __device__ __forceinline__ uint32_t code_word_8lanes(float (&x)[16], unsigned l8
 
 struct EstShared {
   float2 cs[kHeadDim / 2];
-  int cum[kEstMaxBatch + 1];   // token tiles of the sequences before
 };
 
-// Dynamic shared memory: rings | planes [rows of a sequence][2] | counts [rows][kItemCountWords] (count_local).
-// GROUPED: several query heads per cache head (q_group > 1).
-template <typename T, int METRIC, int HP, bool GROUPED>
-__global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const EstimateParams p, int slots) {
+// Dynamic shared memory: rings | planes [seg_rows][2] | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
+// sequences before [batch + 1] (seqs).  GROUPED: several query heads per cache head (q_group > 1).
+// MODE 0: with the append inside (u16 distances); 1: the query codes are given; 2: the same with the XOR metric.
+template <typename T, int MODE, int HP, bool GROUPED>
+__global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items_kernel(const EstimateParams p, int slots, int seg_rows) {
+  constexpr bool APPEND = MODE == 0;
+  constexpr int METRIC = MODE == 2 ? 1 : 0;
   constexpr int TT = 128 / HP;          // tokens of an item
   constexpr int kGroups = TT / 32;      // ... in groups of 32
   constexpr int CPR = 2 * HP;           // 16-byte chunks per token of an item
+  constexpr int kTables = item_tables(HP, GROUPED);
   extern __shared__ __align__(128) uint8_t item_smem[];
   __shared__ EstShared sh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int threads = blockDim.x, warps = threads >> 5;
+  const int len0 = p.seq_len_dev && !p.seqs ? __ldg(p.seq_len_dev) - 1 : p.n_tokens;   // (on its way while the rest is set up)
   const int q_group = GROUPED ? p.q_group : 1;
   const int rows = p.H * q_group;       // query rows of a sequence
-  QPlanes* planes = reinterpret_cast<QPlanes*>(item_smem + warps * slots * kItemBytes);
-  uint32_t* counts = reinterpret_cast<uint32_t*>(planes + 2 * rows);
+  QPlanes* planes = reinterpret_cast<QPlanes*>(item_smem + kItemWarps * slots * kItemBytes);
+  uint32_t* counts = reinterpret_cast<uint32_t*>(planes + 2 * seg_rows);
+  int* cum = reinterpret_cast<int*>(counts + (p.hist ? kTables * seg_rows * kItemCountWords : 0));
   uint4* ring = reinterpret_cast<uint4*>(item_smem + warp * (slots * kItemBytes));
+  // (the position's rotation is formed by warps that have nothing else to do for the query)
+  const int cs_pair = tid - 4 * 32;
+  const bool cs_here = APPEND && p.ap.rope_on && cs_pair >= 0 && cs_pair < kHeadDim / 2;
+  const float cs_freq = cs_here ? rope_inv_freq(cs_pair, p.ap.rp) : 0.f;
 
-  // ---- the line of items: token tile after token tile, `pieces` each: HP heads with a part of their query heads ---
+  // ---- the line of items: sequence after sequence, in it piece after piece (HP cache heads with a part of their query heads),
+  // in it token tile after token tile -----------------------------------------------------------------------------------
   int tiles_all;
   if (p.seqs) {
-    if (warp == 0) est_line(p, TT, lane, sh.cum);
+    if (warp == 0) est_line(p, TT, lane, cum);
     __syncthreads();
-    tiles_all = sh.cum[p.batch];
+    tiles_all = cum[p.batch];
   } else {
-    tiles_all = est_tiles(p.seq_len_dev ? __ldg(p.seq_len_dev) - 1 : p.n_tokens, TT);
+    tiles_all = est_tiles(len0, TT);
   }
   const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
   const int q_split = q_part == q_group ? 1 : (q_group + q_part - 1) / q_part, pieces = p.H / HP * q_split;
-  const float split_inv = 1.f / static_cast<float>(q_split);
-  auto heads_of = [&](int piece) { return q_split == 1 ? piece : __float2int_rz((static_cast<float>(piece) + 0.5f) * split_inv); };   // piece / q_split (exact: pieces <= 1024)
   const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
   if (total == 0) return;
-  // (with the lengths on the device there may be fewer items than blocks: every block that takes part has some)
-  const int b = blockIdx.x, B = min(static_cast<int>(gridDim.x), total);
-  auto line_start = [&](int blk) { return static_cast<int>(static_cast<int64_t>(blk) * total / B); };
+  const int b = blockIdx.x, segments = p.batch * pieces;
+  auto seg_start = [&](int g) {   // where segment g (a piece of a sequence) starts on the line
+    if (!p.seqs) return g * tiles_all;
+    const int s = g / pieces;
+    return s == p.batch ? total : cum[s] * pieces + (g - s * pieces) * (cum[s + 1] - cum[s]);
+  };
   int pos, line_end;
-  int nblk = B, my_blk = b;   // blocks that share out the appends of a piece's sequence, and which of them this one is
-  // A batch with little work: every block takes a piece of ONE sequence, the blocks dealt out in proportion to the items.  (A
-  // block that the line takes into a second sequence codes two queries, one after the other, and the launch waits for it:
-  // 2 sequences of 1250 and 2500 tokens, 32 query heads over 8: 15.2 us, 9.2 this way.)
-  const bool apart = p.seqs && p.batch <= static_cast<int>(gridDim.x) && total <= 2 * p.chip_warps;
-  if (apart) {
-    const int spare = gridDim.x - p.batch;
-    auto first_block = [&](int s) { return s + static_cast<int>(static_cast<int64_t>(sh.cum[s]) * spare / tiles_all); };
-    int lo = 0, hi = p.batch - 1;
-    while (lo < hi) {   // the last sequence that starts at or before this block
-      const int mid = (lo + hi + 1) >> 1;
-      if (first_block(mid) <= b) lo = mid; else hi = mid - 1;
+  // With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the uneven
+  // shares is less than a second segment costs (queries to load and code behind a barrier, counts to add up).
+  if (segments <= static_cast<int>(gridDim.x) && static_cast<int64_t>(total) * segments <= static_cast<int64_t>(kItemApart) * gridDim.x * gridDim.x) {
+    // (the rule keeps every product below 2^31)
+    const int spare = gridDim.x - segments;
+    auto first_block = [&](int g) { return g + (p.seqs ? seg_start(g) * spare / total : g * spare / segments); };
+    int g = b * segments / static_cast<int>(gridDim.x);   // the last segment that starts at or before this block
+    if (p.seqs) {
+      int lo = 0, hi = segments - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (first_block(mid) <= b) lo = mid; else hi = mid - 1;
+      }
+      g = lo;
+    } else {
+      while (first_block(g) > b) --g;
+      while (g + 1 < segments && first_block(g + 1) <= b) ++g;
     }
-    const int seq_items = (sh.cum[lo + 1] - sh.cum[lo]) * pieces;
-    nblk = min(first_block(lo + 1) - first_block(lo), seq_items);
-    my_blk = b - first_block(lo);
-    if (my_blk >= nblk) return;
-    pos = sh.cum[lo] * pieces + static_cast<int>(static_cast<int64_t>(seq_items) * my_blk / nblk);
-    line_end = sh.cum[lo] * pieces + static_cast<int>(static_cast<int64_t>(seq_items) * (my_blk + 1) / nblk);
+    const int start = seg_start(g), n_items = seg_start(g + 1) - start, f = first_block(g), nblk = min(first_block(g + 1) - f, n_items);
+    if (b - f >= nblk) return;
+    pos = start + n_items * (b - f) / nblk;
+    line_end = start + n_items * (b - f + 1) / nblk;
   } else {
+    const int B = min(static_cast<int>(gridDim.x), total);   // (every block that takes part has some)
     if (b >= B) return;
-    pos = line_start(b);
-    line_end = line_start(b + 1);
+    const int q = total / B, r = total - q * B;
+    pos = b * q + b * r / B;   // b * total / B
+    line_end = (b + 1) * q + (b + 1) * r / B;
   }
   bool waited = false;
 
   while (pos < line_end) {
-    // ---- this block's next piece of a sequence: items [first, end) ------------------------------------------
-    int s = 0, seq0 = 0, seq1 = total;
+    // ---- this block's next segment: tiles [first, end) of a piece of a sequence ----------------------------------------
+    int s = 0, tiles = tiles_all, at = pos, n = len0;
+    const uint4* codes = p.codes;
+    const int32_t* table = p.page_table;
     if (p.seqs) {
       int lo = 0, hi = p.batch - 1;
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
-        if (sh.cum[mid] * pieces <= pos) lo = mid; else hi = mid - 1;
+        if (cum[mid] * pieces <= pos) lo = mid; else hi = mid - 1;
       }
       s = lo;
-      seq0 = sh.cum[s] * pieces;
-      seq1 = sh.cum[s + 1] * pieces;
-    }
-    const int end = min(seq1, line_end) - seq0, first = pos - seq0;
-    pos = seq0 + end;
-    const int n = p.seq_len_dev ? __ldg(p.seq_len_dev + s) - 1 : p.n_tokens;
-    const uint4* codes = p.codes;
-    const int32_t* table = p.page_table;
-    if (p.seqs) {
+      tiles = cum[s + 1] - cum[s];
+      at = pos - cum[s] * pieces;
+      n = __ldg(p.seq_len_dev + s) - 1;
       codes = static_cast<const uint4*>(p.seqs[s].code_data);
       table = p.seqs[s].code_table;
     }
+    const int piece = at / tiles, first = at - piece * tiles, end = min(tiles, first + line_end - pos);
+    pos += end - first;
+    const int head0 = (GROUPED ? piece / q_split : piece) * HP;                   // first cache head
+    const int part0 = GROUPED ? (piece - head0 / HP * q_split) * q_part : 0;       // first query head of each of them
+    const int heads = GROUPED ? min(q_part, q_group - part0) : 1;                  // query heads of each
 
     // ---- copies -----------------------------------------------------------------------------------------------
     // the page numbers of an item's tokens (lane = token of each group of 32) are fetched one item ahead of its copies
-    int item_q = first + warp, tile_q = item_q / pieces, piece_q = item_q - tile_q * pieces;
-    const int dt = warps / pieces, dp = warps - dt * pieces;
-    auto step = [&](int& tile, int& piece) {
-      tile += dt;
-      piece += dp;
-      if (piece >= pieces) {
-        piece -= pieces;
-        ++tile;
-      }
-    };
-    int entry[kGroups];
-    auto fetch_entries = [&](int tile) {
+    auto fetch_entries = [&](int tile, int (&entry)[kGroups]) {
 #pragma unroll
       for (int k = 0; k < kGroups; ++k) {
         const unsigned t = static_cast<unsigned>(min(tile * TT + k * 32 + lane, max(n - 1, 0)));   // (absent tokens: the last one's codes)
         entry[k] = __ldg(table + (p.ps_shift >= 0 ? t >> p.ps_shift : t / static_cast<unsigned>(p.page_size)));
       }
     };
-    auto request = [&](int tile, int piece, uint4* slot) {
+    const int64_t stride = 2 * p.H;
+    const uint4* base = codes + head0 * 2 + (lane & (CPR - 1));
+    auto request = [&](int tile, const int (&entry)[kGroups], uint4* slot) {
       int tok[kGroups];
 #pragma unroll
       for (int k = 0; k < kGroups; ++k) {
@@ -224,8 +246,6 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
       }
       constexpr int RPI = 32 / CPR;   // tokens per copy instruction
       const int c = lane & (CPR - 1), r0 = lane / CPR;
-      const uint4* base = codes + heads_of(piece) * CPR + c;
-      const int64_t stride = 2 * p.H;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int r = i * RPI + r0;   // r / 32 == i * RPI / 32
@@ -234,69 +254,70 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
         cp_async_16(slot + r * CPR + (c ^ f), base + slot_of * stride);
       }
     };
-    auto request_next = [&](int slot) {
-      if (item_q < end) {
-        request(tile_q, piece_q, ring + slot * (kItemBytes / 16));
-        step(tile_q, piece_q);
-        item_q += warps;
-        if (item_q < end) fetch_entries(tile_q);
-      }
-      cp_async_commit();
-    };
-    int tile_u = tile_q, piece_u = piece_q;   // the item in use
+    // (the page numbers of the first items are on their way together)
+    int entry[kGroups], first_entry[kItemMaxSlots][kGroups];
 #pragma unroll
-    for (int k = 0; k < kGroups; ++k) entry[k] = 0;
-    if (item_q < end) fetch_entries(tile_q);
-    for (int i = 0; i < slots; ++i) request_next(i);
+    for (int i = 0; i < kItemMaxSlots; ++i)
+      if (i < slots && first + warp + i * kItemWarps < end) fetch_entries(first + warp + i * kItemWarps, first_entry[i]);
+    int next = first + warp + slots * kItemWarps;   // the item to be requested next
+    if (next < end) fetch_entries(next, entry);
+    // (the new token sits at position n = tokens before it)
+    if (cs_here) sh.cs[cs_pair] = rope_cos_sin_at(cs_freq, static_cast<float>(n));
+#pragma unroll
+    for (int i = 0; i < kItemMaxSlots; ++i) {
+      if (i < slots) {
+        if (first + warp + i * kItemWarps < end) request(first + warp + i * kItemWarps, first_entry[i], ring + i * (kItemBytes / 16));
+        cp_async_commit();
+      }
+    }
 
     // ---- the sequence's query: codes, planes; the new token's rows ---------------------------------------------
-    if (p.ap.rope_on) {
-      // the new token sits at position n (= tokens before it)
-      if (tid < kHeadDim / 2) sh.cs[tid] = rope_cos_sin(tid, static_cast<float>(n), p.ap.rp);
-    }
-    if (p.count_local)
-      for (int i = tid; i < rows * (kItemCountWords / 4); i += threads) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
-    if (p.ap.rope_on) __syncthreads();
     if (!waited) {
       grid_dependency_wait();   // q, k, v or the query codes are the preceding kernel's output
       grid_launch_dependents();
       waited = true;
     }
-    if (p.ap.q) {
+    const int64_t seq_row = static_cast<int64_t>(s) * rows;
+    auto query_row = [&](int r) {   // row of the sequence that the segment's row r stands for
+      return GROUPED ? (head0 + r / q_part) * q_group + part0 + r % q_part : head0 + r;
+    };
+    const int my_rows = HP * q_part;       // (of a short last part each cache head's last ones are absent)
+    const unsigned l8 = lane & 7;
+    const int cr = tid >> 3;               // the row that these eight threads code (a pass of the block holds all rows)
+    const bool coding = warp * 4 < my_rows, live_row = cr < my_rows && (!GROUPED || cr % q_part < heads);
+    const int64_t code_row = seq_row + (live_row ? query_row(cr) : 0);
+    uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
+    if (APPEND && coding) {
+      const T* src = static_cast<const T*>(p.ap.q) + code_row * kHeadDim + l8 * 16;
+      q0 = ld_16(src);
+      q1 = ld_16(src + 8);
+    }
+    // (while the query is on its way)
+    const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
+    const int slice0 = p.hist ? first * TT / slice_tokens : 0;
+    const int used = p.hist ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
+    for (int i = tid; i < used * seg_rows * (kItemCountWords / 4); i += kItemThreads) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
+    if (APPEND && p.ap.rope_on) __syncthreads();
+    if (APPEND) {
       const StepAppend& ap = p.ap;
-      const unsigned l8 = lane & 7;
       const bool scaled = ap.rp.inv_freq != nullptr;
-      if (p.seqs && !apart) {
-        auto block_of = [&](int item) {
-          int k = static_cast<int>(static_cast<int64_t>(item) * B / total);
-          while (line_start(k + 1) <= item) ++k;
-          return k;
-        };
-        const int bf = block_of(seq0);
-        nblk = block_of(seq1 - 1) - bf + 1;
-        my_blk = b - bf;
-      }
-      for (int r0 = 0; r0 < rows; r0 += threads / 8) {
-        if (r0 + warp * 4 >= rows) break;   // (warp-uniform)
-        const int r = r0 + (tid >> 3);
-        const bool live = r < rows;
-        const T* src = static_cast<const T*>(ap.q) + (static_cast<int64_t>(s) * rows + (live ? r : 0)) * kHeadDim + l8 * 16;
+      if (coding) {   // (warp-uniform)
         float x[16];
-        unpack16<T>(ld_16(src), ld_16(src + 8), x);
+        unpack16<T>(q0, q1, x);
         if (ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, ap.rp.mscale);
         const uint32_t w = code_word_8lanes<T>(x, l8, ap.scale, ap.th);
-        if (live) {
-          uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * r + (l8 >> 2)) + (l8 & 3);
+        if (live_row) {
+          uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * cr + (l8 >> 2)) + (l8 & 3);
           qp[0] = w;
           qp[4] = qplane_d(w);
-          if ((r / q_group) % nblk == my_blk)
-            reinterpret_cast<uint32_t*>(ap.q_code_out)[(static_cast<int64_t>(s) * rows + r) * (kCodeWords / 2) + l8] = w;
+          if (first == 0) reinterpret_cast<uint32_t*>(ap.q_code_out)[code_row * (kCodeWords / 2) + l8] = w;
         }
       }
-      for (int h = my_blk + nblk * (tid >> 3); h - nblk * ((tid >> 3) & 3) < p.H; h += nblk * (threads / 8)) {
-        // (warp-uniform trip count: the four rows of a warp advance together)
-        const bool live = h < p.H;
-        const int64_t in_off = (static_cast<int64_t>(s) * p.H + (live ? h : 0)) * kHeadDim + l8 * 16;
+      // the new token's rows of the piece's cache heads, by the last warp of the block that has the piece's first tile
+      if (first == 0 && part0 == 0 && warp == kItemWarps - 1) {
+        const bool live = (lane >> 3) < HP;
+        const int h = head0 + (live ? lane >> 3 : 0);
+        const int64_t in_off = (static_cast<int64_t>(s) * p.H + h) * kHeadDim + l8 * 16;
         T* ksrc = static_cast<T*>(ap.k) + in_off;
         const T* vsrc = static_cast<const T*>(ap.v) + in_off;
         uint4 k0 = ld_16(ksrc), k1 = ld_16(ksrc + 8);
@@ -323,6 +344,7 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
           const float c[8] = {x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15]};
           k0 = pack8<T>(a);
           k1 = pack8<T>(c);
+          __syncwarp();   // (lanes without a row of their own have read the first one)
           if (live) {
             st_16(ksrc, k0);
             st_16(ksrc + 8, k1);
@@ -340,110 +362,95 @@ __global__ void __launch_bounds__(kItemThreads, 1) estimate_items_kernel(const E
         }
       }
     } else {
-      for (int c = tid; c < 2 * rows; c += threads) planes[c] = make_qplanes(__ldg(p.q_code + static_cast<int64_t>(s) * 2 * rows + c));
+      for (int c = tid; c < 2 * my_rows; c += kItemThreads) {
+        const int r = c >> 1;
+        if (!GROUPED || r % q_part < heads) planes[c] = make_qplanes(__ldg(p.q_code + (seq_row + query_row(r)) * 2 + (c & 1)));
+      }
     }
     __syncthreads();   // planes and zeroed counts are visible
 
     // ---- scan -----------------------------------------------------------------------------------------------------
-    const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
-    // the counts in shared memory are those of the slice in which this piece starts; tokens of later slices (few, unless
-    // the sequences are far shorter than a block's share) are counted in global memory one by one
-    const int slice0 = p.hist ? first / pieces * TT / slice_tokens : 0;
-    // (a 16-bit count must not overflow)
-    const int slice0_end = p.count_local ? min((slice0 + 1) * slice_tokens, first / pieces * TT + 65504) : 0;
-    uint32_t* hist = p.hist ? p.hist + static_cast<size_t>(s) * rows * kSaScratchWordsPerHead : nullptr;
-    uint16_t* out = static_cast<uint16_t*>(p.out) + static_cast<int64_t>(s) * rows * p.out_stride;
-    auto to_out = [&](unsigned d) { return p.out_half ? __half_as_ushort(__uint2half_rn(d)) : static_cast<uint16_t>(d); };   // (exact: d <= 384)
-    auto count_here = [&](int r, unsigned d) { atomicAdd(counts + r * kItemCountWords + (d >> 1), 1u << ((d & 1) * 16)); };
-    auto count_there = [&](int r, int t0, unsigned d) { hist_count(hist, r, t0 / slice_tokens, d); };
+    // the counts in shared memory are those of the first `used` slices that the segment touches; anything behind them is counted
+    // in global memory one by one
+    uint32_t* hist = p.hist ? p.hist + seq_row * kSaScratchWordsPerHead : nullptr;
+    uint16_t* out = static_cast<uint16_t*>(p.out) + seq_row * p.out_stride;
+    auto to_out = [&](unsigned d) { return !APPEND && p.out_half ? __half_as_ushort(__uint2half_rn(d)) : static_cast<uint16_t>(d); };   // (exact: d <= 384)
     const int f = HP == 4 ? (lane & 7) : HP == 2 ? ((lane >> 1) & 3) : ((lane >> 2) & 1);
     int use = 0;
-    for (int item = first + warp; item < end; item += warps) {
+    for (int tile = first + warp; tile < end; tile += kItemWarps) {
       if (slots == 3) cp_async_wait<2>(); else if (slots == 2) cp_async_wait<1>(); else cp_async_wait<0>();
       __syncwarp();
       const uint4* lrow = ring + use * (kItemBytes / 16) + lane * CPR;
-      if (!GROUPED) {
-        const int r_first = piece_u * HP;                        // first query row of the item
-        const QPlanes* qp0 = planes + 2 * r_first;
 #pragma unroll
-        for (int k = 0; k < kGroups; ++k) {
-          const int t0 = tile_u * TT + k * 32, t = t0 + lane;
+      for (int k = 0; k < kGroups; ++k) {
+        const int t0 = tile * TT + k * 32, t = t0 + lane;
+        uint32_t* tab = counts;   // (a group never straddles two slices)
+        bool here = p.hist != nullptr;
+        if (here) {
+#pragma unroll
+          for (int u = 1; u < kTables; ++u)
+            if (t0 >= (slice0 + u) * slice_tokens) tab += seg_rows * kItemCountWords;
+          here = t0 < (slice0 + kTables) * slice_tokens;
+        }
+        auto emit = [&](int r, uint16_t* o, unsigned d) {   // r: row of the segment
+          *o = to_out(d);
+          if (here) atomicAdd(tab + r * kItemCountWords + d, 1u);
+          else if (p.hist) hist_count(hist, query_row(r), t0 / slice_tokens, d);
+        };
+        if (!GROUPED) {
           unsigned d[HP];
 #pragma unroll
           for (int hh = 0; hh < HP; ++hh)
-            d[hh] = chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh) ^ f)], qp0[2 * hh]) +
-                    chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)], qp0[2 * hh + 1]);
+            d[hh] = chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh) ^ f)], planes[2 * hh]) +
+                    chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)], planes[2 * hh + 1]);
           if (t < n) {
-            uint16_t* o = out + r_first * p.out_stride + t;
+            uint16_t* o = out + head0 * p.out_stride + t;
 #pragma unroll
             for (int hh = 0; hh < HP; ++hh) {
-              *o = to_out(d[hh]);
+              emit(hh, o, d[hh]);
               o += p.out_stride;
             }
-            if (t0 < slice0_end) {   // (a group never straddles two slices)
-#pragma unroll
-              for (int hh = 0; hh < HP; ++hh) count_here(r_first + hh, d[hh]);
-            } else if (hist) {
-#pragma unroll
-              for (int hh = 0; hh < HP; ++hh) count_there(r_first + hh, t0, d[hh]);
-            }
           }
-        }
-      } else {
-        // grouped queries: a code is read once for the item's query heads of its cache head
-        auto grouped = [&](int r_first, int heads) {
-#pragma unroll
-          for (int k = 0; k < kGroups; ++k) {
-            const int t0 = tile_u * TT + k * 32, t = t0 + lane;
-#pragma unroll
-            for (int hh = 0; hh < HP; ++hh) {
-              const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
-              const int r1 = r_first + hh * q_group;
-              uint16_t* o = out + r1 * p.out_stride + t;
-#pragma unroll 4
-              for (int g = 0; g < heads; ++g) {
-                const int r = r1 + g;
-                const unsigned d = chunk_distance<METRIC>(k0, planes[2 * r]) + chunk_distance<METRIC>(k1, planes[2 * r + 1]);
-                if (t < n) {
-                  *o = to_out(d);
-                  if (t0 < slice0_end) count_here(r, d);
-                  else if (hist) count_there(r, t0, d);
-                }
-                o += p.out_stride;
-              }
-            }
-          }
-        };
-        if (q_split == 1) {
-          grouped(piece_u * HP * q_group, q_group);   // (a trip count that is the same for all warps)
         } else {
-          const int heads0 = heads_of(piece_u), g0 = (piece_u - heads0 * q_split) * q_part;
-          grouped(heads0 * HP * q_group + g0, min(q_part, q_group - g0));
+          // grouped queries: a code is read once for the piece's query heads of its cache head
+#pragma unroll
+          for (int hh = 0; hh < HP; ++hh) {
+            const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
+            uint16_t* o = out + ((head0 + hh) * q_group + part0) * p.out_stride + t;
+#pragma unroll 4
+            for (int g = 0; g < heads; ++g) {
+              const int r = hh * q_part + g;
+              const unsigned d = chunk_distance<METRIC>(k0, planes[2 * r]) + chunk_distance<METRIC>(k1, planes[2 * r + 1]);
+              if (t < n) emit(r, o, d);
+              o += p.out_stride;
+            }
+          }
         }
       }
       __syncwarp();   // the slot may be filled again
-      request_next(use);
-      step(tile_u, piece_u);
+      if (next < end) {
+        request(next, entry, ring + use * (kItemBytes / 16));
+        next += kItemWarps;
+        if (next < end) fetch_entries(next, entry);
+      }
+      cp_async_commit();
       if (++use == slots) use = 0;
     }
     cp_async_wait<0>();
     if (p.hist || pos < line_end) __syncthreads();
-    if (p.count_local) {
-      uint32_t* dst = hist + slice0 * kSaBins;
-      for (int i = tid; i < rows * (kItemCountWords / 4); i += threads) {
+    if (p.hist) {
+      for (int i = tid; i < used * seg_rows * (kItemCountWords / 4); i += kItemThreads) {
         const uint4 c4 = reinterpret_cast<const uint4*>(counts)[i];
         if (c4.x | c4.y | c4.z | c4.w) {
-          const int r = i / (kItemCountWords / 4);
-          uint32_t* at = dst + static_cast<size_t>(r) * kSaScratchWordsPerHead + (i - r * (kItemCountWords / 4)) * 8;
-          const uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-          for (int w = 0; w < 4; ++w) {
-            if (c[w] & 0xffffu) atomicAdd(at + 2 * w, c[w] & 0xffffu);
-            if (c[w] >> 16) atomicAdd(at + 2 * w + 1, c[w] >> 16);
-          }
+          const int tr = i / (kItemCountWords / 4), u = tr / seg_rows, r = tr - u * seg_rows;
+          uint32_t* dst = hist + static_cast<size_t>(query_row(r)) * kSaScratchWordsPerHead + (slice0 + u) * kSaBins + (i - tr * (kItemCountWords / 4)) * 4;
+          if (c4.x) atomicAdd(dst, c4.x);
+          if (c4.y) atomicAdd(dst + 1, c4.y);
+          if (c4.z) atomicAdd(dst + 2, c4.z);
+          if (c4.w) atomicAdd(dst + 3, c4.w);
         }
       }
-      if (pos < line_end) __syncthreads();   // the counts may be cleared for the next sequence
+      if (pos < line_end) __syncthreads();   // the counts may be cleared for the next segment
     }
   }
 }

@@ -72,12 +72,17 @@ struct RopeParams {
 
 // (cos, sin) of dimension pair j at position pos: the one expression every kernel that rotates a decode
 // token uses, so that all of them produce the same bits.
-__device__ __forceinline__ float2 rope_cos_sin(int j, float pos, const RopeParams& rp) {
-  const float inv_freq = rp.inv_freq ? __ldg(rp.inv_freq + j)
-                                     : rp.rcp_scale / powf(rp.theta, static_cast<float>(2 * j) * (1.0f / kHeadDim));
+// (In two parts: the frequency does not depend on the position, which may still be on its way from memory.)
+__device__ __forceinline__ float rope_inv_freq(int j, const RopeParams& rp) {
+  return rp.inv_freq ? __ldg(rp.inv_freq + j) : rp.rcp_scale / powf(rp.theta, static_cast<float>(2 * j) * (1.0f / kHeadDim));
+}
+__device__ __forceinline__ float2 rope_cos_sin_at(float inv_freq, float pos) {
   float sn, cs;
   sincosf(pos * inv_freq, &sn, &cs);
   return make_float2(cs, sn);
+}
+__device__ __forceinline__ float2 rope_cos_sin(int j, float pos, const RopeParams& rp) {
+  return rope_cos_sin_at(rope_inv_freq(j, rp), pos);
 }
 
 // The same rotation with the 64 (cos, sin) pairs of the position given (shared memory): what the decode
