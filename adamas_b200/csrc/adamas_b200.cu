@@ -546,7 +546,7 @@ static bool many_distances(int q_heads, int batch, int n) {
 }
 // Which estimate kernel.  The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of
 // its heads in registers; the item kernel takes the rest, and long single sequences, where it counts in shared memory.  Whole step,
-// us a layer, tiles / items: 32 heads 4K 12.0 / 13.1, 32K 20.5 / 21.0, 128K 48.9 / 47.7; 8 x 32K 79.7 / 82.4; 32 x 4-8K 75.0 / 74.7.
+// us a layer, tiles / items: 32 heads 4K 12.0 / 13.1, 32K 20.5 / 21.0, 128K 48.9 / 45.7; 8 x 32K 79.7 / 81.3; 32 x 4-8K 75.0 / 72.7.
 static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n) {
   return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64) && (batch > 1 || !many_distances(q_heads, 1, n));
 }
@@ -581,7 +581,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   prm.n_tokens = n;
   prm.H = num_heads;
   prm.q_group = q_heads / num_heads;
-  prm.chip_warps = kItemWarps * kItemBlocksPerSm * di->num_sms;
+  prm.q_part = 1;
   prm.page_size = page_size;
   prm.ps_shift = log2_exact(page_size);
   prm.batch = batch;
@@ -626,15 +626,21 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   }
   ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0, "q_code must be 16-byte aligned");
   const int hp = item_cache_heads(num_heads, prm.q_group);
-  int64_t items = static_cast<int64_t>(n / (128 / hp) + 1) * (num_heads / hp) * batch;
+  const int64_t tiles = n / (128 / hp) + 1;   // of a sequence
+  int64_t items = tiles * (num_heads / hp) * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
-  const int q_part = item_query_heads(static_cast<int>(items), prm.q_group, prm.chip_warps);
-  items *= (prm.q_group + q_part - 1) / q_part;
+  const int slots_all = est_blocks_per_sm() * di->num_sms;   // resident blocks
+  prm.q_part = item_query_heads(static_cast<int>(items), prm.q_group, kItemWarps * kItemBlocksPerSm * di->num_sms);
+  const int pieces = num_heads / hp * ((prm.q_group + prm.q_part - 1) / prm.q_part);
+  items = tiles * pieces * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
-  const dim3 grid(static_cast<unsigned>(std::min<int64_t>(static_cast<int64_t>(est_blocks_per_sm()) * di->num_sms, items)));
-  const int64_t per_block = (items + grid.x - 1) / grid.x;
-  // (with the length on the device a shorter sequence's groups may be cut into smaller parts, never into larger ones)
-  const int seg_rows = hp * q_part;
+  dim3 grid(static_cast<unsigned>(std::min<int64_t>(slots_all, items)));
+  int64_t per_block = (items + grid.x - 1) / grid.x;
+  if (!seqs) {   // an equal number of blocks for every piece (a remainder of the chip's stays idle: at most 3 % for up to 64 heads)
+    grid = dim3(static_cast<unsigned>(std::min<int64_t>(std::max(1, slots_all / pieces), tiles)), static_cast<unsigned>(pieces));
+    per_block = (tiles + grid.x - 1) / grid.x;
+  }
+  const int seg_rows = hp * prm.q_part;
   const size_t room = static_cast<size_t>(di->smem_per_sm / kItemBlocksPerSm - 1024 - kItemStatic);
   size_t smem = static_cast<size_t>(seg_rows) * 2 * sizeof(QPlanes);
   if (hist) smem += static_cast<size_t>(item_tables(hp, prm.q_group > 1)) * seg_rows * kItemCountWords * sizeof(uint32_t);

@@ -2,7 +2,10 @@
 // for 16, 32 and 64 heads is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (56 instructions, 12 of them population counts at quarter rate, per 32 distances) for grouped
-// queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM; every warp works alone:
+// queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the
+// query while the others' first items are on their way, and appends the new token while they scan (a block that starts late, next
+// to the last blocks of the kernel in front, had its query 4.5 us after its start when the scanning warps coded it themselves
+// behind their requests; now the codes are there 0.6 us after that kernel's end).  The other seven work alone:
 //   * its unit of work is an item of 4 KB of codes: 128 / HP tokens x HP heads (HP = 4, 2 or 1, see item_cache_heads).
 //     Its own 16-byte asynchronous copies bring items into its own ring of two or three slots: no
 //     producer warp, no barrier between warps.  (A bulk copy with a different address in every lane is issued lane after
@@ -16,21 +19,23 @@
 //     the global per-slice histograms once per block.  One L2 atomic per distance runs at 90 to 165 per ns on the whole chip, which
 //     made 1 M distances 6 to 8 us; additions of the constant 1 in shared memory take 1 to 2 cycles per warp, those of packed
 //     16-bit counts 4 to 13 (lanes that meet in a word are taken one after the other).
-// All items of a launch form one line: sequence after sequence, in it piece after piece (HP cache heads), in it token after token.
-// So a block works on a few rows over many tokens: it codes 4 to 16 query rows instead of all, its tables are small, and it adds up as
-// many distances as there are before a table goes out.  The line is cut evenly over the blocks, or, with few segments (a piece of a
-// sequence), every block takes a part of one.  The first items are requested before the kernel's dependency resolves (the cached
-// codes are final).
+// A piece is HP cache heads (with a part of their query heads, item_query_heads).  A block works on one piece of a sequence over
+// many tokens: it codes 4 to 16 query rows instead of all, its tables are small, and it adds up as many distances as there are before
+// a table goes out.  One sequence: every piece has the same number of blocks, which share its tokens evenly (nothing but a division lies
+// between a block's start and its first request).  A batch: sequence after sequence, in it piece after piece, in it token after
+// token forms one line that is cut evenly over the blocks, or, with few segments (a piece of a sequence), every block takes a part
+// of one.  The first items are requested before the kernel's dependency resolves (the cached codes are final).
 // Measured, the whole step, us a layer, against token after token with all heads in it and one block of 16 warps per SM: 40 heads,
-// 12K 18.1 -> 16.7; 32 query heads over 8, 30K 24.6 -> 23.7; 4 sequences x 128K x 4 heads 35.6 -> 34.1; 32 heads, 128K 49.1 -> 47.4
-// (tile pipeline and a counting launch).  Lane = head with four tokens per lane (one 4 KB run of codes per warp) was slower than lane = token.
+// 12K 18.1 -> 15.9; 32 query heads over 8, 30K 24.6 -> 23.7; 4 sequences x 128K x 4 heads 35.6 -> 32.5; 32 heads, 128K 49.1 -> 45.7
+// (tile pipeline and a counting launch).  Eight scanning warps and a ninth leave 96 registers: 26.2 for the grouped case.
+// Lane = head with four tokens per lane (one 4 KB run of codes per warp) was slower than lane = token.
 #pragma once
 #include "estimate.cuh"
 
 namespace adamas {
 
-constexpr int kItemWarps = 8;
-constexpr int kItemThreads = kItemWarps * 32;
+constexpr int kItemWarps = 7;            // that scan
+constexpr int kItemThreads = kItemWarps * 32 + 32;   // (one more warp: the query and the append)
 constexpr int kItemBlocksPerSm = 2;
 constexpr int kItemMaxSlots = 3;         // ring slots per warp at most
 constexpr int kItemBytes = 4096;
@@ -42,12 +47,12 @@ constexpr int kItemCountWords = 388;     // counts per query row and table (a di
 // that works on it).  The group of a cache head is halved as long as every part still
 // finds a warp of its own (`warps` on the chip; `items` are those of undivided groups): a second round costs more than it saves.
 constexpr int kItemRows = 8;
-__host__ __device__ __forceinline__ int item_cache_heads(int kv_heads, int q_group) {
+inline int item_cache_heads(int kv_heads, int q_group) {
   int hp = 4;
   while (hp > 1 && (kv_heads % hp != 0 || (q_group > 1 && hp * q_group > kItemRows))) hp /= 2;
   return hp;
 }
-__host__ __device__ __forceinline__ int item_query_heads(int items, int q_group, int warps) {
+inline int item_query_heads(int items, int q_group, int warps) {
   int heads = q_group;
   for (; heads > 2 * kItemRows; items *= 2) heads = (heads + 1) / 2;
   for (; heads > 1 && items <= warps / 2; items *= 2) heads = (heads + 1) / 2;
@@ -145,66 +150,60 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   uint32_t* counts = reinterpret_cast<uint32_t*>(planes + 2 * seg_rows);
   int* cum = reinterpret_cast<int*>(counts + (p.hist ? kTables * seg_rows * kItemCountWords : 0));
   uint4* ring = reinterpret_cast<uint4*>(item_smem + warp * (slots * kItemBytes));
-  // (the position's rotation is formed by warps that have nothing else to do for the query)
-  const int cs_pair = tid - 4 * 32;
-  const bool cs_here = APPEND && p.ap.rope_on && cs_pair >= 0 && cs_pair < kHeadDim / 2;
+  // The last warp codes the query, while the others request the first items, and appends the new token while they scan.
+  const bool scanning = warp < kItemWarps;
+  // (the position's rotation: two of the other warps)
+  const int cs_pair = tid - (kItemWarps - 2) * 32;
+  const bool cs_here = APPEND && p.ap.rope_on && scanning && cs_pair >= 0;
   const float cs_freq = cs_here ? rope_inv_freq(cs_pair, p.ap.rp) : 0.f;
+  const int q_part = GROUPED ? p.q_part : 1;
+  const int q_split = GROUPED ? (q_group + q_part - 1) / q_part : 1;
 
-  // ---- the line of items: sequence after sequence, in it piece after piece (HP cache heads with a part of their query heads),
-  // in it token tile after token tile -----------------------------------------------------------------------------------
-  int tiles_all;
+  // ---- this block's part of the work ------------------------------------------------------------------------------------
+  // One sequence: blockIdx.y is the piece (HP cache heads with a part of their query heads), blockIdx.x an equal part of its tiles.
+  // A batch: all items form a line, sequence after sequence, in it piece after piece, in it token tile after token tile.
+  int pieces = gridDim.y, tiles_all, pos = 0, line_end = 1;
   if (p.seqs) {
+    pieces = p.H / HP * q_split;
     if (warp == 0) est_line(p, TT, lane, cum);
     __syncthreads();
     tiles_all = cum[p.batch];
-  } else {
-    tiles_all = est_tiles(len0, TT);
-  }
-  const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
-  const int q_split = q_part == q_group ? 1 : (q_group + q_part - 1) / q_part, pieces = p.H / HP * q_split;
-  const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
-  if (total == 0) return;
-  const int b = blockIdx.x, segments = p.batch * pieces;
-  auto seg_start = [&](int g) {   // where segment g (a piece of a sequence) starts on the line
-    if (!p.seqs) return g * tiles_all;
-    const int s = g / pieces;
-    return s == p.batch ? total : cum[s] * pieces + (g - s * pieces) * (cum[s + 1] - cum[s]);
-  };
-  int pos, line_end;
-  // With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the uneven
-  // shares is less than a second segment costs (queries to load and code behind a barrier, counts to add up).
-  if (segments <= static_cast<int>(gridDim.x) && static_cast<int64_t>(total) * segments <= static_cast<int64_t>(kItemApart) * gridDim.x * gridDim.x) {
-    // (the rule keeps every product below 2^31)
-    const int spare = gridDim.x - segments;
-    auto first_block = [&](int g) { return g + (p.seqs ? seg_start(g) * spare / total : g * spare / segments); };
-    int g = b * segments / static_cast<int>(gridDim.x);   // the last segment that starts at or before this block
-    if (p.seqs) {
+    const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
+    const int b = blockIdx.x, segments = p.batch * pieces;
+    auto seg_start = [&](int g) {   // where segment g (a piece of a sequence) starts on the line
+      const int s = g / pieces;
+      return s == p.batch ? total : cum[s] * pieces + (g - s * pieces) * (cum[s + 1] - cum[s]);
+    };
+    // With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the
+    // uneven shares is less than a second segment costs (queries to load and code behind a barrier, counts to add up).
+    if (segments <= static_cast<int>(gridDim.x) && static_cast<int64_t>(total) * segments <= static_cast<int64_t>(kItemApart) * gridDim.x * gridDim.x) {
+      // (the rule keeps every product below 2^31)
+      const int spare = gridDim.x - segments;
+      auto first_block = [&](int g) { return g + seg_start(g) * spare / total; };
       int lo = 0, hi = segments - 1;
-      while (lo < hi) {
+      while (lo < hi) {   // the last segment that starts at or before this block
         const int mid = (lo + hi + 1) >> 1;
         if (first_block(mid) <= b) lo = mid; else hi = mid - 1;
       }
-      g = lo;
+      const int start = seg_start(lo), n_items = seg_start(lo + 1) - start, f = first_block(lo), nblk = min(first_block(lo + 1) - f, n_items);
+      if (b - f >= nblk) return;
+      pos = start + n_items * (b - f) / nblk;
+      line_end = start + n_items * (b - f + 1) / nblk;
     } else {
-      while (first_block(g) > b) --g;
-      while (g + 1 < segments && first_block(g + 1) <= b) ++g;
+      const int B = min(static_cast<int>(gridDim.x), total);   // (every block that takes part has some)
+      if (b >= B) return;
+      const int q = total / B, r = total - q * B;
+      pos = b * q + b * r / B;   // b * total / B
+      line_end = (b + 1) * q + (b + 1) * r / B;
     }
-    const int start = seg_start(g), n_items = seg_start(g + 1) - start, f = first_block(g), nblk = min(first_block(g + 1) - f, n_items);
-    if (b - f >= nblk) return;
-    pos = start + n_items * (b - f) / nblk;
-    line_end = start + n_items * (b - f + 1) / nblk;
   } else {
-    const int B = min(static_cast<int>(gridDim.x), total);   // (every block that takes part has some)
-    if (b >= B) return;
-    const int q = total / B, r = total - q * B;
-    pos = b * q + b * r / B;   // b * total / B
-    line_end = (b + 1) * q + (b + 1) * r / B;
+    tiles_all = est_tiles(len0, TT);
   }
   bool waited = false;
 
   while (pos < line_end) {
     // ---- this block's next segment: tiles [first, end) of a piece of a sequence ----------------------------------------
-    int s = 0, tiles = tiles_all, at = pos, n = len0;
+    int s = 0, n = len0, piece, first, end;
     const uint4* codes = p.codes;
     const int32_t* table = p.page_table;
     if (p.seqs) {
@@ -214,14 +213,22 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
         if (cum[mid] * pieces <= pos) lo = mid; else hi = mid - 1;
       }
       s = lo;
-      tiles = cum[s + 1] - cum[s];
-      at = pos - cum[s] * pieces;
+      const int tiles = cum[s + 1] - cum[s], at = pos - cum[s] * pieces;
+      piece = at / tiles;
+      first = at - piece * tiles;
+      end = min(tiles, first + line_end - pos);
+      pos += end - first;
       n = __ldg(p.seq_len_dev + s) - 1;
       codes = static_cast<const uint4*>(p.seqs[s].code_data);
       table = p.seqs[s].code_table;
+    } else {
+      const int share = (tiles_all + gridDim.x - 1) / gridDim.x;
+      piece = blockIdx.y;
+      first = blockIdx.x * share;
+      end = min(tiles_all, first + share);
+      pos = line_end;
+      if (first >= end) return;
     }
-    const int piece = at / tiles, first = at - piece * tiles, end = min(tiles, first + line_end - pos);
-    pos += end - first;
     const int head0 = (GROUPED ? piece / q_split : piece) * HP;                   // first cache head
     const int part0 = GROUPED ? (piece - head0 / HP * q_split) * q_part : 0;       // first query head of each of them
     const int heads = GROUPED ? min(q_part, q_group - part0) : 1;                  // query heads of each
@@ -258,15 +265,18 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     int entry[kGroups], first_entry[kItemMaxSlots][kGroups];
 #pragma unroll
     for (int i = 0; i < kItemMaxSlots; ++i)
-      if (i < slots && first + warp + i * kItemWarps < end) fetch_entries(first + warp + i * kItemWarps, first_entry[i]);
+      if (i < slots && scanning && first + warp + i * kItemWarps < end) fetch_entries(first + warp + i * kItemWarps, first_entry[i]);
     int next = first + warp + slots * kItemWarps;   // the item to be requested next
-    if (next < end) fetch_entries(next, entry);
+    if (scanning && next < end) fetch_entries(next, entry);
     // (the new token sits at position n = tokens before it)
-    if (cs_here) sh.cs[cs_pair] = rope_cos_sin_at(cs_freq, static_cast<float>(n));
+    if (cs_here) {
+      sh.cs[cs_pair] = rope_cos_sin_at(cs_freq, static_cast<float>(n));
+      asm volatile("bar.arrive 1, 96;" ::: "memory");   // (these two warps and the last one)
+    }
 #pragma unroll
     for (int i = 0; i < kItemMaxSlots; ++i) {
       if (i < slots) {
-        if (first + warp + i * kItemWarps < end) request(first + warp + i * kItemWarps, first_entry[i], ring + i * (kItemBytes / 16));
+        if (scanning && first + warp + i * kItemWarps < end) request(first + warp + i * kItemWarps, first_entry[i], ring + i * (kItemBytes / 16));
         cp_async_commit();
       }
     }
@@ -283,91 +293,103 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     };
     const int my_rows = HP * q_part;       // (of a short last part each cache head's last ones are absent)
     const unsigned l8 = lane & 7;
-    const int cr = tid >> 3;               // the row that these eight threads code (a pass of the block holds all rows)
-    const bool coding = warp * 4 < my_rows, live_row = cr < my_rows && (!GROUPED || cr % q_part < heads);
-    const int64_t code_row = seq_row + (live_row ? query_row(cr) : 0);
-    uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
-    if (APPEND && coding) {
-      const T* src = static_cast<const T*>(p.ap.q) + code_row * kHeadDim + l8 * 16;
-      q0 = ld_16(src);
-      q1 = ld_16(src + 8);
-    }
-    // (while the query is on its way)
+    const bool scaled = p.ap.rp.inv_freq != nullptr;
     const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
     const int slice0 = p.hist ? first * TT / slice_tokens : 0;
     const int used = p.hist ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
-    for (int i = tid; i < used * seg_rows * (kItemCountWords / 4); i += kItemThreads) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
-    if (APPEND && p.ap.rope_on) __syncthreads();
-    if (APPEND) {
-      const StepAppend& ap = p.ap;
-      const bool scaled = ap.rp.inv_freq != nullptr;
-      if (coding) {   // (warp-uniform)
-        float x[16];
-        unpack16<T>(q0, q1, x);
-        if (ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, ap.rp.mscale);
-        const uint32_t w = code_word_8lanes<T>(x, l8, ap.scale, ap.th);
-        if (live_row) {
-          uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * cr + (l8 >> 2)) + (l8 & 3);
-          qp[0] = w;
-          qp[4] = qplane_d(w);
-          if (first == 0) reinterpret_cast<uint32_t*>(ap.q_code_out)[code_row * (kCodeWords / 2) + l8] = w;
-        }
-      }
-      // the new token's rows of the piece's cache heads, by the last warp of the block that has the piece's first tile
-      if (first == 0 && part0 == 0 && warp == kItemWarps - 1) {
-        const bool live = (lane >> 3) < HP;
-        const int h = head0 + (live ? lane >> 3 : 0);
-        const int64_t in_off = (static_cast<int64_t>(s) * p.H + h) * kHeadDim + l8 * 16;
-        T* ksrc = static_cast<T*>(ap.k) + in_off;
-        const T* vsrc = static_cast<const T*>(ap.v) + in_off;
-        uint4 k0 = ld_16(ksrc), k1 = ld_16(ksrc + 8);
-        const uint4 v0 = ld_16(vsrc), v1 = ld_16(vsrc + 8);
-        PagedTarget tgt = ap.tgt;
-        if (p.seqs) {
-          tgt.kv_data = p.seqs[s].kv_data;
-          tgt.kv_table = p.seqs[s].kv_table;
-          tgt.code_data = static_cast<uint16_t*>(p.seqs[s].code_data);
-          tgt.code_table = p.seqs[s].code_table;
-        }
-        const int ps = tgt.page_size;
-        int kv_last_page = ap.kv_last_page, kv_entry = ap.kv_entry, code_last_page = ap.code_last_page, code_entry = ap.code_entry;
-        if (p.seq_len_dev) {
-          kv_last_page = code_last_page = n / ps;
-          kv_entry = code_entry = n - kv_last_page * ps;
-        }
-        const int64_t kv_page = __ldg(tgt.kv_table + kv_last_page), code_page = __ldg(tgt.code_table + code_last_page);
-        float x[16];
-        unpack16<T>(k0, k1, x);
-        if (ap.rope_on) {
-          rope_8lanes<T>(x, l8, sh.cs, scaled, ap.rp.mscale);
-          const float a[8] = {x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
-          const float c[8] = {x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15]};
-          k0 = pack8<T>(a);
-          k1 = pack8<T>(c);
-          __syncwarp();   // (lanes without a row of their own have read the first one)
-          if (live) {
-            st_16(ksrc, k0);
-            st_16(ksrc + 8, k1);
+    if (scanning) {
+      for (int i = tid; i < used * seg_rows * (kItemCountWords / 4); i += kItemWarps * 32) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
+    } else if (APPEND) {
+      // eight lanes per row, four rows at a time, two times four on their way together
+      for (int r0 = 0; r0 < my_rows; r0 += 8) {
+        uint4 q[2][2];
+        int64_t code_row[2];
+        bool live[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int r = r0 + 4 * u + (lane >> 3);
+          live[u] = r < my_rows && (!GROUPED || r % q_part < heads);
+          code_row[u] = seq_row + (live[u] ? query_row(r) : 0);
+          if (r0 + 4 * u < my_rows) {
+            const T* src = static_cast<const T*>(p.ap.q) + code_row[u] * kHeadDim + l8 * 16;
+            q[u][0] = ld_16(src);
+            q[u][1] = ld_16(src + 8);
           }
         }
-        const uint32_t w = code_word_8lanes<T>(x, l8, ap.scale, ap.th);
-        if (live) {
-          T* dst = static_cast<T*>(tgt.kv_data) + ((kv_page * 2 * ps + kv_entry) * p.H + h) * kHeadDim + l8 * 16;
-          st_16(dst, k0);
-          st_16(dst + 8, k1);
-          dst += static_cast<int64_t>(ps) * p.H * kHeadDim;
-          st_16(dst, v0);
-          st_16(dst + 8, v1);
-          reinterpret_cast<uint32_t*>(tgt.code_data)[((code_page * ps + code_entry) * p.H + h) * (kCodeWords / 2) + l8] = w;
+        if (r0 == 0 && p.ap.rope_on) asm volatile("bar.sync 1, 96;" ::: "memory");   // (the rotation is there)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (r0 + 4 * u < my_rows) {   // (warp-uniform)
+            float x[16];
+            unpack16<T>(q[u][0], q[u][1], x);
+            if (p.ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, p.ap.rp.mscale);
+            const uint32_t w = code_word_8lanes<T>(x, l8, p.ap.scale, p.ap.th);
+            if (live[u]) {
+              uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * (r0 + 4 * u + (lane >> 3)) + (l8 >> 2)) + (l8 & 3);
+              qp[0] = w;
+              qp[4] = qplane_d(w);
+              if (first == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[code_row[u] * (kCodeWords / 2) + l8] = w;
+            }
+          }
         }
       }
     } else {
-      for (int c = tid; c < 2 * my_rows; c += kItemThreads) {
+      for (int c = lane; c < 2 * my_rows; c += 32) {
         const int r = c >> 1;
         if (!GROUPED || r % q_part < heads) planes[c] = make_qplanes(__ldg(p.q_code + (seq_row + query_row(r)) * 2 + (c & 1)));
       }
     }
     __syncthreads();   // planes and zeroed counts are visible
+
+    // ---- the new token's rows of the piece's cache heads, in the block that has the piece's first tile ----------------------
+    if (APPEND && !scanning && first == 0 && part0 == 0) {
+      const StepAppend& ap = p.ap;
+      const bool live = (lane >> 3) < HP;
+      const int h = head0 + (live ? lane >> 3 : 0);
+      const int64_t in_off = (static_cast<int64_t>(s) * p.H + h) * kHeadDim + l8 * 16;
+      T* ksrc = static_cast<T*>(ap.k) + in_off;
+      const T* vsrc = static_cast<const T*>(ap.v) + in_off;
+      uint4 k0 = ld_16(ksrc), k1 = ld_16(ksrc + 8);
+      const uint4 v0 = ld_16(vsrc), v1 = ld_16(vsrc + 8);
+      PagedTarget tgt = ap.tgt;
+      if (p.seqs) {
+        tgt.kv_data = p.seqs[s].kv_data;
+        tgt.kv_table = p.seqs[s].kv_table;
+        tgt.code_data = static_cast<uint16_t*>(p.seqs[s].code_data);
+        tgt.code_table = p.seqs[s].code_table;
+      }
+      const int ps = tgt.page_size;
+      int kv_last_page = ap.kv_last_page, kv_entry = ap.kv_entry, code_last_page = ap.code_last_page, code_entry = ap.code_entry;
+      if (p.seq_len_dev) {
+        kv_last_page = code_last_page = n / ps;
+        kv_entry = code_entry = n - kv_last_page * ps;
+      }
+      const int64_t kv_page = __ldg(tgt.kv_table + kv_last_page), code_page = __ldg(tgt.code_table + code_last_page);
+      float x[16];
+      unpack16<T>(k0, k1, x);
+      if (ap.rope_on) {
+        rope_8lanes<T>(x, l8, sh.cs, scaled, ap.rp.mscale);
+        const float a[8] = {x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
+        const float c[8] = {x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15]};
+        k0 = pack8<T>(a);
+        k1 = pack8<T>(c);
+        __syncwarp();   // (lanes without a row of their own have read the first one)
+        if (live) {
+          st_16(ksrc, k0);
+          st_16(ksrc + 8, k1);
+        }
+      }
+      const uint32_t w = code_word_8lanes<T>(x, l8, ap.scale, ap.th);
+      if (live) {
+        T* dst = static_cast<T*>(tgt.kv_data) + ((kv_page * 2 * ps + kv_entry) * p.H + h) * kHeadDim + l8 * 16;
+        st_16(dst, k0);
+        st_16(dst + 8, k1);
+        dst += static_cast<int64_t>(ps) * p.H * kHeadDim;
+        st_16(dst, v0);
+        st_16(dst + 8, v1);
+        reinterpret_cast<uint32_t*>(tgt.code_data)[((code_page * ps + code_entry) * p.H + h) * (kCodeWords / 2) + l8] = w;
+      }
+    }
 
     // ---- scan -----------------------------------------------------------------------------------------------------
     // the counts in shared memory are those of the first `used` slices that the segment touches; anything behind them is counted
@@ -377,7 +399,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     auto to_out = [&](unsigned d) { return !APPEND && p.out_half ? __half_as_ushort(__uint2half_rn(d)) : static_cast<uint16_t>(d); };   // (exact: d <= 384)
     const int f = HP == 4 ? (lane & 7) : HP == 2 ? ((lane >> 1) & 3) : ((lane >> 2) & 1);
     int use = 0;
-    for (int tile = first + warp; tile < end; tile += kItemWarps) {
+    for (int tile = scanning ? first + warp : end; tile < end; tile += kItemWarps) {
       if (slots == 3) cp_async_wait<2>(); else if (slots == 2) cp_async_wait<1>(); else cp_async_wait<0>();
       __syncwarp();
       const uint4* lrow = ring + use * (kItemBytes / 16) + lane * CPR;
@@ -392,37 +414,43 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
             if (t0 >= (slice0 + u) * slice_tokens) tab += seg_rows * kItemCountWords;
           here = t0 < (slice0 + kTables) * slice_tokens;
         }
-        auto emit = [&](int r, uint16_t* o, unsigned d) {   // r: row of the segment
-          *o = to_out(d);
-          if (here) atomicAdd(tab + r * kItemCountWords + d, 1u);
-          else if (p.hist) hist_count(hist, query_row(r), t0 / slice_tokens, d);
+        // up to four rows' distances: segment rows r .., output rows `row` ..
+        auto emit = [&](int r, int row, const unsigned* d, int many) {
+          if (t >= n) return;
+          uint16_t* o = out + row * p.out_stride + t;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (u < many) o[u * p.out_stride] = to_out(d[u]);
+          if (here) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (u < many) atomicAdd(tab + (r + u) * kItemCountWords + d[u], 1u);
+          } else if (p.hist) {
+            const int slice = t0 / slice_tokens;
+#pragma unroll 1
+            for (int u = 0; u < many; ++u) hist_count(hist, row + u, slice, u == 0 ? d[0] : u == 1 ? d[1] : u == 2 ? d[2] : d[3]);
+          }
         };
         if (!GROUPED) {
-          unsigned d[HP];
+          unsigned d[4];
 #pragma unroll
           for (int hh = 0; hh < HP; ++hh)
             d[hh] = chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh) ^ f)], planes[2 * hh]) +
                     chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)], planes[2 * hh + 1]);
-          if (t < n) {
-            uint16_t* o = out + head0 * p.out_stride + t;
-#pragma unroll
-            for (int hh = 0; hh < HP; ++hh) {
-              emit(hh, o, d[hh]);
-              o += p.out_stride;
-            }
-          }
+          emit(0, head0, d, HP);
         } else {
           // grouped queries: a code is read once for the piece's query heads of its cache head
 #pragma unroll
           for (int hh = 0; hh < HP; ++hh) {
             const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
-            uint16_t* o = out + ((head0 + hh) * q_group + part0) * p.out_stride + t;
-#pragma unroll 4
-            for (int g = 0; g < heads; ++g) {
-              const int r = hh * q_part + g;
-              const unsigned d = chunk_distance<METRIC>(k0, planes[2 * r]) + chunk_distance<METRIC>(k1, planes[2 * r + 1]);
-              if (t < n) emit(r, o, d);
-              o += p.out_stride;
+            // (four distances, then their stores and counts: the counts keep the compiler from moving reads of shared memory across them)
+            for (int g = 0; g < heads; g += 4) {
+              const QPlanes* qp = planes + 2 * (hh * q_part + g);
+              unsigned d[4] = {0, 0, 0, 0};
+#pragma unroll
+              for (int u = 0; u < 4; ++u)
+                if (g + u < heads) d[u] = chunk_distance<METRIC>(k0, qp[2 * u]) + chunk_distance<METRIC>(k1, qp[2 * u + 1]);
+              emit(hh * q_part + g, (head0 + hh) * q_group + part0 + g, d, min(4, heads - g));
             }
           }
         }
