@@ -317,11 +317,11 @@ int adamas_hadamard_transform(const void* x, void* y, int64_t rows, int head_dim
   ADAMAS_REQUIRE(rows < (int64_t(1) << 31) * 16, "too many rows");
   const unsigned blocks = rows_to_blocks(rows);
   if (dtype == ADAMAS_F16)
-    hadamard_kernel<__half><<<blocks, 256, 0, to_stream(stream)>>>(
-        static_cast<const __half*>(x), static_cast<__half*>(y), rows, scale);
+    ADAMAS_LAUNCH("hadamard_kernel", hadamard_kernel<__half>, dim3(blocks), dim3(256), 0, to_stream(stream), 1,
+                  static_cast<const __half*>(x), static_cast<__half*>(y), rows, scale);
   else
-    hadamard_kernel<__nv_bfloat16><<<blocks, 256, 0, to_stream(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), rows, scale);
+    ADAMAS_LAUNCH("hadamard_kernel", hadamard_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, to_stream(stream), 1,
+                  static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), rows, scale);
   return check_launch("hadamard_kernel");
 }
 
@@ -473,11 +473,11 @@ static int rope_impl(void* q, void* k, int64_t seq_len, int num_q_heads, int num
   const unsigned blocks = static_cast<unsigned>((seq_len + tpb - 1) / tpb);
   const int seq = static_cast<int>(seq_len), past = static_cast<int>(past_kv_len);
   if (dtype == ADAMAS_F16)
-    rope_kernel<__half><<<blocks, kRopeThreads, 0, to_stream(stream)>>>(
-        static_cast<__half*>(q), static_cast<__half*>(k), seq, num_q_heads, num_kv_heads, past, tpb, rp);
+    ADAMAS_LAUNCH("rope_kernel", rope_kernel<__half>, dim3(blocks), dim3(kRopeThreads), 0, to_stream(stream), 1,
+                  static_cast<__half*>(q), static_cast<__half*>(k), seq, num_q_heads, num_kv_heads, past, tpb, rp);
   else
-    rope_kernel<__nv_bfloat16><<<blocks, kRopeThreads, 0, to_stream(stream)>>>(
-        static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), seq, num_q_heads, num_kv_heads, past, tpb, rp);
+    ADAMAS_LAUNCH("rope_kernel", rope_kernel<__nv_bfloat16>, dim3(blocks), dim3(kRopeThreads), 0, to_stream(stream), 1,
+                  static_cast<__nv_bfloat16*>(q), static_cast<__nv_bfloat16*>(k), seq, num_q_heads, num_kv_heads, past, tpb, rp);
   return check_launch("rope_kernel");
 }
 
@@ -524,11 +524,9 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
   const unsigned blocks = rows_to_blocks(rows);
   const int64_t start = seq_len - n_tokens;
   cudaStream_t st = to_stream(stream);
-#define LAUNCH_AP(T, F)                                                                            \
-  append_prefill_kernel<T, F><<<blocks, 256, 0, st>>>(static_cast<const T*>(k),                    \
-                                                      static_cast<const T*>(v),                    \
-                                                      static_cast<const T*>(h), rows, start, tgt,  \
-                                                      scale, th)
+#define LAUNCH_AP(T, F)                                                                                                  \
+  ADAMAS_LAUNCH("append_prefill_kernel", (append_prefill_kernel<T, F>), dim3(blocks), dim3(256), 0, st, 1,               \
+                static_cast<const T*>(k), static_cast<const T*>(v), static_cast<const T*>(h), rows, start, tgt, scale, th)
   if (dtype == ADAMAS_F16) {
     if (h) LAUNCH_AP(__half, false); else LAUNCH_AP(__half, true);
   } else {

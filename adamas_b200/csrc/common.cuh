@@ -23,12 +23,14 @@ constexpr int kHeadDim = 128;           // the only head dimension the path supp
 constexpr int kCodeWords = kHeadDim / 8;  // 16-bit words per (token, head) code = 32 bytes
 
 // ---- 16-byte global loads / stores ---------------------------------------------------------
-// Streaming read of data that is read once (code cache): bypass L1 allocation.
+// Streaming read of data that is read once: bypass L1 allocation.  (Not through the non-coherent path: the kernel in front may
+// still be writing when a dependent launch starts.)
 __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
+               : "l"(p)
+               : "memory");
   return v;
 }
 __device__ __forceinline__ uint4 ld_16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
