@@ -444,14 +444,17 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
           for (int hh = 0; hh < HP; ++hh) {
             const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
             // (four distances, then their stores and counts: the counts keep the compiler from moving reads of shared memory across them)
-            for (int g = 0; g < heads; g += 4) {
+            auto four = [&](int g, int many) {
               const QPlanes* qp = planes + 2 * (hh * q_part + g);
               unsigned d[4] = {0, 0, 0, 0};
 #pragma unroll
               for (int u = 0; u < 4; ++u)
-                if (g + u < heads) d[u] = chunk_distance<METRIC>(k0, qp[2 * u]) + chunk_distance<METRIC>(k1, qp[2 * u + 1]);
-              emit(hh * q_part + g, (head0 + hh) * q_group + part0 + g, d, min(4, heads - g));
-            }
+                if (u < many) d[u] = chunk_distance<METRIC>(k0, qp[2 * u]) + chunk_distance<METRIC>(k1, qp[2 * u + 1]);
+              emit(hh * q_part + g, (head0 + hh) * q_group + part0 + g, d, many);
+            };
+            int g = 0;
+            for (; g + 4 <= heads; g += 4) four(g, 4);
+            if (g < heads) four(g, heads - g);
           }
         }
       }
