@@ -538,15 +538,23 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 
 // ---------------------------------------------------------------------------------------------
 // Launches of 3 M distances and more (a 128K context of 32 heads, three 32K sequences): there one L2 atomic per distance from
-// inside the estimate bounds it (the estimate of one 128K sequence: 31.7 us with the counts, 23.7 without).
+// inside the tile pipeline bounds it (the estimate of one 128K sequence: 31.7 us with the counts, 23.7 without).
 static bool many_distances(int q_heads, int batch, int n) {
   return static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20);
 }
 // Which estimate kernel.  The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of
-// its heads in registers; the item kernel takes the rest, and long single sequences, where it counts in shared memory.  Whole step,
-// us a layer, tiles / items: 32 heads 4K 12.0 / 13.1, 32K 20.5 / 21.0, 128K 48.9 / 45.7; 8 x 32K 79.7 / 81.3; 32 x 4-8K 75.0 / 72.7.
+// its heads in registers, as long as its L2 atomics, one per distance, do not bound it; the item kernel, which counts in shared
+// memory, takes the rest.  Whole step, us a layer, tiles / items.  One sequence, 32 heads: 4K 12.0 / 13.1, 32K 20.5 / 21.0, 64K 27.4 / 26.0, 88K
+// 34.9 / 30.9, 128K 48.9 / 45.7; 64 heads, 32K 28.9 / 27.1; 16 heads, 64K 23.5 / 20.1.  Batches of 32 heads: 2 x 8K 16.9 / 17.4,
+// 8 x 4K 25.8 / 27.8, 16 x 2-4K 33.7 / 35.5, 4 x 16K 29.8 / 30.1, 32 x 3K 61.8 / 58.9, 12 x 8K 43.5 / 41.6, 8 x 8-16K 41.8 / 40.1, 24 x 3-6K
+// 61.5 / 59.3, 32 x 4-8K 75.0 / 72.5, 16 x 16K 81.2 / 80.0, but 8 x 32K 79.7 / 81.3 (both at the rate of HBM); of 16 heads: 8 x 8K
+// 26.8 / 22.5, 32 x 8K 68.7 / 50.3, 4 x 64K 59.4 / 41.4.
 static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n) {
-  return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64) && (batch > 1 || !many_distances(q_heads, 1, n));
+  if (q_heads != num_heads) return false;
+  const int64_t distances = static_cast<int64_t>(q_heads) * batch * n;
+  if (num_heads == 16) return distances < (int64_t(1) << 20);
+  if (num_heads != 32 && num_heads != 64) return false;
+  return batch == 1 ? distances < (int64_t(3) << 19) : !many_distances(q_heads, batch, n) || n > 24576;
 }
 
 // Launches the estimate.  n: distances per row, or their upper bound when seq_len_dev gives the length on the device

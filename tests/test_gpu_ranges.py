@@ -115,6 +115,12 @@ def test_estimate_items_shapes(H, Hq, L, ps):
             assert torch.equal(counts[r, sl].to(torch.int64), torch.bincount(want[r, sl * per:(sl + 1) * per], minlength=512))
 
 
+@pytest.mark.parametrize("H,L", [(16, 65536), (16, 65537), (32, 49152), (32, 49153), (64, 24576), (64, 24577)])
+def test_estimate_on_both_sides_of_the_kernels_line(H, L):
+    """16, 32 and 64 heads: the last length of the tile pipeline and the first one of the item kernel; exact."""
+    test_estimate_items_shapes(H, H, L, 16)
+
+
 @pytest.mark.parametrize("H,Hq", [(40, 40), (8, 64), (4, 4), (1000, 1000)])   # (1000: too many query planes for half an SM's memory)
 def test_estimate_leaves_half_of_every_sm(H, Hq):
     """One estimate block per SM as the setting: the same distances and counts, from half of the SM's registers and shared
