@@ -33,6 +33,12 @@ __device__ __forceinline__ uint4 ld_stream_16(const void* p) {
                : "memory");
   return v;
 }
+// Read of a value that another kernel may have written shortly before: through L2, in program order.
+__device__ __forceinline__ float ld_coherent(const float* p) {
+  float v;
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint4 ld_16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st_16(void* p, uint4 v) { *reinterpret_cast<uint4*>(p) = v; }
 

@@ -72,9 +72,10 @@ struct RopeParams {
 
 // (cos, sin) of dimension pair j at position pos: the one expression every kernel that rotates a decode
 // token uses, so that all of them produce the same bits.
-// (In two parts: the frequency does not depend on the position, which may still be on its way from memory.)
+// (In two parts: the frequency does not depend on the position, which may still be on its way from memory.  A table is read where
+// the call stands: its maker may be the kernel in front.)
 __device__ __forceinline__ float rope_inv_freq(int j, const RopeParams& rp) {
-  return rp.inv_freq ? __ldg(rp.inv_freq + j) : rp.rcp_scale / powf(rp.theta, static_cast<float>(2 * j) * (1.0f / kHeadDim));
+  return rp.inv_freq ? ld_coherent(rp.inv_freq + j) : rp.rcp_scale / powf(rp.theta, static_cast<float>(2 * j) * (1.0f / kHeadDim));
 }
 __device__ __forceinline__ float2 rope_cos_sin_at(float inv_freq, float pos) {
   float sn, cs;
@@ -154,13 +155,15 @@ __global__ void __launch_bounds__(kRopeThreads) rope_kernel(T* __restrict__ q, T
     for (int i = tid; i < nt * (kHeadDim / 2); i += kRopeThreads)
       s_cs[i >> 6][i & 7][(i & 63) >> 3] = rope_cos_sin(i & 63, static_cast<float>(past_len + tok0 + (i >> 6)), rp);
   };
-  // (a short call forms the table while the kernel in front ends, a long one while its first rows are on their way)
-  if (tokens_per_block == 1) form_table();
+  // (a short call forms the table while the kernel in front ends, a long one while its first rows are on their way; a caller's
+  // frequencies may be what the kernel in front writes)
+  const bool early = tokens_per_block == 1 && !scaled;
+  if (early) form_table();
   grid_dependency_wait();
   grid_launch_dependents();
   int r0 = tid >> 3;
   load(r0);
-  if (tokens_per_block > 1) form_table();
+  if (!early) form_table();
   __syncthreads();
   while (true) {
 #pragma unroll

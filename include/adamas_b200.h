@@ -389,7 +389,9 @@ int adamas_decode_step(void* q, void* k, const void* v, void* o, float* lse, voi
  * Rules: *seq_len_dev <= max_seq_len; the page tables hold an entry for every page of the current
  * length before the step runs; the value must not be written by the kernel that directly precedes
  * a step in the stream (parts of a step start early and read it before that kernel has finished):
- * advance it at the END of a token's work, not in front of the next step. */
+ * advance it at the END of a token's work, not in front of the next step.  The same holds for the page tables and
+ * rope_inv_freq of a decode step; adamas_append_decode_rope_fused and adamas_apply_rope_table_in_place read their frequencies in
+ * stream order. */
 
 /* adamas_decode_step with the length on the device.  Needs *seq_len_dev > budget.
  * rope_inv_freq (optional, device, 64 floats): per-pair rotation frequencies with any position
@@ -461,7 +463,8 @@ int adamas_dense_step_batch_dev(adamas_decode_handler_t* handler, void* q, void*
                                 adamas_stream_t stream);
 
 /* adamas_apply_rope_in_place with a table of rotation frequencies (device, 64 floats) and a factor on
- * the rotated values instead of (rope_scale, rope_theta): the prefill side of YaRN-scaled models.  The
+ * the rotated values instead of (rope_scale, rope_theta): the prefill side of YaRN-scaled models.  The table may come from the
+ * call in front.  The
  * reference's kernel knows linear scaling only (kernels/include/decode/decode_page.cuh:650-659). */
 int adamas_apply_rope_table_in_place(void* q, void* k, int64_t seq_len, int num_q_heads, int num_kv_heads,
                                      int head_dim, int64_t past_kv_len, const float* inv_freq_dev, float mscale,

@@ -207,6 +207,27 @@ def test_rope_table_in_place_yarn(dtype, past_kv_len, seq_len):
     torch.testing.assert_close(kd.cpu().float(), ref.rope_table(k, past_kv_len, want_inv, want_scale).float(), rtol=tol, atol=tol)
 
 
+@pytest.mark.parametrize("tokens", [1, 300, 6000])     # (6000: several tokens per block)
+def test_rope_table_from_the_kernel_in_front(tokens):
+    """The rotation launch may start while the one in front runs; it must not read a frequency table that this one still writes.
+    Here the transform of many rows leaves the table in the last one: bf16 (0, c) pairs, 64 floats of value c."""
+    _, K, U = _mods()
+    rows = 1 << 18
+    x = torch.randn(rows, 128, device=DEV).to(torch.bfloat16)
+    q = _randn((tokens, 4, 128), 1, torch.float16).to(DEV)
+    k = _randn((tokens, 2, 128), 2, torch.float16).to(DEV)
+    want_q, want_k = q.clone(), k.clone()
+    K.apply_rope_table_in_place(want_q, want_k, 100, torch.full((64,), 2.0 ** -7, device=DEV), 1.5)
+    for _ in range(10):
+        got_q, got_k = q.clone(), k.clone()
+        x[-1] = 0
+        x[-1, 0], x[-1, 1] = 2.0 ** -8, -2.0 ** -8        # transformed: 0 at even, 2^-7 at odd dimensions
+        torch.cuda.synchronize()
+        K.hadamard_transform(x, inplace=True, scale=1.0)
+        K.apply_rope_table_in_place(got_q, got_k, 100, x[-1].view(torch.float32), 1.5)
+        assert torch.equal(got_q, want_q) and torch.equal(got_k, want_k)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_yarn_fused_append_equals_separate_launches(dtype):
     """The append launch with the frequency table rotates exactly as the stand-alone table operator."""
