@@ -402,8 +402,9 @@ static int append_decode_impl(const void* k, const void* v, const void* qh, cons
   const RopeParams rp{rope.scale > 0.f ? 1.0f / rope.scale : 1.f, rope.theta, rope.inv_freq, rope.mscale};
 #define LAUNCH_AD(T, F, R)                                                                            \
   ADAMAS_LAUNCH("append_decode_kernel", (append_decode_kernel<T, F, R>), dim3(blocks, seqs ? batch : 1), dim3(256), 0,  \
-                st, 1, static_cast<const T*>(k), static_cast<const T*>(v), static_cast<const T*>(qh), \
-                static_cast<const T*>(kh), static_cast<uint16_t*>(q_code_out), tgt, kv_num_pages - 1, \
+                st, 1, static_cast<T*>(const_cast<void*>(k)), static_cast<const T*>(v),               \
+                static_cast<T*>(const_cast<void*>(qh)), static_cast<const T*>(kh),                    \
+                static_cast<uint16_t*>(q_code_out), tgt, kv_num_pages - 1, \
                 kv_last_page_len - 1, code_num_pages - 1, code_last_page_len - 1, scale, th, pos, rp, \
                 seq_len_dev, q_heads, seqs)
   if (dtype == ADAMAS_F16) {

@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(kEstThreads) estimate_kernel(const EstimatePar
   QPlanes qp[HPW][2];
 #pragma unroll
   for (int hh = 0; hh < HPW; ++hh) {
-    qp[hh][0] = make_qplanes(__ldg(q_code + 2 * (warp * HPW + hh)));
-    qp[hh][1] = make_qplanes(__ldg(q_code + 2 * (warp * HPW + hh) + 1));
+    qp[hh][0] = make_qplanes(ld_16(q_code + 2 * (warp * HPW + hh)));
+    qp[hh][1] = make_qplanes(ld_16(q_code + 2 * (warp * HPW + hh) + 1));
   }
   est_consume<METRIC, OutT, HPW>(p, geom, ring, my_tiles, lane, warp, qp);
 }

@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     } else {
       for (int c = lane; c < 2 * my_rows; c += 32) {
         const int r = c >> 1;
-        if (!GROUPED || r % q_part < heads) planes[c] = make_qplanes(__ldg(p.q_code + (seq_row + query_row(r)) * 2 + (c & 1)));
+        if (!GROUPED || r % q_part < heads) planes[c] = make_qplanes(ld_16(p.q_code + (seq_row + query_row(r)) * 2 + (c & 1)));
       }
     }
     __syncthreads();   // planes and zeroed counts are visible

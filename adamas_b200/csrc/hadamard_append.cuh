@@ -124,7 +124,7 @@ __device__ __forceinline__ T* rope_row(T* q, T* k, int64_t tok, int r, int hq, i
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRopeThreads) rope_kernel(T* __restrict__ q, T* __restrict__ k, int seq, int hq, int hk,
+__global__ void __launch_bounds__(kRopeThreads) rope_kernel(T* q, T* k, int seq, int hq, int hk,
                                                             int past_len, int tokens_per_block, RopeParams rp) {
   constexpr int kRows = kRopeThreads / 8;   // rows per pass of the block
   __shared__ float2 s_cs[kRopeTokens][8][8];   // [token][i][l8]: the pair of element i of lane l8 (no bank conflicts)
@@ -241,10 +241,11 @@ struct PagedTarget {
 // where it exists.  ROPE (needs FUSED): q and k arrive
 // un-rotated; they are rotated for position `pos`, written back in place (the attention reads the
 // rotated q, the caller's k stays consistent with the cache) and then coded.
+// (The rows may be what a rotation or transform in front is still writing when this launch starts, and k and kh are one buffer
+// in the FUSED form: no restrict qualifiers, which would let their reads move in front of the wait.)
 template <typename T, bool FUSED, bool ROPE = false>
 __global__ void __launch_bounds__(256)
-append_decode_kernel(const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ qh,
-                     const T* __restrict__ kh, uint16_t* __restrict__ q_code_out, PagedTarget tgt,
+append_decode_kernel(T* k, const T* v, T* qh, const T* kh, uint16_t* q_code_out, PagedTarget tgt,
                      int kv_last_page, int kv_entry, int code_last_page, int code_entry, float scale,
                      Thresholds th, float pos, RopeParams rp, const int32_t* seq_len_dev, int q_heads,
                      const SeqDesc* seqs) {
@@ -313,8 +314,8 @@ append_decode_kernel(const T* __restrict__ k, const T* __restrict__ v, const T* 
     rope_halfwarp_cs<T>(a, l16, s_cs, rp.inv_freq != nullptr, rp.mscale);
     rope_halfwarp_cs<T>(b, l16, s_cs, rp.inv_freq != nullptr, rp.mscale);
     kraw = pack8<T>(b);
-    if (valid_q) st_16(const_cast<T*>(qh) + q_off, pack8<T>(a));
-    if (valid) st_16(const_cast<T*>(k) + in_off, kraw);
+    if (valid_q) st_16(qh + q_off, pack8<T>(a));
+    if (valid) st_16(k + in_off, kraw);
   }
   if (valid) {
     st_16(kv + k_off, kraw);

@@ -228,6 +228,43 @@ def test_rope_table_from_the_kernel_in_front(tokens):
         assert torch.equal(got_q, want_q) and torch.equal(got_k, want_k)
 
 
+@pytest.mark.parametrize("fused", [False, True])
+def test_chained_launches_with_and_without_overlap(fused):
+    """Rotation, transform, append and estimate directly behind one another, many tokens without a wait of the host: the caches
+    and distances are the same whether the launches may overlap or not."""
+    _, K, U = _mods()
+    from adamas_b200 import _lib
+    L, H, tokens, ps = 40, 8, 48, 16
+    results = []
+    for overlap in (1, 0):
+        st = State(L, H, ps, torch.float16, seed=9, fused=True, max_seq_len=L + tokens + ps)
+        c = st.c
+        c.end_forward()
+        rows = _randn((tokens, 2, H, 128), 5, torch.float16, 3.0).to(DEV)     # q and k of every token
+        v = _randn((tokens, 1, H, 128), 6, torch.float16).to(DEV)
+        dist = []
+        _lib.lib.adamas_set_pdl(overlap)
+        try:
+            for t in range(tokens):
+                c.prepare_hadamard(1)
+                c.begin_forward(1)
+                q, k = rows[t, :1], rows[t, 1:]
+                U.apply_rope_in_place(q, k, L + t)
+                if fused:
+                    code = U.append_qkv_fused(q, k, v[t], c, 0)
+                else:
+                    code = U.append_kvh(k, v[t], K.hadamard_transform(rows[t]), c, 0)
+                dist.append(U.decode_estimate(code, c, 0).clone())
+                c.end_forward()
+        finally:
+            _lib.lib.adamas_set_pdl(1)
+        t = np.arange(L + tokens)
+        kv_pages, code_pages = np.asarray(c.kv_cache.indicies)[t // ps], np.asarray(c.hadamard_cache.indicies)[t // ps]
+        results.append([rows, c.kv_cache.buf_layer(0)[kv_pages, :, t % ps], c.hadamard_cache.buf_layer(0)[code_pages, 0, t % ps]] + dist)
+    for a, b in zip(*results):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 def test_yarn_fused_append_equals_separate_launches(dtype):
     """The append launch with the frequency table rotates exactly as the stand-alone table operator."""
