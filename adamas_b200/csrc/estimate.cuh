@@ -21,6 +21,7 @@
 #pragma once
 #include "common.cuh"
 #include "hadamard_append.cuh"
+#include "item_split.h"
 #include "select_attend.cuh"
 
 namespace adamas {
@@ -138,9 +139,6 @@ struct EstimateParams {
   const SeqDesc* seqs;
   StepAppend ap;
 };
-
-// Tiles of n tokens.  A sequence whose first token is being appended (n = 0) has an empty one: somebody has to append.
-__device__ __forceinline__ int est_tiles(int n, int tile_tokens) { return n == 0 ? 1 : (n + tile_tokens - 1) / tile_tokens; }
 
 // Tiles of `tile_tokens` tokens of the batch's sequences in front of each one -> cum[0 .. batch]; one warp.
 __device__ __forceinline__ void est_line(const EstimateParams& p, int tile_tokens, int lane, int* cum) {

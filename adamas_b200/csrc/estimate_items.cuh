@@ -34,30 +34,11 @@
 
 namespace adamas {
 
-constexpr int kItemWarps = 7;            // that scan
 constexpr int kItemThreads = kItemWarps * 32 + 32;   // (one more warp: the query and the append)
-constexpr int kItemBlocksPerSm = 2;
 constexpr int kItemMaxSlots = 3;         // ring slots per warp at most
 constexpr int kItemBytes = 4096;
-constexpr int kItemApart = 4;            // items per block that keeping to one segment may cost
 constexpr int kItemCountWords = 388;     // counts per query row and table (a distance is at most 384)
 
-// Cache heads of an item, and the query heads of a cache head that a warp takes at a time.  An item has as long a run of a
-// token's codes as divides the cache heads, but not more than kItemRows query rows (every row has count tables in every block
-// that works on it).  The group of a cache head is halved as long as every part still
-// finds a warp of its own (`warps` on the chip; `items` are those of undivided groups): a second round costs more than it saves.
-constexpr int kItemRows = 8;
-inline int item_cache_heads(int kv_heads, int q_group) {
-  int hp = 4;
-  while (hp > 1 && (kv_heads % hp != 0 || (q_group > 1 && hp * q_group > kItemRows))) hp /= 2;
-  return hp;
-}
-inline int item_query_heads(int items, int q_group, int warps) {
-  int heads = q_group;
-  for (; heads > 2 * kItemRows; items *= 2) heads = (heads + 1) / 2;
-  for (; heads > 1 && items <= warps / 2; items *= 2) heads = (heads + 1) / 2;
-  return heads;
-}
 // Count tables of a block: the slices that its tokens may fall into.
 __host__ __device__ __forceinline__ constexpr int item_tables(int hp, bool grouped) { return hp == 1 && !grouped ? 4 : 2; }
 
@@ -169,33 +150,11 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     __syncthreads();
     tiles_all = cum[p.batch];
     const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
-    const int b = blockIdx.x, segments = p.batch * pieces;
-    auto seg_start = [&](int g) {   // where segment g (a piece of a sequence) starts on the line
-      const int s = g / pieces;
-      return s == p.batch ? total : cum[s] * pieces + (g - s * pieces) * (cum[s + 1] - cum[s]);
-    };
-    // With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the
-    // uneven shares is less than a second segment costs (queries to load and code behind a barrier, counts to add up).
-    if (segments <= static_cast<int>(gridDim.x) && static_cast<int64_t>(total) * segments <= static_cast<int64_t>(kItemApart) * gridDim.x * gridDim.x) {
-      // (the rule keeps every product below 2^31)
-      const int spare = gridDim.x - segments;
-      auto first_block = [&](int g) { return g + seg_start(g) * spare / total; };
-      int lo = 0, hi = segments - 1;
-      while (lo < hi) {   // the last segment that starts at or before this block
-        const int mid = (lo + hi + 1) >> 1;
-        if (first_block(mid) <= b) lo = mid; else hi = mid - 1;
-      }
-      const int start = seg_start(lo), n_items = seg_start(lo + 1) - start, f = first_block(lo), nblk = min(first_block(lo + 1) - f, n_items);
-      if (b - f >= nblk) return;
-      pos = start + n_items * (b - f) / nblk;
-      line_end = start + n_items * (b - f + 1) / nblk;
-    } else {
-      const int B = min(static_cast<int>(gridDim.x), total);   // (every block that takes part has some)
-      if (b >= B) return;
-      const int q = total / B, r = total - q * B;
-      pos = b * q + b * r / B;   // b * total / B
-      line_end = (b + 1) * q + (b + 1) * r / B;
-    }
+    const ItemShare work = item_apart(total, p.batch * pieces, gridDim.x) ? item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x)
+                                                                          : item_share_even(total, gridDim.x, blockIdx.x);
+    pos = work.pos;
+    line_end = work.end;
+    if (total == 0) grid_dependency_wait();   // (lengths that are all zero: the kernel behind must not overtake the one in front)
   } else {
     tiles_all = est_tiles(len0, TT);
   }
@@ -227,7 +186,10 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       first = blockIdx.x * share;
       end = min(tiles_all, first + share);
       pos = line_end;
-      if (first >= end) return;
+      if (first >= end) {
+        if (tiles_all == 0) grid_dependency_wait();
+        return;
+      }
     }
     const int head0 = (GROUPED ? piece / q_split : piece) * HP;                   // first cache head
     const int part0 = GROUPED ? (piece - head0 / HP * q_split) * q_part : 0;       // first query head of each of them

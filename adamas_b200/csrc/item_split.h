@@ -1,0 +1,78 @@
+// How the work of the item estimate (estimate_items.cuh) is cut: what an item is, which of them a block takes.  Plain C++ but for
+// the qualifiers, so that the cuts can be checked without a GPU.
+//
+// An item is 128 / HP tokens (a tile) x HP cache heads; a piece is HP cache heads with a part of their query heads.  The items of
+// a launch form a line: sequence after sequence, in it piece after piece, in it tile after tile.  A segment is a piece of a sequence.
+#pragma once
+
+#ifdef __CUDACC__
+#define ADAMAS_HD __host__ __device__ __forceinline__
+#else
+#define ADAMAS_HD inline
+#endif
+
+namespace adamas {
+
+constexpr int kItemWarps = 7;            // of a block, that scan
+constexpr int kItemBlocksPerSm = 2;
+constexpr int kItemApart = 4;            // items per block that keeping to one segment may cost
+
+// Cache heads of an item, and the query heads of a cache head that a warp takes at a time.  An item has as long a run of a
+// token's codes as divides the cache heads, but not more than kItemRows query rows (every row has count tables in every block
+// that works on it).  The group of a cache head is halved as long as every part still
+// finds a warp of its own (`warps` on the chip; `items` are those of undivided groups): a second round costs more than it saves.
+constexpr int kItemRows = 8;
+ADAMAS_HD int item_cache_heads(int kv_heads, int q_group) {
+  int hp = 4;
+  while (hp > 1 && (kv_heads % hp != 0 || (q_group > 1 && hp * q_group > kItemRows))) hp /= 2;
+  return hp;
+}
+ADAMAS_HD int item_query_heads(int items, int q_group, int warps) {
+  int heads = q_group;
+  for (; heads > 2 * kItemRows; items *= 2) heads = (heads + 1) / 2;
+  for (; heads > 1 && items <= warps / 2; items *= 2) heads = (heads + 1) / 2;
+  return heads;
+}
+
+// Tiles of n tokens.  A sequence whose first token is being appended (n = 0) has an empty one: somebody has to append.
+ADAMAS_HD int est_tiles(int n, int tile_tokens) { return n == 0 ? 1 : (n + tile_tokens - 1) / tile_tokens; }
+
+struct ItemShare {
+  int pos, end;   // items of the line; none where pos == end
+};
+
+// An even cut of the line: block b of `blocks`.
+ADAMAS_HD ItemShare item_share_even(int total, int blocks, int b) {
+  const int B = blocks < total ? blocks : total;   // (every block that takes part has some)
+  if (b >= B) return {0, 0};
+  const int q = total / B, r = total - q * B;
+  return {b * q + b * r / B, (b + 1) * q + (b + 1) * r / B};   // b * total / B
+}
+
+// A batch: cum[s] tiles lie in front of sequence s.
+//
+// With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the
+// uneven shares is less than a second segment costs (queries to load and code behind a barrier, counts to add up).
+// (The rule keeps every product of the cut below 2^31.  Lengths that are all zero leave nothing to deal out.)
+ADAMAS_HD bool item_apart(int total, int segments, int blocks) {
+  return total > 0 && segments <= blocks && static_cast<long long>(total) * segments <= static_cast<long long>(kItemApart) * blocks * blocks;
+}
+ADAMAS_HD ItemShare item_share_apart(const int* cum, int batch, int pieces, int blocks, int b) {
+  const int segments = batch * pieces, total = cum[batch] * pieces, spare = blocks - segments;
+  auto seg_start = [&](int g) {   // where segment g starts on the line
+    const int s = g / pieces;
+    return s == batch ? total : cum[s] * pieces + (g - s * pieces) * (cum[s + 1] - cum[s]);
+  };
+  auto first_block = [&](int g) { return g + seg_start(g) * spare / total; };
+  int lo = 0, hi = segments - 1;
+  while (lo < hi) {   // the last segment that starts at or before this block
+    const int mid = (lo + hi + 1) >> 1;
+    if (first_block(mid) <= b) lo = mid; else hi = mid - 1;
+  }
+  const int start = seg_start(lo), n_items = seg_start(lo + 1) - start, f = first_block(lo), all = first_block(lo + 1) - f;
+  const int nblk = all < n_items ? all : n_items;
+  if (b - f >= nblk) return {0, 0};
+  return {start + n_items * (b - f) / nblk, start + n_items * (b - f + 1) / nblk};
+}
+
+}  // namespace adamas

@@ -1,0 +1,91 @@
+"""How the item estimate cuts its work (csrc/item_split.h): compiled for the host, every item of a launch must belong to exactly
+one block, whatever the lengths, heads and blocks."""
+import ctypes
+import os
+import random
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+WARPS, BLOCKS = 7, 296      # scanning warps of a block; blocks of a launch on 148 SMs
+
+SHIM = """
+#include <algorithm>
+#include "item_split.h"
+using namespace adamas;
+extern "C" {
+int cache_heads(int h, int group) { return item_cache_heads(h, group); }
+int query_heads(int items, int group, int warps) { return item_query_heads(items, group, warps); }
+int tiles_of(int n, int t) { return est_tiles(n, t); }
+int share_batch(const int* cum, int batch, int pieces, int q_part, int blocks, int* out) {
+  const int total = cum[batch] * pieces;
+  const bool apart = item_apart(total, batch * pieces, blocks);
+  for (int b = 0; b < blocks; ++b) {
+    const ItemShare w = apart ? item_share_apart(cum, batch, pieces, blocks, b) : item_share_even(total, blocks, b);
+    out[2 * b] = w.pos; out[2 * b + 1] = w.end;
+  }
+  return apart;
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def split(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no host compiler")
+    d = tmp_path_factory.mktemp("split")
+    (d / "shim.cpp").write_text(SHIM)
+    # (-ftrapv: a product beyond 31 bits ends the test)
+    subprocess.run([gxx, "-O1", "-std=c++17", "-fPIC", "-shared", "-ftrapv", "-I", os.path.join(ROOT, "adamas_b200", "csrc"),
+                    "-o", str(d / "shim.so"), str(d / "shim.cpp")], check=True)
+    return ctypes.CDLL(str(d / "shim.so"))
+
+
+def _batch(split, tiles, pieces, q_part, blocks=BLOCKS):
+    cum = np.concatenate([[0], np.cumsum(tiles)]).astype(np.int32)
+    out = np.full((blocks, 2), -1, dtype=np.int32)
+    apart = split.share_batch(cum.ctypes.data_as(ctypes.c_void_p), len(tiles), pieces, q_part, blocks,
+                              out.ctypes.data_as(ctypes.c_void_p))
+    return out, bool(apart)
+
+
+def _covers(shares, total):
+    busy = sorted((int(a), int(b)) for a, b in shares if a != b)
+    assert all(a < b for a, b in busy)
+    assert busy[0][0] == 0 and busy[-1][1] == total
+    assert all(x[1] == y[0] for x, y in zip(busy, busy[1:]))
+
+
+@pytest.mark.parametrize("batch,pieces", [(1, 1), (3, 10), (32, 8), (40, 8), (1024, 1)])
+def test_batch_without_tokens(split, batch, pieces):
+    """Lengths that are all zero (a batch before its lengths are set): no block has anything, and nothing is divided by the total."""
+    shares, apart = _batch(split, [0] * batch, pieces, 1)
+    assert not apart and (shares[:, 0] == shares[:, 1]).all()
+
+
+@pytest.mark.parametrize("heads,group", [(4, 1), (40, 1), (32, 1), (7, 1), (8, 4), (4, 7), (8, 8), (1, 16)])
+def test_batches_every_item_once(split, heads, group):
+    rng = random.Random(heads * 100 + group)
+    for case in range(60):
+        batch = rng.choice([1, 2, 3, 8, 31, 32, 33, 100, 256, 1024])
+        top = rng.choice([1, 40, 700, 5000, 60000])
+        lengths = [rng.randrange(0, top + 1) for _ in range(batch)]
+        hp = split.cache_heads(heads, group)
+        # (a length of 0 tokens besides the newest still has its append; an absent sequence has nothing)
+        tiles = [0 if rng.random() < 0.1 else split.tiles_of(n, 128 // hp) for n in lengths]
+        if sum(tiles) == 0:
+            tiles[-1] = 1
+        q_part = split.query_heads(sum(tiles) * (heads // hp), group, WARPS * BLOCKS)
+        pieces = heads // hp * -(-group // q_part)
+        shares, apart = _batch(split, tiles, pieces, q_part)
+        _covers(shares, sum(tiles) * pieces)
+        if apart:    # nobody has more than one segment
+            ends = np.cumsum(np.repeat(tiles, pieces))
+            for a, b in shares:
+                if a != b:
+                    assert np.searchsorted(ends, a, "right") == np.searchsorted(ends, b - 1, "right")
