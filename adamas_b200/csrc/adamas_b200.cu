@@ -588,7 +588,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   prm.n_tokens = n;
   prm.H = num_heads;
   prm.q_group = q_heads / num_heads;
-  prm.q_part = 1;
+  prm.chip_warps = 0;
   prm.page_size = page_size;
   prm.ps_shift = log2_exact(page_size);
   prm.batch = batch;
@@ -637,17 +637,18 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   int64_t items = tiles * (num_heads / hp) * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
   const int slots_all = est_blocks_per_sm() * di->num_sms;   // resident blocks
-  prm.q_part = item_query_heads(static_cast<int>(items), prm.q_group, kItemWarps * kItemBlocksPerSm * di->num_sms);
-  const int pieces = num_heads / hp * ((prm.q_group + prm.q_part - 1) / prm.q_part);
+  prm.chip_warps = kItemWarps * slots_all;
+  const int q_part = item_query_heads(static_cast<int>(items), prm.q_group, prm.chip_warps);   // (at most; fewer for a shorter length)
+  const int pieces = num_heads / hp * ((prm.q_group + q_part - 1) / q_part);
   items = tiles * pieces * batch;
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
   dim3 grid(static_cast<unsigned>(std::min<int64_t>(slots_all, items)));
   int64_t per_block = (items + grid.x - 1) / grid.x;
-  if (!seqs) {   // an equal number of blocks for every piece (a remainder of the chip's stays idle: at most 3 % for up to 64 heads)
+  if (!seqs && prm.q_group == 1) {   // an equal number of blocks for every piece
     grid = dim3(static_cast<unsigned>(std::min<int64_t>(std::max(1, slots_all / pieces), tiles)), static_cast<unsigned>(pieces));
     per_block = (tiles + grid.x - 1) / grid.x;
   }
-  const int seg_rows = hp * prm.q_part;
+  const int seg_rows = hp * q_part;
   const size_t room = static_cast<size_t>(di->smem_per_sm / kItemBlocksPerSm - 1024 - kItemStatic);
   size_t smem = static_cast<size_t>(seg_rows) * 2 * sizeof(QPlanes);
   if (hist) smem += static_cast<size_t>(item_tables(hp, prm.q_group > 1)) * seg_rows * kItemCountWords * sizeof(uint32_t);

@@ -121,7 +121,7 @@ struct EstimateParams {
   int out_half;
   int n_tokens;     // distances per row (host lengths)
   int H;            // heads of the code cache
-  int q_part;       // estimate_items_kernel: query heads of a cache head in a piece
+  int chip_warps;   // estimate_items_kernel: scanning warps that are resident at once on the device
   int q_group;      // query heads per cache head: out, hist, q and q_code have H * q_group rows per sequence
   int page_size;
   int ps_shift;     // log2(page_size) or -1

@@ -137,26 +137,36 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   const int cs_pair = tid - (kItemWarps - 2) * 32;
   const bool cs_here = APPEND && p.ap.rope_on && scanning && cs_pair >= 0;
   const float cs_freq = cs_here ? rope_inv_freq(cs_pair, p.ap.rp) : 0.f;
-  const int q_part = GROUPED ? p.q_part : 1;
-  const int q_split = GROUPED ? (q_group + q_part - 1) / q_part : 1;
 
   // ---- this block's part of the work ------------------------------------------------------------------------------------
-  // One sequence: blockIdx.y is the piece (HP cache heads with a part of their query heads), blockIdx.x an equal part of its tiles.
-  // A batch: all items form a line, sequence after sequence, in it piece after piece, in it token tile after token tile.
-  int pieces = gridDim.y, tiles_all, pos = 0, line_end = 1;
+  int tiles_all;
   if (p.seqs) {
-    pieces = p.H / HP * q_split;
     if (warp == 0) est_line(p, TT, lane, cum);
     __syncthreads();
     tiles_all = cum[p.batch];
-    const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
-    const ItemShare work = item_apart(total, p.batch * pieces, gridDim.x) ? item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x)
-                                                                          : item_share_even(total, gridDim.x, blockIdx.x);
-    pos = work.pos;
-    line_end = work.end;
-    if (total == 0) grid_dependency_wait();   // (lengths that are all zero: the kernel behind must not overtake the one in front)
   } else {
     tiles_all = est_tiles(len0, TT);
+  }
+  // The group is divided by the length, not by its upper bound: a short sequence in a large cache like one in a small cache (28
+  // query heads over 4, 3K tokens in a cache of 128K: 15.8 us a layer, 20.0 with the division for 128K).
+  const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
+  const int q_split = GROUPED ? (q_group + q_part - 1) / q_part : 1;
+  const int pieces = p.H / HP * q_split;
+  // One sequence, no grouped queries: blockIdx.y is the piece, blockIdx.x an equal part of its tiles.
+  const bool grid_of_pieces = !GROUPED && !p.seqs;
+  int pos = 0, line_end = 1;
+  if (!grid_of_pieces) {
+    const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
+    if (total == 0) {   // (lengths that are all zero: the kernel behind must not overtake the one in front)
+      grid_dependency_wait();
+      return;
+    }
+    ItemShare work;
+    if (!p.seqs) work = item_share_one(tiles_all, pieces, q_part, gridDim.x, blockIdx.x);
+    else if (item_apart(total, p.batch * pieces, gridDim.x)) work = item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x);
+    else work = item_share_even(total, gridDim.x, blockIdx.x);
+    pos = work.pos;
+    line_end = work.end;
   }
   bool waited = false;
 
@@ -165,22 +175,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     int s = 0, n = len0, piece, first, end;
     const uint4* codes = p.codes;
     const int32_t* table = p.page_table;
-    if (p.seqs) {
-      int lo = 0, hi = p.batch - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (cum[mid] * pieces <= pos) lo = mid; else hi = mid - 1;
-      }
-      s = lo;
-      const int tiles = cum[s + 1] - cum[s], at = pos - cum[s] * pieces;
-      piece = at / tiles;
-      first = at - piece * tiles;
-      end = min(tiles, first + line_end - pos);
-      pos += end - first;
-      n = __ldg(p.seq_len_dev + s) - 1;
-      codes = static_cast<const uint4*>(p.seqs[s].code_data);
-      table = p.seqs[s].code_table;
-    } else {
+    if (grid_of_pieces) {
       const int share = (tiles_all + gridDim.x - 1) / gridDim.x;
       piece = blockIdx.y;
       first = blockIdx.x * share;
@@ -190,6 +185,25 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
         if (tiles_all == 0) grid_dependency_wait();
         return;
       }
+    } else {
+      int tiles = tiles_all, at = pos;
+      if (p.seqs) {
+        int lo = 0, hi = p.batch - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (cum[mid] * pieces <= pos) lo = mid; else hi = mid - 1;
+        }
+        s = lo;
+        tiles = cum[s + 1] - cum[s];
+        at = pos - cum[s] * pieces;
+        n = __ldg(p.seq_len_dev + s) - 1;
+        codes = static_cast<const uint4*>(p.seqs[s].code_data);
+        table = p.seqs[s].code_table;
+      }
+      piece = at / tiles;
+      first = at - piece * tiles;
+      end = min(tiles, first + line_end - pos);
+      pos += end - first;
     }
     const int head0 = (GROUPED ? piece / q_split : piece) * HP;                   // first cache head
     const int part0 = GROUPED ? (piece - head0 / HP * q_split) * q_part : 0;       // first query head of each of them
@@ -254,13 +268,14 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       return GROUPED ? (head0 + r / q_part) * q_group + part0 + r % q_part : head0 + r;
     };
     const int my_rows = HP * q_part;       // (of a short last part each cache head's last ones are absent)
+    const int tab_rows = GROUPED ? my_rows : seg_rows;   // rows of a count table
     const unsigned l8 = lane & 7;
     const bool scaled = p.ap.rp.inv_freq != nullptr;
     const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
     const int slice0 = p.hist ? first * TT / slice_tokens : 0;
     const int used = p.hist ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
     if (scanning) {
-      for (int i = tid; i < used * seg_rows * (kItemCountWords / 4); i += kItemWarps * 32) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
+      for (int i = tid; i < used * tab_rows * (kItemCountWords / 4); i += kItemWarps * 32) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
     } else if (APPEND) {
       // eight lanes per row, four rows at a time, two times four on their way together
       for (int r0 = 0; r0 < my_rows; r0 += 8) {
@@ -357,10 +372,11 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     // the counts in shared memory are those of the first `used` slices that the segment touches; anything behind them is counted
     // in global memory one by one
     uint32_t* hist = p.hist ? p.hist + seq_row * kSaScratchWordsPerHead : nullptr;
-    uint16_t* out = static_cast<uint16_t*>(p.out) + seq_row * p.out_stride;
+    uint16_t* out = static_cast<uint16_t*>(p.out) + (seq_row + (GROUPED ? 0 : head0)) * p.out_stride;
     auto to_out = [&](unsigned d) { return !APPEND && p.out_half ? __half_as_ushort(__uint2half_rn(d)) : static_cast<uint16_t>(d); };   // (exact: d <= 384)
     const int f = HP == 4 ? (lane & 7) : HP == 2 ? ((lane >> 1) & 3) : ((lane >> 2) & 1);
-    int use = 0;
+    uint32_t* tab = counts;   // the table of the present tokens, the token behind its slice, the tables that are left
+    int use = 0, left = p.hist ? kTables : 0, tab_end = (slice0 + 1) * slice_tokens;
     for (int tile = scanning ? first + warp : end; tile < end; tile += kItemWarps) {
       if (slots == 3) cp_async_wait<2>(); else if (slots == 2) cp_async_wait<1>(); else cp_async_wait<0>();
       __syncwarp();
@@ -368,18 +384,15 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
 #pragma unroll (GROUPED ? 1 : kGroups)
       for (int k = 0; k < kGroups; ++k) {
         const int t0 = tile * TT + k * 32, t = t0 + lane;
-        uint32_t* tab = counts;   // (a group never straddles two slices)
-        bool here = p.hist != nullptr;
-        if (here) {
-#pragma unroll
-          for (int u = 1; u < kTables; ++u)
-            if (t0 >= (slice0 + u) * slice_tokens) tab += seg_rows * kItemCountWords;
-          here = t0 < (slice0 + kTables) * slice_tokens;
+        for (; left > 0 && t0 >= tab_end; --left) {   // (a group never straddles two slices)
+          tab += tab_rows * kItemCountWords;
+          tab_end += slice_tokens;
         }
+        const bool here = left > 0;
         // up to four rows' distances: segment rows r .., output rows `row` ..
         auto emit = [&](int r, int row, const unsigned* d, int many) {
           if (t >= n) return;
-          uint16_t* o = out + row * p.out_stride + t;
+          uint16_t* o = (GROUPED ? out + row * p.out_stride : out) + t;
 #pragma unroll
           for (int u = 0; u < 4; ++u)
             if (u < many) o[u * p.out_stride] = to_out(d[u]);
@@ -435,10 +448,10 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     cp_async_wait<0>();
     if (p.hist || pos < line_end) __syncthreads();
     if (p.hist) {
-      for (int i = tid; i < used * seg_rows * (kItemCountWords / 4); i += kItemThreads) {
+      for (int i = tid; i < used * tab_rows * (kItemCountWords / 4); i += kItemThreads) {
         const uint4 c4 = reinterpret_cast<const uint4*>(counts)[i];
         if (c4.x | c4.y | c4.z | c4.w) {
-          const int tr = i / (kItemCountWords / 4), u = tr / seg_rows, r = tr - u * seg_rows;
+          const int tr = i / (kItemCountWords / 4), u = tr / tab_rows, r = tr - u * tab_rows;
           uint32_t* dst = hist + static_cast<size_t>(query_row(r)) * kSaScratchWordsPerHead + (slice0 + u) * kSaBins + (i - tr * (kItemCountWords / 4)) * 4;
           if (c4.x) atomicAdd(dst, c4.x);
           if (c4.y) atomicAdd(dst + 1, c4.y);

@@ -49,6 +49,22 @@ ADAMAS_HD ItemShare item_share_even(int total, int blocks, int b) {
   return {b * q + b * r / B, (b + 1) * q + (b + 1) * r / B};   // b * total / B
 }
 
+// What keeping to one segment may cost a block of one sequence: this many items (times the query heads of a cache head in them)
+// more than an even cut would give it.
+constexpr int kItemMore = 16;
+
+// One sequence.  Every piece has the same number of blocks, which share its tiles evenly; a remainder of the blocks stays idle.  An
+// even cut of the line instead with more pieces than blocks, or where more than a quarter of the blocks would stay idle and
+// that costs more than a second segment does.
+ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks, int b) {
+  const int per = blocks / pieces, idle = blocks - per * pieces;
+  if (per == 0 || (idle > blocks / 4 && static_cast<long long>(tiles) * idle * q_part > static_cast<long long>(kItemMore) * per * blocks))
+    return item_share_even(tiles * pieces, blocks, b);
+  const int share = (tiles + per - 1) / per, piece = b / per, first = (b - piece * per) * share;
+  if (piece >= pieces || first >= tiles) return {0, 0};
+  return {piece * tiles + first, piece * tiles + (share < tiles - first ? first + share : tiles)};
+}
+
 // A batch: cum[s] tiles lie in front of sequence s.
 //
 // With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the

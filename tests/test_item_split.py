@@ -20,6 +20,12 @@ extern "C" {
 int cache_heads(int h, int group) { return item_cache_heads(h, group); }
 int query_heads(int items, int group, int warps) { return item_query_heads(items, group, warps); }
 int tiles_of(int n, int t) { return est_tiles(n, t); }
+void share_one(int tiles, int pieces, int q_part, int blocks, int* out) {
+  for (int b = 0; b < blocks; ++b) {
+    const ItemShare w = item_share_one(tiles, pieces, q_part, blocks, b);
+    out[2 * b] = w.pos; out[2 * b + 1] = w.end;
+  }
+}
 int share_batch(const int* cum, int batch, int pieces, int q_part, int blocks, int* out) {
   const int total = cum[batch] * pieces;
   const bool apart = item_apart(total, batch * pieces, blocks);
@@ -46,6 +52,12 @@ def split(tmp_path_factory):
     return ctypes.CDLL(str(d / "shim.so"))
 
 
+def _one(split, tiles, pieces, q_part, blocks=BLOCKS):
+    out = np.full((blocks, 2), -1, dtype=np.int32)
+    split.share_one(tiles, pieces, q_part, blocks, out.ctypes.data_as(ctypes.c_void_p))
+    return out
+
+
 def _batch(split, tiles, pieces, q_part, blocks=BLOCKS):
     cum = np.concatenate([[0], np.cumsum(tiles)]).astype(np.int32)
     out = np.full((blocks, 2), -1, dtype=np.int32)
@@ -59,6 +71,37 @@ def _covers(shares, total):
     assert all(a < b for a, b in busy)
     assert busy[0][0] == 0 and busy[-1][1] == total
     assert all(x[1] == y[0] for x, y in zip(busy, busy[1:]))
+
+
+GROUPED = [(1, 16), (1, 128), (1, 1024), (2, 32), (4, 7), (8, 4), (8, 8), (8, 12), (5, 3), (128, 8), (301, 3)]
+
+
+@pytest.mark.parametrize("blocks", [BLOCKS, BLOCKS // 2])
+@pytest.mark.parametrize("heads,group", GROUPED)
+def test_one_grouped_sequence_every_item_once(split, heads, group, blocks):
+    rng = random.Random(heads * group)
+    hp = split.cache_heads(heads, group)
+    most = 0
+    for n in sorted([0, 1, 31, 32, 33, 127, 128, 129, 4095] + [int(2 ** rng.uniform(5, 20)) for _ in range(12)]):
+        tiles = split.tiles_of(n, 128 // hp)
+        q_part = split.query_heads(tiles * (heads // hp), group, WARPS * blocks)
+        pieces = heads // hp * -(-group // q_part)
+        _covers(_one(split, tiles, pieces, q_part, blocks), tiles * pieces)
+        # a launch has shared memory for the rows of its longest sequence: a shorter one must not need more
+        assert q_part >= most
+        most = q_part
+
+
+@pytest.mark.parametrize("heads,group", [(4, 7), (8, 4), (8, 8), (1, 16), (4, 8)])
+def test_short_sequence_in_a_large_cache(split, heads, group):
+    """What a block gets follows from the length alone: 3000 tokens keep at least as many warps busy as in a cache of their size."""
+    src = open(os.path.join(ROOT, "adamas_b200", "csrc", "estimate_items.cuh")).read()
+    assert "item_query_heads(tiles_all * (p.H / HP), q_group" in src    # (the kernel divides by its own tiles)
+    hp = split.cache_heads(heads, group)
+    tiles = split.tiles_of(2999, 128 // hp)
+    q_part = split.query_heads(tiles * (heads // hp), group, WARPS * BLOCKS)
+    shares = _one(split, tiles, heads // hp * -(-group // q_part), q_part)
+    assert (shares[:, 1] > shares[:, 0]).sum() >= min(BLOCKS // 2, tiles * heads // hp * group)
 
 
 @pytest.mark.parametrize("batch,pieces", [(1, 1), (3, 10), (32, 8), (40, 8), (1024, 1)])
