@@ -644,9 +644,12 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   ADAMAS_REQUIRE(items < (int64_t(1) << 31), "too many tokens for one estimate launch");
   dim3 grid(static_cast<unsigned>(std::min<int64_t>(slots_all, items)));
   int64_t per_block = (items + grid.x - 1) / grid.x;
-  if (!seqs && prm.q_group == 1) {   // an equal number of blocks for every piece
-    grid = dim3(static_cast<unsigned>(std::min<int64_t>(std::max(1, slots_all / pieces), tiles)), static_cast<unsigned>(pieces));
-    per_block = (tiles + grid.x - 1) / grid.x;
+  if (!seqs && prm.q_group == 1) {
+    const int per = item_blocks_per_piece(static_cast<int>(tiles), pieces, 1, static_cast<int>(grid.x));
+    if (per > 0) {
+      grid = dim3(static_cast<unsigned>(per), static_cast<unsigned>(pieces));
+      per_block = (tiles + per - 1) / per;
+    }
   }
   const int seg_rows = hp * q_part;
   const size_t room = static_cast<size_t>(di->smem_per_sm / kItemBlocksPerSm - 1024 - kItemStatic);

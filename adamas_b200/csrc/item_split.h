@@ -53,13 +53,17 @@ ADAMAS_HD ItemShare item_share_even(int total, int blocks, int b) {
 // more than an even cut would give it.
 constexpr int kItemMore = 16;
 
-// One sequence.  Every piece has the same number of blocks, which share its tiles evenly; a remainder of the blocks stays idle.  An
-// even cut of the line instead with more pieces than blocks, or where more than a quarter of the blocks would stay idle and
-// that costs more than a second segment does.
-ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks, int b) {
+// One sequence.  Every piece has the same number of blocks, which share its tiles evenly; a remainder of the blocks stays idle
+// (of 296: 11 % with 33 pieces, 18 % with 61, at most a quarter).  0, an even cut of the line instead, with more pieces than blocks, or where more
+// than a quarter would stay idle and that costs more than a second segment does (151 heads: 48K tokens 112 us a layer with a block
+// per piece, 82 cut evenly, 12K 41 / 35; 61 heads, 48K: 41 with a remainder of 18 %, 49 cut evenly).
+ADAMAS_HD int item_blocks_per_piece(int tiles, int pieces, int q_part, int blocks) {
   const int per = blocks / pieces, idle = blocks - per * pieces;
-  if (per == 0 || (idle > blocks / 4 && static_cast<long long>(tiles) * idle * q_part > static_cast<long long>(kItemMore) * per * blocks))
-    return item_share_even(tiles * pieces, blocks, b);
+  return idle > blocks / 4 && static_cast<long long>(tiles) * idle * q_part > static_cast<long long>(kItemMore) * per * blocks ? 0 : per;
+}
+ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks, int b) {
+  const int per = item_blocks_per_piece(tiles, pieces, q_part, blocks);
+  if (per == 0) return item_share_even(tiles * pieces, blocks, b);
   const int share = (tiles + per - 1) / per, piece = b / per, first = (b - piece * per) * share;
   if (piece >= pieces || first >= tiles) return {0, 0};
   return {piece * tiles + first, piece * tiles + (share < tiles - first ? first + share : tiles)};

@@ -20,6 +20,7 @@ extern "C" {
 int cache_heads(int h, int group) { return item_cache_heads(h, group); }
 int query_heads(int items, int group, int warps) { return item_query_heads(items, group, warps); }
 int tiles_of(int n, int t) { return est_tiles(n, t); }
+int per_piece(int tiles, int pieces, int blocks) { return item_blocks_per_piece(tiles, pieces, 1, blocks); }
 void share_one(int tiles, int pieces, int q_part, int blocks, int* out) {
   for (int b = 0; b < blocks; ++b) {
     const ItemShare w = item_share_one(tiles, pieces, q_part, blocks, b);
@@ -90,6 +91,23 @@ def test_one_grouped_sequence_every_item_once(split, heads, group, blocks):
         # a launch has shared memory for the rows of its longest sequence: a shorter one must not need more
         assert q_part >= most
         most = q_part
+
+
+@pytest.mark.parametrize("blocks", [BLOCKS, BLOCKS // 2])
+@pytest.mark.parametrize("heads", [1, 2, 3, 7, 28, 33, 40, 61, 96, 101, 147, 148, 149, 151, 295, 297, 600, 1000, 1024])
+def test_one_sequence_every_item_once(split, heads, blocks):
+    """No grouped queries: a grid of pieces, or the line; never more blocks than may be resident."""
+    rng = random.Random(heads)
+    hp = split.cache_heads(heads, 1)
+    for n in [1, 31, 32, 33, 127, 128, 129, 4095] + [int(2 ** rng.uniform(5, 20)) for _ in range(12)]:
+        tiles, pieces = split.tiles_of(n, 128 // hp), heads // hp
+        grid = min(blocks, tiles * pieces)
+        per = split.per_piece(tiles, pieces, grid)
+        assert per * pieces <= grid and (per > 0 or pieces > grid * 3 // 4 or grid % pieces > grid // 4)
+        if per > 0:
+            # a long row leaves no more than a quarter of the blocks idle
+            assert tiles < 1000 or (grid - per * pieces) * 4 <= grid
+        _covers(_one(split, tiles, pieces, 1, grid), tiles * pieces)
 
 
 @pytest.mark.parametrize("heads,group", [(4, 7), (8, 4), (8, 8), (1, 16), (4, 8)])
