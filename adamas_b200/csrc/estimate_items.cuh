@@ -110,6 +110,15 @@ struct EstShared {
   float2 cs[kHeadDim / 2];
 };
 
+// Whether a batch keeps to one segment a block.  (Out of line: inlined, it cost the launches of one sequence 0.3 us through the
+// registers of what follows.)
+__device__ __noinline__ bool item_batch_apart(const int* cum, int batch, int pieces, int q_part) {
+  const int total = cum[batch] * pieces, blocks = gridDim.x;
+  int most = 0;
+  for (int s = threadIdx.x & 31; s < batch; s += 32) most = max(most, item_apart_most(cum[s + 1] - cum[s], total, blocks - batch * pieces));
+  return item_apart_pays(__reduce_max_sync(0xffffffffu, most), total, q_part, blocks);
+}
+
 // Dynamic shared memory: rings | planes [seg_rows][2] | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
 // sequences before [batch + 1] (seqs).  GROUPED: several query heads per cache head (q_group > 1).
 // MODE 0: with the append inside (u16 distances); 1: the query codes are given; 2: the same with the XOR metric.
@@ -164,7 +173,9 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     }
     ItemShare work;
     if (!p.seqs) work = GROUPED ? item_share_one(tiles_all, pieces, q_part, gridDim.x, blockIdx.x) : item_share_even(total, gridDim.x, blockIdx.x);
-    else if (item_apart(total, p.batch * pieces, gridDim.x)) work = item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x);
+    else if (item_apart_possible(total, p.batch * pieces, gridDim.x) &&
+             (item_apart_small(total, p.batch * pieces, gridDim.x) || item_batch_apart(cum, p.batch, pieces, q_part)))
+      work = item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x);
     else work = item_share_even(total, gridDim.x, blockIdx.x);
     pos = work.pos;
     line_end = work.end;

@@ -15,7 +15,6 @@ namespace adamas {
 
 constexpr int kItemWarps = 7;            // of a block, that scan
 constexpr int kItemBlocksPerSm = 2;
-constexpr int kItemApart = 4;            // items per block that keeping to one segment may cost
 
 // Cache heads of an item, and the query heads of a cache head that a warp takes at a time.  An item has as long a run of a
 // token's codes as divides the cache heads, but not more than kItemRows query rows (every row has count tables in every block
@@ -71,12 +70,21 @@ ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks
 
 // A batch: cum[s] tiles lie in front of sequence s.
 //
-// With few segments every block takes a part of ONE, the blocks dealt out in proportion to the items: what is lost to the
-// uneven shares is less than a second segment costs (queries to load and code behind a barrier, counts to add up).
-// (The rule keeps every product of the cut below 2^31.  Lengths that are all zero leave nothing to deal out.)
-ADAMAS_HD bool item_apart(int total, int segments, int blocks) {
-  return total > 0 && segments <= blocks && static_cast<long long>(total) * segments <= static_cast<long long>(kItemApart) * blocks * blocks;
+// Where the segments are no more than the blocks, every block may take a part of ONE, the blocks dealt out in proportion to the
+// items.  A second segment costs a block about 4 us (a query to load and code behind a barrier, counts to add up), a larger share its items:
+// up to kItemApart more than an even cut gives, times the query heads of a cache head in them (64 sequences x 2K x 28 over
+// 4: 80.8 us a layer cut evenly, 79.3 apart with 2 items of 7 heads more; 32 x 2K x 32 over 8 52.3 / 49.7; 20 x 3K x 40 heads 50.8 / 53.9 with
+// 31 more).  A launch with little work does not ask what the most is, which takes 0.35 us in front of its first request.
+// (Products stay below 2^31.  Lengths that are all zero leave nothing to deal out.)
+constexpr int kItemApart = 24;
+ADAMAS_HD bool item_apart_possible(int total, int segments, int blocks) { return total > 0 && segments <= blocks && total <= 0x7fffffff / blocks; }
+ADAMAS_HD bool item_apart_small(int total, int segments, int blocks) { return static_cast<long long>(total) * segments <= 4LL * blocks * blocks; }
+// the most that a block gets of the segments of a sequence of `tiles` tiles; spare = blocks - segments
+ADAMAS_HD int item_apart_most(int tiles, int total, int spare) {
+  const int blocks = 1 + tiles * spare / total;   // of each segment, at least
+  return (tiles + blocks - 1) / blocks;
 }
+ADAMAS_HD bool item_apart_pays(int most, int total, int q_part, int blocks) { return (most - total / blocks) * q_part <= kItemApart; }
 ADAMAS_HD ItemShare item_share_apart(const int* cum, int batch, int pieces, int blocks, int b) {
   const int segments = batch * pieces, total = cum[batch] * pieces, spare = blocks - segments;
   auto seg_start = [&](int g) {   // where segment g starts on the line

@@ -29,7 +29,13 @@ void share_one(int tiles, int pieces, int q_part, int blocks, int* out) {
 }
 int share_batch(const int* cum, int batch, int pieces, int q_part, int blocks, int* out) {
   const int total = cum[batch] * pieces;
-  const bool apart = item_apart(total, batch * pieces, blocks);
+  const int segments = batch * pieces;
+  bool apart = item_apart_possible(total, segments, blocks);
+  if (apart && !item_apart_small(total, segments, blocks)) {
+    int most = 0;
+    for (int s = 0; s < batch; ++s) most = std::max(most, item_apart_most(cum[s + 1] - cum[s], total, blocks - segments));
+    apart = item_apart_pays(most, total, q_part, blocks);
+  }
   for (int b = 0; b < blocks; ++b) {
     const ItemShare w = apart ? item_share_apart(cum, batch, pieces, blocks, b) : item_share_even(total, blocks, b);
     out[2 * b] = w.pos; out[2 * b + 1] = w.end;
@@ -145,8 +151,20 @@ def test_batches_every_item_once(split, heads, group):
         pieces = heads // hp * -(-group // q_part)
         shares, apart = _batch(split, tiles, pieces, q_part)
         _covers(shares, sum(tiles) * pieces)
-        if apart:    # nobody has more than one segment
+        if apart:    # nobody has more than one segment, nor much more than an even share
             ends = np.cumsum(np.repeat(tiles, pieces))
             for a, b in shares:
                 if a != b:
                     assert np.searchsorted(ends, a, "right") == np.searchsorted(ends, b - 1, "right")
+            total, blocks = sum(tiles) * pieces, BLOCKS
+            if total * batch * pieces > 4 * blocks * blocks:
+                assert ((shares[:, 1] - shares[:, 0]).max() - total // blocks) * q_part <= 24 + q_part
+
+
+@pytest.mark.parametrize("batch,n,heads,group,want", [(64, 2000, 4, 7, True), (32, 4000, 4, 7, True), (32, 2000, 8, 8, True),
+                                                      (24, 1500, 40, 1, True), (20, 3000, 40, 1, False), (20, 16000, 40, 1, False)])
+def test_batches_that_keep_to_one_segment(split, batch, n, heads, group, want):
+    hp = split.cache_heads(heads, group)
+    tiles = [split.tiles_of(n - 1, 128 // hp)] * batch
+    q_part = split.query_heads(sum(tiles) * (heads // hp), group, WARPS * BLOCKS)
+    assert _batch(split, tiles, heads // hp * -(-group // q_part), q_part)[1] is want
