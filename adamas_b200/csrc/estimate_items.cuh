@@ -38,6 +38,11 @@ constexpr int kItemThreads = kItemWarps * 32 + 32;   // (one more warp: the quer
 constexpr int kItemMaxSlots = 3;         // ring slots per warp at most
 constexpr int kItemBytes = 4096;
 constexpr int kItemCountWords = 388;     // counts per query row and table (a distance is at most 384)
+// A block with up to so many tokens in all counts them in global memory one by one: clearing and adding up tables costs more (16
+// heads, 2K tokens in a cache of 64K: 13.8 us a layer with tables, 13.6 without; 32 sequences x 600 x 4 heads 14.6 / 14.3).  Not with
+// grouped queries, where a piece has more rows (64 sequences x 2K x 28 over 4: 81.0 / 81.9), nor between a block's other segments (256 x 400
+// x 40 heads: 237.4 / 239.2).
+constexpr int kItemDirect = 256;
 
 // Count tables of a block: the slices that its tokens may fall into.
 __host__ __device__ __forceinline__ constexpr int item_tables(int hp, bool grouped) { return hp == 1 && !grouped ? 4 : 2; }
@@ -184,7 +189,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
 
   while (pos < line_end) {
     // ---- this block's next segment: tiles [first, end) of a piece of a sequence ----------------------------------------
-    int s = 0, n = len0, piece, first, end;
+    int s = 0, n = len0, piece, first, end, rest;   // (rest: tiles of the block from here on)
     const uint4* codes = p.codes;
     const int32_t* table = p.page_table;
     if (grid_of_pieces) {
@@ -192,6 +197,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       piece = blockIdx.y;
       first = blockIdx.x * share;
       end = min(tiles_all, first + share);
+      rest = end - first;
       pos = line_end;
       if (first >= end) {
         if (tiles_all == 0) grid_dependency_wait();
@@ -214,7 +220,8 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       }
       piece = at / tiles;
       first = at - piece * tiles;
-      end = min(tiles, first + line_end - pos);
+      rest = line_end - pos;
+      end = min(tiles, first + rest);
       pos += end - first;
     }
     const int head0 = (GROUPED ? piece / q_split : piece) * HP;                   // first cache head
@@ -285,7 +292,8 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     const bool scaled = p.ap.rp.inv_freq != nullptr;
     const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
     const int slice0 = p.hist ? first * TT / slice_tokens : 0;
-    const int used = p.hist ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
+    const bool tables = p.hist && (GROUPED || rest * TT > kItemDirect);
+    const int used = tables ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
     if (scanning) {
       for (int i = tid; i < used * tab_rows * (kItemCountWords / 4); i += kItemWarps * 32) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
     } else if (APPEND) {
@@ -388,7 +396,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     auto to_out = [&](unsigned d) { return !APPEND && p.out_half ? __half_as_ushort(__uint2half_rn(d)) : static_cast<uint16_t>(d); };   // (exact: d <= 384)
     const int f = HP == 4 ? (lane & 7) : HP == 2 ? ((lane >> 1) & 3) : ((lane >> 2) & 1);
     uint32_t* tab = counts;   // the table of the present tokens, the token behind its slice, the tables that are left
-    int use = 0, left = p.hist ? kTables : 0, tab_end = (slice0 + 1) * slice_tokens;
+    int use = 0, left = tables ? kTables : 0, tab_end = (slice0 + 1) * slice_tokens;
     for (int tile = scanning ? first + warp : end; tile < end; tile += kItemWarps) {
       if (slots == 3) cp_async_wait<2>(); else if (slots == 2) cp_async_wait<1>(); else cp_async_wait<0>();
       __syncwarp();
@@ -458,8 +466,8 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       if (++use == slots) use = 0;
     }
     cp_async_wait<0>();
-    if (p.hist || pos < line_end) __syncthreads();
-    if (p.hist) {
+    if (tables || pos < line_end) __syncthreads();
+    if (tables) {
       for (int i = tid; i < used * tab_rows * (kItemCountWords / 4); i += kItemThreads) {
         const uint4 c4 = reinterpret_cast<const uint4*>(counts)[i];
         if (c4.x | c4.y | c4.z | c4.w) {
