@@ -326,8 +326,8 @@ int adamas_select_attend_slices(int n, int k, int num_heads, int* slices);
  * an adamas_estimate call has filled: the shard's 512-bin histogram per head, ready to be exchanged. */
 /* Counts rows of integer distances (ADAMAS_VAL_U16, as adamas_estimate writes them) into the histogram
  * scratch, `slices` per-slice histograms per row, the layout adamas_select_attend(..., hist_ready = 1)
- * reads: what adamas_estimate does on the side when it is given `hist`, as a launch of its own that counts
- * in shared memory.  Cheaper than counting inside the estimate from about 3 M distances per call. */
+ * reads: what adamas_estimate does on the side, and for less, when it is given `hist`, as a launch of its own for distances that exist
+ * already. */
 int adamas_dist_histograms(const void* dist, int64_t dist_stride, int n, int num_heads, int slices,
                            uint32_t* hist, adamas_stream_t stream);
 

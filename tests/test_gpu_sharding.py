@@ -51,6 +51,28 @@ def _make_shard(dev, q, k, v, t0, t1, L, ps, dtype):
     return sharding.CudaOps(c, 0, q_code, owns_tail), qd
 
 
+@pytest.mark.parametrize("H,n", [(32, 100001), (16, 200000), (8, 30000)])
+def test_shard_counts_inside_its_estimate(H, n, monkeypatch):
+    """A shard's histograms come from its one estimate launch at every length (beyond 3 M distances too): right counts, no
+    second pass over the distances."""
+    import adamas_b200.utils as U
+    from adamas_b200 import _kernels as K, sharding
+    dev = "cuda:0"
+    monkeypatch.setattr(K, "dist_histograms", lambda *a: pytest.fail("a counting launch of its own"))
+    gen = torch.Generator(device=dev).manual_seed(n)
+    c = U.InferenceController(1, H, 128, 16, 1 << 20, n + 16, torch.float16, dev)
+    k = torch.randn(n, H, 128, device=dev, dtype=torch.float16, generator=gen)
+    c.prepare_hadamard(n)
+    c.begin_forward(n)
+    U.append_kvh(k, k, None, c, 0)
+    c.end_forward()
+    q_code = torch.empty(1, H, 16, dtype=torch.float16, device=dev)
+    K.bucketize_pack(K.hadamard_transform(torch.randn(1, H, 128, device=dev, dtype=torch.float16, generator=gen)), q_code)
+    got = sharding.CudaOps(c, 0, q_code, False).local_histograms(1024)
+    dist = c.distance_scratch(n).long()
+    assert torch.equal(got.long(), torch.stack([torch.bincount(d, minlength=512) for d in dist]))
+
+
 @pytest.mark.parametrize("world", [1, 2, 4, 8])
 @pytest.mark.parametrize("L,budget,ps,dtype", [(3000, 257, 16, torch.float16), (1200, 1024, 16, torch.bfloat16),
                                                 (500, 64, 1, torch.float16)])
