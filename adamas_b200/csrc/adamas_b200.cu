@@ -636,7 +636,9 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
 #undef LAUNCH_EST
     return check_launch("estimate_kernel");
   }
-  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0, "q_code must be 16-byte aligned");
+  // (for the head counts that the tile pipeline takes at other lengths, the query codes may start on any 16-bit word as there)
+  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0 || (q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64)),
+                 "q_code must be 16-byte aligned");
   const int hp = item_cache_heads(num_heads, prm.q_group);
   const int64_t tiles = n / (128 / hp) + 1;   // of a sequence
   int64_t items = tiles * (num_heads / hp) * batch;

@@ -218,3 +218,30 @@ def test_append_estimate_tiles(H, L):
         results.append([t.cpu() for t in (kv_cache, code_cache, q_code, dist)])
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,L", [(16, 70001), (32, 50001), (64, 26001), (32, 20001)])
+def test_query_codes_on_any_16_bit_word(H, L):
+    """Estimate with the append inside for 16, 32 and 64 heads, by the item kernel and (the last one) by the tiles: the query
+    codes may start on any 16-bit word."""
+    _, K, _ = _mods()
+    ps, n = 16, L - 1
+    pages = (L + ps - 1) // ps
+    gen = torch.Generator(device=DEV).manual_seed(L)
+    table = torch.randperm(pages, device=DEV, generator=gen).to(torch.int32)
+    codes = torch.randint(-32768, 32768, (pages, 1, ps, H, 16), device=DEV, generator=gen).to(torch.int16)
+    q, k, v = (torch.randn(1, H, 128, device=DEV, generator=gen).to(torch.float16) for _ in range(3))
+    results = []
+    for off in (0, 1, 2):
+        code_cache, kv_cache = codes.clone(), torch.zeros(pages, 2, ps, H, 128, dtype=torch.float16, device=DEV)
+        store = torch.zeros(H * 16 + 8, dtype=torch.int16, device=DEV)
+        q_code = store[off:off + H * 16].view(1, H, 16)
+        dist = torch.zeros(H, (n + 7) // 8 * 8, dtype=torch.int16, device=DEV)
+        hist = K.histogram_scratch(H, DEV)
+        last = L - (pages - 1) * ps
+        K.append_estimate(q, k, v, q_code, kv_cache, table, last, code_cache, table, last, dist[:, :n], scale=1.0, hist=hist, hist_slices=8)
+        assert int(store[:off].abs().sum()) == 0 and int(store[off + H * 16:].abs().sum()) == 0
+        results.append([q_code.clone(), dist, code_cache, kv_cache, hist])
+    for other in results[1:]:
+        for a, b in zip(results[0], other):
+            assert torch.equal(a, b)
