@@ -115,7 +115,7 @@ struct EstShared {
   float2 cs[kHeadDim / 2];
 };
 
-// Whether a batch keeps to one segment a block.  (Out of line: inlined, it cost the launches of one sequence 0.3 us through the
+// Whether a batch with grouped queries keeps to one segment a block.  (Out of line: inlined, it cost the launches of one sequence 0.3 us through the
 // registers of what follows.)
 __device__ __noinline__ bool item_batch_apart(const int* cum, int batch, int pieces, int q_part) {
   const int total = cum[batch] * pieces, blocks = gridDim.x;
@@ -179,7 +179,8 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     ItemShare work;
     if (!p.seqs) work = GROUPED ? item_share_one(tiles_all, pieces, q_part, gridDim.x, blockIdx.x) : item_share_even(total, gridDim.x, blockIdx.x);
     else if (item_apart_possible(total, p.batch * pieces, gridDim.x) &&
-             (item_apart_small(total, p.batch * pieces, gridDim.x) || item_batch_apart(cum, p.batch, pieces, q_part)))
+             (item_apart_simple(total, p.batch * pieces, gridDim.x) ||
+              (GROUPED && !item_apart_hopeless(total, p.batch * pieces, q_part, gridDim.x) && item_batch_apart(cum, p.batch, pieces, q_part))))
       work = item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x);
     else work = item_share_even(total, gridDim.x, blockIdx.x);
     pos = work.pos;

@@ -71,14 +71,25 @@ ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks
 // A batch: cum[s] tiles lie in front of sequence s.
 //
 // Where the segments are no more than the blocks, every block may take a part of ONE, the blocks dealt out in proportion to the
-// items.  A second segment costs a block about 4 us (a query to load and code behind a barrier, counts to add up), a larger share its items:
-// up to kItemApart more than an even cut gives, times the query heads of a cache head in them (64 sequences x 2K x 28 over
-// 4: 80.8 us a layer cut evenly, 79.3 apart with 2 items of 7 heads more; 32 x 2K x 32 over 8 52.3 / 49.7; 20 x 3K x 40 heads 50.8 / 53.9 with
-// 31 more).  A launch with little work does not ask what the most is, which takes 0.35 us in front of its first request.
+// items.  A second segment costs a block about 4 us (a query to load and code behind a barrier, counts to add up), a larger share its
+// items.  They are kept apart
+//  * where there is little work, or an eighth as many segments as blocks: shares differ by an eighth at most (4 sequences x 64K x 32
+//    heads 71.3 us a layer cut evenly, 67.7 apart);
+//  * with grouped queries, where the largest share is up to kItemApart items more than an even one, times the query heads of a
+//    cache head in them (64 x 2K x 28 over 4: 80.8 cut evenly, 79.3 apart with 2 items of 7 heads more; 32 x 2K x 32 over 8 52.3 / 49.7).
+//    What the largest share is costs about 2 us to find, once per launch.  Without grouped queries that is
+//    more than it gains (40 heads, 12 x 8K 46.1 / 48.4).
 // (Products stay below 2^31.  Lengths that are all zero leave nothing to deal out.)
 constexpr int kItemApart = 24;
 ADAMAS_HD bool item_apart_possible(int total, int segments, int blocks) { return total > 0 && segments <= blocks && total <= 0x7fffffff / blocks; }
-ADAMAS_HD bool item_apart_small(int total, int segments, int blocks) { return static_cast<long long>(total) * segments <= 4LL * blocks * blocks; }
+ADAMAS_HD bool item_apart_few(int segments, int blocks) { return segments * 8 <= blocks; }
+ADAMAS_HD bool item_apart_simple(int total, int segments, int blocks) {
+  return static_cast<long long>(total) * segments <= 4LL * blocks * blocks || item_apart_few(segments, blocks);
+}
+// (with about one block per segment, and an average one too much for it, there is nothing to ask)
+ADAMAS_HD bool item_apart_hopeless(int total, int segments, int q_part, int blocks) {
+  return 2 * segments > blocks && static_cast<long long>(total) * (blocks - segments) * q_part > static_cast<long long>(kItemApart) * segments * blocks;
+}
 // the most that a block gets of the segments of a sequence of `tiles` tiles; spare = blocks - segments
 ADAMAS_HD int item_apart_most(int tiles, int total, int spare) {
   const int blocks = 1 + tiles * spare / total;   // of each segment, at least

@@ -31,10 +31,10 @@ int share_batch(const int* cum, int batch, int pieces, int q_part, int blocks, i
   const int total = cum[batch] * pieces;
   const int segments = batch * pieces;
   bool apart = item_apart_possible(total, segments, blocks);
-  if (apart && !item_apart_small(total, segments, blocks)) {
+  if (apart && !item_apart_simple(total, segments, blocks)) {
     int most = 0;
     for (int s = 0; s < batch; ++s) most = std::max(most, item_apart_most(cum[s + 1] - cum[s], total, blocks - segments));
-    apart = item_apart_pays(most, total, q_part, blocks);
+    apart = q_part > 1 && !item_apart_hopeless(total, segments, q_part, blocks) && item_apart_pays(most, total, q_part, blocks);
   }
   for (int b = 0; b < blocks; ++b) {
     const ItemShare w = apart ? item_share_apart(cum, batch, pieces, blocks, b) : item_share_even(total, blocks, b);
@@ -157,12 +157,15 @@ def test_batches_every_item_once(split, heads, group):
                 if a != b:
                     assert np.searchsorted(ends, a, "right") == np.searchsorted(ends, b - 1, "right")
             total, blocks = sum(tiles) * pieces, BLOCKS
-            if total * batch * pieces > 4 * blocks * blocks:
+            if batch * pieces * 8 <= blocks:
+                assert (shares[:, 1] - shares[:, 0]).max() <= -(-total // blocks) * 1.15 + 1
+            elif total * batch * pieces > 4 * blocks * blocks:
                 assert ((shares[:, 1] - shares[:, 0]).max() - total // blocks) * q_part <= 24 + q_part
 
 
 @pytest.mark.parametrize("batch,n,heads,group,want", [(64, 2000, 4, 7, True), (32, 4000, 4, 7, True), (32, 2000, 8, 8, True),
-                                                      (24, 1500, 40, 1, True), (20, 3000, 40, 1, False), (20, 16000, 40, 1, False)])
+                                                      (24, 1500, 40, 1, False), (20, 16000, 40, 1, False), (12, 8000, 40, 1, False),
+                                                      (32, 6000, 32, 1, False), (8, 32768, 32, 1, False), (4, 64000, 32, 1, True)])
 def test_batches_that_keep_to_one_segment(split, batch, n, heads, group, want):
     hp = split.cache_heads(heads, group)
     tiles = [split.tiles_of(n - 1, 128 // hp)] * batch
