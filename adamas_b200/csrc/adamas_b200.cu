@@ -554,11 +554,11 @@ static bool many_distances(int q_heads, int batch, int n) {
 // 26.8 / 22.5, 32 x 8K 68.7 / 50.3, 4 x 64K 59.4 / 41.4.
 // Without counts (counts false) there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
 // 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
+static bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
 static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts) {
-  if (q_heads != num_heads) return false;
+  if (!tile_heads(num_heads, q_heads)) return false;
   const int64_t distances = static_cast<int64_t>(q_heads) * batch * n;
   if (num_heads == 16) return distances < (int64_t(1) << 20);
-  if (num_heads != 32 && num_heads != 64) return false;
   if (!counts) return true;
   return batch == 1 ? distances < (int64_t(3) << 19) : !many_distances(q_heads, batch, n) || n > 24576;
 }
@@ -603,7 +603,9 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   prm.seqs = seqs;
   prm.ap = ap;
   cudaStream_t st = to_stream(stream);
-  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr)) {
+  // (the tiles store query codes on any 16-bit word, at every length)
+  const bool codes_aligned = (reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0;
+  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr) || (!codes_aligned && tile_heads(num_heads, q_heads))) {
     const int num_tiles = (n + kEstTile - 1) / kEstTile;
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
@@ -636,9 +638,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
 #undef LAUNCH_EST
     return check_launch("estimate_kernel");
   }
-  // (for the head counts that the tile pipeline takes at other lengths, the query codes may start on any 16-bit word as there)
-  ADAMAS_REQUIRE((reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0 || (q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64)),
-                 "q_code must be 16-byte aligned");
+  ADAMAS_REQUIRE(codes_aligned, "q_code must be 16-byte aligned");
   const int hp = item_cache_heads(num_heads, prm.q_group);
   const int64_t tiles = n / (128 / hp) + 1;   // of a sequence
   int64_t items = tiles * (num_heads / hp) * batch;

@@ -326,11 +326,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
               uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * (r0 + 4 * u + (lane >> 3)) + (l8 >> 2)) + (l8 & 3);
               qp[0] = w;
               qp[4] = qplane_d(w);
-              if (first == 0) {   // (on any 16-bit word)
-                uint16_t* dst = p.ap.q_code_out + code_row[u] * kCodeWords + 2 * l8;
-                dst[0] = static_cast<uint16_t>(w);
-                dst[1] = static_cast<uint16_t>(w >> 16);
-              }
+              if (first == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[code_row[u] * (kCodeWords / 2) + l8] = w;
             }
           }
         }

@@ -222,8 +222,8 @@ def test_append_estimate_tiles(H, L):
 
 @pytest.mark.parametrize("H,L", [(16, 70001), (32, 50001), (64, 26001), (32, 20001)])
 def test_query_codes_on_any_16_bit_word(H, L):
-    """Estimate with the append inside for 16, 32 and 64 heads, by the item kernel and (the last one) by the tiles: the query
-    codes may start on any 16-bit word."""
+    """Estimate with the append inside for 16, 32 and 64 heads, at lengths of the item kernel and (the last one) of the tiles: the
+    query codes may start on any 16-bit word."""
     _, K, _ = _mods()
     ps, n = 16, L - 1
     pages = (L + ps - 1) // ps
