@@ -543,24 +543,33 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 static bool many_distances(int q_heads, int batch, int n) {
   return static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20);
 }
-// Which estimate kernel.  n is the length, or the cache's capacity where the length is on the device (a short sequence in a large cache
-// loses nothing by it but 16 heads: 32 heads, 4K tokens in 98K 14.7 tiles / 14.5 items, 16K 16.7 / 16.9; 64 heads, 8K in 66K 18.9 / 16.6; 16 heads, 2K
-// in 66K 13.3 / 13.6, 8K 14.2 / 14.0).  The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of
-// its heads in registers, as long as its L2 atomics, one per distance, do not bound it; the item kernel, which counts in shared
-// memory, takes the rest.  Whole step, us a layer, tiles / items.  One sequence, 32 heads: 4K 12.0 / 13.1, 32K 20.5 / 21.0, 64K 27.4 / 26.0, 88K
-// 34.9 / 30.9, 128K 48.9 / 45.7; 64 heads, 32K 28.9 / 27.1; 16 heads, 64K 23.5 / 20.1.  Batches of 32 heads: 2 x 8K 16.9 / 17.4,
-// 8 x 4K 25.8 / 27.8, 16 x 2-4K 33.7 / 35.5, 4 x 16K 29.8 / 30.1, 32 x 3K 61.8 / 58.9, 12 x 8K 43.5 / 41.6, 8 x 8-16K 41.8 / 40.1, 24 x 3-6K
-// 61.5 / 59.3, 32 x 4-8K 75.0 / 72.5, 16 x 16K 81.2 / 80.0, but 8 x 32K 79.7 / 81.3 (both at the rate of HBM); of 16 heads: 8 x 8K
-// 26.8 / 22.5, 32 x 8K 68.7 / 50.3, 4 x 64K 59.4 / 41.4.
+// Which estimate kernel.  n is the length, or the cache's capacity where the length is on the device.
+//
+// The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of its heads in registers,
+// as long as its L2 atomics, one per distance, do not bound it; the item kernel, which counts in shared memory, takes the rest.
+// Whole step, us a layer, tiles / items.  One sequence, 32 heads: 4K 12.0 / 13.1, 32K 20.5 / 21.0, 64K 27.4 / 26.0, 88K 34.9 /
+// 30.9, 128K 48.9 / 45.7; 64 heads, 32K 28.9 / 27.1; 16 heads, 64K 23.5 / 20.1.  Batches of 32 heads: 2 x 8K 16.9 / 17.4, 8 x
+// 4K 25.8 / 27.8, 16 x 2-4K 33.7 / 35.5, 4 x 16K 29.8 / 30.1, 12 x 8K 43.5 / 41.6, 8 x 8-16K 41.8 / 40.1, 32 x 4-8K 75.0 / 72.5,
+// 16 x 16K 81.2 / 80.0; of 16 heads: 8 x 8K 26.8 / 22.5, 32 x 8K 68.7 / 50.3, 4 x 64K 59.4 / 41.4.
+//
+// Long rows of a batch (beyond 24K) go to the tiles, with the counts in a launch of their own, unless there are so few segments
+// (a piece of 4 heads of a sequence) that the item kernel keeps them apart.  Otherwise a block's two segments of hundreds of tiles read pieces of
+// the same tokens far apart in time: 32 heads, 8 x 32K 79.0 / 81.3.  Where they are few: 2 x 48K 34.7 / 34.6, 3 x 36K 37.5 / 36.6, 2 x 128K 68.1 / 66.6, 4 x
+// 64K 71.5 / 66.8; 64 heads, 2 x 28K 42.4 / 38.0, 2 x 66K 75.0 / 68.9.
+//
+// Short sequences in large caches: 32 heads, 4K in 98K 14.7 / 14.5, 16K 16.7 / 16.9; 64 heads, 8K in 66K 18.9 / 16.6; 16 heads, 2K in 66K 13.3 /
+// 13.5, 8K 14.2 / 14.0; batches of 32 heads, 8 x 4K in 32K 27.4 / 27.1, 4 x 8K in 64K 23.8 / 22.2, 16 x 3K in 32K 35.9 / 36.9.
+//
 // Without counts (counts false) there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
 // 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
 static bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
-static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts) {
+static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, int blocks) {
   if (!tile_heads(num_heads, q_heads)) return false;
   const int64_t distances = static_cast<int64_t>(q_heads) * batch * n;
   if (num_heads == 16) return distances < (int64_t(1) << 20);
   if (!counts) return true;
-  return batch == 1 ? distances < (int64_t(3) << 19) : !many_distances(q_heads, batch, n) || n > 24576;
+  if (batch == 1) return distances < (int64_t(3) << 19);
+  return !many_distances(q_heads, batch, n) || (n > 24576 && !item_apart_few(batch * (num_heads / 4), blocks));
 }
 
 // Launches the estimate.  n: distances per row, or their upper bound when seq_len_dev gives the length on the device
@@ -605,7 +614,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   cudaStream_t st = to_stream(stream);
   // (the tiles store query codes on any 16-bit word, at every length)
   const bool codes_aligned = (reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0;
-  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr) || (!codes_aligned && tile_heads(num_heads, q_heads))) {
+  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, est_blocks_per_sm() * di->num_sms) || (!codes_aligned && tile_heads(num_heads, q_heads))) {
     const int num_tiles = (n + kEstTile - 1) / kEstTile;
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
@@ -1431,7 +1440,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   int rc;
   // The histogram counts.  Item kernel: in shared memory.  Tile pipeline: one L2 atomic per distance from inside the estimate, or,
   // with many distances, a launch of its own that counts in shared memory.
-  const bool count_apart = estimate_by_tiles(num_heads, q_heads, batch, n, true) && many_distances(q_heads, batch, n);
+  const bool count_apart = estimate_by_tiles(num_heads, q_heads, batch, n, true, est_blocks_per_sm() * di->num_sms) && many_distances(q_heads, batch, n);
   uint32_t* est_hist = count_apart ? nullptr : hist;
   const bool two_launches = fused_append_enabled();
   if (two_launches) {
