@@ -160,11 +160,10 @@ def test_batched_graph_replay_over_tokens():
     assert _lib.device_error(clear=False) == 0
 
 
-def test_large_launches_count_their_histograms_in_a_launch_of_their_own():
-    """From 3 M distances per launch the fused step counts the histograms in a separate launch instead of
-    inside the estimate.  Four sequences of 33K tokens x 32 heads cross that line as a batch and stay below
-    it one by one: both forms must select the same slots; one 66K sequence of 64 heads is checked against
-    the oracle."""
+def test_large_launches_count_their_histograms_in_shared_memory():
+    """Launches with many distances count the histograms in shared memory (the item kernel) instead of by one atomic per distance
+    from inside the tile pipeline.  Four sequences of 33K tokens x 32 heads do as a batch and not one by one: both forms must
+    select the same slots; one 66K sequence of 64 heads is checked against the oracle."""
     _, K, U = _mods()
     lengths, Hq, H, ps, budget, dtype = [33100, 32900, 33500, 33001], 32, 32, 16, 1024, torch.float16
     B = len(lengths)
@@ -212,17 +211,25 @@ def test_large_launches_count_their_histograms_in_a_launch_of_their_own():
 
 @pytest.mark.parametrize("fused_append", [True, False])
 @pytest.mark.parametrize("lengths,Hq,H,budget", [
-    ([90000, 70001, 85000, 77777], 4, 4, 2048),         # blocks take pieces of two sequences
+    ([90000, 70001, 85000, 77777], 4, 4, 2048),         # every block a piece of one sequence
     ([40000, 9001, 3000, 35000], 32, 8, 512),           # ... of grouped queries
-    ([20000, 9001, 3000, 15000, 600], 32, 8, 512),      # every block a piece of one sequence
+    ([20000, 9001, 3000, 15000, 600], 32, 8, 512),
     ([21000] + [300] * 40, 40, 40, 256),                # short sequences: several in a block, several slices in a piece
+    ([2000 + 7 * i for i in range(64)], 28, 4, 256),    # as many pieces as a launch has blocks, kept apart
+    ([3000 + 50 * i for i in range(20)], 40, 40, 256),  # ... and cut evenly
+    ([700 + 3 * i for i in range(40)], 7, 7, 128),      # few tokens a block
+    # 16, 32 and 64 heads: batches with many distances leave the tile pipeline
+    ([8000, 4001, 8192, 7777, 6500, 5003, 8100, 4097, 7000, 6001, 8003, 5555, 7321], 32, 32, 128),
+    ([9000, 4501, 8999, 9001, 700, 8500, 7001, 9500], 16, 16, 256),
+    ([13001, 12000, 6501, 13100], 64, 64, 256),
+    ([25100, 24701], 64, 64, 512),
+    ([24700, 24601, 24000, 23001, 24699, 24688, 12000, 24100], 32, 32, 256),   # long rows, two segments a block: the tiles and a counting launch
 ])
 def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
-    """From 1 M distances on a batch is counted in shared memory (head counts other than 16, 32 and 64, and grouped queries): the
-    same selection as each sequence by itself, and a table that is zero afterwards."""
+    """A batch whose distances are counted in shared memory: the same selection as each sequence by itself, and a table
+    that is zero afterwards."""
     _, K, U = _mods()
     B, ps, cap = len(lengths), 16, max(lengths) + 16
-    assert Hq * B * cap >= 1 << 20
     gen = torch.Generator(device=DEV).manual_seed(B)
     rand = lambda *shape: torch.randn(*shape, device=DEV, dtype=torch.float16, generator=gen)
     both = [[U.InferenceController(1, H, 128, ps, budget // ps, cap, torch.float16, DEV, num_q_heads=Hq) for _ in lengths] for _ in range(2)]
@@ -235,16 +242,17 @@ def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
             cs[i].end_forward()
     q, k, v = rand(B, Hq, 128), rand(B, H, 128), rand(B, H, 128)
     K.set_fused_append(fused_append)
+    rope = (8.0, 1e4) if Hq in (16, 28, 32, 64) else None
     batch = U.SequenceBatch(both[0])
     batch.prepare(1)
     batch.sync_seq_lens()
     idx = torch.full((B * Hq, budget - 1), -1, dtype=torch.int32, device=DEV)
-    o = batch.decode_step_dev(q, k, v, 0, indices_out=idx)
+    o = batch.decode_step_dev(q.clone(), k.clone(), v, 0, indices_out=idx, rope=rope)
     assert int(K.histogram_counts(batch._hist).abs().sum()) == 0
     for i, c in enumerate(both[1]):
         c.prepare_hadamard(1)
         c.begin_forward(1)
-        want = U.decode_step(q[i:i + 1], k[i:i + 1], v[i:i + 1], c, 0)
+        want = U.decode_step(q[i:i + 1].clone(), k[i:i + 1].clone(), v[i:i + 1], c, 0, rope=rope)
         assert torch.equal(idx[i * Hq:(i + 1) * Hq], c.topk_dindices_buffer), f"sequence {i}"
         _assert_attn_close(o[i], want[0])
         c.end_forward()

@@ -79,8 +79,8 @@ def test_sparse_decode_list_with_holes():
 @pytest.mark.parametrize("H,Hq", [(1, 1), (2, 2), (3, 9), (4, 4), (5, 5), (8, 64), (4, 28), (2, 32), (12, 12), (28, 28), (40, 40), (6, 48), (96, 96)])
 @pytest.mark.parametrize("L,ps", [(2, 16), (33, 1), (130, 16), (257, 7), (5000, 32), (40001, 16)])
 def test_estimate_items_shapes(H, Hq, L, ps):
-    """The estimate for any head count: remainders of its items, one item, several per warp, and (from 1 M distances
-    on) the counts in shared memory; distances and per-slice counts exact, grouped queries included."""
+    """The estimate for any head count: remainders of its items, one item, several per warp, counts in shared memory and, with few
+    tokens a block, in global memory; distances and per-slice counts exact, grouped queries included."""
     _, K, _ = _mods()
     if Hq * L > 1 << 22:
         pytest.skip("larger than the range this is about")
@@ -121,10 +121,42 @@ def test_estimate_on_both_sides_of_the_kernels_line(H, L):
     test_estimate_items_shapes(H, H, L, 16)
 
 
-@pytest.mark.parametrize("H,Hq", [(40, 40), (8, 64), (4, 4), (1000, 1000)])   # (1000: too many query planes for half an SM's memory)
+@pytest.mark.parametrize("H,L,dtype", [(16, 65536, torch.float16), (16, 65537, torch.bfloat16), (32, 49152, torch.float16), (32, 49153, torch.bfloat16),
+                                       (64, 24576, torch.float16), (64, 24577, torch.float16), (151, 6000, torch.float16)])
+def test_step_on_both_sides_of_the_kernels_line(H, L, dtype):
+    """The fused step (append, rotation and counts inside the estimate) selects what the separate operators do, at the last length of the
+    tile pipeline and the first one of the item kernel; 151 heads: more pieces than half of the blocks."""
+    _, K, U = _mods()
+    budget, ps, rope = 256, 16, (8.0, 1e4)
+    gen = torch.Generator(device=DEV).manual_seed(L)
+    rand = lambda n: torch.randn(n, H, 128, device=DEV, generator=gen).to(dtype)
+    k, v = rand(L), rand(L)
+    q, k1, v1 = rand(1), rand(1), rand(1)
+    found = []
+    for fused in (True, False):
+        c = U.InferenceController(1, H, 128, ps, budget // ps, L + 1, dtype, DEV)
+        c.prepare_hadamard(L)
+        c.begin_forward(L)
+        U.append_kvh(k, v, None, c, 0)
+        c.end_forward()
+        c.prepare_hadamard(1)
+        c.begin_forward(1)
+        qd, kd = q.clone(), k1.clone()
+        if fused:
+            U.decode_step(qd, kd, v1, c, 0, rope=rope)
+        else:
+            U.decode_topk(U.decode_estimate(U.append_qkv_fused(qd, kd, v1, c, 0, rope=rope), c, 0), c)
+        code = c.hadamard_cache.buf_layer(0)[c.hadamard_cache.indicies[-1], 0, L % ps].view(torch.int16)
+        found.append((c.topk_dindices_buffer.sort(1).values, qd.view(torch.int16), kd.view(torch.int16), code.clone()))
+        c.end_forward()
+    for a, b in zip(*found):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H,Hq", [(40, 40), (8, 64), (4, 4), (1000, 1000)])   # (1000: more pieces than blocks)
 def test_estimate_leaves_half_of_every_sm(H, Hq):
     """One estimate block per SM as the setting: the same distances and counts, from half of the SM's registers and shared
-    memory."""
+    memory.  (How many blocks a launch has is checked by the CPU test of the cuts.)"""
     _, K, _ = _mods()
     L, ps = 9001 if H < 1000 else 1100, 16
     g = torch.Generator().manual_seed(H)

@@ -118,9 +118,8 @@ def test_one_sequence_every_item_once(split, heads, blocks):
 
 @pytest.mark.parametrize("heads,group", [(4, 7), (8, 4), (8, 8), (1, 16), (4, 8)])
 def test_short_sequence_in_a_large_cache(split, heads, group):
-    """What a block gets follows from the length alone: 3000 tokens keep at least as many warps busy as in a cache of their size."""
-    src = open(os.path.join(ROOT, "adamas_b200", "csrc", "estimate_items.cuh")).read()
-    assert "item_query_heads(tiles_all * (p.H / HP), q_group" in src    # (the kernel divides by its own tiles)
+    """What a block gets follows from the length, which the kernel reads, and not from the capacity: at 3000 tokens half of the
+    blocks and more have something, or every tile and query head is on its own."""
     hp = split.cache_heads(heads, group)
     tiles = split.tiles_of(2999, 128 // hp)
     q_part = split.query_heads(tiles * (heads // hp), group, WARPS * BLOCKS)
