@@ -166,9 +166,9 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
   const int q_split = GROUPED ? (q_group + q_part - 1) / q_part : 1;
   const int pieces = p.H / HP * q_split;
-  // One sequence, no grouped queries: blockIdx.y is the piece, blockIdx.x an equal part of its tiles (or, a grid of one row, an even
-  // cut of the line).
-  const bool grid_of_pieces = !GROUPED && gridDim.y > 1;
+  // One sequence, no grouped queries: blockIdx.y is the piece, blockIdx.x an equal part of its tiles (or, a grid of one row with
+  // several pieces, an even cut of the line).
+  const bool grid_of_pieces = !GROUPED && !p.seqs && (gridDim.y > 1 || pieces == 1);
   int pos = 0, line_end = 1;
   if (!grid_of_pieces) {
     const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
