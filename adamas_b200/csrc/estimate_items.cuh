@@ -42,7 +42,8 @@ constexpr int kItemCountWords = 388;     // counts per query row and table (a di
 // heads, 2K tokens in a cache of 64K: 13.8 us a layer with tables, 13.6 without; 32 sequences x 600 x 4 heads 14.6 / 14.3).  Not with
 // grouped queries, where a piece has more rows (64 sequences x 2K x 28 over 4: 81.0 / 81.9), nor between a block's other segments (256 x 400
 // x 40 heads: 237.4 / 239.2).
-constexpr int kItemDirect = 256;
+// Long rows keep their tables: too many blocks would add to the same few counts (4 heads, 60K 13.35 / 13.7, 8 heads, 16K 12.5 / 12.65).
+constexpr int kItemDirect = 256, kItemDirectRow = 8192;
 
 // Count tables of a block: the slices that its tokens may fall into.
 __host__ __device__ __forceinline__ constexpr int item_tables(int hp, bool grouped) { return hp == 1 && !grouped ? 4 : 2; }
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     const bool scaled = p.ap.rp.inv_freq != nullptr;
     const int slice_tokens = p.hist ? 8 * sa_granules_per_block(max(n, 1), p.hist_cl) : 1;
     const int slice0 = p.hist ? first * TT / slice_tokens : 0;
-    const bool tables = p.hist && (GROUPED || rest * TT > kItemDirect);
+    const bool tables = p.hist && (GROUPED || rest * TT > kItemDirect || n > kItemDirectRow);
     const int used = tables ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
     if (scanning) {
       for (int i = tid; i < used * tab_rows * (kItemCountWords / 4); i += kItemWarps * 32) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
