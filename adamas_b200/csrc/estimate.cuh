@@ -3,7 +3,8 @@
 //
 // The code of (token t, head h) is 32 bytes at ((page*page_size + entry)*H + h)*32 in the code cache.  Two kernels:
 //
-// estimate_kernel / estimate_append_kernel (here): 16, 32 or 64 heads without grouped queries.  Persistent, two blocks per SM; the blocks of a sequence walk its tiles of kEstTile = 32 consecutive tokens round-robin.
+// estimate_kernel / estimate_append_kernel (here): 16, 32 or 64 heads without grouped queries, up to as many distances as the
+//   atomics below can count in time (estimate_by_tiles).  Persistent, two blocks per SM; the blocks of a sequence walk its tiles of kEstTile = 32 consecutive tokens round-robin.
 //   (Contiguous runs of tiles per block measured slower: 7.5 us against 6.8 for 32K tokens x 32 heads.)
 //   * Two producer warps issue one bulk (TMA) copy per token (the token's H codes, H*32 contiguous bytes) into a
 //     kEstStages-deep shared-memory ring; rows are padded by 16 bytes.  A "full" mbarrier per slot counts the bytes, an
@@ -14,7 +15,7 @@
 //     of one head, so the [H, n] output needs no transpose, no shuffle and no block barrier.  Histogram counts, where
 //     they are wanted, are one L2 atomic per distance.
 //
-// estimate_items_kernel (estimate_items.cuh): other head counts and grouped queries.
+// estimate_items_kernel (estimate_items.cuh): everything else.
 //
 // All mbarrier waits are bounded; one that runs out sets a device error flag and the kernel finishes (with wrong
 // results, which the flag reports).  The distance arithmetic on packed 2-bit codes is described at chunk_distance().

@@ -1,5 +1,5 @@
-// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline
-// for 16, 32 and 64 heads is in estimate.cuh, with the parameters and the distance arithmetic.
+// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes 16, 32 and
+// 64 heads as long as its atomics do not bound it, is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (56 instructions, 12 of them population counts at quarter rate, per 32 distances) for grouped
 // queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the
@@ -20,14 +20,12 @@
 //     made 1 M distances 6 to 8 us; additions of the constant 1 in shared memory take 1 to 2 cycles per warp, those of packed
 //     16-bit counts 4 to 13 (lanes that meet in a word are taken one after the other).
 // A piece is HP cache heads (with a part of their query heads, item_query_heads).  A block works on one piece of a sequence over
-// many tokens: it codes 4 to 16 query rows instead of all, its tables are small, and it adds up as many distances as there are before
-// a table goes out.  One sequence: every piece has the same number of blocks, which share its tokens evenly (nothing but a division lies
-// between a block's start and its first request).  A batch: sequence after sequence, in it piece after piece, in it token after
-// token forms one line that is cut evenly over the blocks, or, with few segments (a piece of a sequence), every block takes a part
-// of one.  The first items are requested before the kernel's dependency resolves (the cached codes are final).
+// many tokens: it codes 1 to 16 query rows instead of all, its tables are small, and it adds up as many distances as there are before
+// a table goes out.  How the items are dealt out is in item_split.h.  The first items are requested before the kernel's dependency
+// resolves (the cached codes are final).
 // Measured, the whole step, us a layer, against token after token with all heads in it and one block of 16 warps per SM: 40 heads,
-// 12K 18.1 -> 15.9; 32 query heads over 8, 30K 24.6 -> 23.7; 4 sequences x 128K x 4 heads 35.6 -> 32.5; 32 heads, 128K 49.1 -> 45.7
-// (tile pipeline and a counting launch).  Eight scanning warps and a ninth leave 96 registers: 26.2 for the grouped case.
+// 12K 18.1 -> 15.9; 32 query heads over 8, 30K 24.6 -> 22.9; 4 sequences x 128K x 4 heads 35.6 -> 32.5; 32 heads, 128K 49.1 -> 45.7
+// (tile pipeline and a counting launch).  Eight scanning warps and a ninth leave 96 registers: 26.2 against 23.7 for the grouped case.
 // Lane = head with four tokens per lane (one 4 KB run of codes per warp) was slower than lane = token.
 #pragma once
 #include "estimate.cuh"

@@ -526,9 +526,9 @@ struct DistHistogramParams {
 };
 
 // Per-slice histograms of given distance rows: grid (slices, rows[, sequences]).  Used where the rows exist
-// already (the stand-alone select_attend call) and, in the fused step, for launches with so many distances
-// that one L2 atomic per distance from inside the estimate would bound it (3 M and more per launch): a
-// block counts its slice in shared memory and stores 512 totals.
+// already (the stand-alone select_attend call) and, in the fused step, for the batches of long rows that stay with the tile
+// pipeline although one L2 atomic per distance from inside it would bound it (estimate_by_tiles): a block counts its
+// slice in shared memory and stores 512 totals.
 __global__ void __launch_bounds__(kSaBins) dist_histogram_kernel(const DistHistogramParams p) {
   __shared__ unsigned h_local[kSaBins];
   const int tid = threadIdx.x;
