@@ -356,9 +356,9 @@ int adamas_append_estimate(const void* q, const void* k, const void* v, void* q_
                            const float* thresholds3_host, uint32_t* hist, int hist_slices,
                            adamas_stream_t stream);
 
-/* One layer's whole decode step in one call: two launches (the estimate with the append inside, then
- * select+attend) for 32 or 64 heads and rotated inputs, three (fused append, estimate,
- * select+attend) otherwise:
+/* One layer's whole decode step in one call: two launches (the estimate with the append, and the rotary embedding if one is
+ * asked for, inside, then select+attend; one more for batches of long rows whose counts are a launch of their own), or as
+ * adamas_set_fused_append chooses:
  * what adamas/models/Adamas.py:145-200 does with seven launches.  q, k, v, o [1,H,D]; q_code
  * [1,H,D/8] scratch/output; dist_scratch [H, dist_stride] 16-bit, rows on 16-byte boundaries,
  * dist_stride >= context - 1; hist_scratch: see ADAMAS_HIST_WORDS_PER_HEAD.  Requires context > budget

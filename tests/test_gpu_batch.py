@@ -30,7 +30,7 @@ def _controllers(lengths, Hq, H, ps, budget_pages, dtype, cap, seed):
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("rope", [None, (8.0, 1e4)])
 @pytest.mark.parametrize("lengths,Hq,H,ps,budget", [
-    ([700, 300, 1500, 701], 32, 32, 16, 64),      # two-launch step (32 heads, no rotation) or three (with)
+    ([700, 300, 1500, 701], 32, 32, 16, 64),
     ([40000, 33000], 32, 32, 16, 1024),           # beyond 32768 tokens: several granules per thread
     ([900, 2000, 500], 8, 8, 1, 96),              # page size 1, page-copy estimate
     ([700, 1300], 32, 8, 16, 64),                 # grouped queries
