@@ -18,7 +18,7 @@
 // estimate_items_kernel (estimate_items.cuh): everything else.
 //
 // All mbarrier waits are bounded; one that runs out sets a device error flag and the kernel finishes (with wrong
-// results, which the flag reports).  The distance arithmetic on packed 2-bit codes is described at chunk_distance().
+// results, which the flag reports).  The distance arithmetic on packed 2-bit codes is described at code_distance().
 #pragma once
 #include "common.cuh"
 #include "hadamard_append.cuh"
@@ -34,50 +34,56 @@ constexpr int kEstThreads = (kEstConsumerWarps + kEstProducerWarps) * 32;
 constexpr int kEstStages = 3;     // ring depth (tiles in flight per block: kEstStages - 1)
 constexpr int kEstMaxBatch = 1024;
 
-// One 16-byte half of a query row's packed code and, for METRIC 0, (q_hi ^ q_lo) of every dimension at the hi bit positions.
+// A code's 128 dimensions as two bit planes (hi: value bit 1, lo: value bit 0) of four words: word i holds the dimensions of code words
+// 2i (at the odd bits) and 2i + 1 (at the even bits).
+struct CodePlanes {
+  uint32_t hi[4], lo[4];
+};
+// A query row's planes and their difference.
 struct __align__(16) QPlanes {
-  uint4 qw, qd;
+  uint4 hi, lo, d;   // d = hi ^ lo
 };
 
-__device__ __forceinline__ uint32_t lop3_70(uint32_t a, uint32_t b, uint32_t c) {  // a & ~(b & c)
+__device__ __forceinline__ uint32_t odd_even(uint32_t a, uint32_t b) {  // the odd bits of a, the even bits of b
   uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0x70;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(a), "r"(b), "r"(0xAAAAAAAAu));
   return d;
 }
-__device__ __forceinline__ uint32_t lop3_e4(uint32_t a, uint32_t b, uint32_t c) {  // (a & c) | (b & ~c)
-  uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0xE4;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-  return d;
+__device__ __forceinline__ uint32_t plane_hi(uint32_t w0, uint32_t w1) { return odd_even(w0, w1 >> 1); }
+__device__ __forceinline__ uint32_t plane_lo(uint32_t w0, uint32_t w1) { return odd_even(w0 << 1, w1); }
+__device__ __forceinline__ CodePlanes code_planes(uint4 a, uint4 b) {   // words 0 .. 3, 4 .. 7
+  return CodePlanes{{plane_hi(a.x, a.y), plane_hi(a.z, a.w), plane_hi(b.x, b.y), plane_hi(b.z, b.w)},
+                    {plane_lo(a.x, a.y), plane_lo(a.z, a.w), plane_lo(b.x, b.y), plane_lo(b.z, b.w)}};
+}
+__device__ __forceinline__ QPlanes query_planes(uint4 a, uint4 b) {
+  const CodePlanes c = code_planes(a, b);
+  return QPlanes{make_uint4(c.hi[0], c.hi[1], c.hi[2], c.hi[3]), make_uint4(c.lo[0], c.lo[1], c.lo[2], c.lo[3]),
+                 make_uint4(c.hi[0] ^ c.lo[0], c.hi[1] ^ c.lo[1], c.hi[2] ^ c.lo[2], c.hi[3] ^ c.lo[3])};
 }
 
-__device__ __forceinline__ uint32_t qplane_d(uint32_t qw) { return ((qw << 1) ^ qw) & 0xAAAAAAAAu; }
-__device__ __forceinline__ QPlanes make_qplanes(uint4 q) {
-  return QPlanes{q, make_uint4(qplane_d(q.x), qplane_d(q.y), qplane_d(q.z), qplane_d(q.w))};
-}
-
-// Distance contribution of one 16-byte chunk (64 dimensions), 25 integer instructions.
-// With x = k ^ q per dimension (x1, x0):  |k - q| = x0 + 2*x1 - 2*[x1 & x0 & (q1 ^ q0)]
-// (the correction fires exactly for the code pairs {1, 2}).  Clearing x1 where the bracket holds
-// gives y with |k - q| = y0 + 2*y1, so a word contributes popc(y) + popc(y & HI); the second terms of
-// two words share one popc.  The XOR metric of the reference's CUDA kernel is the same without the
-// correction.
+// Distance of two codes.  With x = k ^ q per dimension (x1, x0):  |k - q| = x0 + 2 * (x1 & ~(x0 & (q1 ^ q0)))  (the bracket clears
+// x1 for the code pairs {1, 2}); the XOR metric of the reference's CUDA kernel is the same without the bracket.  So four words
+// count once and four count twice; three full adders leave five of them to count.
+// Bound: logic instructions at half rate and population counts at an eighth of the issue rate.  Packed words, with x and y = x & ~... of
+// whole code words and 12 counts, took 78 cycles per 32 distances and scheduler, this form 57 (with 8 counts and no adders 58; of which the
+// query rows of a group share the key's planes).  The step, us a layer: 32 heads, 32K 20.2 -> 19.9; 32 query heads over 8, 30K 22.5 -> 21.1;
+// 40 heads, 12K 15.8 -> 15.5.
 template <int METRIC>
-__device__ __forceinline__ unsigned chunk_distance(uint4 kc, const QPlanes& q) {
-  const uint4 qw = q.qw, qd = q.qd;
-  const uint32_t x[4] = {kc.x ^ qw.x, kc.y ^ qw.y, kc.z ^ qw.z, kc.w ^ qw.w};
-  uint32_t y[4];
-  if (METRIC == 0) {
-    y[0] = lop3_70(x[0], x[0] << 1, qd.x);
-    y[1] = lop3_70(x[1], x[1] << 1, qd.y);
-    y[2] = lop3_70(x[2], x[2] << 1, qd.z);
-    y[3] = lop3_70(x[3], x[3] << 1, qd.w);
-  } else {
+__device__ __forceinline__ unsigned code_distance(const CodePlanes& k, const QPlanes& q) {
+  const uint32_t qh[4] = {q.hi.x, q.hi.y, q.hi.z, q.hi.w}, ql[4] = {q.lo.x, q.lo.y, q.lo.z, q.lo.w}, qd[4] = {q.d.x, q.d.y, q.d.z, q.d.w};
+  uint32_t one[4], two[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) y[i] = x[i];
+  for (int i = 0; i < 4; ++i) {
+    one[i] = k.lo[i] ^ ql[i];
+    two[i] = k.hi[i] ^ qh[i];
+    if (METRIC == 0) two[i] &= ~(one[i] & qd[i]);
   }
-  const uint32_t z0 = lop3_e4(y[0], y[1] >> 1, 0xAAAAAAAAu);
-  const uint32_t z1 = lop3_e4(y[2], y[3] >> 1, 0xAAAAAAAAu);
-  return (__popc(y[0]) + __popc(y[1]) + __popc(y[2])) + (__popc(y[3]) + __popc(z0) + __popc(z1));
+  auto sum = [](uint32_t a, uint32_t b, uint32_t c) { return a ^ b ^ c; };
+  auto carry = [](uint32_t a, uint32_t b, uint32_t c) { return (a & b) | (a & c) | (b & c); };
+  const uint32_t s1 = sum(one[0], one[1], one[2]), c1 = carry(one[0], one[1], one[2]);
+  const uint32_t s2 = sum(two[0], two[1], two[2]), c2 = carry(two[0], two[1], two[2]);
+  const uint32_t s3 = sum(s2, two[3], c1), c3 = carry(s2, two[3], c1);
+  return (__popc(s1) + __popc(one[3])) + 2 * __popc(s3) + 4 * (__popc(c2) + __popc(c3));
 }
 
 template <typename OutT>
@@ -293,7 +299,7 @@ __device__ __forceinline__ void est_produce(const EstimateParams& p, const EstGe
 // Consumer warp: lane = token of the tile; the warp covers heads warp*HPW .. (query planes in registers).
 template <int METRIC, typename OutT, int HPW>
 __device__ __forceinline__ void est_consume(const EstimateParams& p, const EstGeom& g, const EstRing& r, int my_tiles,
-                                            int lane, int warp, const QPlanes (&qp)[HPW][2]) {
+                                            int lane, int warp, const QPlanes (&qp)[HPW]) {
   OutT* out = static_cast<OutT*>(p.out) + static_cast<int64_t>(g.row0) * p.out_stride;   // this sequence's rows
   uint32_t* hist = p.hist ? p.hist + static_cast<size_t>(g.row0) * kSaScratchWordsPerHead : nullptr;
   int slot = 0;
@@ -311,7 +317,7 @@ __device__ __forceinline__ void est_consume(const EstimateParams& p, const EstGe
 #pragma unroll
     for (int hh = 0; hh < HPW; ++hh) {
       const int h = warp * HPW + hh;
-      d[hh] = chunk_distance<METRIC>(row[2 * h], qp[hh][0]) + chunk_distance<METRIC>(row[2 * h + 1], qp[hh][1]);
+      d[hh] = code_distance<METRIC>(code_planes(row[2 * h], row[2 * h + 1]), qp[hh]);
     }
     if (lane < tile_tokens) {
 #pragma unroll
@@ -376,12 +382,9 @@ __global__ void __launch_bounds__(kEstThreads) estimate_kernel(const EstimatePar
   // code is that kernel's output, so the consumers wait for it here (the producers do not).
   grid_dependency_wait();
   grid_launch_dependents();
-  QPlanes qp[HPW][2];
+  QPlanes qp[HPW];
 #pragma unroll
-  for (int hh = 0; hh < HPW; ++hh) {
-    qp[hh][0] = make_qplanes(ld_16(q_code + 2 * (warp * HPW + hh)));
-    qp[hh][1] = make_qplanes(ld_16(q_code + 2 * (warp * HPW + hh) + 1));
-  }
+  for (int hh = 0; hh < HPW; ++hh) qp[hh] = query_planes(ld_16(q_code + 2 * (warp * HPW + hh)), ld_16(q_code + 2 * (warp * HPW + hh) + 1));
   est_consume<METRIC, OutT, HPW>(p, geom, ring, my_tiles, lane, warp, qp);
 }
 
@@ -472,7 +475,7 @@ __global__ void __launch_bounds__(kEstThreads) estimate_append_kernel(const Esti
     }
   }
   if (geom.rank >= geom.blocks) return;
-  QPlanes qp[HPW][2];
+  QPlanes qp[HPW];
 #pragma unroll
   for (int pass = 0; pass < kPasses; ++pass) {
     float x[8];
@@ -491,8 +494,7 @@ __global__ void __launch_bounds__(kEstThreads) estimate_append_kernel(const Esti
     for (int s = 0; s < (HPW == 1 ? 1 : 2); ++s) {
       const uint4* cw = reinterpret_cast<const uint4*>(&s_code[warp][16 * s]);
       const int hh = (HPW == 1) ? 0 : 2 * pass + s;
-      qp[hh][0] = make_qplanes(cw[0]);
-      qp[hh][1] = make_qplanes(cw[1]);
+      qp[hh] = query_planes(cw[0], cw[1]);
     }
   }
   est_consume<0, uint16_t, HPW>(p, geom, ring, my_tiles, lane, warp, qp);

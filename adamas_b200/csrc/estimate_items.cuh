@@ -1,7 +1,7 @@
 // The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes 16, 32 and
 // 64 heads as long as its atomics do not bound it, is in estimate.cuh, with the parameters and the distance arithmetic.
 //
-// Bound: integer issue (56 instructions, 12 of them population counts at quarter rate, per 32 distances) for grouped
+// Bound: integer issue (logic at half rate and 5 population counts at an eighth, code_distance) for grouped
 // queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the
 // query while the others' first items are on their way, and appends the new token while they scan (a block that starts late, next
 // to the last blocks of the kernel in front, had its query 4.5 us after its start when the scanning warps coded it themselves
@@ -123,7 +123,7 @@ __device__ __noinline__ bool item_batch_apart(const int* cum, int batch, int pie
   return item_apart_pays(__reduce_max_sync(0xffffffffu, most), total, q_part, blocks);
 }
 
-// Dynamic shared memory: rings | planes [seg_rows][2] | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
+// Dynamic shared memory: rings | planes [seg_rows] | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
 // sequences before [batch + 1] (seqs).  GROUPED: several query heads per cache head (q_group > 1).
 // MODE 0: with the append inside (u16 distances); 1: the query codes are given; 2: the same with the XOR metric.
 template <typename T, int MODE, int HP, bool GROUPED>
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   const int q_group = GROUPED ? p.q_group : 1;
   const int rows = p.H * q_group;       // query rows of a sequence
   QPlanes* planes = reinterpret_cast<QPlanes*>(item_smem + kItemWarps * slots * kItemBytes);
-  uint32_t* counts = reinterpret_cast<uint32_t*>(planes + 2 * seg_rows);
+  uint32_t* counts = reinterpret_cast<uint32_t*>(planes + seg_rows);
   int* cum = reinterpret_cast<int*>(counts + (p.hist ? kTables * seg_rows * kItemCountWords : 0));
   uint4* ring = reinterpret_cast<uint4*>(item_smem + warp * (slots * kItemBytes));
   // The last warp codes the query, while the others request the first items, and appends the new token while they scan.
@@ -321,19 +321,24 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
             unpack16<T>(q[u][0], q[u][1], x);
             if (p.ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, p.ap.rp.mscale);
             const uint32_t w = code_word_8lanes<T>(x, l8, p.ap.scale, p.ap.th);
+            const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);   // (words 2i and 2i + 1 make word i of a plane)
             if (live[u]) {
-              uint32_t* qp = reinterpret_cast<uint32_t*>(planes + 2 * (r0 + 4 * u + (lane >> 3)) + (l8 >> 2)) + (l8 & 3);
-              qp[0] = w;
-              qp[4] = qplane_d(w);
+              if (!(l8 & 1)) {
+                const uint32_t hi = plane_hi(w, next), lo = plane_lo(w, next);
+                uint32_t* qp = reinterpret_cast<uint32_t*>(planes + r0 + 4 * u + (lane >> 3)) + (l8 >> 1);
+                qp[0] = hi;
+                qp[4] = lo;
+                qp[8] = hi ^ lo;
+              }
               if (first == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[code_row[u] * (kCodeWords / 2) + l8] = w;
             }
           }
         }
       }
     } else {
-      for (int c = lane; c < 2 * my_rows; c += 32) {
-        const int r = c >> 1;
-        if (!GROUPED || r % q_part < heads) planes[c] = make_qplanes(ld_16(p.q_code + (seq_row + query_row(r)) * 2 + (c & 1)));
+      for (int r = lane; r < my_rows; r += 32) {
+        const uint4* code = p.q_code + (seq_row + query_row(r)) * 2;
+        if (!GROUPED || r % q_part < heads) planes[r] = query_planes(ld_16(code), ld_16(code + 1));
       }
     }
     __syncthreads();   // planes and zeroed counts are visible
@@ -430,8 +435,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
           unsigned d[4];
 #pragma unroll
           for (int hh = 0; hh < HP; ++hh)
-            d[hh] = chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh) ^ f)], planes[2 * hh]) +
-                    chunk_distance<METRIC>(lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)], planes[2 * hh + 1]);
+            d[hh] = code_distance<METRIC>(code_planes(lrow[k * 32 * CPR + ((2 * hh) ^ f)], lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)]), planes[hh]);
           emit(0, head0, d, HP);
         } else {
           // Grouped queries: a code is read once for the piece's query heads of its cache head.  The loops over groups and heads stay
@@ -440,14 +444,14 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
           // 3K 16.8 / 13.2; 64 sequences x 2K x 28 over 4 103 / 81).
 #pragma unroll 1
           for (int hh = 0; hh < HP; ++hh) {
-            const uint4 k0 = lrow[k * 32 * CPR + ((2 * hh) ^ f)], k1 = lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)];
+            const CodePlanes key = code_planes(lrow[k * 32 * CPR + ((2 * hh) ^ f)], lrow[k * 32 * CPR + ((2 * hh + 1) ^ f)]);
             // (four distances, then their stores and counts: the counts keep the compiler from moving reads of shared memory across them)
             auto four = [&](int g, int many) {
-              const QPlanes* qp = planes + 2 * (hh * q_part + g);
+              const QPlanes* qp = planes + hh * q_part + g;
               unsigned d[4] = {0, 0, 0, 0};
 #pragma unroll
               for (int u = 0; u < 4; ++u)
-                if (u < many) d[u] = chunk_distance<METRIC>(k0, qp[2 * u]) + chunk_distance<METRIC>(k1, qp[2 * u + 1]);
+                if (u < many) d[u] = code_distance<METRIC>(key, qp[u]);
               emit(hh * q_part + g, (head0 + hh) * q_group + part0 + g, d, many);
             };
             int g = 0;
