@@ -83,6 +83,19 @@ __device__ __forceinline__ void tile_copy(const T* kbase, int64_t v_delta, int64
   }
 }
 
+// 8 rows of such a tile (kSaRows rows of one kind behind `slot`): lane l holds the cache row of token l, in units of row_bytes
+// behind `base`; FIRST: which 8.
+template <int FIRST>
+__device__ __forceinline__ void tile_copy8(const uint8_t* base, uint32_t row_bytes, int row, uint8_t* slot, int lane) {
+  const int half = lane >> 4, c = lane & 15;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {   // a half-warp per row
+    const int rr = FIRST + 2 * i + half;
+    const uint32_t r = static_cast<uint32_t>(__shfl_sync(0xffffffffu, row, rr));
+    cp_async_16(slot + rr * 256 + ((c ^ tile_swizzle(rr)) << 4), base + static_cast<uint64_t>(r) * row_bytes + c * 16);
+  }
+}
+
 // Scaled logits of a tile of ROWS tokens: s[2u], s[2u + 1] are head g's for tokens 8u + 2t, 8u + 2t + 1; -inf for tokens
 // outside `mask`.
 template <typename T, int ROWS>
@@ -105,6 +118,30 @@ __device__ __forceinline__ void tile_logits(const uint8_t* slot, const uint4 (&q
   for (int u = 0; u < ROWS / 4; ++u) {
     const int tok = 8 * (u >> 1) + 2 * t + (u & 1);
     s[u] = (mask >> tok) & 1u ? (c[u >> 1][0][u & 1] + c[u >> 1][1][u & 1]) * scale_log2 : -INFINITY;
+  }
+}
+
+// The same for one query row and the first `rem` tokens (8 at a time; ROWS at most).
+template <typename T, int ROWS>
+__device__ __forceinline__ void tile_logits8(const uint8_t* slot, const uint4 (&q)[4], int rem, float scale_log2, int lane, float (&s)[ROWS / 4]) {
+  const int g = lane >> 2, t = lane & 3;
+  const uint8_t* krow = slot + g * 256;
+  const int ksw = tile_swizzle(g);
+#pragma unroll
+  for (int u = 0; u < ROWS / 8; ++u) {
+    s[2 * u] = s[2 * u + 1] = -INFINITY;
+    if (u == 0 || rem > 8 * u) {
+      float c[2][4] = {};   // (two accumulators: shorter chains)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint4 k = *reinterpret_cast<const uint4*>(krow + u * 2048 + (((4 * j + t) ^ ksw) << 4));
+        Mma<T>::run(c[0], q[j].x, 0u, q[j].y, 0u, k.x, k.y);
+        Mma<T>::run(c[1], q[j].z, 0u, q[j].w, 0u, k.z, k.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        if (8 * u + 2 * t + i < rem) s[2 * u + i] = (c[0][i] + c[1][i]) * scale_log2;
+    }
   }
 }
 

@@ -31,6 +31,10 @@
 // Measured, the whole step: blocks of 512 threads with the distances in registers, two to an SM, took 22.7 us per layer for
 // one sequence (32 heads, 32K tokens, budget 1024), 103 us for 8 x 32K and 125 us for 32 x 4-8K; this form 20.7, 79 and 81.
 // (Blocks of 256 threads, three to an SM: 26.0 / - / 122.  16 rows per tile: a second round for half of the warps.)
+// A warp has few others to hide behind (four to a scheduler), so its instructions count: rows are copied, multiplied and weighted
+// eight at a time, as many as there are, P.V runs on paired fp32 multiply-adds with the weights from shared memory instead of a
+// shuffle per row, and half of the histogram loads are behind one branch (us a layer: 40 heads, 12K 15.5 -> 14.9; 32 over 8, 30K 21.1 -> 20.7; 32 x
+// 4-8K 69.0 -> 67.9; 32 heads, 32K 19.9 -> 19.7).
 #pragma once
 #include "attend_tile.cuh"
 #include "common.cuh"
@@ -205,17 +209,28 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   uint16_t q_own, q_pair = 0;                          // the query's element tid, and the one it rotates with
   {
     const uint4* hrow = reinterpret_cast<const uint4*>(head_scratch) + tid;
+    constexpr unsigned kHalf = kSaMaxSlices / 2;
     uint4 c[kSaMaxSlices];
+    auto load = [&](unsigned r) { c[r] = r < static_cast<unsigned>(p.slices) && tid < p.bin_threads ? __ldcg(hrow + r * (kSaBins / 4)) : make_uint4(0u, 0u, 0u, 0u); };
+    auto add = [&](unsigned r) {
+      tot.x += c[r].x; tot.y += c[r].y; tot.z += c[r].z; tot.w += c[r].w;
+      if (r < static_cast<unsigned>(slice)) { low.x += c[r].x; low.y += c[r].y; low.z += c[r].z; low.w += c[r].w; }
+    };
 #pragma unroll
-    for (unsigned r = 0; r < kSaMaxSlices; ++r) c[r] = r < static_cast<unsigned>(p.slices) && tid < p.bin_threads ? __ldcg(hrow + r * (kSaBins / 4)) : make_uint4(0u, 0u, 0u, 0u);
+    for (unsigned r = 0; r < kHalf; ++r) load(r);
+    if (p.slices > static_cast<int>(kHalf)) {
+#pragma unroll
+      for (unsigned r = kHalf; r < kSaMaxSlices; ++r) load(r);
+    }
     q_own = reinterpret_cast<const uint16_t*>(q_row)[tid];
     if (p.rope_on) q_pair = reinterpret_cast<const uint16_t*>(q_row)[tid ^ (kHeadDim / 2)];
     for (int g = tid; g < n_staged; g += kSaThreads) cp_async_16(staged + g + (g >> 3), gbase + g);
     cp_async_commit();
 #pragma unroll
-    for (unsigned r = 0; r < kSaMaxSlices; ++r) {
-      tot.x += c[r].x; tot.y += c[r].y; tot.z += c[r].z; tot.w += c[r].w;
-      if (r < static_cast<unsigned>(slice)) { low.x += c[r].x; low.y += c[r].y; low.z += c[r].z; low.w += c[r].w; }
+    for (unsigned r = 0; r < kHalf; ++r) add(r);
+    if (p.slices > static_cast<int>(kHalf)) {
+#pragma unroll
+      for (unsigned r = kHalf; r < kSaMaxSlices; ++r) add(r);
     }
   }
 
@@ -385,13 +400,14 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   // ---- attend: warp w takes rows w*rpw .. of the list, 24 at a time --------------------------------------
   uint8_t* tile = sa_smem + warp * kSaWarpBytes;
   float m_run = -INFINITY, l_run = 0.f;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);   // dimensions 4 * lane ..
+  float2 acc_lo = make_float2(0.f, 0.f), acc_hi = acc_lo;   // dimensions 4 * lane ..
   const int rpw = (n_loc + kSaWarps - 1) / kSaWarps;
   const int my_first = warp * rpw;
   const int my_total = max(0, min(rpw, n_loc - my_first));
   if (my_total > 0) {
-    const int64_t row_elems = static_cast<int64_t>(H) * kHeadDim, v_delta = p.page_size * row_elems;
-    const T* kbase = static_cast<const T*>(kv_base) + head_kv * kHeadDim;
+    const uint32_t row_bytes = static_cast<uint32_t>(H) * kHeadDim * 2;   // (H <= 1024)
+    const uint8_t* kbase = reinterpret_cast<const uint8_t*>(static_cast<const T*>(kv_base) + head_kv * kHeadDim);
+    const uint8_t* vbase = kbase + static_cast<uint64_t>(p.page_size) * row_bytes;
     int32_t* oi = p.out_idx ? p.out_idx + static_cast<int64_t>(head) * p.out_stride + lt_before + min(eq_before, need_eq) : nullptr;
     uint4 q[4];
 #pragma unroll
@@ -409,16 +425,19 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
         slot = sh.tail_slot;
       }
       const int row = static_cast<int>(slot + page_of(slot) * ps);   // page * 2 ps + entry
-      tile_copy<T, kSaRows, true, false>(kbase, v_delta, row_elems, row, tile, lane);
-      cp_async_commit();
-      tile_copy<T, kSaRows, false, true>(kbase, v_delta, row_elems, row, tile, lane);
-      cp_async_commit();
+      const int rem = my_total - done;
+      auto copy = [&](const uint8_t* base, uint8_t* to) {   // (eight rows at a time, as many as there are)
+        tile_copy8<0>(base, row_bytes, row, to, lane);
+        if (rem > 8) tile_copy8<8>(base, row_bytes, row, to, lane);
+        if (rem > 16) tile_copy8<16>(base, row_bytes, row, to, lane);
+        cp_async_commit();
+      };
+      copy(kbase, tile);
+      copy(vbase, tile + kSaRows * 256);
       float sc[kSaRows / 4];
       cp_async_wait<1>();
       __syncwarp();
-      tile_logits<T, kSaRows>(tile, q, my_total - done >= kSaRows ? (1u << kSaRows) - 1u : (1u << (my_total - done)) - 1u, p.scale_log2, lane, sc);
-      cp_async_wait<0>();
-      __syncwarp();
+      tile_logits8<T, kSaRows>(tile, q, rem, p.scale_log2, lane, sc);
       // softmax in base 2 (the head's logits are in lanes 0 .. 3) and P.V with four
       // dimensions per lane: one query row leaves the matrix form an eighth used and its accumulators cost 28 registers
       float m_new = sc[0];
@@ -431,24 +450,40 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
       const float rescale = exp2f(m_run - base);
       m_run = m_new;
       l_run *= rescale;
-      acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
+      acc_lo.x *= rescale; acc_lo.y *= rescale; acc_hi.x *= rescale; acc_hi.y *= rescale;
 #pragma unroll
       for (int u = 0; u < kSaRows / 4; ++u) {
         sc[u] = exp2f(sc[u] - base);
         l_run += sc[u];
         sc[u] = fmaxf(sc[u], 1.4e-45f);   // (0 times an infinity, in the row that an absent one borrows, would be a NaN)
       }
-      const uint8_t* vbase = tile + kSaRows * 256 + (lane & 1) * 8;
+      // the weights go through shared memory (the K rows' place: they are read), each twice: a pair of them is an operand of the paired
+      // multiply-add
+      float4* weights = reinterpret_cast<float4*>(tile);
+      __syncwarp();
+      if (lane < 4) {
 #pragma unroll
-      for (int j = 0; j < kSaRows; ++j) {
-        const float pj = __shfl_sync(0xffffffffu, sc[(j & 1) + 2 * (j >> 3)], (j & 7) >> 1);
-        const uint2 vv = *reinterpret_cast<const uint2*>(vbase + j * 256 + (((lane >> 1) ^ tile_swizzle(j)) << 4));
-        const float2 a = Elem<T>::to_f2(vv.x), b = Elem<T>::to_f2(vv.y);
-        acc.x = fmaf(pj, a.x, acc.x);
-        acc.y = fmaf(pj, a.y, acc.y);
-        acc.z = fmaf(pj, b.x, acc.z);
-        acc.w = fmaf(pj, b.y, acc.w);
+        for (int u = 0; u < kSaRows / 8; ++u) weights[4 * u + lane] = make_float4(sc[2 * u], sc[2 * u], sc[2 * u + 1], sc[2 * u + 1]);
       }
+      cp_async_wait<0>();
+      __syncwarp();
+      const uint8_t* vrow = tile + kSaRows * 256 + (lane & 1) * 8;
+      auto weigh8 = [&](int first) {
+#pragma unroll
+        for (int j = first; j < first + 8; j += 2) {
+          const float4 pp = weights[j >> 1];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint2 vv = *reinterpret_cast<const uint2*>(vrow + (j + i) * 256 + (((lane >> 1) ^ tile_swizzle(j + i)) << 4));
+            const float2 pj = i == 0 ? make_float2(pp.x, pp.y) : make_float2(pp.z, pp.w);
+            acc_lo = fma2(pj, Elem<T>::to_f2(vv.x), acc_lo);
+            acc_hi = fma2(pj, Elem<T>::to_f2(vv.y), acc_hi);
+          }
+        }
+      };
+      weigh8(0);
+      if (rem > 8) weigh8(8);
+      if (rem > 16) weigh8(16);
       __syncwarp();   // the tile may be filled again
     }
   }
@@ -457,7 +492,7 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);   // (lanes 0 .. 3)
   l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
   __syncwarp();
-  reinterpret_cast<float4*>(tile)[lane] = acc;
+  reinterpret_cast<float4*>(tile)[lane] = make_float4(acc_lo.x, acc_lo.y, acc_hi.x, acc_hi.y);
   if (lane == 0) {
     sh.ml[warp][0] = m_run;
     sh.ml[warp][1] = l_run;
