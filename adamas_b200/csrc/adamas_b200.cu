@@ -669,7 +669,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   }
   const int seg_rows = hp * q_part;
   const size_t room = static_cast<size_t>(di->smem_per_sm / kItemBlocksPerSm - 1024 - kItemStatic);
-  size_t smem = static_cast<size_t>(seg_rows) * sizeof(QPlanes);
+  size_t smem = static_cast<size_t>(seg_rows) * sizeof(QPlanes) + (ap.q && prm.q_group > 1 ? static_cast<size_t>(seg_rows + hp) * kHeadDim * 2 : 0);
   if (hist) smem += static_cast<size_t>(item_tables(hp, prm.q_group > 1)) * seg_rows * kItemCountWords * sizeof(uint32_t);
   if (seqs) smem += static_cast<size_t>(batch + 1) * sizeof(int);
   const size_t slot = static_cast<size_t>(kItemWarps) * kItemBytes;

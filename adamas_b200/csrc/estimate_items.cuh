@@ -5,7 +5,9 @@
 // queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the
 // query while the others' first items are on their way, and appends the new token while they scan (a block that starts late, next
 // to the last blocks of the kernel in front, had its query 4.5 us after its start when the scanning warps coded it themselves
-// behind their requests; now the codes are there 0.6 us after that kernel's end).  The other seven work alone:
+// behind their requests).  With grouped queries (up to 16 rows a block) it only loads the rows and all warps code them, one each:
+// the last warp alone took 2 us longer for eight (32 query heads over 8, 30K: 20.7 us a layer, 18.2 this way; with one row per warp for the four
+// rows of other blocks batches and long rows took 1-3 % longer, for the blocks that start late).  The other seven work alone:
 //   * its unit of work is an item of 4 KB of codes: 128 / HP tokens x HP heads (HP = 4, 2 or 1, see item_cache_heads).
 //     Its own 16-byte asynchronous copies bring items into its own ring of two or three slots: no
 //     producer warp, no barrier between warps.  (A bulk copy with a different address in every lane is issued lane after
@@ -110,7 +112,57 @@ __device__ __forceinline__ uint32_t code_word_8lanes(float (&x)[16], unsigned l8
   return static_cast<uint32_t>(bucketize_pack8(lo, th)) | (static_cast<uint32_t>(bucketize_pack8(hi, th)) << 16);
 }
 
+// A 128-element row spread over a warp, dimensions 4 * lane .. in a lane: the rotation, transform and code of a half-warp
+// (hadamard_append.cuh) with the same operations in the same order, so the same bits.
+template <typename T>
+__device__ __forceinline__ void unpack4(uint2 v, float (&x)[4]) {
+  const float2 a = Elem<T>::to_f2(v.x), b = Elem<T>::to_f2(v.y);
+  x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+}
+template <typename T>
+__device__ __forceinline__ void rope_warp(float (&x)[4], int lane, const float2* cs_table, bool scaled, float mscale) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {   // dimension pairs sit in lanes l and l ^ 16
+    const float other = __shfl_xor_sync(0xffffffffu, x[i], 16);
+    const float2 cs = cs_table[(lane & 15) * 4 + i];
+    float r = lane >= 16 ? fmaf(other, cs.y, x[i] * cs.x) : fmaf(-other, cs.y, x[i] * cs.x);
+    if (scaled) r *= mscale;
+    x[i] = Elem<T>::round(r);
+  }
+}
+// The row's code: lanes 4j .. 4j + 3 get its 32-bit word j.
+template <typename T>
+__device__ __forceinline__ uint32_t code_word_warp(float (&x)[4], int lane, float scale, const Thresholds& th) {
+#pragma unroll
+  for (int s = 1; s < 4; s <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if ((i & s) == 0) {
+        const float a = x[i], b = x[i + s];
+        x[i] = __fadd_rn(a, b);
+        x[i + s] = __fsub_rn(a, b);
+      }
+    }
+  }
+#pragma unroll
+  for (int m = 1; m < 32; m <<= 1) {
+    const float sgn = (lane & m) != 0 ? -1.0f : 1.0f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = __fmaf_rn(x[i], sgn, __shfl_xor_sync(0xffffffffu, x[i], m));
+  }
+  uint32_t w = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float v = Elem<T>::round(__fmul_rn(x[i], scale));
+    w |= static_cast<uint32_t>((v > th.t0) + (v > th.t1) + (v > th.t2)) << (2 * i);
+  }
+  w <<= 8 * (lane & 3);
+  w |= __shfl_xor_sync(0xffffffffu, w, 1);
+  return w | __shfl_xor_sync(0xffffffffu, w, 2);
+}
+
 struct EstShared {
+  int64_t kv_row, code_row;   // GROUPED: the new token's first row of the block's piece in the caches
   float2 cs[kHeadDim / 2];
 };
 
@@ -123,7 +175,7 @@ __device__ __noinline__ bool item_batch_apart(const int* cum, int batch, int pie
   return item_apart_pays(__reduce_max_sync(0xffffffffu, most), total, q_part, blocks);
 }
 
-// Dynamic shared memory: rings | planes [seg_rows] | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
+// Dynamic shared memory: rings | planes [seg_rows] | query rows and new key rows [seg_rows + HP][128] (append, GROUPED) | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
 // sequences before [batch + 1] (seqs).  GROUPED: several query heads per cache head (q_group > 1).
 // MODE 0: with the append inside (u16 distances); 1: the query codes are given; 2: the same with the XOR metric.
 template <typename T, int MODE, int HP, bool GROUPED>
@@ -141,7 +193,8 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   const int q_group = GROUPED ? p.q_group : 1;
   const int rows = p.H * q_group;       // query rows of a sequence
   QPlanes* planes = reinterpret_cast<QPlanes*>(item_smem + kItemWarps * slots * kItemBytes);
-  uint32_t* counts = reinterpret_cast<uint32_t*>(planes + seg_rows);
+  uint4* q_rows = reinterpret_cast<uint4*>(planes + seg_rows);
+  uint32_t* counts = reinterpret_cast<uint32_t*>(q_rows + (APPEND && GROUPED ? (seg_rows + HP) * (kHeadDim / 8) : 0));
   int* cum = reinterpret_cast<int*>(counts + (p.hist ? kTables * seg_rows * kItemCountWords : 0));
   uint4* ring = reinterpret_cast<uint4*>(item_smem + warp * (slots * kItemBytes));
   // The last warp codes the query, while the others request the first items, and appends the new token while they scan.
@@ -266,7 +319,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     // (the new token sits at position n = tokens before it)
     if (cs_here) {
       sh.cs[cs_pair] = rope_cos_sin_at(cs_freq, static_cast<float>(n));
-      asm volatile("bar.arrive 1, 96;" ::: "memory");   // (these two warps and the last one)
+      if (!GROUPED) asm volatile("bar.arrive 1, 96;" ::: "memory");   // (these two warps and the last one)
     }
 #pragma unroll
     for (int i = 0; i < kItemMaxSlots; ++i) {
@@ -276,17 +329,18 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       }
     }
 
-    // ---- the sequence's query: codes, planes; the new token's rows ---------------------------------------------
-    if (!waited) {
-      grid_dependency_wait();   // q, k, v or the query codes are the preceding kernel's output
-      grid_launch_dependents();
-      waited = true;
-    }
     const int64_t seq_row = static_cast<int64_t>(s) * rows;
+    // (r / q_part: both are at most 16)
+    const unsigned per_part = GROUPED ? 65536u / q_part + 1u : 0u;
+    auto head_of = [&](int r) { return GROUPED ? static_cast<int>(r * per_part >> 16) : r; };
     auto query_row = [&](int r) {   // row of the sequence that the segment's row r stands for
-      return GROUPED ? (head0 + r / q_part) * q_group + part0 + r % q_part : head0 + r;
+      const int h = head_of(r);
+      return GROUPED ? (head0 + h) * q_group + part0 + r - h * q_part : head0 + r;
     };
-    const int my_rows = HP * q_part;       // (of a short last part each cache head's last ones are absent)
+    auto absent = [&](int r) { return GROUPED && r - head_of(r) * q_part >= heads; };   // (of a short last part)
+    const int my_rows = HP * q_part;
+    // The block with the piece's first tile appends the new token's rows of the piece's cache heads.
+    const bool appends = APPEND && first == 0 && part0 == 0;
     const int tab_rows = GROUPED ? my_rows : seg_rows;   // rows of a count table
     const unsigned l8 = lane & 7;
     const bool scaled = p.ap.rp.inv_freq != nullptr;
@@ -294,57 +348,121 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     const int slice0 = p.hist ? first * TT / slice_tokens : 0;
     const bool tables = p.hist && (GROUPED || rest * TT > kItemDirect || n > kItemDirectRow);
     const int used = tables ? min(kTables, (end * TT - 1) / slice_tokens - slice0 + 1) : 0;   // count tables of this segment
+    constexpr int kPairs = (HP + 1) / 2;
+    uint4 v_row[kPairs];   // (GROUPED, last warp, appending: the new V rows, one in each half)
+    if (GROUPED && appends && !scanning && lane == 0) {   // (the page tables are final as well)
+      const StepAppend& ap = p.ap;
+      const int ps = ap.tgt.page_size;
+      const int32_t* kv_table = p.seqs ? p.seqs[s].kv_table : ap.tgt.kv_table;
+      const int32_t* code_table = p.seqs ? p.seqs[s].code_table : ap.tgt.code_table;
+      int kv_last_page = ap.kv_last_page, kv_entry = ap.kv_entry, code_last_page = ap.code_last_page, code_entry = ap.code_entry;
+      if (p.seq_len_dev) {
+        kv_last_page = code_last_page = n / ps;
+        kv_entry = code_entry = n - kv_last_page * ps;
+      }
+      const int64_t kv_page = __ldg(kv_table + kv_last_page), code_page = __ldg(code_table + code_last_page);
+      sh.kv_row = (kv_page * 2 * ps + kv_entry) * p.H + head0;
+      sh.code_row = (code_page * ps + code_entry) * p.H + head0;
+    }
+
+    // ---- the sequence's query: codes, planes; the new token's rows ---------------------------------------------
+    if (!waited) {
+      grid_dependency_wait();   // q, k, v or the query codes are the preceding kernel's output
+      grid_launch_dependents();
+      waited = true;
+    }
     if (scanning) {
       for (int i = tid; i < used * tab_rows * (kItemCountWords / 4); i += kItemWarps * 32) reinterpret_cast<uint4*>(counts)[i] = make_uint4(0, 0, 0, 0);
+    } else if (APPEND && GROUPED) {
+      const int c = lane & 15;   // (a half-warp per row)
+#pragma unroll 2
+      for (int r = lane >> 4; r < my_rows; r += 2)
+        if (!absent(r)) cp_async_16(q_rows + r * 16 + c, static_cast<const T*>(p.ap.q) + (seq_row + query_row(r)) * kHeadDim + c * 8);
+      if (appends) {
+#pragma unroll
+        for (int i = 0; i < kPairs; ++i) {
+          const int h = 2 * i + (lane >> 4);
+          if (h >= HP) continue;
+          cp_async_16(q_rows + (my_rows + h) * 16 + c, static_cast<const T*>(p.ap.k) + (static_cast<int64_t>(s) * p.H + head0 + h) * kHeadDim + c * 8);
+          v_row[i] = ld_16(static_cast<const T*>(p.ap.v) + (static_cast<int64_t>(s) * p.H + head0 + h) * kHeadDim + c * 8);
+        }
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
     } else if (APPEND) {
-      // eight lanes per row, four rows at a time, two times four on their way together
-      for (int r0 = 0; r0 < my_rows; r0 += 8) {
-        uint4 q[2][2];
-        int64_t code_row[2];
-        bool live[2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int r = r0 + 4 * u + (lane >> 3);
-          live[u] = r < my_rows && (!GROUPED || r % q_part < heads);
-          code_row[u] = seq_row + (live[u] ? query_row(r) : 0);
-          if (r0 + 4 * u < my_rows) {
-            const T* src = static_cast<const T*>(p.ap.q) + code_row[u] * kHeadDim + l8 * 16;
-            q[u][0] = ld_16(src);
-            q[u][1] = ld_16(src + 8);
-          }
+      // eight lanes per row, all (at most four) at a time
+      const int row = lane >> 3;
+      const int64_t code_row = seq_row + query_row(row < HP ? row : 0);
+      const T* src = static_cast<const T*>(p.ap.q) + code_row * kHeadDim + l8 * 16;
+      const uint4 q0 = ld_16(src), q1 = ld_16(src + 8);
+      if (p.ap.rope_on) asm volatile("bar.sync 1, 96;" ::: "memory");   // (the rotation is there)
+      float x[16];
+      unpack16<T>(q0, q1, x);
+      if (p.ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, p.ap.rp.mscale);
+      const uint32_t w = code_word_8lanes<T>(x, l8, p.ap.scale, p.ap.th);
+      const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);   // (words 2i and 2i + 1 make word i of a plane)
+      if (row < HP) {
+        if (!(l8 & 1)) {
+          const uint32_t hi = plane_hi(w, next), lo = plane_lo(w, next);
+          uint32_t* qp = reinterpret_cast<uint32_t*>(planes + row) + (l8 >> 1);
+          qp[0] = hi;
+          qp[4] = lo;
+          qp[8] = hi ^ lo;
         }
-        if (r0 == 0 && p.ap.rope_on) asm volatile("bar.sync 1, 96;" ::: "memory");   // (the rotation is there)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (r0 + 4 * u < my_rows) {   // (warp-uniform)
-            float x[16];
-            unpack16<T>(q[u][0], q[u][1], x);
-            if (p.ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, p.ap.rp.mscale);
-            const uint32_t w = code_word_8lanes<T>(x, l8, p.ap.scale, p.ap.th);
-            const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);   // (words 2i and 2i + 1 make word i of a plane)
-            if (live[u]) {
-              if (!(l8 & 1)) {
-                const uint32_t hi = plane_hi(w, next), lo = plane_lo(w, next);
-                uint32_t* qp = reinterpret_cast<uint32_t*>(planes + r0 + 4 * u + (lane >> 3)) + (l8 >> 1);
-                qp[0] = hi;
-                qp[4] = lo;
-                qp[8] = hi ^ lo;
-              }
-              if (first == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[code_row[u] * (kCodeWords / 2) + l8] = w;
-            }
-          }
-        }
+        if (first == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[code_row * (kCodeWords / 2) + l8] = w;
       }
     } else {
       for (int r = lane; r < my_rows; r += 32) {
         const uint4* code = p.q_code + (seq_row + query_row(r)) * 2;
-        if (!GROUPED || r % q_part < heads) planes[r] = query_planes(ld_16(code), ld_16(code + 1));
+        if (!absent(r)) planes[r] = query_planes(ld_16(code), ld_16(code + 1));
       }
     }
-    __syncthreads();   // planes and zeroed counts are visible
+    __syncthreads();
+    if (APPEND && GROUPED) {   // a warp per row
+#pragma unroll 1
+      for (int r = warp; r < my_rows + (appends ? HP : 0); r += kItemWarps + 1) {
+        const int h = r - my_rows;   // (a new key row)
+        if (h < 0 && absent(r)) continue;
+        uint2 raw = reinterpret_cast<const uint2*>(q_rows)[r * 32 + lane];
+        float x[4];
+        unpack4<T>(raw, x);
+        if (p.ap.rope_on) {
+          rope_warp<T>(x, lane, sh.cs, scaled, p.ap.rp.mscale);
+          raw = make_uint2(Elem<T>::from_f2(x[0], x[1]), Elem<T>::from_f2(x[2], x[3]));
+        }
+        const uint32_t w = code_word_warp<T>(x, lane, p.ap.scale, p.ap.th);
+        if (h < 0) {   // planes and, by the piece's first block, the code
+          const uint32_t next = __shfl_down_sync(0xffffffffu, w, 4);
+          if (first == 0 && (lane & 3) == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[(seq_row + query_row(r)) * (kCodeWords / 2) + (lane >> 2)] = w;
+          if ((lane & 7) == 0) {   // (words 2i and 2i + 1 make word i of a plane)
+            const uint32_t hi = plane_hi(w, next), lo = plane_lo(w, next);
+            uint32_t* qp = reinterpret_cast<uint32_t*>(planes + r) + (lane >> 3);
+            qp[0] = hi;
+            qp[4] = lo;
+            qp[8] = hi ^ lo;
+          }
+        } else {
+          if (p.ap.rope_on) (static_cast<uint2*>(p.ap.k) + (static_cast<int64_t>(s) * p.H + head0 + h) * (kHeadDim / 4))[lane] = raw;
+          void* kv_data = p.seqs ? p.seqs[s].kv_data : p.ap.tgt.kv_data;
+          void* code_data = p.seqs ? p.seqs[s].code_data : p.ap.tgt.code_data;
+          (static_cast<uint2*>(kv_data) + (sh.kv_row + h) * (kHeadDim / 4))[lane] = raw;
+          if ((lane & 3) == 0) (static_cast<uint32_t*>(code_data) + (sh.code_row + h) * (kCodeWords / 2))[lane >> 2] = w;
+        }
+      }
+      __syncthreads();
+    }
+    // (planes and zeroed counts are visible)
+    if (GROUPED && appends && !scanning) {
+      uint4* kv_data = static_cast<uint4*>(p.seqs ? p.seqs[s].kv_data : p.ap.tgt.kv_data);
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) {
+        const int h = 2 * i + (lane >> 4);
+        if (h < HP) kv_data[(sh.kv_row + static_cast<int64_t>(p.page_size) * p.H + h) * 16 + (lane & 15)] = v_row[i];
+      }
+    }
 
     // ---- the new token's rows of the piece's cache heads, in the block that has the piece's first tile ----------------------
-    if (APPEND && !scanning && first == 0 && part0 == 0) {
+    if (!GROUPED && appends && !scanning) {
       const StepAppend& ap = p.ap;
       const bool live = (lane >> 3) < HP;
       const int h = head0 + (live ? lane >> 3 : 0);

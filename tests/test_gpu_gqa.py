@@ -113,6 +113,39 @@ def test_gqa_decode_step(Hq, H, L, ps, budget, rope, dtype):
     c.end_forward()
 
 
+@pytest.mark.parametrize("Hq,H,L,dtype", [(32, 2, 70000, torch.float16), (48, 3, 4000, torch.bfloat16), (20, 4, 9000, torch.float16),
+                                          (16, 4, 30001, torch.bfloat16), (40, 1, 1500, torch.float16)])
+def test_gqa_step_selects_what_the_operators_do(Hq, H, L, dtype):
+    """1 to 16 query rows in a block of the estimate (and the new key rows behind them), parts of a group that are short of a row: the
+    fused step's selection, rotated rows, cache rows and codes are those of the separate operators."""
+    _, K, U = _mods()
+    budget, ps, rope = 128, 16, (8.0, 1e4)
+    gen = torch.Generator(device=DEV).manual_seed(L)
+    rand = lambda n, h: torch.randn(n, h, 128, device=DEV, generator=gen).to(dtype)
+    k, v, q, k1, v1 = rand(L, H), rand(L, H), rand(1, Hq), rand(1, H), rand(1, H)
+    found = []
+    for fused in (True, False):
+        c = U.InferenceController(1, H, 128, ps, budget // ps, L + 1, dtype, DEV, num_q_heads=Hq)
+        c.prepare_hadamard(L)
+        c.begin_forward(L)
+        U.append_kvh(k, v, None, c, 0)
+        c.end_forward()
+        c.prepare_hadamard(1)
+        c.begin_forward(1)
+        qd, kd = q.clone(), k1.clone()
+        if fused:
+            U.decode_step(qd, kd, v1, c, 0, rope=rope)
+        else:
+            U.decode_topk(U.decode_estimate(U.append_qkv_fused(qd, kd, v1, c, 0, rope=rope), c, 0), c)
+        page, at = c.kv_cache.indicies[-1], L % ps
+        code = c.hadamard_cache.buf_layer(0)[c.hadamard_cache.indicies[-1], 0, at].view(torch.int16)
+        found.append((c.topk_dindices_buffer.sort(1).values, qd.view(torch.int16), kd.view(torch.int16), code.clone(),
+                      c.kv_cache.buf_layer(0)[page, :, at].view(torch.int16).clone()))
+        c.end_forward()
+    for a, b in zip(*found):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("Hq,H,ps", [(32, 8, 16), (8, 2, 1), (12, 4, 16)])
 def test_gqa_graph_replay_equals_eager_loop(Hq, H, ps):
     """Device-resident sequence length with grouped queries: one captured sparse step and one captured
