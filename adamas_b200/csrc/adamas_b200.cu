@@ -538,38 +538,23 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 }
 
 // ---------------------------------------------------------------------------------------------
-// Launches of 3 M distances and more (a 128K context of 32 heads, three 32K sequences): there one L2 atomic per distance from
-// inside the tile pipeline bounds it (the estimate of one 128K sequence: 31.7 us with the counts, 23.7 without).
-static bool many_distances(int q_heads, int batch, int n) {
-  return static_cast<int64_t>(q_heads) * batch * n >= (int64_t(3) << 20);
-}
 // Which estimate kernel.  n is the length, or the cache's capacity where the length is on the device.
 //
-// The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of its heads in registers,
-// as long as its L2 atomics, one per distance, do not bound it; the item kernel, which counts in shared memory, takes the rest.
-// Whole step, us a layer, tiles / items.  One sequence, 32 heads: 4K 12.0 / 13.1, 32K 20.5 / 21.0, 64K 27.4 / 26.0, 88K 34.9 /
-// 30.9, 128K 48.9 / 45.7; 64 heads, 32K 28.9 / 27.1; 16 heads, 64K 23.5 / 20.1.  Batches of 32 heads: 2 x 8K 16.9 / 17.4, 8 x
-// 4K 25.8 / 27.8, 16 x 2-4K 33.7 / 35.5, 4 x 16K 29.8 / 30.1, 12 x 8K 43.5 / 41.6, 8 x 8-16K 41.8 / 40.1, 32 x 4-8K 75.0 / 72.5,
-// 16 x 16K 81.2 / 80.0; of 16 heads: 8 x 8K 26.8 / 22.5, 32 x 8K 68.7 / 50.3, 4 x 64K 59.4 / 41.4.
+// The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of its heads in registers.  With
+// counts, one L2 atomic per distance in it, it is ahead only where a block of the item kernel has next to nothing to scan and its query
+// decides (us a layer, tiles / items): 16 heads, 1.5K 8.4 / 9.0, 2K with rotation 9.2 / 9.7, 4K 10.8 / 10.1; 32 heads, 1.5K 9.1 / 9.7, 4K 10.8 / 11.0,
+// 8K 12.3 / 11.7, with rotation 2K 10.6 / 10.3, 4K 12.0 / 11.3, 32K 20.6 / 20.2; 64 heads, 1.5K 12.0 / 11.8; 2 x 3K of 16 heads 11.8 / 12.1, of 32 heads
+// without rotation 11.5 / 12.1, 4 x 4K of 16 heads 15.8 / 14.5.
 //
-// Long rows of a batch (beyond 24K) go to the tiles, with the counts in a launch of their own, unless there are so few segments
-// (a piece of 4 heads of a sequence) that the item kernel keeps them apart.  Otherwise a block's two segments of hundreds of tiles read pieces of
-// the same tokens far apart in time: 32 heads, 8 x 32K 79.0 / 81.3.  Where they are few: 2 x 48K 34.7 / 34.6, 3 x 36K 37.5 / 36.6, 2 x 128K 68.1 / 66.6, 4 x
-// 64K 71.5 / 66.8; 64 heads, 2 x 28K 42.4 / 38.0, 2 x 66K 75.0 / 68.9.
-//
-// Short sequences in large caches: 32 heads, 4K in 98K 14.7 / 14.5, 16K 16.7 / 16.9; 64 heads, 8K in 66K 18.9 / 16.6; 16 heads, 2K in 66K 13.3 /
-// 13.5, 8K 14.2 / 14.0; batches of 32 heads, 8 x 4K in 32K 27.4 / 27.1, 4 x 8K in 64K 23.8 / 22.2, 16 x 3K in 32K 35.9 / 36.9.
-//
-// Without counts (counts false) there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
+// Without counts there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
 // 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
 static bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
-static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, int blocks) {
+static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope) {
   if (!tile_heads(num_heads, q_heads)) return false;
-  const int64_t distances = static_cast<int64_t>(q_heads) * batch * n;
-  if (num_heads == 16) return distances < (int64_t(1) << 20);
-  if (!counts) return true;
-  if (batch == 1) return distances < (int64_t(3) << 19);
-  return !many_distances(q_heads, batch, n) || (n > 24576 && !item_apart_few(batch * (num_heads / 4), blocks));
+  const int64_t tokens = static_cast<int64_t>(batch) * n;
+  if (!counts) return num_heads != 16 || tokens < 65536;
+  if (num_heads == 16) return n <= 3584 && tokens <= 7168;
+  return num_heads == 32 && !rope && n <= 4608 && tokens <= 7168;
 }
 
 // Launches the estimate.  n: distances per row, or their upper bound when seq_len_dev gives the length on the device
@@ -614,7 +599,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   cudaStream_t st = to_stream(stream);
   // (the tiles store query codes on any 16-bit word, at every length)
   const bool codes_aligned = (reinterpret_cast<uintptr_t>(ap.q_code_out) & 15) == 0;
-  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, est_blocks_per_sm() * di->num_sms) || (!codes_aligned && tile_heads(num_heads, q_heads))) {
+  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, ap.rope_on != 0) || (!codes_aligned && tile_heads(num_heads, q_heads))) {
     const int num_tiles = (n + kEstTile - 1) / kEstTile;
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
@@ -661,9 +646,9 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   dim3 grid(static_cast<unsigned>(std::min<int64_t>(slots_all, items)));
   int64_t per_block = (items + grid.x - 1) / grid.x;
   if (!seqs && prm.q_group == 1) {
-    const int per = item_blocks_per_piece(static_cast<int>(tiles), pieces, 1, static_cast<int>(grid.x));
+    const int per = std::min<int>(item_blocks_per_piece(static_cast<int>(tiles), pieces, 1, static_cast<int>(grid.x)), (tiles + kItemWarps - 1) / kItemWarps);
     if (per > 0) {
-      grid = dim3(static_cast<unsigned>(per), static_cast<unsigned>(pieces));
+      grid = dim3(static_cast<unsigned>(pieces), static_cast<unsigned>(per));
       per_block = (tiles + per - 1) / per;
     }
   }
@@ -671,7 +656,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   const size_t room = static_cast<size_t>(di->smem_per_sm / kItemBlocksPerSm - 1024 - kItemStatic);
   size_t smem = static_cast<size_t>(seg_rows) * sizeof(QPlanes) + (ap.q && prm.q_group > 1 ? static_cast<size_t>(seg_rows + hp) * kHeadDim * 2 : 0);
   if (hist) smem += static_cast<size_t>(item_tables(hp, prm.q_group > 1)) * seg_rows * kItemCountWords * sizeof(uint32_t);
-  if (seqs) smem += static_cast<size_t>(batch + 1) * sizeof(int);
+  if (seqs) smem += static_cast<size_t>(batch + 2) * sizeof(int);
   const size_t slot = static_cast<size_t>(kItemWarps) * kItemBytes;
   int slots = static_cast<int>(std::min<int64_t>(kItemMaxSlots, (per_block + kItemWarps - 1) / kItemWarps));
   while (slots > 1 && smem + slots * slot > room) --slots;
@@ -1295,7 +1280,6 @@ int adamas_select_attend(const void* dist, int64_t dist_stride, int n, int k, co
     hp.hist = hist;
     hp.n = n;
     hp.cl = pl.slices;
-    hp.seq_len_dev = nullptr;
     ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.slices, num_heads), dim3(kSaBins), 0,
                   to_stream(stream), 1, hp);
   }
@@ -1317,7 +1301,6 @@ int adamas_dist_histograms(const void* dist, int64_t dist_stride, int n, int num
   hp.hist = hist;
   hp.n = n;
   hp.cl = slices;
-  hp.seq_len_dev = nullptr;
   ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(slices, num_heads), dim3(kSaBins), 0,
                 to_stream(stream), 1, hp);
   return check_launch("dist_histogram_kernel");
@@ -1438,16 +1421,12 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   SaPlan pl;
   if (int rc = sa_plan(n, budget - 1, q_heads * batch, page_size, di, &pl)) return rc;
   int rc;
-  // The histogram counts.  Item kernel: in shared memory.  Tile pipeline: one L2 atomic per distance from inside the estimate, or,
-  // with many distances, a launch of its own that counts in shared memory.
-  const bool count_apart = estimate_by_tiles(num_heads, q_heads, batch, n, true, est_blocks_per_sm() * di->num_sms) && many_distances(q_heads, batch, n);
-  uint32_t* est_hist = count_apart ? nullptr : hist;
   const bool two_launches = fused_append_enabled();
   if (two_launches) {
     // two launches: the estimate with the append (and, with RoPE, the rotation) inside, then select + attend
     rc = estimate_append_launch(q, k, v, q_code, kv_data, kv_page_table, pages, last_len, code_data,
                                 code_page_table, pages, last_len, n, num_heads, q_heads, page_size, dtype, dist_scratch,
-                                dist_stride, hadamard_scale, thresholds3_host, seq_len_dev, est_hist, pl.slices, stream, seqs,
+                                dist_stride, hadamard_scale, thresholds3_host, seq_len_dev, hist, pl.slices, stream, seqs,
                                 batch, rope);
     if (rc) return rc;
   } else {
@@ -1456,20 +1435,8 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
                             thresholds3_host, dtype, stream, rope, seq_len_dev, q_heads, seqs, batch);
     if (rc) return rc;
     rc = launch_estimate(q_code, StepAppend{}, dtype, code_data, code_page_table, n, page_size, num_heads, q_heads, dist_scratch,
-                         dist_stride, ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, est_hist, pl.slices, stream, seqs, batch);
+                         dist_stride, ADAMAS_VAL_U16, ADAMAS_METRIC_L1, seq_len_dev, hist, pl.slices, stream, seqs, batch);
     if (rc) return rc;
-  }
-  if (count_apart) {
-    DistHistogramParams hp;
-    hp.dist = static_cast<const uint16_t*>(dist_scratch);
-    hp.dist_stride = dist_stride;
-    hp.hist = hist;
-    hp.n = n;
-    hp.cl = pl.slices;
-    hp.seq_len_dev = seq_len_dev;
-    ADAMAS_LAUNCH("dist_histogram_kernel", dist_histogram_kernel, dim3(pl.slices, q_heads, batch), dim3(kSaBins), 0,
-                  to_stream(stream), 1, hp);
-    if (int rc2 = check_launch("dist_histogram_kernel")) return rc2;
   }
   const int64_t tail = static_cast<int64_t>(kv_last_page_idx) * page_size + last_len - 1;
   rc = select_attend_impl(dist_scratch, dist_stride, n, budget - 1, q, o, nullptr, lse, kv_data, kv_page_table,

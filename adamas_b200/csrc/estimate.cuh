@@ -3,8 +3,8 @@
 //
 // The code of (token t, head h) is 32 bytes at ((page*page_size + entry)*H + h)*32 in the code cache.  Two kernels:
 //
-// estimate_kernel / estimate_append_kernel (here): 16, 32 or 64 heads without grouped queries, up to as many distances as the
-//   atomics below can count in time (estimate_by_tiles).  Persistent, two blocks per SM; the blocks of a sequence walk its tiles of kEstTile = 32 consecutive tokens round-robin.
+// estimate_kernel / estimate_append_kernel (here): 16, 32 or 64 heads without grouped queries, for short rows with counts and, 32 and 64
+//   heads, for all without (estimate_by_tiles).  Persistent, two blocks per SM; the blocks of a sequence walk its tiles of kEstTile = 32 consecutive tokens round-robin.
 //   (Contiguous runs of tiles per block measured slower: 7.5 us against 6.8 for 32K tokens x 32 heads.)
 //   * Two producer warps issue one bulk (TMA) copy per token (the token's H codes, H*32 contiguous bytes) into a
 //     kEstStages-deep shared-memory ring; rows are padded by 16 bytes.  A "full" mbarrier per slot counts the bytes, an
@@ -147,11 +147,14 @@ struct EstimateParams {
   StepAppend ap;
 };
 
-// Tiles of `tile_tokens` tokens of the batch's sequences in front of each one -> cum[0 .. batch]; one warp.
+// Tiles of `tile_tokens` tokens of the batch's sequences in front of each one -> cum[0 .. batch], and, MOST, the most that one has ->
+// cum[batch + 1]; one warp.
+template <bool MOST = false>
 __device__ __forceinline__ void est_line(const EstimateParams& p, int tile_tokens, int lane, int* cum) {
-  int base = 0;
+  int base = 0, most = 0;
   for (int s0 = 0; s0 < p.batch; s0 += 32) {
     int v = s0 + lane < p.batch ? est_tiles(__ldg(p.seq_len_dev + s0 + lane) - 1, tile_tokens) : 0;
+    most = max(most, v);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int u = __shfl_up_sync(0xffffffffu, v, o);
@@ -161,6 +164,10 @@ __device__ __forceinline__ void est_line(const EstimateParams& p, int tile_token
     base += __shfl_sync(0xffffffffu, v, 31);
   }
   if (lane == 0) cum[0] = 0;
+  if (MOST) {
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 0) cum[p.batch + 1] = most;
+  }
 }
 
 // What a block works on: tiles rank, rank + blocks, ... of one sequence; nothing to scan where rank == blocks.

@@ -1,5 +1,5 @@
-// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes 16, 32 and
-// 64 heads as long as its atomics do not bound it, is in estimate.cuh, with the parameters and the distance arithmetic.
+// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes the short rows of 16 and
+// 32 heads and estimates without counts, is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (logic at half rate and 5 population counts at an eighth, code_distance) for grouped
 // queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the
@@ -166,17 +166,8 @@ struct EstShared {
   float2 cs[kHeadDim / 2];
 };
 
-// Whether a batch with grouped queries keeps to one segment a block.  (Out of line: inlined, it cost the launches of one sequence 0.3 us through the
-// registers of what follows.)
-__device__ __noinline__ bool item_batch_apart(const int* cum, int batch, int pieces, int q_part) {
-  const int total = cum[batch] * pieces, blocks = gridDim.x;
-  int most = 0;
-  for (int s = threadIdx.x & 31; s < batch; s += 32) most = max(most, item_apart_most(cum[s + 1] - cum[s], total, blocks - batch * pieces));
-  return item_apart_pays(__reduce_max_sync(0xffffffffu, most), total, q_part, blocks);
-}
-
 // Dynamic shared memory: rings | planes [seg_rows] | query rows and new key rows [seg_rows + HP][128] (append, GROUPED) | counts [tables][seg_rows][kItemCountWords] (hist) | token tiles of the
-// sequences before [batch + 1] (seqs).  GROUPED: several query heads per cache head (q_group > 1).
+// sequences before [batch + 1], the most of one (seqs).  GROUPED: several query heads per cache head (q_group > 1).
 // MODE 0: with the append inside (u16 distances); 1: the query codes are given; 2: the same with the XOR metric.
 template <typename T, int MODE, int HP, bool GROUPED>
 __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items_kernel(const EstimateParams p, int slots, int seg_rows) {
@@ -207,7 +198,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   // ---- this block's part of the work ------------------------------------------------------------------------------------
   int tiles_all;
   if (p.seqs) {
-    if (warp == 0) est_line(p, TT, lane, cum);
+    if (warp == 0) est_line<true>(p, TT, lane, cum);
     __syncthreads();
     tiles_all = cum[p.batch];
   } else {
@@ -218,10 +209,11 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
   const int q_part = GROUPED ? item_query_heads(tiles_all * (p.H / HP), q_group, p.chip_warps) : 1;
   const int q_split = GROUPED ? (q_group + q_part - 1) / q_part : 1;
   const int pieces = p.H / HP * q_split;
-  // One sequence, no grouped queries: blockIdx.y is the piece, blockIdx.x an equal part of its tiles (or, a grid of one row with
-  // several pieces, an even cut of the line).
-  const bool grid_of_pieces = !GROUPED && !p.seqs && (gridDim.y > 1 || pieces == 1);
-  int pos = 0, line_end = 1;
+  // One sequence, no grouped queries: blockIdx.x is the piece, blockIdx.y an equal part of its tiles (or, where the grid's rows are not the
+  // pieces, an even cut of the line).
+  const bool grid_of_pieces = !GROUPED && !p.seqs && static_cast<int>(gridDim.x) == pieces;
+  // Several sequences: columns of a block per piece, which share the line of one piece's tiles.
+  int pos = 0, line_end = 1, column_piece = -1;
   if (!grid_of_pieces) {
     const int total = tiles_all * pieces;   // (below 2^31: checked on the host)
     if (total == 0) {   // (lengths that are all zero: the kernel behind must not overtake the one in front)
@@ -229,12 +221,20 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       return;
     }
     ItemShare work;
-    if (!p.seqs) work = GROUPED ? item_share_one(tiles_all, pieces, q_part, gridDim.x, blockIdx.x) : item_share_even(total, gridDim.x, blockIdx.x);
-    else if (item_apart_possible(total, p.batch * pieces, gridDim.x) &&
-             (item_apart_simple(total, p.batch * pieces, gridDim.x) ||
-              (GROUPED && !item_apart_hopeless(total, p.batch * pieces, q_part, gridDim.x) && item_batch_apart(cum, p.batch, pieces, q_part))))
-      work = item_share_apart(cum, p.batch, pieces, gridDim.x, blockIdx.x);
-    else work = item_share_even(total, gridDim.x, blockIdx.x);
+    const int columns = p.seqs ? item_blocks_per_piece(tiles_all, pieces, q_part, gridDim.x) : 0;
+    if (columns > 0) {
+      const int column = blockIdx.x / pieces, alike = item_columns_alike(cum, p.batch, columns);
+      column_piece = blockIdx.x - column * pieces;
+      if (column >= columns) work = ItemShare{0, 0};
+      else if (alike > 0) work = item_share_alike(cum[1], p.batch, alike, column);
+      else if (item_columns_apart(tiles_all, cum[p.batch + 1], p.batch, q_part, columns))
+        work = item_share_apart(cum, p.batch, 1, columns, column);
+      else work = item_share_even(tiles_all, columns, column);
+    } else if (GROUPED && !p.seqs) {
+      work = item_share_one(tiles_all, pieces, q_part, gridDim.x, blockIdx.x);
+    } else {
+      work = item_share_even(total, gridDim.x, blockIdx.x);
+    }
     pos = work.pos;
     line_end = work.end;
   }
@@ -246,9 +246,9 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     const uint4* codes = p.codes;
     const int32_t* table = p.page_table;
     if (grid_of_pieces) {
-      const int share = (tiles_all + gridDim.x - 1) / gridDim.x;
-      piece = blockIdx.y;
-      first = blockIdx.x * share;
+      const int share = (tiles_all + gridDim.y - 1) / gridDim.y;
+      piece = blockIdx.x;
+      first = blockIdx.y * share;
       end = min(tiles_all, first + share);
       rest = end - first;
       pos = line_end;
@@ -259,20 +259,21 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     } else {
       int tiles = tiles_all, at = pos;
       if (p.seqs) {
+        const int line_pieces = column_piece >= 0 ? 1 : pieces;
         int lo = 0, hi = p.batch - 1;
         while (lo < hi) {
           const int mid = (lo + hi + 1) >> 1;
-          if (cum[mid] * pieces <= pos) lo = mid; else hi = mid - 1;
+          if (cum[mid] * line_pieces <= pos) lo = mid; else hi = mid - 1;
         }
         s = lo;
         tiles = cum[s + 1] - cum[s];
-        at = pos - cum[s] * pieces;
+        at = pos - cum[s] * line_pieces;
         n = __ldg(p.seq_len_dev + s) - 1;
         codes = static_cast<const uint4*>(p.seqs[s].code_data);
         table = p.seqs[s].code_table;
       }
-      piece = at / tiles;
-      first = at - piece * tiles;
+      piece = column_piece >= 0 ? column_piece : at / tiles;
+      first = column_piece >= 0 ? at : at - piece * tiles;
       rest = line_end - pos;
       end = min(tiles, first + rest);
       pos += end - first;

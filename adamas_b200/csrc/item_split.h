@@ -63,23 +63,33 @@ ADAMAS_HD int item_blocks_per_piece(int tiles, int pieces, int q_part, int block
 ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks, int b) {
   const int per = item_blocks_per_piece(tiles, pieces, q_part, blocks);
   if (per == 0) return item_share_even(tiles * pieces, blocks, b);
-  const int share = (tiles + per - 1) / per, piece = b / per, first = (b - piece * per) * share;
-  if (piece >= pieces || first >= tiles) return {0, 0};
+  const int share = (tiles + per - 1) / per;
+  // (Long shares: the pieces of a range of tokens in neighbouring blocks, as in a batch's columns, 28 query heads over 4, 100K 24.3 -> 23.6 us a
+  // layer.  Short ones: the blocks that have something spread over the launch, 3K 11.8 / 11.0.)
+  const int part = share > kItemWarps ? b / pieces : b % per, piece = share > kItemWarps ? b % pieces : b / per, first = part * share;
+  if (piece >= pieces || part >= per || first >= tiles) return {0, 0};
   return {piece * tiles + first, piece * tiles + (share < tiles - first ? first + share : tiles)};
 }
 
 // A batch: cum[s] tiles lie in front of sequence s.
 //
-// Where the segments are no more than the blocks, every block may take a part of ONE, the blocks dealt out in proportion to the
-// items.  A second segment costs a block about 4 us (a query to load and code behind a barrier, counts to add up), a larger share its
+// The blocks form columns of one block per piece (item_blocks_per_piece of them, neighbours in the launch; none, an even cut of the whole
+// line, where too many blocks would be left over).  The columns share the line of ONE piece's tiles, so that the pieces of a token's codes,
+// which lie side by side, are read at about the same time: with the pieces of a sequence one after the other on the line, blocks read pieces
+// of the same tokens far apart (32 heads, us a layer: 8 x 32K 76.0 -> 72.2, 32 x 4-8K 67.9 -> 63.0, 16 x 15-30K 58.4 -> 56.2; 4 x 30K of 64 heads
+// 69.7 -> 63.4; all columns of a piece next to one another 72.9, 64.0, 58.1 and 64.0).
+//
+// Where the sequences are no more than the columns, every column may take a part of ONE, the columns dealt out in proportion to the
+// tiles.  A second segment costs a block about 4 us (a query to load and code behind a barrier, counts to add up), a larger share its
 // items.  They are kept apart
-//  * where there is little work, or an eighth as many segments as blocks: shares differ by an eighth at most (4 sequences x 64K x 32
+//  * with equal lengths, where a seventh of the columns at most stays without any: the shares are equal as well (8 x 32K 72.8 a layer, 73.4
+//    cut evenly; 20 x 16K of 8 heads 30.7 / 33.1; 10 x 26K of 32 heads, where a fifth would stay idle, 82.2 / 82.0);
+//  * where there is little work, or an eighth as many sequences as columns: shares differ by an eighth at most (4 sequences x 64K x 32
 //    heads 71.3 us a layer cut evenly, 67.7 apart);
-//  * with grouped queries, where the largest share is up to kItemApart items more than an even one, times the query heads of a
-//    cache head in them (64 x 2K x 28 over 4: 80.8 cut evenly, 79.3 apart with 2 items of 7 heads more; 32 x 2K x 32 over 8 52.3 / 49.7).
-//    What the largest share is costs about 2 us to find, once per launch.  Without grouped queries that is
-//    more than it gains (40 heads, 12 x 8K 46.1 / 48.4).
-// (Products stay below 2^31.  Lengths that are all zero leave nothing to deal out.)
+//  * where the largest share cannot be much more than an even one.  It is at most that of the longest sequence with a column of its own, and at
+//    most tiles / (columns - sequences): item_columns_apart.
+// (Products stay below 2^31.  Lengths that are all zero leave nothing to deal out.)  In what follows a segment is a sequence and a block a
+// column; with the whole line cut (pieces > 1) a piece of a sequence and a block.
 constexpr int kItemApart = 24;
 ADAMAS_HD bool item_apart_possible(int total, int segments, int blocks) { return total > 0 && segments <= blocks && total <= 0x7fffffff / blocks; }
 ADAMAS_HD bool item_apart_few(int segments, int blocks) { return segments * 8 <= blocks; }
@@ -112,6 +122,25 @@ ADAMAS_HD ItemShare item_share_apart(const int* cum, int batch, int pieces, int 
   const int nblk = all < n_items ? all : n_items;
   if (b - f >= nblk) return {0, 0};
   return {start + n_items * (b - f) / nblk, start + n_items * (b - f + 1) / nblk};
+}
+
+constexpr int kItemApartPlain = 40;   // (without grouped queries)
+ADAMAS_HD bool item_columns_apart(int total, int longest, int batch, int q_part, int columns) {
+  if (!item_apart_possible(total, batch, columns)) return false;
+  if (item_apart_simple(total, batch, columns)) return true;
+  const int spare = columns - batch, most = static_cast<long long>(longest) * spare <= total ? longest : total / spare + 1;
+  return (most - total / columns) * q_part <= (q_part > 1 ? kItemApart : kItemApartPlain);
+}
+// Equal lengths (cum[1] of them tiles each): `per` columns a sequence, or 0.
+ADAMAS_HD int item_columns_alike(const int* cum, int batch, int columns) {
+  if (batch > columns || static_cast<long long>(cum[1]) * batch != cum[batch] || columns % batch > columns / 7) return 0;
+  return columns / batch;
+}
+ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
+  const int s = c / per, nblk = per < tiles ? per : tiles, i = c - s * per;
+  if (s >= batch || i >= nblk) return {0, 0};
+  const int q = tiles / nblk, r = tiles - q * nblk;
+  return {s * tiles + i * q + i * r / nblk, s * tiles + (i + 1) * q + (i + 1) * r / nblk};
 }
 
 }  // namespace adamas

@@ -570,26 +570,22 @@ struct DistHistogramParams {
   const uint16_t* dist;
   int64_t dist_stride;
   uint32_t* hist;
-  int n;                        // distances per row, or their upper bound with seq_len_dev
+  int n;                        // distances per row
   int cl;
-  const int32_t* seq_len_dev;   // optional: n = *seq_len_dev - 1 (grid.z = sequence: seq_len_dev[z], rows (z, y))
 };
 
-// Per-slice histograms of given distance rows: grid (slices, rows[, sequences]).  Used where the rows exist
-// already (the stand-alone select_attend call) and, in the fused step, for the batches of long rows that stay with the tile
-// pipeline although one L2 atomic per distance from inside it would bound it (estimate_by_tiles): a block counts its
-// slice in shared memory and stores 512 totals.
+// Per-slice histograms of given distance rows: grid (slices, rows).  Used where the rows exist already (the stand-alone
+// select_attend call): a block counts its slice in shared memory and stores 512 totals.
 __global__ void __launch_bounds__(kSaBins) dist_histogram_kernel(const DistHistogramParams p) {
   __shared__ unsigned h_local[kSaBins];
   const int tid = threadIdx.x;
   const int r = blockIdx.x;
-  const int head = blockIdx.z * gridDim.y + blockIdx.y;
+  const int head = blockIdx.y;
   h_local[tid] = 0;
   __syncthreads();
   grid_dependency_wait();
   grid_launch_dependents();
-  const int n = p.seq_len_dev ? __ldg(p.seq_len_dev + blockIdx.z) - 1 : p.n;
-  const int G = (n + 7) >> 3;
+  const int n = p.n, G = (n + 7) >> 3;
   const int gpb = sa_granules_per_block(n, p.cl);
   const int g_end = min(G, (r + 1) * gpb);
   const uint4* gbase = reinterpret_cast<const uint4*>(p.dist + static_cast<int64_t>(head) * p.dist_stride);

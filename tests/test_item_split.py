@@ -42,6 +42,20 @@ int share_batch(const int* cum, int batch, int pieces, int q_part, int blocks, i
   }
   return apart;
 }
+int share_columns(const int* cum, int batch, int pieces, int q_part, int blocks, int* out) {   // column shares, piece after piece
+  const int columns = item_blocks_per_piece(cum[batch], pieces, q_part, blocks);
+  int longest = 0;
+  for (int s = 0; s < batch; ++s) longest = std::max(longest, cum[s + 1] - cum[s]);
+  const int alike = columns > 0 ? item_columns_alike(cum, batch, columns) : 0;
+  const bool apart = columns > 0 && item_columns_apart(cum[batch], longest, batch, q_part, columns);
+  for (int b = 0; b < blocks && columns > 0; ++b) {
+    const int c = b / pieces;
+    ItemShare w{0, 0};
+    if (c < columns) w = alike > 0 ? item_share_alike(cum[1], batch, alike, c) : apart ? item_share_apart(cum, batch, 1, columns, c) : item_share_even(cum[batch], columns, c);
+    out[2 * b] = w.pos; out[2 * b + 1] = w.end;
+  }
+  return columns == 0 ? 0 : alike > 0 ? 1 : apart ? 2 : 3;
+}
 }
 """
 
@@ -170,3 +184,39 @@ def test_batches_that_keep_to_one_segment(split, batch, n, heads, group, want):
     tiles = [split.tiles_of(n - 1, 128 // hp)] * batch
     q_part = split.query_heads(sum(tiles) * (heads // hp), group, WARPS * BLOCKS)
     assert _batch(split, tiles, heads // hp * -(-group // q_part), q_part)[1] is want
+
+
+@pytest.mark.parametrize("blocks", [BLOCKS, BLOCKS // 2])
+@pytest.mark.parametrize("heads,group", [(4, 1), (40, 1), (32, 1), (7, 1), (151, 1), (8, 4), (4, 7), (8, 8), (1, 16)])
+def test_columns_of_a_batch_every_item_once(split, heads, group, blocks):
+    """Every piece's blocks cover all sequences' tiles; equal lengths get equal shares of one sequence; columns of ragged lengths that
+    are kept apart have one sequence each and not much more than an even share."""
+    rng = random.Random(heads * 10 + group + blocks)
+    for case in range(80):
+        batch = rng.choice([1, 2, 3, 8, 16, 31, 37, 100, 256, 1024])
+        top = rng.choice([1, 40, 700, 5000, 60000])
+        hp = split.cache_heads(heads, group)
+        alike = case % 4 == 0
+        lengths = [top] * batch if alike else [rng.randrange(0, top + 1) for _ in range(batch)]
+        tiles = [0 if not alike and rng.random() < 0.1 else split.tiles_of(n, 128 // hp) for n in lengths]
+        if sum(tiles) == 0:
+            tiles[-1] = 1
+        q_part = split.query_heads(sum(tiles) * (heads // hp), group, WARPS * blocks)
+        pieces = heads // hp * -(-group // q_part)
+        grid = min(blocks, sum(tiles) * pieces)
+        cum = np.concatenate([[0], np.cumsum(tiles)]).astype(np.int32)
+        out = np.full((grid, 2), -1, dtype=np.int32)
+        mode = split.share_columns(cum.ctypes.data_as(ctypes.c_void_p), batch, pieces, q_part, grid, out.ctypes.data_as(ctypes.c_void_p))
+        if mode == 0:
+            continue
+        columns = split.per_piece(int(cum[-1]), pieces, grid) if q_part == 1 else None
+        for piece in range(pieces):
+            mine = out[piece::pieces]
+            _covers(mine[:columns], int(cum[-1]))
+        sizes = out[:, 1] - out[:, 0]
+        if mode in (1, 2):
+            for a, b in out:
+                if a != b:
+                    assert np.searchsorted(cum[1:], a, "right") == np.searchsorted(cum[1:], b - 1, "right")
+        if mode == 1:
+            assert sizes.max() - sizes[sizes > 0].min() <= 1
