@@ -522,7 +522,7 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
   PagedTarget tgt{kv_data, kv_page_table, static_cast<uint16_t*>(code_data), code_page_table, page_size,
                   num_heads};
   const Thresholds th = make_thresholds(thresholds3_host);
-  const unsigned blocks = rows_to_blocks(rows);
+  const unsigned blocks = static_cast<unsigned>((rows + 31) / 32);   // (eight lanes a row)
   const int64_t start = seq_len - n_tokens;
   cudaStream_t st = to_stream(stream);
 #define LAUNCH_AP(T, F)                                                                                                  \

@@ -126,6 +126,14 @@ struct Elem<__half> {
     return *reinterpret_cast<uint32_t*>(&h);
   }
   static __device__ __forceinline__ float round(float a) { return __half2float(__float2half_rn(a)); }
+  // two copies of the largest number of the type up to a; which halves of v are above those of t
+  static __device__ __forceinline__ uint32_t floor2(float a) {
+    const __half2 h = __half2half2(__float2half_rd(a));
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  static __device__ __forceinline__ uint32_t above2(uint32_t v, uint32_t t) {
+    return __hgt2_mask(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&t));
+  }
   // c + a.lo * b.lo + a.hi * b.hi on two packed pairs, in that order, each step one fused multiply-add
   // in fp32 on the 16-bit operands (mixed-precision fma of sm_100: the same result as converting
   // first, without the conversions)
@@ -153,6 +161,13 @@ struct Elem<__nv_bfloat16> {
   }
   static __device__ __forceinline__ float round(float a) {
     return __bfloat162float(__float2bfloat16_rn(a));
+  }
+  static __device__ __forceinline__ uint32_t floor2(float a) {
+    const __nv_bfloat162 h = __bfloat162bfloat162(__float2bfloat16_rd(a));
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  static __device__ __forceinline__ uint32_t above2(uint32_t v, uint32_t t) {
+    return __hgt2_mask(*reinterpret_cast<const __nv_bfloat162*>(&v), *reinterpret_cast<const __nv_bfloat162*>(&t));
   }
   static __device__ __forceinline__ float dot2(uint32_t a, uint32_t b, float c) {
     float d;
@@ -184,8 +199,23 @@ __device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
   return v;
 }
 
-// a * b + c on both halves, one instruction on sm_100.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+// Arithmetic on both halves of a pair, one instruction on sm_100 (each half rounded like the scalar one).
+#define ADAMAS_PAIR_OP(name, op)                                                      \
+  __device__ __forceinline__ float2 name(float2 a, float2 b) {                        \
+    float2 d;                                                                         \
+    asm("{\n\t.reg .b64 x, y;\n\t"                                                   \
+        "mov.b64 x, {%2, %3};\n\t"                                                    \
+        "mov.b64 y, {%4, %5};\n\t" op " x, x, y;\n\t"                                \
+        "mov.b64 {%0, %1}, x;\n\t}"                                                   \
+        : "=f"(d.x), "=f"(d.y)                                                        \
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                    \
+    return d;                                                                         \
+  }
+ADAMAS_PAIR_OP(add2, "add.rn.f32x2")
+ADAMAS_PAIR_OP(sub2, "sub.rn.f32x2")
+ADAMAS_PAIR_OP(mul2, "mul.rn.f32x2")
+#undef ADAMAS_PAIR_OP
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {   // a * b + c
   float2 d;
   asm("{\n\t.reg .b64 x, y, z;\n\t"
       "mov.b64 x, {%2, %3};\n\t"

@@ -277,3 +277,29 @@ def test_query_codes_on_any_16_bit_word(H, L):
     for other in results[1:]:
         for a, b in zip(results[0], other):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("thresholds", [(-10.0, 0.0, 10.0), (-1.0001, 0.10007, 3.14159), (float("-inf"), 0.0, float("inf")), (-1e6, 70000.0, 1e30),
+                                        (0.5, float("nan"), 0.25)])
+def test_prefill_codes_at_any_thresholds(thresholds, dtype):
+    """The fused prefill append compares in the storage type with thresholds rounded down: the codes are those of a comparison in fp32,
+    for thresholds that the type does not have, beyond its range, infinite and in any order, and values up to infinities."""
+    from adamas_b200 import hadamard_transform
+    _, K, _ = _mods()
+    N, H, ps = 37, 3, 16
+    k = _randn((N, H, 128), 5, dtype)
+    k[:5] *= 3000.0
+    k[5] = 60000.0   # (the first coefficient overflows fp16)
+    pages = (N + ps - 1) // ps
+    kd, table = k.to(DEV), torch.arange(pages, dtype=torch.int32, device=DEV)
+    kv = torch.zeros(pages, 2, ps, H, 128, dtype=dtype, device=DEV)
+    codes = torch.zeros(pages, 1, ps, H, 16, dtype=torch.int16, device=DEV)
+    last = (N - 1) % ps + 1
+    K.append_kv_cache_prefill(kd, kd, None, kv, table, None, last, 0, codes, table, None, last, 0, 0, None, thresholds)
+    h = hadamard_transform(kd).float().cpu()
+    bucket = sum((h > torch.tensor(t)).to(torch.int32) for t in thresholds).view(N, H, 16, 8)
+    want = sum(bucket[..., i] << (2 * i) for i in range(8)).to(torch.int16)
+    assert torch.equal(codes.view(pages * ps, H, 16)[:N].cpu(), want)
+    assert torch.equal(kv.permute(0, 2, 1, 3, 4).reshape(pages * ps, 2, H, 128)[:N].cpu().view(torch.int16),
+                       torch.stack([k, k], 1).view(torch.int16))
