@@ -48,70 +48,6 @@ constexpr int kItemDirect = 256, kItemDirectRow = 8192;
 // Count tables of a block: the slices that its tokens may fall into.
 __host__ __device__ __forceinline__ constexpr int item_tables(int hp, bool grouped) { return hp == 1 && !grouped ? 4 : 2; }
 
-// 128-point transform of a row spread over 8 lanes, 16 elements each: the butterflies of wht128_halfwarp in the
-// same order, so the same bits.
-__device__ __forceinline__ void wht128_8lanes(float (&x)[16], unsigned l8) {
-#pragma unroll
-  for (int s = 1; s < 16; s <<= 1) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      if ((i & s) == 0) {
-        const float a = x[i], b = x[i + s];
-        x[i] = __fadd_rn(a, b);
-        x[i + s] = __fsub_rn(a, b);
-      }
-    }
-  }
-#pragma unroll
-  for (unsigned m = 1; m < 8; m <<= 1) {
-    const float sgn = (l8 & m) != 0 ? -1.0f : 1.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float other = __shfl_xor_sync(0xffffffffu, x[i], m);
-      x[i] = __fmaf_rn(x[i], sgn, other);
-    }
-  }
-}
-
-// rope_halfwarp_cs for a row spread over 8 lanes: dimension pairs sit in lanes l and l ^ 4.
-template <typename T>
-__device__ __forceinline__ void rope_8lanes(float (&x)[16], unsigned l8, const float2* cs_table, bool scaled, float mscale) {
-  const bool upper = (l8 & 4) != 0;
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    const float other = __shfl_xor_sync(0xffffffffu, x[i], 4);
-    const float2 cs = cs_table[static_cast<int>(l8 & 3) * 16 + i];
-    float r = upper ? fmaf(other, cs.y, x[i] * cs.x) : fmaf(-other, cs.y, x[i] * cs.x);
-    if (scaled) r *= mscale;
-    x[i] = Elem<T>::round(r);
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void unpack16(uint4 a, uint4 b, float (&x)[16]) {
-  float lo[8], hi[8];
-  unpack8<T>(a, lo);
-  unpack8<T>(b, hi);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    x[i] = lo[i];
-    x[8 + i] = hi[i];
-  }
-}
-
-// transform, scale, bucketize: this lane's 32-bit word of the row's code
-template <typename T>
-__device__ __forceinline__ uint32_t code_word_8lanes(float (&x)[16], unsigned l8, float scale, const Thresholds& th) {
-  wht128_8lanes(x, l8);
-  float lo[8], hi[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    lo[i] = Elem<T>::round(__fmul_rn(x[i], scale));
-    hi[i] = Elem<T>::round(__fmul_rn(x[8 + i], scale));
-  }
-  return static_cast<uint32_t>(bucketize_pack8(lo, th)) | (static_cast<uint32_t>(bucketize_pack8(hi, th)) << 16);
-}
-
 // A 128-element row spread over a warp, dimensions 4 * lane .. in a lane: the rotation, transform and code of a half-warp
 // (hadamard_append.cuh) with the same operations in the same order, so the same bits.
 template <typename T>
@@ -132,7 +68,7 @@ __device__ __forceinline__ void rope_warp(float (&x)[4], int lane, const float2*
 }
 // The row's code: lanes 4j .. 4j + 3 get its 32-bit word j.
 template <typename T>
-__device__ __forceinline__ uint32_t code_word_warp(float (&x)[4], int lane, float scale, const Thresholds& th) {
+__device__ __forceinline__ uint32_t code_word_warp(float (&x)[4], int lane, float scale, const PairThresholds<T>& th) {
 #pragma unroll
   for (int s = 1; s < 4; s <<= 1) {
 #pragma unroll
@@ -152,10 +88,8 @@ __device__ __forceinline__ uint32_t code_word_warp(float (&x)[4], int lane, floa
   }
   uint32_t w = 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float v = Elem<T>::round(__fmul_rn(x[i], scale));
-    w |= static_cast<uint32_t>((v > th.t0) + (v > th.t1) + (v > th.t2)) << (2 * i);
-  }
+  for (int j = 0; j < 2; ++j) w |= buckets2<T>(Elem<T>::from_f2(__fmul_rn(x[2 * j], scale), __fmul_rn(x[2 * j + 1], scale)), th, 4 * j);
+  w = (w | (w >> 16)) & 0xffu;
   w <<= 8 * (lane & 3);
   w |= __shfl_xor_sync(0xffffffffu, w, 1);
   return w | __shfl_xor_sync(0xffffffffu, w, 2);
@@ -394,23 +328,33 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       // eight lanes per row, all (at most four) at a time
       const int row = lane >> 3;
       const int64_t code_row = seq_row + query_row(row < HP ? row : 0);
-      const T* src = static_cast<const T*>(p.ap.q) + code_row * kHeadDim + l8 * 16;
-      const uint4 q0 = ld_16(src), q1 = ld_16(src + 8);
+      const T* src = static_cast<const T*>(p.ap.q) + code_row * kHeadDim + l8 * 8;
+      const uint4 q0 = ld_16(src), q1 = ld_16(src + kHeadDim / 2);
       if (p.ap.rope_on) asm volatile("bar.sync 1, 96;" ::: "memory");   // (the rotation is there)
-      float x[16];
-      unpack16<T>(q0, q1, x);
-      if (p.ap.rope_on) rope_8lanes<T>(x, l8, sh.cs, scaled, p.ap.rp.mscale);
-      const uint32_t w = code_word_8lanes<T>(x, l8, p.ap.scale, p.ap.th);
-      const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);   // (words 2i and 2i + 1 make word i of a plane)
+      float2 x[8];
+      unpack_pairs<T>(q0, q1, x);
+      if (p.ap.rope_on) rope_pairs<T>(x, l8, sh.cs, scaled, p.ap.rp.mscale);
+      const uint32_t w = code_pairs<T>(x, l8, p.ap.scale, PairThresholds<T>(p.ap.th));
+      // 32-bit words l8 / 2 and 4 + l8 / 2 of the code in the even lanes, and words i and 2 + i, i = l8 / 4, of a plane in every fourth
+      const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);
+      const uint32_t c0 = __byte_perm(w, next, 0x5410), c1 = __byte_perm(w, next, 0x7632);
+      const uint32_t d0 = __shfl_down_sync(0xffffffffu, c0, 2), d1 = __shfl_down_sync(0xffffffffu, c1, 2);
       if (row < HP) {
-        if (!(l8 & 1)) {
-          const uint32_t hi = plane_hi(w, next), lo = plane_lo(w, next);
-          uint32_t* qp = reinterpret_cast<uint32_t*>(planes + row) + (l8 >> 1);
-          qp[0] = hi;
-          qp[4] = lo;
-          qp[8] = hi ^ lo;
+        if (first == 0 && !(l8 & 1)) {
+          uint32_t* dst = reinterpret_cast<uint32_t*>(p.ap.q_code_out) + code_row * (kCodeWords / 2) + (l8 >> 1);
+          dst[0] = c0;
+          dst[4] = c1;
         }
-        if (first == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[code_row * (kCodeWords / 2) + l8] = w;
+        if (!(l8 & 3)) {
+          const uint32_t hi0 = plane_hi(c0, d0), lo0 = plane_lo(c0, d0), hi1 = plane_hi(c1, d1), lo1 = plane_lo(c1, d1);
+          uint32_t* qp = reinterpret_cast<uint32_t*>(planes + row) + (l8 >> 2);
+          qp[0] = hi0;
+          qp[2] = hi1;
+          qp[4] = lo0;
+          qp[6] = lo1;
+          qp[8] = hi0 ^ lo0;
+          qp[10] = hi1 ^ lo1;
+        }
       }
     } else {
       for (int r = lane; r < my_rows; r += 32) {
@@ -431,7 +375,7 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
           rope_warp<T>(x, lane, sh.cs, scaled, p.ap.rp.mscale);
           raw = make_uint2(Elem<T>::from_f2(x[0], x[1]), Elem<T>::from_f2(x[2], x[3]));
         }
-        const uint32_t w = code_word_warp<T>(x, lane, p.ap.scale, p.ap.th);
+        const uint32_t w = code_word_warp<T>(x, lane, p.ap.scale, PairThresholds<T>(p.ap.th));
         if (h < 0) {   // planes and, by the piece's first block, the code
           const uint32_t next = __shfl_down_sync(0xffffffffu, w, 4);
           if (first == 0 && (lane & 3) == 0) reinterpret_cast<uint32_t*>(p.ap.q_code_out)[(seq_row + query_row(r)) * (kCodeWords / 2) + (lane >> 2)] = w;
@@ -467,11 +411,12 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       const StepAppend& ap = p.ap;
       const bool live = (lane >> 3) < HP;
       const int h = head0 + (live ? lane >> 3 : 0);
-      const int64_t in_off = (static_cast<int64_t>(s) * p.H + h) * kHeadDim + l8 * 16;
+      constexpr int kHalf = kHeadDim / 2;
+      const int64_t in_off = (static_cast<int64_t>(s) * p.H + h) * kHeadDim + l8 * 8;
       T* ksrc = static_cast<T*>(ap.k) + in_off;
       const T* vsrc = static_cast<const T*>(ap.v) + in_off;
-      uint4 k0 = ld_16(ksrc), k1 = ld_16(ksrc + 8);
-      const uint4 v0 = ld_16(vsrc), v1 = ld_16(vsrc + 8);
+      uint4 k0 = ld_16(ksrc), k1 = ld_16(ksrc + kHalf);
+      const uint4 v0 = ld_16(vsrc), v1 = ld_16(vsrc + kHalf);
       PagedTarget tgt = ap.tgt;
       if (p.seqs) {
         tgt.kv_data = p.seqs[s].kv_data;
@@ -486,29 +431,28 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
         kv_entry = code_entry = n - kv_last_page * ps;
       }
       const int64_t kv_page = __ldg(tgt.kv_table + kv_last_page), code_page = __ldg(tgt.code_table + code_last_page);
-      float x[16];
-      unpack16<T>(k0, k1, x);
+      float2 x[8];
+      unpack_pairs<T>(k0, k1, x);
       if (ap.rope_on) {
-        rope_8lanes<T>(x, l8, sh.cs, scaled, ap.rp.mscale);
-        const float a[8] = {x[0], x[1], x[2], x[3], x[4], x[5], x[6], x[7]};
-        const float c[8] = {x[8], x[9], x[10], x[11], x[12], x[13], x[14], x[15]};
-        k0 = pack8<T>(a);
-        k1 = pack8<T>(c);
+        rope_pairs<T>(x, l8, sh.cs, scaled, ap.rp.mscale);
+        pack_pairs<T>(x, &k0, &k1);
         __syncwarp();   // (lanes without a row of their own have read the first one)
         if (live) {
           st_16(ksrc, k0);
-          st_16(ksrc + 8, k1);
+          st_16(ksrc + kHalf, k1);
         }
       }
-      const uint32_t w = code_word_8lanes<T>(x, l8, ap.scale, ap.th);
+      const uint32_t w = code_pairs<T>(x, l8, ap.scale, PairThresholds<T>(ap.th));
       if (live) {
-        T* dst = static_cast<T*>(tgt.kv_data) + ((kv_page * 2 * ps + kv_entry) * p.H + h) * kHeadDim + l8 * 16;
+        T* dst = static_cast<T*>(tgt.kv_data) + ((kv_page * 2 * ps + kv_entry) * p.H + h) * kHeadDim + l8 * 8;
         st_16(dst, k0);
-        st_16(dst + 8, k1);
+        st_16(dst + kHalf, k1);
         dst += static_cast<int64_t>(ps) * p.H * kHeadDim;
         st_16(dst, v0);
-        st_16(dst + 8, v1);
-        reinterpret_cast<uint32_t*>(tgt.code_data)[((code_page * ps + code_entry) * p.H + h) * (kCodeWords / 2) + l8] = w;
+        st_16(dst + kHalf, v1);
+        uint16_t* code = tgt.code_data + ((code_page * ps + code_entry) * p.H + h) * kCodeWords + l8;
+        code[0] = static_cast<uint16_t>(w);
+        code[8] = static_cast<uint16_t>(w >> 16);
       }
     }
 

@@ -166,6 +166,13 @@ struct PairThresholds {
   __device__ __forceinline__ explicit PairThresholds(const Thresholds& th)
       : t0(Elem<T>::floor2(th.t0)), t1(Elem<T>::floor2(th.t1)), t2(Elem<T>::floor2(th.t2)) {}
 };
+// How many thresholds each half of v is above, at bits `at` .. (low half) and 16 + 2 + `at` .. (high half).
+template <typename T>
+__device__ __forceinline__ uint32_t buckets2(uint32_t v, const PairThresholds<T>& th, int at) {
+  const uint32_t m0 = Elem<T>::above2(v, th.t0), m1 = Elem<T>::above2(v, th.t1), m2 = Elem<T>::above2(v, th.t2);
+  const uint32_t odd = m0 ^ m1 ^ m2, two = (m0 & m1) | (m0 & m2) | (m1 & m2);
+  return (odd & (0x00040001u << at)) | (two & (0x00080002u << at));
+}
 // Transform, scale, round, bucketize: code word l8 in the low half, word 8 + l8 in the high one.
 template <typename T>
 __device__ __forceinline__ uint32_t code_pairs(float2 (&x)[8], unsigned l8, float scale, const PairThresholds<T>& th) {
@@ -176,13 +183,8 @@ __device__ __forceinline__ uint32_t code_pairs(float2 (&x)[8], unsigned l8, floa
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {   // values 2j and 2j + 1: how many thresholds each is above, to bits 4j .. and 16 + 4j + 2 ..
-      const uint32_t v = h == 0 ? Elem<T>::from_f2(x[2 * j].x, x[2 * j + 1].x) : Elem<T>::from_f2(x[2 * j].y, x[2 * j + 1].y);
-      const uint32_t m0 = Elem<T>::above2(v, th.t0), m1 = Elem<T>::above2(v, th.t1), m2 = Elem<T>::above2(v, th.t2);
-      const uint32_t odd = m0 ^ m1 ^ m2, two = (m0 & m1) | (m0 & m2) | (m1 & m2);
-      w[h] |= odd & (0x00040001u << (4 * j));
-      w[h] |= two & (0x00080002u << (4 * j));
-    }
+    for (int j = 0; j < 4; ++j)
+      w[h] |= buckets2<T>(h == 0 ? Elem<T>::from_f2(x[2 * j].x, x[2 * j + 1].x) : Elem<T>::from_f2(x[2 * j].y, x[2 * j + 1].y), th, 4 * j);
     w[h] |= w[h] >> 16;
   }
   return __byte_perm(w[0], w[1], 0x5410);
