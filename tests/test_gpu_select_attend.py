@@ -211,3 +211,41 @@ def test_stale_histogram_table_is_reported_not_followed():
     assert _lib.device_error(clear=True) == 8
     want = st.v[n].float()          # softmax over one token
     _assert_attn_close(o[0], want)
+
+
+@pytest.mark.parametrize("distinct", [3, 40, 100000])
+@pytest.mark.parametrize("n,k,H", [(32768, 1023, 4), (30001, 1100, 3), (131072, 2047, 2), (100003, 1500, 1), (32768, 2560, 2), (32768, 2561, 2)])
+def test_step_with_first_slices_shared_by_one_block_more(n, k, H, distinct):
+    """The fused step with sixteen blocks per head and up to 2560 winners: three (or, long rows, two) blocks share each of the first slices of
+    the histograms.  Keys of a few kinds, so that ties fill the front of the row; the selection is that of the separate operators (ties to the
+    lower position) and the result that of attention over it."""
+    _, K, U = _mods()
+    g = torch.Generator(device=DEV).manual_seed(n + k)
+    kinds = torch.randn(distinct, H, 128, device=DEV, generator=g).half()
+    keys = kinds[torch.randint(0, distinct, (n + 1,), device=DEV, generator=g)]
+    values = torch.randn(n + 1, H, 128, device=DEV, generator=g).half()
+    q = torch.randn(1, H, 128, device=DEV, generator=g).half()
+    found = []
+    for fused in (True, False):
+        c = U.InferenceController(1, H, 128, 1, k + 1, n + 1, torch.float16, DEV)
+        c.prepare_hadamard(n)
+        c.begin_forward(n)
+        U.append_kvh(keys[:n], values[:n], None, c, 0)
+        c.end_forward()
+        c.prepare_hadamard(1)
+        c.begin_forward(1)
+        if fused:
+            out = U.decode_step(q.clone(), keys[n:], values[n:], c, 0)
+            assert int(K.histogram_counts(c.hist_scratch).abs().sum().item()) == 0
+        else:
+            U.decode_topk(U.decode_estimate(U.append_qkv_fused(q.clone(), keys[n:], values[n:], c, 0), c, 0), c)
+        sel = c.topk_dindices_buffer.cpu()
+        found.append(sel)
+        c.end_forward()
+    assert torch.equal(found[0], found[1])      # (page size 1: slots are positions here)
+    full = np.concatenate([found[0].numpy().astype(np.int64), np.full((H, 1), n, dtype=np.int64)], 1)
+    table = np.asarray(c.kv_cache.indicies)
+    where = np.empty(table.max() + 1, dtype=np.int64)
+    where[table] = np.arange(len(table))
+    full[:, :-1] = where[full[:, :-1]]
+    _assert_attn_close(out[0], ref.sparse_attention(q[0].cpu(), keys.cpu(), values.cpu(), full))
