@@ -1,4 +1,4 @@
-// A warp's attention over a tile of 16 (or 24) gathered K and V rows, on the tensor cores (mma.sync m16n8k16, fp32
+// A warp's attention over a tile of 16 (select+attend: up to 24) gathered K and V rows, on the tensor cores (mma.sync m16n8k16, fp32
 // accumulation): up to 8 query rows at once.  Used by the decode attention (all query heads of a cache head) and by
 // select+attend (one query row: q.K only).
 //
@@ -68,23 +68,23 @@ __device__ __forceinline__ int tile_swizzle(int r) { return (r & 6) ^ ((r & 1) <
 
 __device__ __forceinline__ uint32_t word_of(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// Requests a tile's K and / or V rows with 16-byte asynchronous copies: lane l holds the cache row of token l (of 16 tokens:
+// Requests a tile's K and V rows with 16-byte asynchronous copies: lane l holds the cache row of token l (of 16 tokens:
 // lanes l and l + 16), in units of row_elems elements behind kbase; its V row lies v_delta elements behind its K row.
-template <typename T, int ROWS, bool K, bool V>
+template <typename T>
 __device__ __forceinline__ void tile_copy(const T* kbase, int64_t v_delta, int64_t row_elems, int row, uint8_t* slot, int lane) {
   const int half = lane >> 4, c = lane & 15;
 #pragma unroll
-  for (int i = 0; i < ROWS / 2; ++i) {   // a half-warp per row
+  for (int i = 0; i < kTileRows / 2; ++i) {   // a half-warp per row
     const int rr = 2 * i + half;
     const T* src = kbase + __shfl_sync(0xffffffffu, row, rr) * row_elems + c * 8;
     uint8_t* dst = slot + rr * 256 + ((c ^ tile_swizzle(rr)) << 4);
-    if (K) cp_async_16(dst, src);
-    if (V) cp_async_16(dst + ROWS * 256, src + v_delta);
+    cp_async_16(dst, src);
+    cp_async_16(dst + kTileRows * 256, src + v_delta);
   }
 }
 
-// 8 rows of such a tile (kSaRows rows of one kind behind `slot`): lane l holds the cache row of token l, in units of row_bytes
-// behind `base`; FIRST: which 8.
+// 8 rows of one kind (select+attend): lane l holds the cache row of token l, in units of row_bytes
+// behind `base`; the copies go behind `slot`.  FIRST: which 8.
 template <int FIRST>
 __device__ __forceinline__ void tile_copy8(const uint8_t* base, uint32_t row_bytes, int row, uint8_t* slot, int lane) {
   const int half = lane >> 4, c = lane & 15;
@@ -96,11 +96,12 @@ __device__ __forceinline__ void tile_copy8(const uint8_t* base, uint32_t row_byt
   }
 }
 
-// Scaled logits of a tile of ROWS tokens: s[2u], s[2u + 1] are head g's for tokens 8u + 2t, 8u + 2t + 1; -inf for tokens
+// Scaled logits of a tile: s[2u], s[2u + 1] are head g's for tokens 8u + 2t, 8u + 2t + 1; -inf for tokens
 // outside `mask`.
-template <typename T, int ROWS>
+template <typename T>
 __device__ __forceinline__ void tile_logits(const uint8_t* slot, const uint4 (&q)[4], unsigned mask, float scale_log2, int lane,
-                                            float (&s)[ROWS / 4]) {
+                                            float (&s)[kTileRows / 4]) {
+  constexpr int ROWS = kTileRows;
   const int g = lane >> 2, t = lane & 3;
   float c[ROWS / 8][2][4] = {};   // (two accumulators per 8 rows: shorter chains)
   const uint8_t* krow = slot + g * 256;

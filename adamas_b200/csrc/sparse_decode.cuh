@@ -123,7 +123,7 @@ __device__ __forceinline__ unsigned dec_request(const DecodeParams& p, const Dec
   const unsigned mask = __ballot_sync(0xffffffffu, row >= 0) & 0xffffu;
   const int safe = __shfl_sync(0xffffffffu, row, mask ? __ffs(mask) - 1 : 0);
   row = max(row >= 0 ? row : safe, 0);
-  tile_copy<T, kDecTile, true, true>(kbase, p.page_size * row_elems, row_elems, row, slot, lane);
+  tile_copy<T>(kbase, p.page_size * row_elems, row_elems, row, slot, lane);
   return mask;
 }
 
@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(kDecThreads, kDecBlocksPerSm) paged_decode_ker
         __syncwarp();
         if (masks[0]) {
           float sc[4];
-          tile_logits<T, kDecTile>(ring + use * kDecTileBytes, q, masks[0], p.scale_log2, lane, sc);
+          tile_logits<T>(ring + use * kDecTileBytes, q, masks[0], p.scale_log2, lane, sc);
           tile_softmax_pv<T>(st, ring + use * kDecTileBytes, sc, lane);
         }
         __syncwarp();   // the slot may be filled again
