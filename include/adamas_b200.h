@@ -357,7 +357,7 @@ int adamas_append_estimate(const void* q, const void* k, const void* v, void* q_
                            adamas_stream_t stream);
 
 /* One layer's whole decode step in one call: two launches (the estimate with the append, and the rotary embedding if one is
- * asked for, inside, then select+attend; one more for batches of long rows whose counts are a launch of their own), or as
+ * asked for, inside, then select+attend), or as
  * adamas_set_fused_append chooses:
  * what adamas/models/Adamas.py:145-200 does with seven launches.  q, k, v, o [1,H,D]; q_code
  * [1,H,D/8] scratch/output; dist_scratch [H, dist_stride] 16-bit, rows on 16-byte boundaries,
