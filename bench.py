@@ -583,7 +583,7 @@ def run_ours(args):
         both = stage_time("select_attend", pre="estimate")
         stage_us["estimate_then_select_attend"] = both
         stage_us["select_attend"] = both - stage_us["estimate"]
-        by_tiles = args.heads in (16, 32, 64)
+        by_tiles = args.heads in (16, 32) and args.ctx <= 3584   # (short rows; about where the library's line lies)
         kernels = {first: "estimate_items_kernel" if not by_tiles else "estimate_append_kernel" if first == "append_estimate" else "estimate_kernel",
                    "select_attend": "select_attend_kernel"}
         if first == "estimate":
