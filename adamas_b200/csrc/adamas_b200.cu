@@ -1125,25 +1125,21 @@ int launch_select_attend(const SelectAttendParams& prm, int cl, int num_heads, i
 // Shape of a select_attend launch: blocks per head, histogram slices, and dynamic shared memory (the tiles | winner list |
 // page numbers).  Planned for rows of up to n distances; shorter rows run in the same shape.
 struct SaPlan {
-  int cl, slices, sharing, shared_more, tokens, list_capacity, staged_granules, pages_at;   // tokens: of a block at most
+  int cl, slices, sharing, tokens, list_capacity, staged_granules, pages_at;   // tokens: of a block at most
   size_t smem;
 };
 
 // For `cl` blocks per head: everything but the staged page numbers.
-void sa_shape(int n, int k, int cl, bool uneven, SaPlan* pl) {
+void sa_shape(int n, int k, int cl, SaPlan* pl) {
   pl->cl = cl;
   // Every block reads every histogram slice of its head, 2 KB each: with 16 blocks and slices of 32 heads 17 MB from L2, 1.8 us.
   // Two blocks share a slice where the second one can count what lies in front of it in a few instructions.
   const int sharing = pl->sharing = cl >= 8 && cl % 2 == 0 && sa_granules_per_block(n, cl / 2) <= 4 * kSaThreads ? 2 : 1;
-  // The distances that equal the cut are taken from the front of the row, and they are many (whole numbers, a few units of spread): with
-  // equal blocks the first two to four of sixteen had 1.6 to 2 times the winners of the others (32K tokens, budget 1024: 100, 98, 80, 68,
-  // then 57) and a round of gathers more.  The first slices are therefore shared by one block more.  us a layer: 32 heads, 32K 19.0 ->
-  // 18.3, 128K with budget 2048 42.4 -> 41.0, 20K with 2048 20.5 -> 20.1; not with many more winners, where the ties are few among them
-  // (60K with 4096 33.6 / 35.1), nor with fewer blocks, whose winners fit one round (3K with 256 10.3 / 10.7).
-  // (The stand-alone call keeps equal blocks: its callers count the histograms' slices by themselves.)
-  pl->shared_more = uneven && cl == kSaMaxSlices && k <= 10 * kSaWarps * kSaRows * 8 / 3 ? 4 : 0;
-  if (sa_granules_per_block(n, (cl - pl->shared_more) / sharing) * 8 > kSaMaxBlockTokens) pl->shared_more = 0;
-  pl->slices = (cl - pl->shared_more) / sharing;
+  // (Every block has the same part of the row.  One block more on each of the first slices, where the ties are taken, was 3 % faster for
+  // independent keys with many ties and 4 to 20 % slower for selections that lean to the end of the row, as recent tokens do.  us a layer, equal / one
+  // more, 32 heads: budget 1024 of 32K, all in the last quarter 22.0 / 23.4, in the last tenth 27.5 / 29.9; 2048 of 128K, in the last tenth 60.4 / 67.6;
+  // 2048 of 20K, in the last tenth 31.6 / 39.0.)
+  pl->slices = cl / sharing;
   const int granules = sa_granules_per_block(n, pl->slices);
   pl->tokens = std::min(n, (granules + sharing - 1) / sharing * 8);
   pl->list_capacity = std::min(k, pl->tokens) + 1;   // winners of one block at most, plus the newest token
@@ -1157,7 +1153,7 @@ int sa_resident(size_t smem, const DeviceInfo* di) {   // blocks per SM
 }
 
 // (page_size plays no part in the number of blocks and slices: adamas_select_attend_slices does not know it)
-int sa_plan(int n, int k, int num_heads, int page_size, const DeviceInfo* di, bool uneven, SaPlan* pl) {
+int sa_plan(int n, int k, int num_heads, int page_size, const DeviceInfo* di, SaPlan* pl) {
   // Blocks per head: any number up to 16 (the blocks of a head do not wait for one another).  num_heads counts the rows of
   // the launch (query heads x sequences).  A block's work is a chain of short dependent steps, so what counts is that
   // a block's winners fit the tiles of its warps, that a thread has a granule or two, and that the whole launch is
@@ -1172,7 +1168,7 @@ int sa_plan(int n, int k, int num_heads, int page_size, const DeviceInfo* di, bo
   int wanted = std::max((g_total + 2 * kSaThreads - 1) / (2 * kSaThreads), (k + winners - 1) / winners);
   if (wanted >= 8) wanted = (wanted + 1) & ~1;   // (two blocks then share a slice)
   for (int cl = std::min(std::max(wanted, least), cl_limit);; --cl) {
-    sa_shape(n, k, cl, uneven, pl);
+    sa_shape(n, k, cl, pl);
     if (cl == std::max(least, 1) || cl * num_heads <= sa_resident(pl->smem, di) * di->num_sms) break;
   }
   const int page_bytes = ((pl->tokens / page_size + 2) * 4 + 15) & ~15;
@@ -1222,14 +1218,7 @@ int select_attend_impl(const void* dist, int64_t dist_stride, int n, int k, cons
   prm.out_stride = out_stride;
   prm.list_capacity = pl.list_capacity;
   prm.slices = pl.slices;
-  for (int b = 0, sl = 0, part = 0; b < kSaMaxSlices; ++b) {
-    const int parts = pl.sharing + (sl < pl.shared_more ? 1 : 0);
-    prm.place[b] = static_cast<uint8_t>(sl << 4 | part << 2 | parts);
-    if (++part == parts) {
-      part = 0;
-      ++sl;
-    }
-  }
+  prm.share_shift = pl.sharing - 1;
   prm.staged_granules = pl.staged_granules;
   prm.pages_at = pl.pages_at;
   prm.bin_threads = dist_bins > 3 * kHeadDim ? kSaThreads : (3 * kHeadDim + 4) / 4;
@@ -1258,7 +1247,7 @@ int adamas_select_attend_slices(int n, int k, int num_heads, int* slices) {
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
   SaPlan pl;
-  if (int rc = sa_plan(n, k, num_heads, 16, di, false, &pl)) return rc;
+  if (int rc = sa_plan(n, k, num_heads, 16, di, &pl)) return rc;
   *slices = pl.slices;
   return ADAMAS_OK;
 }
@@ -1289,7 +1278,7 @@ int adamas_select_attend(const void* dist, int64_t dist_stride, int n, int k, co
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
   SaPlan pl;
-  if (int rc = sa_plan(n, k, num_heads, page_size, di, false, &pl)) return rc;
+  if (int rc = sa_plan(n, k, num_heads, page_size, di, &pl)) return rc;
   if (!hist_ready) {
     DistHistogramParams hp;
     hp.dist = static_cast<const uint16_t*>(dist);
@@ -1436,7 +1425,7 @@ static int decode_step_impl(void* q, void* k, const void* v, void* o, float* lse
   const DeviceInfo* di = nullptr;
   if (int rc = get_device_info(&di)) return rc;
   SaPlan pl;
-  if (int rc = sa_plan(n, budget - 1, q_heads * batch, page_size, di, true, &pl)) return rc;
+  if (int rc = sa_plan(n, budget - 1, q_heads * batch, page_size, di, &pl)) return rc;
   int rc;
   const bool two_launches = fused_append_enabled();
   if (two_launches) {

@@ -6,7 +6,7 @@
 // The kernel does not count anything itself.  The estimate kernels (or dist_histogram_kernel, for a
 // caller that only has a distance row) leave, per head, one 512-bin histogram per SLICE of the row
 // in a global table [H][kSaMaxSlices][512] u32: a slice covers the granules (8 distances) of one block of
-// the head, or of two or three neighbouring ones.  A distance is at most 3 * 128 = 384; larger values count as 511.
+// the head, or of two neighbouring ones.  A distance is at most 3 * 128 = 384; larger values count as 511.
 //
 // CL <= 16 blocks x 128 threads per head (grid (CL, H)); the blocks of a head never wait for one another.
 // Block `cr`:
@@ -94,7 +94,7 @@ struct SelectAttendParams {
   int32_t* out_idx;         // optional [H, out_stride]: physical slots of the winners, ascending position
   int64_t out_stride;
   int slices;               // histogram rows per head
-  uint8_t place[kSaMaxSlices];   // block -> slice << 4 | part << 2 | parts of the slice (1 to 3)
+  int share_shift;          // 0 or 1: 1 << share_shift blocks share one
   int staged_granules;      // granules of a slice staged in the tiles' memory
   int pages_at;             // where in shared memory the block's page numbers go; 0: they are not staged
   int bin_threads;          // threads that read histogram bins (four each): the bins that can be in use
@@ -173,15 +173,14 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
   if (tid == 0) sh.cut = 0xffffffffu;
   const int n = seq_len_dev ? (__ldg(seq_len_dev) - 1) : p.n;
   const int G = (n + 7) >> 3;
-  // slice of the histograms, and this block's part of it (up to three blocks share a slice; a block counts what lies in front of it in
-  // its slice by itself)
+  // slice of the histograms, and this block's part of it (one or two blocks share a slice; the second one counts what lies in front
+  // of it in the first part by itself)
   const int per_slice = sa_granules_per_block(n, p.slices);
-  const unsigned place = p.place[cr];
-  const int slice = place >> 4, part = (place >> 2) & 3u, parts = place & 3u;
-  const int per_part = parts == 1 ? per_slice : parts == 2 ? (per_slice + 1) >> 1 : static_cast<int>((per_slice + 2) * 43691u >> 17);   // (a third of less than 64K)
+  const int slice = cr >> p.share_shift, per_part = (per_slice + p.share_shift) >> p.share_shift;
+  const bool second = cr & p.share_shift;
   const int seg_first = slice * per_slice, seg_end = min(G, seg_first + per_slice);
-  const int pre = max(0, min(part * per_part, seg_end - seg_first));            // granules of the slice in front of this block's
-  const int blk_first = seg_first + pre, blk_count = max(0, min(per_part, seg_end - blk_first));
+  const int pre = second ? max(0, min(per_part, seg_end - seg_first)) : 0;      // granules of the slice in front of this block's
+  const int blk_first = seg_first + pre, blk_count = max(0, min(second ? per_slice - per_part : per_part, seg_end - blk_first));
   // the page numbers of the block's tokens, where they fit
   const unsigned ps = static_cast<unsigned>(p.page_size);
   auto page_of = [&](unsigned t) { return p.ps_shift >= 0 ? t >> p.ps_shift : t / ps; };
@@ -351,7 +350,7 @@ __global__ void __launch_bounds__(kSaThreads, kSaBlocksPerSm) select_attend_kern
     const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  if (parts > 1) ahead = __reduce_add_sync(0xffffffffu, ahead);
+  if (p.share_shift) ahead = __reduce_add_sync(0xffffffffu, ahead);
   if (lane == 31) sh.warp_sum[warp] = make_uint2(incl, ahead);   // (the readers of the cut phase are past a block barrier)
   if (p.rope_on) {   // (rope_halfwarp_cs, one element per thread)
     const float2 cs = sh.cs[tid & (kHeadDim / 2 - 1)];

@@ -215,10 +215,10 @@ def test_stale_histogram_table_is_reported_not_followed():
 
 @pytest.mark.parametrize("distinct", [3, 40, 100000])
 @pytest.mark.parametrize("n,k,H", [(32768, 1023, 4), (30001, 1100, 3), (131072, 2047, 2), (100003, 1500, 1), (32768, 2560, 2), (32768, 2561, 2)])
-def test_step_with_first_slices_shared_by_one_block_more(n, k, H, distinct):
-    """The fused step with sixteen blocks per head and up to 2560 winners: three (or, long rows, two) blocks share each of the first slices of
-    the histograms.  Keys of a few kinds, so that ties fill the front of the row; the selection is that of the separate operators (ties to the
-    lower position) and the result that of attention over it."""
+def test_step_with_ties_at_the_front(n, k, H, distinct):
+    """The fused step with sixteen blocks per head, two (or, long rows, one) to a slice of the histograms.  Keys of a few kinds, so that
+    ties fill the front of the row; the selection is that of the separate operators (ties to the lower position) and the result that of
+    attention over it."""
     _, K, U = _mods()
     g = torch.Generator(device=DEV).manual_seed(n + k)
     kinds = torch.randn(distinct, H, 128, device=DEV, generator=g).half()
@@ -249,3 +249,31 @@ def test_step_with_first_slices_shared_by_one_block_more(n, k, H, distinct):
     where[table] = np.arange(len(table))
     full[:, :-1] = where[full[:, :-1]]
     _assert_attn_close(out[0], ref.sparse_attention(q[0].cpu(), keys.cpu(), values.cpu(), full))
+
+
+@pytest.mark.parametrize("quarter", [0, 1, 2, 3])
+def test_step_gives_every_block_the_same_part_of_the_row(quarter):
+    """All winners in one quarter of the row, wherever it is: four of the sixteen blocks per head gather them.  (The slots of
+    partial results that hold a sum are those of blocks with rows of their own; the last block has the newest token as well.)"""
+    _, K, U = _mods()
+    n, k, H = 32768, 1023, 4
+    g = torch.Generator(device=DEV).manual_seed(quarter)
+    u = torch.randn(H, 128, device=DEV, generator=g)
+    keys = torch.randn(n + 1, H, 128, device=DEV, generator=g)
+    for h in range(H):
+        keys[quarter * n // 4 + torch.randperm(n // 4, device=DEV, generator=g)[:k], h] += 2.0 * u[h]
+    c = U.InferenceController(1, H, 128, 1, k + 1, n + 1, torch.float16, DEV)
+    c.prepare_hadamard(n)
+    c.begin_forward(n)
+    U.append_kvh(keys[:n].half(), torch.randn(n, H, 128, device=DEV, generator=g).half(), None, c, 0)
+    c.end_forward()
+    c.prepare_hadamard(1)
+    c.begin_forward(1)
+    U.decode_step(u.half()[None], keys[n:].half(), keys[n:].half(), c, 0)
+    slots = c.hist_scratch.view(H, -1)[:, 16 * 512:].view(H, 16, 132)
+    busy = (slots[:, :, 129] != 0).cpu()
+    want = torch.zeros(16, dtype=torch.bool)
+    want[4 * quarter:4 * quarter + 4] = True
+    want[15] = True
+    assert torch.equal(busy, want.expand(H, 16))
+    c.end_forward()
