@@ -538,25 +538,6 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
 }
 
 // ---------------------------------------------------------------------------------------------
-// Which estimate kernel.  n is the length, or the cache's capacity where the length is on the device.
-//
-// The tile pipeline takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of its heads in registers.  With
-// counts, one L2 atomic per distance in it, it is ahead only where a block of the item kernel has next to nothing to scan and its query
-// decides.  us a layer, tiles / items: without rotation 16 heads, 600 tokens 8.2 / 8.7, 1.5K 8.2 / 8.5, 4K 9.5 / 8.5, 2 x 1.5K 9.3 / 10.7, 4 x 1.5K 10.5 /
-// 11.3; 32 heads, 1.5K 8.5 / 8.7, 3K 9.0 / 9.2, 4K 9.9 / 9.7, 2 x 3K 11.5 / 11.9, 4 x 1.5K 13.3 / 12.8; with rotation 16 heads, 1.5K 9.0 / 8.7,
-// 2 x 1.5K 10.2 / 11.0, 4 x 1.5K 11.8 / 11.6; 32 heads, 1.5K 9.4 / 9.0, 3K 10.2 / 9.5; 64 heads, 1.5K 12.0 / 11.8.
-//
-// Without counts there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
-// 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
-static bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
-static bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope) {
-  if (!tile_heads(num_heads, q_heads)) return false;
-  const int64_t tokens = static_cast<int64_t>(batch) * n;
-  if (!counts) return num_heads != 16 || tokens < 65536;
-  if (rope) return num_heads == 16 && batch > 1 && tokens <= 4096;
-  return (num_heads == 16 || (num_heads == 32 && batch <= 2)) && n <= 3584 && tokens <= 7168;
-}
-
 // Launches the estimate.  n: distances per row, or their upper bound when seq_len_dev gives the length on the device
 // (it sizes the grid; each block derives its share from the device value).  num_heads: heads of the code cache; q_heads:
 // query rows per sequence (a multiple of num_heads).  ap.q set: with the append inside (dtype of q, k, v); else q_code is given.

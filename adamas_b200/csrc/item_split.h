@@ -1,5 +1,5 @@
-// How the work of the item estimate (estimate_items.cuh) is cut: what an item is, which of them a block takes.  Plain C++ but for
-// the qualifiers, so that the cuts can be checked without a GPU.
+// How the work of the item estimate (estimate_items.cuh) is cut: what an item is, which of them a block takes; and which launches go
+// to it (estimate_by_tiles).  Plain C++ but for the qualifiers, so that both can be checked without a GPU.
 //
 // An item is 128 / HP tokens (a tile) x HP cache heads; a piece is HP cache heads with a part of their query heads.  The items of
 // a launch form a line: sequence after sequence, in it piece after piece, in it tile after tile.  A segment is a piece of a sequence.
@@ -141,6 +141,32 @@ ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
   if (s >= batch || i >= nblk) return {0, 0};
   const int q = tiles / nblk, r = tiles - q * nblk;
   return {s * tiles + i * q + i * r / nblk, s * tiles + (i + 1) * q + (i + 1) * r / nblk};
+}
+
+// Which estimate kernel.  n is the length, or the cache's capacity where the length is on the device.
+//
+// The tile pipeline (estimate.cuh) takes 16, 32 and 64 heads without grouped queries, where a warp keeps the planes of its heads in registers.
+// With counts, one L2 atomic per distance in it, it is ahead only where a block of the item kernel has next to nothing to scan and its
+// query decides.  us a layer, tiles / items.  One sequence, without rotation: 16 heads, 600 tokens 8.2 / 8.7, 1.5K 8.2 / 8.7, 4K 9.5 / 8.5; 32 heads, 1.5K
+// 8.7 / 8.7, 3.6K 9.3 / 9.5, 4.5K 9.9 / 9.7; with it 16 heads, 1.5K 9.0 / 8.7; 32 heads, 1.5K 9.8 / 9.4.  Batches of 16 heads, without rotation 2 x 3.6K
+// 10.5 / 11.1, 4 x 1.8K 10.9 / 11.4, 5 x 1.5K 11.8 / 11.6, 6 x 1K 11.3 / 11.8, 8 x 1K 12.4 / 11.8; with it 2 x 2.3K 10.8 / 11.4, 2 x 2.7K 11.8 / 11.4, 4 x 1K
+// 11.3 / 11.9, 4 x 1.5K 12.3 / 11.9, 8 x 450 12.1 / 12.3, 8 x 600 12.7 / 12.5.  Batches of 32 heads, where another sequence costs the tiles more, without
+// rotation 2 x 3.6K 11.9 / 11.9, 3 x 1.5K 11.3 / 11.8, 3 x 2.5K 12.8 / 12.3, 4 x 1K 11.4 / 11.8, 4 x 1.5K 12.4 / 12.3, 6 x 450 11.8 / 12.3, 6 x 1K 13.8 / 12.8, 8 x 300
+// 13.0 / 12.8, 10 x 200 13.4 / 14.2; with it 2 x 600 10.3 / 11.8, 2 x 1.25K 10.7 / 11.9, 2 x 1.8K 12.0 / 11.9, 3 x 450 10.8 / 12.3, 3 x 600 12.3 / 12.3, 5 x 200 12.8 /
+// 12.4.  64 heads: one sequence, 1.5K 10.6 / 9.5; batches without rotation 2 x 300 11.3 / 11.8, 4 x 200 12.4 / 12.8, 4 x 600 13.3 / 13.2, 4 x 1.5K 15.9 / 15.3;
+// with it 2 x 300 12.8 / 12.3.
+//
+// Without counts there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
+// 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
+inline bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
+inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope) {
+  if (!tile_heads(num_heads, q_heads)) return false;
+  const long long tokens = static_cast<long long>(batch) * n;
+  if (!counts) return num_heads != 16 || tokens < 65536;
+  if (n > 3584 || (rope && batch == 1)) return false;
+  if (num_heads == 16) return tokens <= (rope ? 4608 : 7424);
+  if (num_heads == 32) return batch * tokens <= (rope ? 5120 : 20736);
+  return !rope && batch > 1 && tokens <= 1024;
 }
 
 }  // namespace adamas

@@ -218,12 +218,12 @@ def test_large_launches_count_their_histograms_in_shared_memory():
     ([2000 + 7 * i for i in range(64)], 28, 4, 256),    # as many pieces as a launch has blocks, kept apart
     ([3000 + 50 * i for i in range(20)], 40, 40, 256),  # ... and cut evenly
     ([700 + 3 * i for i in range(40)], 7, 7, 128),      # few tokens a block
-    # 16, 32 and 64 heads: batches with many distances leave the tile pipeline
+    # 16, 32 and 64 heads: longer than the batches of the tile pipeline
     ([8000, 4001, 8192, 7777, 6500, 5003, 8100, 4097, 7000, 6001, 8003, 5555, 7321], 32, 32, 128),
     ([9000, 4501, 8999, 9001, 700, 8500, 7001, 9500], 16, 16, 256),
     ([13001, 12000, 6501, 13100], 64, 64, 256),
     ([25100, 24701], 64, 64, 512),
-    ([24700, 24601, 24000, 23001, 24699, 24688, 12000, 24100], 32, 32, 256),   # long rows, two segments a block: the tiles and a counting launch
+    ([24700, 24601, 24000, 23001, 24699, 24688, 12000, 24100], 32, 32, 256),   # long rows, two segments a block
 ])
 def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
     """A batch whose distances are counted in shared memory: the same selection as each sequence by itself, and a table
@@ -255,4 +255,40 @@ def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
         want = U.decode_step(q[i:i + 1].clone(), k[i:i + 1].clone(), v[i:i + 1], c, 0, rope=rope)
         assert torch.equal(idx[i * Hq:(i + 1) * Hq], c.topk_dindices_buffer), f"sequence {i}"
         _assert_attn_close(o[i], want[0])
+        c.end_forward()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("H,rope,lengths,cap", [
+    (16, None, [1857, 300, 1500, 70], 1857), (16, None, [1858, 300, 1500, 70], 1858),        # the last tokens of the tile pipeline, one more
+    (16, (8.0, 1e4), [700, 300, 1537], 1537), (16, (8.0, 1e4), [700, 300, 1538], 1538),
+    (32, None, [2305, 2000, 100], 2305), (32, None, [2306, 2000, 100], 2306),
+    (32, (8.0, 1e4), [1281, 65], 1281), (32, (8.0, 1e4), [1282, 65], 1282),
+    (64, None, [257, 200, 100, 65], 257), (64, None, [258, 200, 100, 65], 258),
+])
+def test_batches_on_both_sides_of_the_kernels_line(H, rope, lengths, cap, dtype):
+    """The fused step of a short batch in the tile pipeline and in the item kernel: rotated rows, cache rows, codes and selection of every
+    sequence are those of the separate operators, and the histogram table is zero afterwards."""
+    _, K, U = _mods()
+    B, budget, ps = len(lengths), 64, 1     # (page size 1: the capacity is exact)
+    both = [_controllers(lengths, H, H, ps, budget, dtype, cap, seed=cap)[0] for _ in range(2)]
+    q, k, v = (_randn((B, H, 128), 5 + i, dtype).to(DEV) for i in range(3))
+    batch = U.SequenceBatch(both[0])
+    batch.prepare(1)
+    batch.sync_seq_lens()
+    idx = torch.full((B * H, budget - 1), -1, dtype=torch.int32, device=DEV)
+    qb, kb = q.clone(), k.clone()
+    o = batch.decode_step_dev(qb, kb, v, 0, indices_out=idx, rope=rope)
+    assert int(K.histogram_counts(batch._hist).abs().sum()) == 0
+    for i, (c, mine) in enumerate(zip(both[1], both[0])):
+        c.prepare_hadamard(1)
+        c.begin_forward(1)
+        qi, ki = q[i:i + 1].clone(), k[i:i + 1].clone()
+        U.decode_topk(U.decode_estimate(U.append_qkv_fused(qi, ki, v[i:i + 1], c, 0, rope=rope), c, 0), c)
+        assert torch.equal(idx[i * H:(i + 1) * H].sort(1).values, c.topk_dindices_buffer.sort(1).values), f"sequence {i}"
+        assert torch.equal(qb[i].view(torch.int16), qi[0].view(torch.int16)) and torch.equal(kb[i].view(torch.int16), ki[0].view(torch.int16))
+        for a, b in ((mine.kv_cache, c.kv_cache), (mine.hadamard_cache, c.hadamard_cache)):
+            assert a.indicies == b.indicies
+            assert torch.equal(a.buf_layer(0).view(torch.int16)[a.indicies], b.buf_layer(0).view(torch.int16)[b.indicies])
+        _assert_attn_close(o[i], U.decode_sparse_attn(qi, c, 0, c.topk_dindices_buffer)[0])
         c.end_forward()

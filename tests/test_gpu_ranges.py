@@ -115,19 +115,42 @@ def test_estimate_items_shapes(H, Hq, L, ps):
             assert torch.equal(counts[r, sl].to(torch.int64), torch.bincount(want[r, sl * per:(sl + 1) * per], minlength=512))
 
 
-@pytest.mark.parametrize("H,L", [(16, 65536), (16, 65537), (32, 49152), (32, 49153), (64, 24576), (64, 24577)])
+@pytest.mark.parametrize("H,L", [(16, 3585), (16, 3586), (32, 3585), (32, 3586), (64, 1500), (16, 65537), (32, 49153), (64, 24577)])
 def test_estimate_on_both_sides_of_the_kernels_line(H, L):
-    """16, 32 and 64 heads: the last length of the tile pipeline and the first one of the item kernel; exact."""
+    """16 and 32 heads with counts: the last length of the tile pipeline (3584 tokens in front of the newest) and the first one of the item
+    kernel; 64 heads and long rows, all in the item kernel; exact."""
     test_estimate_items_shapes(H, H, L, 16)
 
 
-@pytest.mark.parametrize("H,L,dtype", [(16, 65536, torch.float16), (16, 65537, torch.bfloat16), (32, 49152, torch.float16), (32, 49153, torch.bfloat16),
-                                       (64, 24576, torch.float16), (64, 24577, torch.float16), (151, 6000, torch.float16)])
-def test_step_on_both_sides_of_the_kernels_line(H, L, dtype):
-    """The fused step (append, rotation and counts inside the estimate) selects what the separate operators do, at the last length of the
-    tile pipeline and the first one of the item kernel; 151 heads: more pieces than half of the blocks."""
+@pytest.mark.parametrize("H,n", [(16, 65535), (16, 65536), (32, 65536), (64, 30000)])
+def test_estimate_without_counts_on_both_sides_of_the_kernels_line(H, n):
+    """16 heads without counts: the last length of the tile pipeline and the first one of the item kernel; 32 and 64: the tile pipeline.
+    The distances are those of the same call with counts."""
+    _, K, _ = _mods()
+    ps = 16
+    pages = n // ps + 1
+    g = torch.Generator(device=DEV).manual_seed(n)
+    codes = torch.randint(-32768, 32768, (pages, 1, ps, H, 16), generator=g, device=DEV).to(torch.int16)
+    q = torch.randint(-32768, 32768, (1, H, 16), generator=g, device=DEV).to(torch.int16)
+    table = torch.randperm(pages, generator=g, device=DEV).to(torch.int32)
+    stores = [torch.zeros(H, (n + 7) // 8 * 8, dtype=torch.int16, device=DEV) for _ in range(2)]
+    last = n + 1 - (pages - 1) * ps
+    K.estimate_attn_score(q, stores[0][:, :n], codes, table, None, last, 0, 0)
+    K.estimate_attn_score(q, stores[1][:, :n], codes, table, None, last, 0, 0, hist=K.histogram_scratch(H, DEV), hist_slices=8)
+    assert torch.equal(stores[0], stores[1]) and int(stores[0].max()) > 0
+
+
+@pytest.mark.parametrize("H,L,rope,dtype", [
+    (16, 3584, None, torch.float16), (16, 3585, None, torch.float16), (32, 3584, None, torch.bfloat16), (32, 3585, None, torch.bfloat16),
+    (16, 65536, (8.0, 1e4), torch.float16), (16, 65537, (8.0, 1e4), torch.bfloat16), (32, 49152, (8.0, 1e4), torch.float16),
+    (32, 49153, (8.0, 1e4), torch.bfloat16), (64, 24576, (8.0, 1e4), torch.float16), (64, 24577, (8.0, 1e4), torch.float16),
+    (16, 600, (8.0, 1e4), torch.bfloat16), (32, 600, (8.0, 1e4), torch.float16), (151, 6000, (8.0, 1e4), torch.float16)])
+def test_step_on_both_sides_of_the_kernels_line(H, L, rope, dtype):
+    """The fused step (append, rotation and counts inside the estimate) selects what the separate operators do, without rotation at the
+    last length of the tile pipeline and the first one of the item kernel, with it at short and long rows of the item kernel; 151 heads: more
+    pieces than half of the blocks."""
     _, K, U = _mods()
-    budget, ps, rope = 256, 16, (8.0, 1e4)
+    budget, ps = 256, 16
     gen = torch.Generator(device=DEV).manual_seed(L)
     rand = lambda n: torch.randn(n, H, 128, device=DEV, generator=gen).to(dtype)
     k, v = rand(L), rand(L)

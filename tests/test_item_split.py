@@ -21,6 +21,7 @@ int cache_heads(int h, int group) { return item_cache_heads(h, group); }
 int query_heads(int items, int group, int warps) { return item_query_heads(items, group, warps); }
 int tiles_of(int n, int t) { return est_tiles(n, t); }
 int per_piece(int tiles, int pieces, int blocks) { return item_blocks_per_piece(tiles, pieces, 1, blocks); }
+int by_tiles(int heads, int q_heads, int batch, int n, int counts, int rope) { return estimate_by_tiles(heads, q_heads, batch, n, counts, rope); }
 void share_one(int tiles, int pieces, int q_part, int blocks, int* out) {
   for (int b = 0; b < blocks; ++b) {
     const ItemShare w = item_share_one(tiles, pieces, q_part, blocks, b);
@@ -220,3 +221,28 @@ def test_columns_of_a_batch_every_item_once(split, heads, group, blocks):
                     assert np.searchsorted(cum[1:], a, "right") == np.searchsorted(cum[1:], b - 1, "right")
         if mode == 1:
             assert sizes.max() - sizes[sizes > 0].min() <= 1
+
+
+@pytest.mark.parametrize("heads,batch,n,rope,want", [
+    # both sides of every line, with counts
+    (16, 1, 3584, False, True), (16, 1, 3585, False, False), (16, 1, 600, True, False), (16, 4, 1856, False, True), (16, 4, 1857, False, False),
+    (16, 3, 1536, True, True), (16, 3, 1537, True, False), (32, 1, 3584, False, True), (32, 1, 3585, False, False), (32, 1, 600, True, False),
+    (32, 2, 3584, False, True), (32, 3, 2304, False, True), (32, 3, 2305, False, False), (32, 2, 1280, True, True), (32, 2, 1281, True, False),
+    (64, 1, 600, False, False), (64, 4, 256, False, True), (64, 4, 257, False, False), (64, 2, 300, True, False),
+    # short batches that were slower in the item kernel by 4 to 15 % (us a layer beside estimate_by_tiles)
+    (32, 2, 600, True, True), (32, 2, 1000, True, True), (32, 2, 1250, True, True), (32, 3, 300, True, True), (32, 3, 450, True, True),
+    (32, 3, 300, False, True), (32, 3, 1500, False, True), (32, 4, 600, False, True), (32, 5, 600, False, True), (32, 6, 450, False, True),
+    (32, 10, 207, False, True), (16, 3, 1500, True, True), (16, 4, 1800, False, True), (64, 2, 200, False, True),
+    # ... and ones that are not
+    (32, 6, 1000, False, False), (32, 4, 1500, False, False), (32, 5, 300, True, False), (16, 8, 1000, False, False), (16, 8, 600, True, False),
+    (32, 1024, 3000, False, False), (16, 1024, 2000000, True, False),
+])
+def test_which_kernel_counts(split, heads, batch, n, rope, want):
+    assert bool(split.by_tiles(heads, heads, batch, n, 1, rope)) is want
+    for h, q in ((heads // 2, heads), (40, 40), (4, 4)):     # grouped queries and other head counts: the item kernel
+        assert not split.by_tiles(h, q, batch, n, 1, rope)
+
+
+@pytest.mark.parametrize("heads,n,want", [(16, 65535, True), (16, 65536, False), (32, 1000000, True), (64, 1000000, True), (8, 100, False)])
+def test_which_kernel_without_counts(split, heads, n, want):
+    assert bool(split.by_tiles(heads, heads, 1, n, 0, 0)) is want
