@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(kEstThreads) estimate_kernel(const EstimatePar
 // through shared memory.
 template <typename T, int HPW, bool ROPE>
 __global__ void __launch_bounds__(kEstThreads) estimate_append_kernel(const EstimateParams p) {
-  static_assert(HPW == 1 || HPW == 2 || HPW == 4, "heads per warp");
+  static_assert(HPW == 1 || HPW == 2 || (HPW == 4 && !ROPE), "heads per warp");
   extern __shared__ uint4 est_smem[];
   __shared__ __align__(8) uint64_t full_bar[kEstStages];
   __shared__ __align__(8) uint64_t empty_bar[kEstStages];

@@ -1,5 +1,5 @@
-// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes the short rows of 16 and
-// 32 heads and estimates without counts, is in estimate.cuh, with the parameters and the distance arithmetic.
+// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes short rows of 16 and 32
+// heads, short batches of 64 and estimates without counts (estimate_by_tiles), is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (logic at half rate and 5 population counts at an eighth, code_distance) for grouped
 // queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the
@@ -340,10 +340,10 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
       const uint32_t c0 = __byte_perm(w, next, 0x5410), c1 = __byte_perm(w, next, 0x7632);
       const uint32_t d0 = __shfl_down_sync(0xffffffffu, c0, 2), d1 = __shfl_down_sync(0xffffffffu, c1, 2);
       if (row < HP) {
-        if (first == 0 && !(l8 & 1)) {
-          uint32_t* dst = reinterpret_cast<uint32_t*>(p.ap.q_code_out) + code_row * (kCodeWords / 2) + (l8 >> 1);
-          dst[0] = c0;
-          dst[4] = c1;
+        if (first == 0) {   // (the codes may start on any 16-bit word)
+          uint16_t* dst = p.ap.q_code_out + code_row * kCodeWords + l8;
+          dst[0] = static_cast<uint16_t>(w);
+          dst[8] = static_cast<uint16_t>(w >> 16);
         }
         if (!(l8 & 3)) {
           const uint32_t hi0 = plane_hi(c0, d0), lo0 = plane_lo(c0, d0), hi1 = plane_hi(c1, d1), lo1 = plane_lo(c1, d1);

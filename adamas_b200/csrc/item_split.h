@@ -160,13 +160,13 @@ ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
 // 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
 inline bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
 inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope) {
-  if (!tile_heads(num_heads, q_heads)) return false;
+  if (!tile_heads(num_heads, q_heads) || (num_heads == 64 && rope)) return false;
   const long long tokens = static_cast<long long>(batch) * n;
   if (!counts) return num_heads != 16 || tokens < 65536;
   if (n > 3584 || (rope && batch == 1)) return false;
   if (num_heads == 16) return tokens <= (rope ? 4608 : 7424);
   if (num_heads == 32) return batch * tokens <= (rope ? 5120 : 20736);
-  return !rope && batch > 1 && tokens <= 1024;
+  return batch > 1 && tokens <= 1024;
 }
 
 }  // namespace adamas

@@ -275,9 +275,9 @@ def test_append_estimate_tiles(H, L):
         assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("H,L", [(16, 70001), (32, 50001), (64, 26001), (32, 20001)])
+@pytest.mark.parametrize("H,L", [(16, 70001), (32, 50001), (64, 26001), (32, 20001), (16, 3000), (32, 3000), (64, 700)])
 def test_query_codes_on_any_16_bit_word(H, L):
-    """Estimate with the append inside for 16, 32 and 64 heads, at lengths of the item kernel and (the last one) of the tiles: the
+    """Estimate with the append inside for 16, 32 and 64 heads, at lengths of the item kernel and (3000 tokens) of the tiles: the
     query codes may start on any 16-bit word."""
     _, K, _ = _mods()
     ps, n = 16, L - 1
@@ -300,6 +300,71 @@ def test_query_codes_on_any_16_bit_word(H, L):
     for other in results[1:]:
         for a, b in zip(results[0], other):
             assert torch.equal(a, b)
+
+
+def _kernels_of(run):
+    """Names of this library's kernels that `run` launches, and how often."""
+    from collections import Counter
+    from torch.profiler import ProfilerActivity, profile
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        run()
+        torch.cuda.synchronize()
+    names = Counter(e.name for e in p.events() if "adamas::" in e.name)
+    assert names, "the profiler saw no kernel"
+    return names
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("H,lengths,rope", [(32, [9000, 8000, 8999], None), (64, [3000, 2000], (8.0, 1e4)), (16, [900, 700, 300], (8.0, 1e4)), (32, [500, 300], (8.0, 1e4)),
+                                            (32, [700, 300], None)])
+def test_step_with_query_codes_on_any_16_bit_word(H, lengths, rope, dtype):
+    """A batch whose query codes start on any 16-bit word: the same kernels as with aligned ones, and the same bits."""
+    _, K, U = _mods()
+    B, budget, ps = len(lengths), 64, 16
+    gen = torch.Generator(device=DEV).manual_seed(H)
+    rand = lambda *shape: torch.randn(*shape, device=DEV, generator=gen).to(dtype)
+    cs = [U.InferenceController(1, H, 128, ps, budget // ps, max(lengths) + 16, dtype, DEV) for _ in lengths]
+    for c, L in zip(cs, lengths):
+        c.prepare_hadamard(L - 1)
+        c.begin_forward(L - 1)
+        U.append_kvh(rand(L - 1, H, 128), rand(L - 1, H, 128), None, c, 0)
+        c.end_forward()
+    batch = U.SequenceBatch(cs)
+    batch.prepare(1)
+    batch.sync_seq_lens()
+    q, k, v = rand(B, H, 128), rand(B, H, 128), rand(B, H, 128)
+    found = []
+    for off in (0, 1, 2, 8):
+        store = torch.zeros(B * H * 16 + 16, dtype=dtype, device=DEV)
+        batch._q_code = store[off:off + B * H * 16].view(B, H, 16)
+        idx = torch.full((B * H, budget - 1), -1, dtype=torch.int32, device=DEV)
+        qd, kd, o = q.clone(), k.clone(), torch.zeros_like(q)
+        names = _kernels_of(lambda: batch.decode_step_dev(qd, kd, v, 0, out=o, rope=rope, indices_out=idx))
+        words = store.view(torch.int16)
+        assert int(words[:off].abs().sum()) == 0 and int(words[off + B * H * 16:].abs().sum()) == 0
+        found.append((names, batch._q_code.view(torch.int16).clone(), qd, kd, o, idx))
+    for other in found[1:]:
+        assert other[0] == found[0][0]
+        for a, b in zip(found[0][1:], other[1:]):
+            assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H", [4, 40])
+def test_query_codes_of_other_heads_start_on_16_bytes(H):
+    """Other head counts refuse a query code that is not 16-byte aligned; the caches and the distances stay as they are."""
+    _, K, _ = _mods()
+    ps, L = 16, 200
+    pages = (L + ps - 1) // ps
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)
+    q, k, v = (_randn((1, H, 128), s, torch.float16).to(DEV) for s in (1, 2, 3))
+    codes = torch.zeros(pages, 1, ps, H, 16, dtype=torch.int16, device=DEV)
+    kv = torch.zeros(pages, 2, ps, H, 128, dtype=torch.float16, device=DEV)
+    dist = torch.zeros(H, 200, dtype=torch.int16, device=DEV)
+    store = torch.zeros(H * 16 + 8, dtype=torch.int16, device=DEV)
+    with pytest.raises(Exception, match="16-byte aligned"):
+        K.append_estimate(q, k, v, store[1:1 + H * 16].view(1, H, 16), kv, table, L - (pages - 1) * ps, codes, table, L - (pages - 1) * ps, dist[:, :L - 1], scale=1.0)
+    assert not any(bool(t.any()) for t in (kv, codes, dist, store))
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])

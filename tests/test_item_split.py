@@ -246,3 +246,4 @@ def test_which_kernel_counts(split, heads, batch, n, rope, want):
 @pytest.mark.parametrize("heads,n,want", [(16, 65535, True), (16, 65536, False), (32, 1000000, True), (64, 1000000, True), (8, 100, False)])
 def test_which_kernel_without_counts(split, heads, n, want):
     assert bool(split.by_tiles(heads, heads, 1, n, 0, 0)) is want
+    assert not split.by_tiles(64, 64, 1, n, 0, 1)      # (the tile pipeline has no rotation for 64 heads)
