@@ -157,10 +157,10 @@ __global__ void __launch_bounds__(kItemThreads, kItemBlocksPerSm) estimate_items
     ItemShare work;
     const int columns = p.seqs ? item_blocks_per_piece(tiles_all, pieces, q_part, gridDim.x) : 0;
     if (columns > 0) {
-      const int column = blockIdx.x / pieces, alike = item_columns_alike(cum, p.batch, columns);
+      const int column = blockIdx.x / pieces, alike = item_columns_alike(tiles_all, cum[p.batch + 1], p.batch, columns);
       column_piece = blockIdx.x - column * pieces;
       if (column >= columns) work = ItemShare{0, 0};
-      else if (alike > 0) work = item_share_alike(cum[1], p.batch, alike, column);
+      else if (alike > 0) work = item_share_alike(cum[p.batch + 1], p.batch, alike, column);
       else if (item_columns_apart(tiles_all, cum[p.batch + 1], p.batch, q_part, columns))
         work = item_share_apart(cum, p.batch, 1, columns, column);
       else work = item_share_even(tiles_all, columns, column);

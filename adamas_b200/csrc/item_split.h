@@ -131,9 +131,9 @@ ADAMAS_HD bool item_columns_apart(int total, int longest, int batch, int q_part,
   const int spare = columns - batch, most = static_cast<long long>(longest) * spare <= total ? longest : total / spare + 1;
   return (most - total / columns) * q_part <= (q_part > 1 ? kItemApart : kItemApartPlain);
 }
-// Equal lengths (cum[1] of them tiles each): `per` columns a sequence, or 0.
-ADAMAS_HD int item_columns_alike(const int* cum, int batch, int columns) {
-  if (batch > columns || static_cast<long long>(cum[1]) * batch != cum[batch] || columns % batch > columns / 7) return 0;
+// Equal lengths (the longest is the average): `per` columns a sequence, or 0.
+ADAMAS_HD int item_columns_alike(int total, int longest, int batch, int columns) {
+  if (batch > columns || static_cast<long long>(longest) * batch != total || columns % batch > columns / 7) return 0;
   return columns / batch;
 }
 ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {

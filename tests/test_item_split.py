@@ -47,12 +47,12 @@ int share_columns(const int* cum, int batch, int pieces, int q_part, int blocks,
   const int columns = item_blocks_per_piece(cum[batch], pieces, q_part, blocks);
   int longest = 0;
   for (int s = 0; s < batch; ++s) longest = std::max(longest, cum[s + 1] - cum[s]);
-  const int alike = columns > 0 ? item_columns_alike(cum, batch, columns) : 0;
+  const int alike = columns > 0 ? item_columns_alike(cum[batch], longest, batch, columns) : 0;
   const bool apart = columns > 0 && item_columns_apart(cum[batch], longest, batch, q_part, columns);
   for (int b = 0; b < blocks && columns > 0; ++b) {
     const int c = b / pieces;
     ItemShare w{0, 0};
-    if (c < columns) w = alike > 0 ? item_share_alike(cum[1], batch, alike, c) : apart ? item_share_apart(cum, batch, 1, columns, c) : item_share_even(cum[batch], columns, c);
+    if (c < columns) w = alike > 0 ? item_share_alike(longest, batch, alike, c) : apart ? item_share_apart(cum, batch, 1, columns, c) : item_share_even(cum[batch], columns, c);
     out[2 * b] = w.pos; out[2 * b + 1] = w.end;
   }
   return columns == 0 ? 0 : alike > 0 ? 1 : apart ? 2 : 3;
@@ -198,16 +198,20 @@ def test_columns_of_a_batch_every_item_once(split, heads, group, blocks):
         top = rng.choice([1, 40, 700, 5000, 60000])
         hp = split.cache_heads(heads, group)
         alike = case % 4 == 0
+        average_first = case % 4 == 1 and batch > 2      # (an average length in front does not make the others equal)
         lengths = [top] * batch if alike else [rng.randrange(0, top + 1) for _ in range(batch)]
         tiles = [0 if not alike and rng.random() < 0.1 else split.tiles_of(n, 128 // hp) for n in lengths]
         if sum(tiles) == 0:
             tiles[-1] = 1
+        if average_first:
+            tiles = [100] + [100 + (40 if i % 2 else -40) for i in range(batch - 2 + batch % 2)] + [100] * (1 - batch % 2)
         q_part = split.query_heads(sum(tiles) * (heads // hp), group, WARPS * blocks)
         pieces = heads // hp * -(-group // q_part)
         grid = min(blocks, sum(tiles) * pieces)
         cum = np.concatenate([[0], np.cumsum(tiles)]).astype(np.int32)
         out = np.full((grid, 2), -1, dtype=np.int32)
         mode = split.share_columns(cum.ctypes.data_as(ctypes.c_void_p), batch, pieces, q_part, grid, out.ctypes.data_as(ctypes.c_void_p))
+        assert mode != 1 or len(set(tiles)) == 1
         if mode == 0:
             continue
         columns = split.per_piece(int(cum[-1]), pieces, grid) if q_part == 1 else None
