@@ -125,14 +125,12 @@ int get_device_info(const DeviceInfo** out) {
   EST_ATTR(estimate_kernel<1, __half, HPW>);                    \
   EST_ATTR(estimate_kernel<1, uint16_t, HPW>);                  \
   EST_ATTR(estimate_append_kernel<__half, HPW, false>);         \
-  EST_ATTR(estimate_append_kernel<__nv_bfloat16, HPW, false>)
+  EST_ATTR(estimate_append_kernel<__half, HPW, true>);          \
+  EST_ATTR(estimate_append_kernel<__nv_bfloat16, HPW, false>);  \
+  EST_ATTR(estimate_append_kernel<__nv_bfloat16, HPW, true>)
     EST_ATTR_HPW(1);
     EST_ATTR_HPW(2);
     EST_ATTR_HPW(4);
-    EST_ATTR(estimate_append_kernel<__half, 1, true>);
-    EST_ATTR(estimate_append_kernel<__nv_bfloat16, 1, true>);
-    EST_ATTR(estimate_append_kernel<__half, 2, true>);
-    EST_ATTR(estimate_append_kernel<__nv_bfloat16, 2, true>);
 #undef EST_ATTR_HPW
 #define EST_ATTR_HP(HP, G)                                  \
   EST_ATTR(estimate_items_kernel<__half, 0, HP, G>);        \
@@ -583,7 +581,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   // (with 16, 32 and 64 heads query codes may start on any 16-bit word, in both kernels)
   const int code_align = tile_heads(num_heads, q_heads) ? 2 : 16;
   ADAMAS_REQUIRE(reinterpret_cast<uintptr_t>(ap.q_code_out) % code_align == 0, "q_code must be %d-byte aligned", code_align);
-  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, ap.rope_on != 0)) {
+  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, ap.rope_on != 0, est_blocks_per_sm() * di->num_sms)) {
     const int num_tiles = (n + kEstTile - 1) / kEstTile;
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);
@@ -591,15 +589,16 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
     // (a batch: one block per sequence at least; with an append, one per sequence that has nothing else to do where there is room)
     const dim3 grid(static_cast<unsigned>(std::max<int64_t>(batch, std::min<int64_t>(static_cast<int64_t>(num_tiles + (ap.q ? 1 : 0)) * batch, di->num_sms * per_sm))));
 #define LAUNCH_EST(...) ADAMAS_LAUNCH("estimate_kernel", (__VA_ARGS__), grid, dim3(kEstThreads), smem, st, 1, prm)
-#define LAUNCH_EST_APPEND(HPW, ROPE)                                                            \
-  do {                                                                                          \
-    if (dtype == ADAMAS_F16) LAUNCH_EST(estimate_append_kernel<__half, HPW, ROPE>);             \
-    else LAUNCH_EST(estimate_append_kernel<__nv_bfloat16, HPW, ROPE>);                          \
-  } while (0)
 #define LAUNCH_EST_HPW(HPW)                                                                     \
   do {                                                                                          \
     if (ap.q) {                                                                                 \
-      LAUNCH_EST_APPEND(HPW, false);                                                            \
+      if (dtype == ADAMAS_F16) {                                                                \
+        if (ap.rope_on) LAUNCH_EST(estimate_append_kernel<__half, HPW, true>);                  \
+        else LAUNCH_EST(estimate_append_kernel<__half, HPW, false>);                            \
+      } else {                                                                                  \
+        if (ap.rope_on) LAUNCH_EST(estimate_append_kernel<__nv_bfloat16, HPW, true>);           \
+        else LAUNCH_EST(estimate_append_kernel<__nv_bfloat16, HPW, false>);                     \
+      }                                                                                         \
     } else if (metric == ADAMAS_METRIC_L1) {                                                    \
       if (prm.out_half) LAUNCH_EST(estimate_kernel<0, __half, HPW>);                            \
       else LAUNCH_EST(estimate_kernel<0, uint16_t, HPW>);                                       \
@@ -608,16 +607,10 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
       else LAUNCH_EST(estimate_kernel<1, uint16_t, HPW>);                                       \
     }                                                                                           \
   } while (0)
-    if (ap.rope_on) {   // (64 heads with rotation are the item kernel's)
-      if (num_heads == 16) LAUNCH_EST_APPEND(1, true);
-      else LAUNCH_EST_APPEND(2, true);
-    } else {
-      if (num_heads == 16) LAUNCH_EST_HPW(1);
-      else if (num_heads == 32) LAUNCH_EST_HPW(2);
-      else LAUNCH_EST_HPW(4);
-    }
+    if (num_heads == 16) LAUNCH_EST_HPW(1);
+    else if (num_heads == 32) LAUNCH_EST_HPW(2);
+    else LAUNCH_EST_HPW(4);
 #undef LAUNCH_EST_HPW
-#undef LAUNCH_EST_APPEND
 #undef LAUNCH_EST
     return check_launch("estimate_kernel");
   }

@@ -1,5 +1,5 @@
-// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes short rows of 16 and 32
-// heads, short batches of 64 and estimates without counts (estimate_by_tiles), is in estimate.cuh, with the parameters and the distance arithmetic.
+// The distance estimate (and decode append) for any head count and for grouped queries; the tile pipeline, which takes short rows of 16, 32 and 64
+// heads and estimates without counts (estimate_by_tiles), is in estimate.cuh, with the parameters and the distance arithmetic.
 //
 // Bound: integer issue (logic at half rate and 5 population counts at an eighth, code_distance) for grouped
 // queries, HBM for long rows, fill and drain for short ones.  Two blocks of 8 warps per SM.  One warp of a block loads, rotates and codes the

@@ -156,17 +156,23 @@ ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
 // 12.4.  64 heads: one sequence, 1.5K 10.6 / 9.5; batches without rotation 2 x 300 11.3 / 11.8, 4 x 200 12.4 / 12.8, 4 x 600 13.3 / 13.2, 4 x 1.5K 15.9 / 15.3;
 // with it 2 x 300 12.8 / 12.3.
 //
+// Where a batch has more segments (of four heads) than the item kernel has blocks, a block codes a query and clears and adds up count
+// tables for each of its segments, and short rows go to the tiles again: 32 heads, 36 x 260 (288 segments on 296 blocks) 30.0 / 28.2, 48 x 300
+// 38.0 / 42.1, 48 x 1.1K 45.6 / 47.7, 128 x 200 81.1 / 90.4, 160 x 540 116.3 / 117.1; with rotation 48 x 300 39.6 / 43.6, 52 x 1.2K 51.2 / 51.5; 64 heads, 64 x
+// 300 81.7 / 90.2, 48 x 1.1K 79.4 / 83.5, with rotation 64 x 260 86.6 / 93.0, 52 x 700 84.6 / 84.0; 16 heads, 112 x 200 45.3 / 47.9, 112 x 420 49.6 / 48.8.
+//
 // Without counts there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
 // 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
 inline bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
-inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope) {
-  if (!tile_heads(num_heads, q_heads) || (num_heads == 64 && rope)) return false;
+inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope, int blocks) {
+  if (!tile_heads(num_heads, q_heads)) return false;
   const long long tokens = static_cast<long long>(batch) * n;
   if (!counts) return num_heads != 16 || tokens < 65536;
   if (n > 3584 || (rope && batch == 1)) return false;
+  if (batch * (num_heads / 4) > blocks) return n <= (num_heads == 16 ? (rope ? 0 : 256) : !rope ? 1024 : num_heads == 32 ? 640 : 320);
   if (num_heads == 16) return tokens <= (rope ? 4608 : 7424);
   if (num_heads == 32) return batch * tokens <= (rope ? 5120 : 20736);
-  return batch > 1 && tokens <= 1024;
+  return !rope && batch > 1 && tokens <= 1024;
 }
 
 }  // namespace adamas

@@ -265,9 +265,13 @@ def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
     (32, None, [2305, 2000, 100], 2305), (32, None, [2306, 2000, 100], 2306),
     (32, (8.0, 1e4), [1281, 65], 1281), (32, (8.0, 1e4), [1282, 65], 1282),
     (64, None, [257, 200, 100, 65], 257), (64, None, [258, 200, 100, 65], 258),
+    # more segments of four heads than blocks
+    (16, None, [257 - 2 * i for i in range(75)], 257), (16, None, [258 - 2 * i for i in range(75)], 258),
+    (32, (8.0, 1e4), [641 - 15 * i for i in range(38)], 641), (32, (8.0, 1e4), [642 - 15 * i for i in range(38)], 642),
+    (64, (8.0, 1e4), [321 - 14 * i for i in range(19)], 321), (64, (8.0, 1e4), [322 - 14 * i for i in range(19)], 322),
 ])
 def test_batches_on_both_sides_of_the_kernels_line(H, rope, lengths, cap, dtype):
-    """The fused step of a short batch in the tile pipeline and in the item kernel: rotated rows, cache rows, codes and selection of every
+    """The fused step of a batch of short rows in the tile pipeline and in the item kernel: rotated rows, cache rows, codes and selection of every
     sequence are those of the separate operators, and the histogram table is zero afterwards."""
     _, K, U = _mods()
     B, budget, ps = len(lengths), 64, 1     # (page size 1: the capacity is exact)
@@ -290,5 +294,7 @@ def test_batches_on_both_sides_of_the_kernels_line(H, rope, lengths, cap, dtype)
         for a, b in ((mine.kv_cache, c.kv_cache), (mine.hadamard_cache, c.hadamard_cache)):
             assert a.indicies == b.indicies
             assert torch.equal(a.buf_layer(0).view(torch.int16)[a.indicies], b.buf_layer(0).view(torch.int16)[b.indicies])
-        _assert_attn_close(o[i], U.decode_sparse_attn(qi, c, 0, c.topk_dindices_buffer)[0])
+        # (two fp32 results a few roundings apart may round to neighbouring numbers: 2^-7 of the value in bf16, 2^-10 in fp16)
+        want = U.decode_sparse_attn(qi, c, 0, c.topk_dindices_buffer)[0].float()
+        torch.testing.assert_close(o[i].float(), want, rtol=2.0 ** -7 if dtype == torch.bfloat16 else 2e-3, atol=2e-3 * float(want.abs().max()))
         c.end_forward()

@@ -316,7 +316,7 @@ def _kernels_of(run):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("H,lengths,rope", [(32, [9000, 8000, 8999], None), (64, [3000, 2000], (8.0, 1e4)), (16, [900, 700, 300], (8.0, 1e4)), (32, [500, 300], (8.0, 1e4)),
+@pytest.mark.parametrize("H,lengths,rope", [(32, [9000, 8000, 8999], None), (64, [3000, 2000], (8.0, 1e4)), (16, [900, 700, 300], (8.0, 1e4)), (32, [500, 300], (8.0, 1e4)), (64, [300 - 10 * i for i in range(19)], (8.0, 1e4)),
                                             (32, [700, 300], None)])
 def test_step_with_query_codes_on_any_16_bit_word(H, lengths, rope, dtype):
     """A batch whose query codes start on any 16-bit word: the same kernels as with aligned ones, and the same bits."""

@@ -21,7 +21,7 @@ int cache_heads(int h, int group) { return item_cache_heads(h, group); }
 int query_heads(int items, int group, int warps) { return item_query_heads(items, group, warps); }
 int tiles_of(int n, int t) { return est_tiles(n, t); }
 int per_piece(int tiles, int pieces, int blocks) { return item_blocks_per_piece(tiles, pieces, 1, blocks); }
-int by_tiles(int heads, int q_heads, int batch, int n, int counts, int rope) { return estimate_by_tiles(heads, q_heads, batch, n, counts, rope); }
+int by_tiles(int heads, int q_heads, int batch, int n, int counts, int rope, int blocks) { return estimate_by_tiles(heads, q_heads, batch, n, counts, rope, blocks); }
 void share_one(int tiles, int pieces, int q_part, int blocks, int* out) {
   for (int b = 0; b < blocks; ++b) {
     const ItemShare w = item_share_one(tiles, pieces, q_part, blocks, b);
@@ -240,14 +240,17 @@ def test_columns_of_a_batch_every_item_once(split, heads, group, blocks):
     # ... and ones that are not
     (32, 6, 1000, False, False), (32, 4, 1500, False, False), (32, 5, 300, True, False), (16, 8, 1000, False, False), (16, 8, 600, True, False),
     (32, 1024, 3000, False, False), (16, 1024, 2000000, True, False),
+    # large batches: more segments of four heads than blocks
+    (32, 37, 300, False, False), (32, 38, 300, False, True), (32, 128, 1024, False, True), (32, 128, 1025, False, False), (32, 96, 640, True, True),
+    (32, 96, 641, True, False), (64, 18, 300, False, False), (64, 19, 300, False, True), (64, 64, 1025, False, False), (64, 64, 320, True, True),
+    (64, 64, 321, True, False), (16, 112, 256, False, True), (16, 112, 257, False, False), (16, 112, 200, True, False),
 ])
 def test_which_kernel_counts(split, heads, batch, n, rope, want):
-    assert bool(split.by_tiles(heads, heads, batch, n, 1, rope)) is want
+    assert bool(split.by_tiles(heads, heads, batch, n, 1, rope, BLOCKS)) is want
     for h, q in ((heads // 2, heads), (40, 40), (4, 4)):     # grouped queries and other head counts: the item kernel
-        assert not split.by_tiles(h, q, batch, n, 1, rope)
+        assert not split.by_tiles(h, q, batch, n, 1, rope, BLOCKS)
 
 
 @pytest.mark.parametrize("heads,n,want", [(16, 65535, True), (16, 65536, False), (32, 1000000, True), (64, 1000000, True), (8, 100, False)])
 def test_which_kernel_without_counts(split, heads, n, want):
-    assert bool(split.by_tiles(heads, heads, 1, n, 0, 0)) is want
-    assert not split.by_tiles(64, 64, 1, n, 0, 1)      # (the tile pipeline has no rotation for 64 heads)
+    assert bool(split.by_tiles(heads, heads, 1, n, 0, 0, BLOCKS)) is want
