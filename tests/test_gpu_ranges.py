@@ -214,7 +214,8 @@ def _blocks_per_head(hist):
     (2047, 96, 32, 16, 2, 2), (2049, 97, 32, 16, 2, 2),
     (30000, 1023, 32, 16, 16, 8), (32768, 2047, 8, 1, 16, 8),   # two blocks share a histogram slice; page numbers not staged (page size 1)
     (40001, 4000, 4, 7, 16, 16),                       # several rounds per warp, a page size that is no power of two
-    (100000, 63, 100, 32, 5, 5),                       # few blocks per row: distances beyond the staged ones
+    (100000, 63, 100, 32, 5, 5),                       # few blocks per row: nearly as many distances as are staged
+    (30000, 63, 600, 16, 1, 1), (30001, 700, 592, 16, 1, 1), (400003, 1000, 2, 16, 16, 16),   # ... beyond the staged ones: 21824 per block
 ])
 @pytest.mark.parametrize("ties", [False, True])
 def test_select_attend_shapes(n, k, H, ps, blocks, slices, ties):
