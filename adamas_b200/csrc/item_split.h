@@ -88,8 +88,10 @@ ADAMAS_HD ItemShare item_share_one(int tiles, int pieces, int q_part, int blocks
 //    heads 71.3 us a layer cut evenly, 67.7 apart);
 //  * where the largest share cannot be much more than an even one.  It is at most that of the longest sequence with a column of its own, and at
 //    most tiles / (columns - sequences): item_columns_apart.
-// (Products stay below 2^31.  Lengths that are all zero leave nothing to deal out.)  In what follows a segment is a sequence and a block a
-// column; with the whole line cut (pieces > 1) a piece of a sequence and a block.
+// (Products stay below 2^31.  Lengths that are all zero leave nothing to deal out.)  In what follows a segment is a sequence, a block a
+// column, and the kernel's calls have pieces = 1.  item_apart_most is the exact largest share, which takes a look at every length (2.7 us a layer
+// on the device): item_columns_apart bounds it instead.  No kernel asks for it, nor for item_apart_hopeless and item_apart_pays, nor cuts several pieces
+// apart on one line: the tests of such cuts do.
 constexpr int kItemApart = 24;
 ADAMAS_HD bool item_apart_possible(int total, int segments, int blocks) { return total > 0 && segments <= blocks && total <= 0x7fffffff / blocks; }
 ADAMAS_HD bool item_apart_few(int segments, int blocks) { return segments * 8 <= blocks; }
@@ -135,6 +137,12 @@ ADAMAS_HD bool item_columns_apart(int total, int longest, int batch, int q_part,
 ADAMAS_HD int item_columns_alike(int total, int longest, int batch, int columns) {
   if (batch > columns || static_cast<long long>(longest) * batch != total || columns % batch > columns / 7) return 0;
   return columns / batch;
+}
+// The same for a host that has the line alone: cum[s] tiles lie in front of sequence s.
+inline int item_columns_alike(const int* cum, int batch, int columns) {
+  int longest = 0;
+  for (int s = 0; s < batch; ++s) longest = cum[s + 1] - cum[s] > longest ? cum[s + 1] - cum[s] : longest;
+  return item_columns_alike(cum[batch], longest, batch, columns);
 }
 ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
   const int s = c / per, nblk = per < tiles ? per : tiles, i = c - s * per;

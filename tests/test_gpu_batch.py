@@ -218,12 +218,13 @@ def test_large_launches_count_their_histograms_in_shared_memory():
     ([2000 + 7 * i for i in range(64)], 28, 4, 256),    # as many pieces as a launch has blocks, kept apart
     ([3000 + 50 * i for i in range(20)], 40, 40, 256),  # ... and cut evenly
     ([700 + 3 * i for i in range(40)], 7, 7, 128),      # few tokens a block
-    # 16, 32 and 64 heads: longer than the batches of the tile pipeline
+    # 16, 32 and 64 heads: batches with many distances leave the tile pipeline
     ([8000, 4001, 8192, 7777, 6500, 5003, 8100, 4097, 7000, 6001, 8003, 5555, 7321], 32, 32, 128),
     ([9000, 4501, 8999, 9001, 700, 8500, 7001, 9500], 16, 16, 256),
     ([13001, 12000, 6501, 13100], 64, 64, 256),
     ([25100, 24701], 64, 64, 512),
-    ([24700, 24601, 24000, 23001, 24699, 24688, 12000, 24100], 32, 32, 256),   # long rows, two segments a block
+    # (there is no counting launch any more: the item kernel, as for the others)
+    ([24700, 24601, 24000, 23001, 24699, 24688, 12000, 24100], 32, 32, 256),   # long rows, two segments a block: the tiles and a counting launch
 ])
 def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
     """A batch whose distances are counted in shared memory: the same selection as each sequence by itself, and a table

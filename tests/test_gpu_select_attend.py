@@ -213,12 +213,13 @@ def test_stale_histogram_table_is_reported_not_followed():
     _assert_attn_close(o[0], want)
 
 
+# (Every block has the same part of the row, so two blocks, or one, share a slice; what is selected does not depend on it.)
 @pytest.mark.parametrize("distinct", [3, 40, 100000])
 @pytest.mark.parametrize("n,k,H", [(32768, 1023, 4), (30001, 1100, 3), (131072, 2047, 2), (100003, 1500, 1), (32768, 2560, 2), (32768, 2561, 2)])
-def test_step_with_ties_at_the_front(n, k, H, distinct):
-    """The fused step with sixteen blocks per head, two (or, long rows, one) to a slice of the histograms.  Keys of a few kinds, so that
-    ties fill the front of the row; the selection is that of the separate operators (ties to the lower position) and the result that of
-    attention over it."""
+def test_step_with_first_slices_shared_by_one_block_more(n, k, H, distinct):
+    """The fused step with sixteen blocks per head and up to 2560 winners: three (or, long rows, two) blocks share each of the first slices of
+    the histograms.  Keys of a few kinds, so that ties fill the front of the row; the selection is that of the separate operators (ties to the
+    lower position) and the result that of attention over it."""
     _, K, U = _mods()
     g = torch.Generator(device=DEV).manual_seed(n + k)
     kinds = torch.randn(distinct, H, 128, device=DEV, generator=g).half()
