@@ -583,7 +583,8 @@ def run_ours(args):
         both = stage_time("select_attend", pre="estimate")
         stage_us["estimate_then_select_attend"] = both
         stage_us["select_attend"] = both - stage_us["estimate"]
-        by_tiles = args.heads in (16, 32) and args.ctx <= 3584   # (short rows; about where the library's line lies)
+        # (the stages are timed with one sequence, host lengths, counts and no rotation: the library's rule for those)
+        by_tiles = args.heads in (16, 32) and c.hadamard_cache.seqlen - 1 <= 3584
         kernels = {first: "estimate_items_kernel" if not by_tiles else "estimate_append_kernel" if first == "append_estimate" else "estimate_kernel",
                    "select_attend": "select_attend_kernel"}
         if first == "estimate":
