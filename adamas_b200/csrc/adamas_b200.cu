@@ -522,11 +522,11 @@ int adamas_append_prefill(const void* k, const void* v, const void* h, int64_t n
   PagedTarget tgt{kv_data, kv_page_table, static_cast<uint16_t*>(code_data), code_page_table, page_size,
                   num_heads};
   const Thresholds th = make_thresholds(thresholds3_host);
-  const unsigned blocks = static_cast<unsigned>((rows + 31) / 32);   // (eight lanes a row)
+  const unsigned blocks = static_cast<unsigned>((rows * 8 + kPrefillThreads - 1) / kPrefillThreads);   // (eight lanes a row)
   const int64_t start = seq_len - n_tokens;
   cudaStream_t st = to_stream(stream);
 #define LAUNCH_AP(T, F)                                                                                                  \
-  ADAMAS_LAUNCH("append_prefill_kernel", (append_prefill_kernel<T, F>), dim3(blocks), dim3(256), 0, st, 1,               \
+  ADAMAS_LAUNCH("append_prefill_kernel", (append_prefill_kernel<T, F>), dim3(blocks), dim3(kPrefillThreads), 0, st, 1,   \
                 static_cast<const T*>(k), static_cast<const T*>(v), static_cast<const T*>(h), rows, start, tgt, scale, th)
   if (dtype == ADAMAS_F16) {
     if (h) LAUNCH_AP(__half, false); else LAUNCH_AP(__half, true);

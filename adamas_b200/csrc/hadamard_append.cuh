@@ -431,8 +431,12 @@ append_decode_kernel(T* k, const T* v, T* qh, const T* kh, uint16_t* q_code_out,
 // and written once, and the codes); with half-warps per row and the codes element by element it was instructions (32768 tokens x 32 heads,
 // us: fp16 199 -> 162, bf16 218 -> 163; 162 without the transform).  (Two or four rows per half-warp in flight, streaming stores, and the rows from the
 // last one to the first, behind a rotation that has left its last ones in L2, measured no better.)
+// Blocks of 16 rows: a lane's transform is 48 shuffles, and with few rows those of a block's warps are what takes time: us for 32 / 256 /
+// 2048 / 16384 rows of 16 heads, a block of 256 threads 1.54 / 1.65 / 1.75 / 3.28, of 128 1.34 / 1.44 / 1.54 / 3.08, of 64 1.34 / 1.44 / 1.54 / 3.20, of 32
+// 1.34 / 1.44 / 1.65 / 4.30; half-warps per row in blocks of 256 took 1.24 / 1.44 / 1.54 / 3.90.
+constexpr int kPrefillThreads = 128;
 template <typename T, bool FUSED>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(kPrefillThreads)
 append_prefill_kernel(const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ h,
                       int64_t rows, int64_t start_pos, PagedTarget tgt, float scale, Thresholds th) {
   const unsigned l8 = threadIdx.x & 7;

@@ -437,3 +437,31 @@ def test_prefill_codes_at_any_thresholds(thresholds, dtype):
     assert torch.equal(codes.view(pages * ps, H, 16)[:N].cpu(), want)
     assert torch.equal(kv.permute(0, 2, 1, 3, 4).reshape(pages * ps, 2, H, 128)[:N].cpu().view(torch.int16),
                        torch.stack([k, k], 1).view(torch.int16))
+
+
+@pytest.mark.parametrize("given", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,H,past", [(1, 1, 0), (15, 1, 3), (16, 1, 0), (17, 1, 5), (3, 5, 16), (11, 3, 2), (31, 33, 1)])
+def test_prefill_around_a_block_of_rows(N, H, past, dtype, given):
+    """Prompts of a few rows, sixteen to a block, behind `past` cached tokens: every row has its codes and its K and V, and no other place of
+    the caches is written."""
+    from adamas_b200 import hadamard_transform
+    _, K, _ = _mods()
+    ps, total = 4, N + past
+    k, v = _randn((N, H, 128), 5, dtype).to(DEV), _randn((N, H, 128), 6, dtype).to(DEV)
+    pages = (total + ps - 1) // ps
+    table = torch.arange(pages - 1, -1, -1, dtype=torch.int32, device=DEV)
+    kv = torch.zeros(pages + 1, 2, ps, H, 128, dtype=dtype, device=DEV)
+    codes = torch.zeros(pages + 1, 1, ps, H, 16, dtype=torch.int16, device=DEV)
+    last = (total - 1) % ps + 1
+    h = hadamard_transform(k)
+    K.append_kv_cache_prefill(k, v, h if given else None, kv, table, None, last, 0, codes, table, None, last, 0, 0, None, (-10.0, 0.0, 10.0))
+    bucket = sum((h.float() > t).to(torch.int32) for t in (-10.0, 0.0, 10.0)).view(N, H, 16, 8)
+    want = sum(bucket[..., i] << (2 * i) for i in range(8)).to(torch.int16)
+    order = table.long()
+    got = codes[order].reshape(pages * ps, H, 16)
+    rows = kv[order].permute(0, 2, 1, 3, 4).reshape(pages * ps, 2, H, 128).view(torch.int16)
+    assert torch.equal(got[past:total], want)
+    assert torch.equal(rows[past:total], torch.stack([k, v], 1).view(torch.int16))
+    for t in (got[:past], got[total:], rows[:past], rows[total:], kv[pages], codes[pages]):
+        assert not bool(t.any())
