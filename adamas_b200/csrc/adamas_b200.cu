@@ -627,7 +627,12 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   dim3 grid(static_cast<unsigned>(std::min<int64_t>(slots_all, items)));
   int64_t per_block = (items + grid.x - 1) / grid.x;
   if (!seqs && prm.q_group == 1) {
-    const int per = std::min<int>(item_blocks_per_piece(static_cast<int>(tiles), pieces, 1, static_cast<int>(grid.x)), (tiles + kItemWarps - 1) / kItemWarps);
+    int per = item_blocks_per_piece(static_cast<int>(tiles), pieces, 1, static_cast<int>(grid.x));
+    // A tile per warp at least, so that no more blocks than that code the query.  Where the codes are given that is only so while it leaves a block an
+    // SM of its own and a block per tile would not (us, by warps / by blocks, with counts: 2 heads, 400 tokens 2.24 / 1.73, 9K 2.06 / 1.92, 14K 2.12 / 2.35; 8
+    // heads, 2K 1.92 / 1.83, 3K 1.92 / 2.05; 28 heads, 600 1.92 / 1.80, 900 1.93 / 2.07; 40 heads, 3K 2.18 / 2.25, 3.5K 2.77 / 2.37).
+    const int by_warps = static_cast<int>((tiles + kItemWarps - 1) / kItemWarps);
+    if (ap.q || (tiles * pieces > di->num_sms && by_warps * pieces <= di->num_sms)) per = std::min(per, by_warps);
     if (per > 0) {
       grid = dim3(static_cast<unsigned>(pieces), static_cast<unsigned>(per));
       per_block = (tiles + per - 1) / per;

@@ -465,3 +465,10 @@ def test_prefill_around_a_block_of_rows(N, H, past, dtype, given):
     assert torch.equal(rows[past:total], torch.stack([k, v], 1).view(torch.int16))
     for t in (got[:past], got[total:], rows[:past], rows[total:], kv[pages], codes[pages]):
         assert not bool(t.any())
+
+
+@pytest.mark.parametrize("H,L", [(1, 18944), (1, 18945), (2, 9472), (2, 9473), (28, 672), (28, 673), (33, 512), (33, 513), (40, 3136), (40, 3137)])
+def test_estimate_with_given_codes_around_a_tile_per_sm(H, L):
+    """Given codes: the last length with a block to a tile (148 of them on the chip) and the first one with a tile per warp; 40 heads, the last one
+    of those and the first one behind it."""
+    test_estimate_items_shapes(H, H, L, 16)
