@@ -581,7 +581,7 @@ static int launch_estimate(const void* q_code, const StepAppend& ap, int dtype, 
   // (with 16, 32 and 64 heads query codes may start on any 16-bit word, in both kernels)
   const int code_align = tile_heads(num_heads, q_heads) ? 2 : 16;
   ADAMAS_REQUIRE(reinterpret_cast<uintptr_t>(ap.q_code_out) % code_align == 0, "q_code must be %d-byte aligned", code_align);
-  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, ap.rope_on != 0, est_blocks_per_sm() * di->num_sms)) {
+  if (estimate_by_tiles(num_heads, q_heads, batch, n, hist != nullptr, ap.rope_on != 0, est_blocks_per_sm() * di->num_sms, ap.q != nullptr)) {
     const int num_tiles = (n + kEstTile - 1) / kEstTile;
     const size_t smem = static_cast<size_t>(kEstStages) * kEstTile * (2 * num_heads + 1) * 16;
     ADAMAS_REQUIRE(smem <= most, "num_heads (%d) too large", num_heads);

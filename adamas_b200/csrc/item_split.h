@@ -169,13 +169,17 @@ ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
 // 38.0 / 42.1, 48 x 1.1K 45.6 / 47.7, 128 x 200 81.1 / 90.4, 160 x 540 116.3 / 117.1; with rotation 48 x 300 39.6 / 43.6, 52 x 1.2K 51.2 / 51.5; 64 heads, 64 x
 // 300 81.7 / 90.2, 48 x 1.1K 79.4 / 83.5, with rotation 64 x 260 86.6 / 93.0, 52 x 700 84.6 / 84.0; 16 heads, 112 x 200 45.3 / 47.9, 112 x 420 49.6 / 48.8.
 //
+// With given codes nobody waits for the query and the tiles keep up longer (us, one sequence, tiles / items): 16 heads, 4.5K 1.86 / 2.05, 6K 2.24 / 2.18; 32
+// heads, 4.5K 2.18 / 2.68, 9K 3.06 / 3.52, 14K 3.96 / 3.97; 64 heads, 3.5K 2.95 / 2.75, 4.5K 3.14 / 3.57, 9K 4.47 / 4.88, 14K 7.27 / 7.00.
+//
 // Without counts there are no atomics: 32 and 64 heads stay with the tiles (one estimate of 32 heads, 64K 11.0 / 11.8, 256K
 // 44.2 / 46.9; 64 heads, 32K 10.8 / 12.2), 16 heads do not (128K 17.8 / 11.9).
 inline bool tile_heads(int num_heads, int q_heads) { return q_heads == num_heads && (num_heads == 16 || num_heads == 32 || num_heads == 64); }
-inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope, int blocks) {
+inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool counts, bool rope, int blocks, bool append = true) {
   if (!tile_heads(num_heads, q_heads)) return false;
   const long long tokens = static_cast<long long>(batch) * n;
   if (!counts) return num_heads != 16 || tokens < 65536;
+  if (!append && batch == 1) return num_heads == 64 ? n > 4096 && n <= 12288 : n <= (num_heads == 16 ? 5120 : 12288);
   if (n > 3584 || (rope && batch == 1)) return false;
   if (batch * (num_heads / 4) > blocks) return n <= (num_heads == 16 ? (rope ? 0 : 256) : !rope ? 1024 : num_heads == 32 ? 640 : 320);
   if (num_heads == 16) return tokens <= (rope ? 4608 : 7424);

@@ -584,7 +584,10 @@ def run_ours(args):
         stage_us["estimate_then_select_attend"] = both
         stage_us["select_attend"] = both - stage_us["estimate"]
         # (the stages are timed with one sequence, host lengths, counts and no rotation: the library's rule for those)
-        by_tiles = args.heads in (16, 32) and c.hadamard_cache.seqlen - 1 <= 3584
+        n = c.hadamard_cache.seqlen - 1
+        by_tiles = args.heads in (16, 32) and n <= 3584
+        if first == "estimate":   # (given codes)
+            by_tiles = n > 4096 and n <= 12288 if args.heads == 64 else n <= {16: 5120, 32: 12288}.get(args.heads, 0)
         kernels = {first: "estimate_items_kernel" if not by_tiles else "estimate_append_kernel" if first == "append_estimate" else "estimate_kernel",
                    "select_attend": "select_attend_kernel"}
         if first == "estimate":

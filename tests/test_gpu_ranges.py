@@ -472,3 +472,9 @@ def test_estimate_with_given_codes_around_a_tile_per_sm(H, L):
     """Given codes: the last length with a block to a tile (148 of them on the chip) and the first one with a tile per warp; 40 heads, the last one
     of those and the first one behind it."""
     test_estimate_items_shapes(H, H, L, 16)
+
+
+@pytest.mark.parametrize("H,L", [(16, 5121), (16, 5122), (32, 12289), (32, 12290), (64, 4097), (64, 4098), (64, 12289), (64, 12290)])
+def test_estimate_with_given_codes_on_both_sides_of_the_kernels_line(H, L):
+    """Given codes and counts: the lengths on both sides of the line between the kernels; exact."""
+    test_estimate_items_shapes(H, H, L, 16)

@@ -22,6 +22,7 @@ int query_heads(int items, int group, int warps) { return item_query_heads(items
 int tiles_of(int n, int t) { return est_tiles(n, t); }
 int per_piece(int tiles, int pieces, int blocks) { return item_blocks_per_piece(tiles, pieces, 1, blocks); }
 int by_tiles(int heads, int q_heads, int batch, int n, int counts, int rope, int blocks) { return estimate_by_tiles(heads, q_heads, batch, n, counts, rope, blocks); }
+int by_tiles_given(int heads, int batch, int n) { return estimate_by_tiles(heads, heads, batch, n, true, false, 296, false); }
 void share_one(int tiles, int pieces, int q_part, int blocks, int* out) {
   for (int b = 0; b < blocks; ++b) {
     const ItemShare w = item_share_one(tiles, pieces, q_part, blocks, b);
@@ -262,3 +263,10 @@ def test_which_kernel_counts(split, heads, batch, n, rope, want):
 @pytest.mark.parametrize("heads,n,want", [(16, 65535, True), (16, 65536, False), (32, 1000000, True), (64, 1000000, True), (8, 100, False)])
 def test_which_kernel_without_counts(split, heads, n, want):
     assert bool(split.by_tiles(heads, heads, 1, n, 0, 0, BLOCKS)) is want
+
+
+@pytest.mark.parametrize("heads,n,want", [(16, 5120, True), (16, 5121, False), (32, 12288, True), (32, 12289, False), (64, 4096, False), (64, 4097, True),
+                                          (64, 12288, True), (64, 12289, False), (8, 100, False)])
+def test_which_kernel_counts_with_given_codes(split, heads, n, want):
+    assert bool(split.by_tiles_given(heads, 1, n)) is want
+    assert not split.by_tiles_given(heads, 8, n)           # (batches: the rule with the append)
