@@ -160,9 +160,11 @@ ADAMAS_HD ItemShare item_share_alike(int tiles, int batch, int per, int c) {
 // 10.5 / 11.1, 4 x 1.8K 10.9 / 11.4, 5 x 1.5K 11.8 / 11.6, 6 x 1K 11.3 / 11.8, 8 x 1K 12.4 / 11.8; with it 2 x 2.3K 10.8 / 11.4, 2 x 2.7K 11.8 / 11.4, 4 x 1K
 // 11.3 / 11.9, 4 x 1.5K 12.3 / 11.9, 8 x 450 12.1 / 12.3, 8 x 600 12.7 / 12.5.  Batches of 32 heads, where another sequence costs the tiles more, without
 // rotation 2 x 3.6K 11.9 / 11.9, 3 x 1.5K 11.3 / 11.8, 3 x 2.5K 12.8 / 12.3, 4 x 1K 11.4 / 11.8, 4 x 1.5K 12.4 / 12.3, 6 x 450 11.8 / 12.3, 6 x 1K 13.8 / 12.8, 8 x 300
-// 13.0 / 12.8, 10 x 200 13.4 / 14.2; with it 2 x 600 10.3 / 11.8, 2 x 1.25K 10.7 / 11.9, 2 x 1.8K 12.0 / 11.9, 3 x 450 10.8 / 12.3, 3 x 600 12.3 / 12.3, 5 x 200 12.8 /
-// 12.4.  64 heads: one sequence, 1.5K 10.6 / 9.5; batches without rotation 2 x 300 11.3 / 11.8, 4 x 200 12.4 / 12.8, 4 x 600 13.3 / 13.2, 4 x 1.5K 15.9 / 15.3;
-// with it 2 x 300 12.8 / 12.3.
+// 13.0 / 12.8, 10 x 200 13.4 / 14.2; with it 2 x 600 10.3 / 11.8, 2 x 1.25K 10.7 / 11.9, 2 x 1.8K 12.0 / 11.9, 3 x 450 10.8 / 12.3, 3 x 600 12.3 / 12.3.
+// 64 heads: one sequence, 1.5K 10.6 / 9.5; batches without rotation 2 x 300 11.3 / 11.8, 4 x 200 12.4 / 12.8, 4 x 600 13.3 / 13.2, 4 x 1.5K 15.9 / 15.3;
+// with it 2 x 300 12.8 / 12.3.  The same with many layers, whose caches do not stay in L2: 32 heads with rotation 3 x 700 12.3 / 12.0 (3 x 350 in caches
+// for 700: 8.0 / 9.5), 3 x 1K 12.4 / 12.1, 4 x 450 12.8 / 12.5, 5 x 300 9.0 / 10.5, 8 x 300 10.6 / 11.2, 8 x 450 14.7 / 14.1, 10 x 200 11.2 / 12.3; 64 heads without 3 x 700
+// 13.2 / 13.1 (350 in 700: 9.6 / 10.3), 5 x 300 10.3 / 11.8, 10 x 300 15.1 / 17.0, 16 x 200 18.4 / 18.3; 16 heads without 16 x 450 14.8 / 13.9, 10 x 700 13.3 / 12.9.
 //
 // Where a batch has more segments (of four heads) than the item kernel has blocks, a block codes a query and clears and adds up count
 // tables for each of its segments, and short rows go to the tiles again: 32 heads, 36 x 260 (288 segments on 296 blocks) 30.0 / 28.2, 48 x 300
@@ -182,9 +184,9 @@ inline bool estimate_by_tiles(int num_heads, int q_heads, int batch, int n, bool
   if (!append && batch == 1) return num_heads == 64 ? n > 4096 && n <= 12288 : n <= (num_heads == 16 ? 5120 : 12288);
   if (n > 3584 || (rope && batch == 1)) return false;
   if (batch * (num_heads / 4) > blocks) return n <= (num_heads == 16 ? (rope ? 0 : 256) : !rope ? 1024 : num_heads == 32 ? 640 : 320);
-  if (num_heads == 16) return tokens <= (rope ? 4608 : 7424);
-  if (num_heads == 32) return batch * tokens <= (rope ? 5120 : 20736);
-  return !rope && batch > 1 && tokens <= 1024;
+  if (num_heads == 16) return rope ? tokens <= 4608 : tokens + 200 * batch <= 8224;
+  if (num_heads == 32) return batch * tokens <= (rope ? 20480 : 20736) && !(rope && tokens > 2560);
+  return !rope && batch > 1 && tokens <= 3072;
 }
 
 }  // namespace adamas

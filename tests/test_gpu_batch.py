@@ -265,7 +265,8 @@ def test_batched_counts_in_shared_memory(lengths, Hq, H, budget, fused_append):
     (16, (8.0, 1e4), [700, 300, 1537], 1537), (16, (8.0, 1e4), [700, 300, 1538], 1538),
     (32, None, [2305, 2000, 100], 2305), (32, None, [2306, 2000, 100], 2306),
     (32, (8.0, 1e4), [1281, 65], 1281), (32, (8.0, 1e4), [1282, 65], 1282),
-    (64, None, [257, 200, 100, 65], 257), (64, None, [258, 200, 100, 65], 258),
+    (64, None, [769, 200, 100, 65], 769), (64, None, [770, 200, 100, 65], 770),
+    (32, (8.0, 1e4), [321, 300, 65, 66, 300, 280, 310, 100], 321), (32, (8.0, 1e4), [322, 300, 65, 66, 300, 280, 310, 100], 322),
     # more segments of four heads than blocks
     (16, None, [257 - 2 * i for i in range(75)], 257), (16, None, [258 - 2 * i for i in range(75)], 258),
     (32, (8.0, 1e4), [641 - 15 * i for i in range(38)], 641), (32, (8.0, 1e4), [642 - 15 * i for i in range(38)], 642),

@@ -241,13 +241,14 @@ def test_an_average_length_in_front_does_not_make_the_others_equal(split, heads,
     (16, 1, 3584, False, True), (16, 1, 3585, False, False), (16, 1, 600, True, False), (16, 4, 1856, False, True), (16, 4, 1857, False, False),
     (16, 3, 1536, True, True), (16, 3, 1537, True, False), (32, 1, 3584, False, True), (32, 1, 3585, False, False), (32, 1, 600, True, False),
     (32, 2, 3584, False, True), (32, 3, 2304, False, True), (32, 3, 2305, False, False), (32, 2, 1280, True, True), (32, 2, 1281, True, False),
-    (64, 1, 600, False, False), (64, 4, 256, False, True), (64, 4, 257, False, False), (64, 2, 300, True, False),
+    (32, 8, 320, True, True), (32, 8, 321, True, False), (32, 10, 204, True, True), (32, 10, 205, True, False), (16, 16, 314, False, True), (16, 16, 315, False, False),
+    (64, 1, 600, False, False), (64, 4, 768, False, True), (64, 4, 769, False, False), (64, 2, 300, True, False),
     # short batches that were slower in the item kernel by 4 to 15 % (us a layer beside estimate_by_tiles)
     (32, 2, 600, True, True), (32, 2, 1000, True, True), (32, 2, 1250, True, True), (32, 3, 300, True, True), (32, 3, 450, True, True),
     (32, 3, 300, False, True), (32, 3, 1500, False, True), (32, 4, 600, False, True), (32, 5, 600, False, True), (32, 6, 450, False, True),
     (32, 10, 207, False, True), (16, 3, 1500, True, True), (16, 4, 1800, False, True), (64, 2, 200, False, True),
     # ... and ones that are not
-    (32, 6, 1000, False, False), (32, 4, 1500, False, False), (32, 5, 300, True, False), (16, 8, 1000, False, False), (16, 8, 600, True, False),
+    (32, 6, 1000, False, False), (32, 4, 1500, False, False), (32, 3, 1000, True, False), (16, 8, 1000, False, False), (16, 8, 600, True, False),
     (32, 1024, 3000, False, False), (16, 1024, 2000000, True, False),
     # large batches: more segments of four heads than blocks
     (32, 37, 300, False, False), (32, 38, 300, False, True), (32, 128, 1024, False, True), (32, 128, 1025, False, False), (32, 96, 640, True, True),
